@@ -57,13 +57,15 @@ enum {
 typedef struct uastar_engine uastar_engine;
 
 typedef struct {
-    int32_t heaps;           /* k parallel binary heaps of the plain engine (0 -> 8192 grid, 16384 puzzle) */
+    int32_t heaps;           /* k parallel binary heaps of the plain engine (0 -> 8192 grid, 16384 puzzle,
+                              rounded up to a whole number of CTAs per SM) */
     int32_t block_threads;   /* CTA size of the plain engine's persistent kernel (0 -> 256) */
     int32_t heap_capacity;   /* entries per heap (0 -> auto, grown on overflow) */
     int32_t hash_log2_slots; /* dedup table = 2^n slots of 32 B, n <= 31 (0 -> sized from the instance and
                               grown 4x in place whenever it is half full) */
     double max_load;         /* dedup table load limit in (0,1) (0 -> 0.8) */
-    int64_t max_rounds;      /* GA* round limit per solve (0 -> 2^31) */
+    int64_t max_rounds;      /* limit on expansion steps per solve (0 -> 2^31): a GA* round is one, and
+                              each further pass of expansions that it makes at once is one more */
     double wait_timeout_s;   /* bound on any device-side barrier wait (0 -> 10 s) */
     int32_t threads_per_heap; /* threads that share one heap's successors (0 -> 4) */
     int32_t heap_top_levels;  /* heap levels kept in shared memory (0 -> as many as fit, -1 -> none) */
@@ -115,7 +117,7 @@ typedef struct {
     int64_t expanded;     /* pops that were neither stale nor the goal */
     int64_t generated;    /* successors generated (dedup probes) */
     int64_t pushed;       /* heap pushes (new or improved nodes) */
-    int64_t rounds;       /* GA* rounds */
+    int64_t rounds;       /* expansion steps: GA* rounds and their further passes */
     int64_t table_used;   /* dedup-table slots in use */
     int64_t path_len;     /* cells on the optimal path, start and goal included */
     double kernel_ms;     /* device time of the search kernel (CUDA events) */

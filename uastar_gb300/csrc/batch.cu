@@ -56,7 +56,7 @@ struct InstDesc {
 
 struct InstOut {
     uint32_t status, goal_slot;
-    unsigned long long goal_best, rounds, expanded, generated, pushed, inserted;
+    unsigned long long goal_best, rounds, steps, expanded, generated, pushed, inserted;
     unsigned long long t_start, t_end;  // device globaltimer around this call's work (ns)
     unsigned long long path_len;        // batch: keys written (goal -> start); key_cap + 1 if cut
 };
@@ -123,55 +123,104 @@ __device__ void clear_partition(Slot *tab, uint64_t slots) {
 
 __device__ void init_state(TeamState *st) { team_state_init(st); }
 
+// The search of one problem type as a function of its own: called, it has the
+// registers to itself and the kernel's state is saved once per call (inlined
+// three times into one kernel the searches spill in their round loops).
+template <class P, class Team>
+__device__ __noinline__ uint32_t search_instance(const P &prob, Team &team, const SearchMem<typename P::Entry> &m,
+                                                 uint32_t H, unsigned char *smem, uint64_t budget) {
+    return ga_search(prob, team, m, H, smem, budget);
+}
+
+// What a search reads of its instance, in shared memory (one copy per CTA):
+// kernel parameters would sit in the constant bank, but these differ from
+// instance to instance, and held in registers they spill.
+union InstanceMem {
+    struct {
+        GridProblem prob;
+        SearchMem<GridEntry> m;
+    } grid;
+    struct {
+        PuzzleProblem<3> prob;
+        SearchMem<PuzzleEntry> m;
+    } p3;
+    struct {
+        PuzzleProblem<4> prob;
+        SearchMem<PuzzleEntry> m;
+    } p4;
+    __device__ InstanceMem() {}
+};
+
 // Runs one instance on this CTA for up to `budget` rounds.
 template <class Team>
 __device__ uint32_t run_instance(const BatchArgs &a, const InstDesc &d, Team &team, Slot *tab, uint8_t *heaps,
                                  uint32_t *hs, Cand *cand, unsigned char *smem, uint64_t budget,
-                                 uint64_t deadline_ns) {
-    const uint64_t slots = 1ull << d.log2_slots;
-    const bool own_geo = a.serving != 0;  // serving requests carry their heap geometry
-    if (d.kind == UASTAR_KIND_GRID) {
-        GridProblem prob;
-        prob.bm = a.bitmaps + d.bm_word;
-        prob.H = d.H;
-        prob.W = d.W;
-        prob.sx = d.sx;
-        prob.sy = d.sy;
-        prob.ex = d.ex;
-        prob.ey = d.ey;
-        SearchMem<GridEntry> m{tab, slots - 1, (uint64_t)(slots * a.max_load), 4096u,
-                               reinterpret_cast<GridEntry *>(heaps),
-                               own_geo ? d.heap_stride : a.stride_grid, own_geo ? d.heap_hcap : a.hcap_grid,
-                               a.L_grid, hs, cand, d.max_rounds};
-        if (d.grow_at) m.grow_at = d.grow_at;
-        m.deadline_ns = deadline_ns;
-        m.split = a.split_grid;
-        return ga_search(prob, team, m, a.H, smem, budget);
+                                 uint64_t deadline_ns, InstanceMem &im) {
+    const bool grid = d.kind == UASTAR_KIND_GRID;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const uint64_t slots = 1ull << d.log2_slots;
+        const bool own_geo = a.serving != 0;  // serving requests carry their heap geometry
+        const auto common = [&](auto &m) {
+            m.tab = tab;
+            m.mask = slots - 1;
+            m.max_inserted = (uint64_t)(slots * a.max_load);
+            m.max_probe = 4096u;
+            m.stride = own_geo ? d.heap_stride : grid ? a.stride_grid : a.stride_puzzle;
+            m.hcap = own_geo ? d.heap_hcap : grid ? a.hcap_grid : a.hcap_puzzle;
+            m.L = grid ? a.L_grid : a.L_puzzle;
+            m.heap_size = hs;
+            m.cand = cand;
+            m.max_rounds = d.max_rounds;
+            m.grow_at = d.grow_at ? d.grow_at : ~0ull;
+            m.deadline_ns = deadline_ns;
+            m.split = grid ? a.split_grid : a.split_puzzle;
+            m.sort_buf = nullptr;
+            m.sort_hist = nullptr;
+            m.sort_bits = 0;
+            // One continuation pass per round, near the least f: these teams pop
+            // close to it anyway, and their rounds are bound by the relaxers.
+            // 96 mixed instances 0 / 1 / 2 passes: 128 / 111 / 120 ms, 160
+            // 15-puzzles 201 / 176 / 176, 64 grids up to 1500^2 57.7 / 54.6 /
+            // 62.1 (slack 4); puzzles with a slack of one f level (2): 228.
+            m.set(Expansion{1u, ~0u, grid ? 4.f : 0.5f});
+        };
+        if (grid) {
+            GridProblem &prob = im.grid.prob;
+            prob.bm = a.bitmaps + d.bm_word;
+            prob.H = d.H;
+            prob.W = d.W;
+            prob.sx = d.sx;
+            prob.sy = d.sy;
+            prob.ex = d.ex;
+            prob.ey = d.ey;
+            prob.w_inv = GridProblem::row_inverse(prob.W);
+            common(im.grid.m);
+            im.grid.m.heaps = reinterpret_cast<GridEntry *>(heaps);
+        } else if (d.n == 4) {
+            im.p4.prob.pdb = a.pdb4;
+            im.p4.prob.start = d.start_key;
+            im.p4.prob.goal = PuzzleProblem<4>::goal_key();
+            common(im.p4.m);
+            im.p4.m.heaps = reinterpret_cast<PuzzleEntry *>(heaps);
+        } else {
+            im.p3.prob.pdb = a.pdb3;
+            im.p3.prob.start = d.start_key;
+            im.p3.prob.goal = PuzzleProblem<3>::goal_key();
+            common(im.p3.m);
+            im.p3.m.heaps = reinterpret_cast<PuzzleEntry *>(heaps);
+        }
     }
-    SearchMem<PuzzleEntry> m{tab, slots - 1, (uint64_t)(slots * a.max_load), 4096u,
-                             reinterpret_cast<PuzzleEntry *>(heaps),
-                             own_geo ? d.heap_stride : a.stride_puzzle, own_geo ? d.heap_hcap : a.hcap_puzzle,
-                             a.L_puzzle, hs, cand, d.max_rounds};
-    if (d.grow_at) m.grow_at = d.grow_at;
-    m.deadline_ns = deadline_ns;
-    m.split = a.split_puzzle;
-    if (d.n == 4) {
-        PuzzleProblem<4> prob;
-        prob.pdb = a.pdb4;
-        prob.start = d.start_key;
-        prob.goal = PuzzleProblem<4>::goal_key();
-        return ga_search(prob, team, m, a.H, smem, budget);
-    }
-    PuzzleProblem<3> prob;
-    prob.pdb = a.pdb3;
-    prob.start = d.start_key;
-    prob.goal = PuzzleProblem<3>::goal_key();
-    return ga_search(prob, team, m, a.H, smem, budget);
+    __syncthreads();
+    if (grid) return search_instance(im.grid.prob, team, im.grid.m, a.H, smem, budget);
+    if (d.n == 4) return search_instance(im.p4.prob, team, im.p4.m, a.H, smem, budget);
+    return search_instance(im.p3.prob, team, im.p3.m, a.H, smem, budget);
 }
 
 __global__ void __launch_bounds__(512, 1) k_batch(BatchArgs a) {
     __shared__ TeamState st;
     __shared__ uint32_t s_next;
+    __shared__ InstanceMem im;
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t H = a.H;
     // batch: each CTA owns a heap slice reused by the instances it takes;
@@ -206,7 +255,7 @@ __global__ void __launch_bounds__(512, 1) k_batch(BatchArgs a) {
         __syncthreads();
         BlockTeam team{&st};
         run_instance(a, d, team, tab, heaps, hs, cand, smem, d.budget ? d.budget : a.budget,
-                     a.quantum_ns ? t_start + a.quantum_ns : 0);
+                     a.quantum_ns ? t_start + a.quantum_ns : 0, im);
         __syncthreads();
         if (threadIdx.x == 0) {
             InstOut o;
@@ -215,6 +264,7 @@ __global__ void __launch_bounds__(512, 1) k_batch(BatchArgs a) {
             o.goal_slot = st.goal_slot;
             o.goal_best = st.goal_best;
             o.rounds = st.round;
+            o.steps = st.steps;
             o.expanded = st.expanded;
             o.generated = st.generated;
             o.pushed = st.pushed;
@@ -259,6 +309,7 @@ __device__ void clear_partition_team(Slot *tab, uint64_t slots, uint32_t rank, u
 // cluster's CTAs are one GA* team (H heaps each); instances come from the
 // device work queue, one per cluster at a time.
 __global__ void __launch_bounds__(512, 1) k_batch_cluster(BatchArgs a) {
+    __shared__ InstanceMem im;
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t crank = ClusterTeam{nullptr}.cta(), csize = ClusterTeam{nullptr}.ctas();
     const uint32_t cid = blockIdx.x / csize;
@@ -293,7 +344,7 @@ __global__ void __launch_bounds__(512, 1) k_batch_cluster(BatchArgs a) {
         }
         team.sync();
         run_instance(a, d, team, tab, heaps, hs, cand, smem, d.budget ? d.budget : a.budget,
-                     a.quantum_ns ? t_start + a.quantum_ns : 0);
+                     a.quantum_ns ? t_start + a.quantum_ns : 0, im);
         team.sync();
         if (crank == 0 && threadIdx.x == 0) {
             InstOut o;
@@ -302,6 +353,7 @@ __global__ void __launch_bounds__(512, 1) k_batch_cluster(BatchArgs a) {
             o.goal_slot = ldcg_u32(&st->goal_slot);
             o.goal_best = ldcg_u64(&st->goal_best);
             o.rounds = ldcg_u64(&st->round);
+            o.steps = ldcg_u64(&st->steps);
             o.expanded = ldcg_u64(&st->expanded);
             o.generated = ldcg_u64(&st->generated);
             o.pushed = ldcg_u64(&st->pushed);
@@ -759,7 +811,7 @@ int32_t run_wave(uastar_engine *eng, const uastar_instance *insts, const std::ve
         r.status = (int32_t)o.status;
         r.expanded += (int64_t)o.expanded;
         r.generated += (int64_t)o.generated;
-        r.rounds += (int64_t)o.rounds;
+        r.rounds += (int64_t)o.steps;
         if (stats) {
             stats->expanded += (int64_t)o.expanded;
             stats->generated += (int64_t)o.generated;
@@ -796,13 +848,8 @@ int32_t run_wave(uastar_engine *eng, const uastar_instance *insts, const std::ve
         } else {
             r.steps = (int32_t)o.goal_best;
             std::vector<int32_t> moves;
-            auto blank = [&](uint64_t k) {
-                for (int c = 0; c < in.n * in.n; ++c)
-                    if (((k >> (4 * c)) & 15) == 0) return c;
-                return -1;
-            };
             for (uint64_t t = len - 1; t >= 1; --t) {
-                const int pb = blank(kk[t]), cb = blank(kk[t - 1]);
+                const int pb = key_blank(kk[t]), cb = key_blank(kk[t - 1]);
                 moves.push_back(cb - pb == in.n ? 0 : cb - pb == -in.n ? 1 : cb - pb == 1 ? 2 : 3);
             }
             if ((int64_t)moves.size() != r.steps ||
@@ -1502,13 +1549,8 @@ static int32_t serve_finish_ok(ServeReq &r, const InstOut &o, const std::vector<
     }
     r.acc.steps = (int32_t)o.goal_best;
     std::vector<int32_t> moves;
-    auto blank = [&](uint64_t k) {
-        for (int c = 0; c < in.n * in.n; ++c)
-            if (((k >> (4 * c)) & 15) == 0) return c;
-        return -1;
-    };
     for (uint64_t u = len - 1; u >= 1; --u) {
-        const int pb = blank(kk[u]), cb = blank(kk[u - 1]);
+        const int pb = key_blank(kk[u]), cb = key_blank(kk[u - 1]);
         moves.push_back(cb - pb == in.n ? 0 : cb - pb == -in.n ? 1 : cb - pb == 1 ? 2 : 3);
     }
     if ((int64_t)moves.size() != r.acc.steps ||
@@ -1769,7 +1811,7 @@ static void serve_retire(ServeState *S, ServeTier &t, std::deque<ServeReq> &to_l
         r.acc.device_ms = (double)(o.t_end - o.t_start) * 1e-6;
         r.acc.expanded += (int64_t)o.expanded;
         r.acc.generated += (int64_t)o.generated;
-        r.acc.rounds += (int64_t)o.rounds;
+        r.acc.rounds += (int64_t)o.steps;
         int32_t status = (int32_t)o.status;
         if (status == ST_OK && o.path_len == kWalkDeferred && serve_walk_issue(S, t, q)) {
             t.descs[q].kind = 0;

@@ -220,6 +220,19 @@ template <class P> uint32_t plain_heaps(const uastar_config &c) {
     return c.heaps > 0 ? (uint32_t)c.heaps : (P::kMoves >= 8 ? 8192u : 16384u);
 }
 
+// The plain engine's launch shape: H heaps per CTA, n CTAs.  Left to the
+// engine, the heaps are rounded up to a whole number of CTAs per SM (9728 in
+// 152 CTAs for 8192, 19456 in 304 for 16384): a round lasts as long with one
+// CTA fewer on some SMs, and every heap more is a pop more.  20000^2 grid
+// 194 -> 179 ms, 60-move 15-puzzle 6.1 -> 5.4 ms.
+template <class P>
+void plain_shape(const uastar_engine *eng, uint32_t block, uint32_t tph, uint32_t *H, uint32_t *n) {
+    *H = std::max(1u, block / std::min(tph, block));
+    *n = (plain_heaps<P>(eng->cfg) + *H - 1) / *H;
+    const uint32_t sms = (uint32_t)std::max(1, eng->sms);
+    if (eng->cfg.heaps <= 0) *n = (*n + sms - 1) / sms * sms;
+}
+
 // Moves a paused search's table to one 4x larger (k_grow_*), swapping it in
 // as eng->tab.  Returns false (and changes nothing) if the memory is not there.
 template <class P>
@@ -264,8 +277,8 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
     const uastar_config &c = eng->cfg;
     const uint32_t block = (uint32_t)c.block_threads;
     const uint32_t tph = c.threads_per_heap > 0 ? (uint32_t)c.threads_per_heap : 4u;
-    const uint32_t H = std::max(1u, block / std::min(tph, block));
-    const uint32_t nblocks = (plain_heaps<P>(c) + H - 1) / H;
+    uint32_t H, nblocks;
+    plain_shape<P>(eng, block, tph, &H, &nblocks);
     const uint32_t k = nblocks * H;
     int log2 = c.hash_log2_slots > 0 ? c.hash_log2_slots : log2_auto;
     if (log2 > 31) {
@@ -368,6 +381,20 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
         m.heap_size = eng->heap_size.as<uint32_t>();
         m.cand = eng->cand.as<Cand>();
         m.max_rounds = (uint64_t)c.max_rounds;
+        if (!sorted) m.set(prob.expansion(k));
+        if constexpr (std::is_same<P, GridProblem>::value) {
+            // An auto-sized table starts at 2^20 slots.  Maps of 2^19 to 2^20
+            // cells keep the open frontier unbounded: their search is expected
+            // to outgrow that table's growth point (2^19 states; the in-place
+            // growth of a grid is pinned by a test on the 1000^2 map), and so
+            // few states stay in L2.  1000^2: 12.6 ms -> 9.7 ms so (2 passes),
+            // 6.4 ms with the bound.
+            const uint64_t cells = (uint64_t)prob.H * (uint64_t)prob.W;
+            if (!sorted && c.hash_log2_slots <= 0 && cells > (1ull << 19) && cells <= (1ull << 20)) {
+                m.slack = 0.f;
+                m.cont = 2;
+            }
+        }
         if (sorted) {
             m.sort_buf = eng->sortb.as<unsigned long long>();
             m.sort_hist = reinterpret_cast<uint32_t *>(m.sort_buf + 2 * sort_n);
@@ -547,6 +574,7 @@ int32_t grid_solve_impl(uastar_engine *eng, const uint64_t *host_words, int32_t 
     prob.sy = sy;
     prob.ex = ex;
     prob.ey = ey;
+    prob.w_inv = GridProblem::row_inverse(prob.W);
     const uint64_t cells = (uint64_t)H * W;
     const int log2_auto = std::min(28, std::max(20, ceil_log2_u64(cells) - 1));
     const uint32_t per_heap =
@@ -559,7 +587,7 @@ int32_t grid_solve_impl(uastar_engine *eng, const uint64_t *host_words, int32_t 
     out->expanded = (int64_t)st.expanded;
     out->generated = (int64_t)st.generated;
     out->pushed = (int64_t)st.pushed;
-    out->rounds = (int64_t)st.round;
+    out->rounds = (int64_t)st.steps;
     out->table_used = (int64_t)st.inserted;
     out->kernel_ms = po.kernel_ms;
     out->table_grows = po.grows;
@@ -653,7 +681,7 @@ int32_t walk_boards(uastar_engine *eng, uint32_t slot, std::vector<std::vector<u
         if (int32_t rc = walk_keys_wide(eng, slot, 4096, &keys)) return rc;
         for (const Key128 &k : keys) {
             std::vector<uint8_t> b(25);
-            for (int c = 0; c < 25; ++c) b[c] = (uint8_t)PuzzleProblem<5>::field(k, c);
+            for (int t = 0; t < 25; ++t) b[PuzzleProblem<5>::cell(k, t)] = (uint8_t)t;
             boards->push_back(b);
         }
     } else {
@@ -661,7 +689,7 @@ int32_t walk_boards(uastar_engine *eng, uint32_t slot, std::vector<std::vector<u
         if (int32_t rc = walk_keys(eng, slot, 4096, &keys, PuzzleProblem<4>::kLink)) return rc;
         for (uint64_t k : keys) {
             std::vector<uint8_t> b(N * N);
-            for (int c = 0; c < N * N; ++c) b[c] = (uint8_t)((k >> (4 * c)) & 15);
+            for (int t = 0; t < N * N; ++t) b[(k >> (4 * t)) & 15] = (uint8_t)t;
             boards->push_back(b);
         }
     }
@@ -884,9 +912,9 @@ int32_t puzzle_bounded_n(uastar_engine *eng, const uint8_t *tiles, int max_log2,
         out->generated += (int64_t)po.st.generated;
         out->kernel_ms += po.kernel_ms;
         std::vector<std::vector<uint8_t>> boards;
-        if (po.st.status == ST_OK) {
-            if (seg == 0) out->lower_bound = (int32_t)po.st.goal_best;
-            if ((rc = walk_boards<N>(eng, po.st.goal_slot, &boards))) return rc;
+        const auto solved = [&](uint64_t cost, uint32_t slot) -> int32_t {
+            if (seg == 0) out->lower_bound = (int32_t)cost;
+            if ((rc = walk_boards<N>(eng, slot, &boards))) return rc;
             boards_to_moves(N, boards, moves);
             // more than one segment: the exact phase, from the first
             // segment's bound up to this solution's length
@@ -894,7 +922,8 @@ int32_t puzzle_bounded_n(uastar_engine *eng, const uint8_t *tiles, int max_log2,
                 return ida_exact<N>(eng, tiles, out->lower_bound, (int32_t)moves->size(),
                                     eng->cfg.exact_ms > 0 ? (double)eng->cfg.exact_ms : 3000.0, moves, out);
             return UASTAR_OK;
-        }
+        };
+        if (po.st.status == ST_OK) return solved(po.st.goal_best, po.st.goal_slot);
         if (po.st.status != ST_RUNNING) return (int32_t)po.st.status;
         // paused with the table full: commit to the best open node
         if ((e = eng->walk.ensure(4096 * 8 + 64)) != cudaSuccess) return fail_cuda(eng, e, "alloc walk");
@@ -906,6 +935,9 @@ int32_t puzzle_bounded_n(uastar_engine *eng, const uint8_t *tiles, int max_log2,
         unsigned long long best = ~0ull;
         cudaMemcpyAsync(&best, d_best, 8, cudaMemcpyDeviceToHost, eng->stream);
         if ((e = cudaStreamSynchronize(eng->stream)) != cudaSuccess) return fail_cuda(eng, e, "best open node");
+        // a goal at or below every open node (the pause came before the decision
+        // that takes it): this segment's optimum
+        if (po.st.goal_best <= best >> 48) return solved(po.st.goal_best, po.st.goal_slot);
         if (best == ~0ull) {
             return fallback(UASTAR_HASH_FULL, "bounded search: no current open node at the memory bound");
         }
@@ -1035,8 +1067,8 @@ int32_t uastar_round_floor(uastar_engine *eng, int32_t rounds, double *us_barrie
     const uastar_config &c = eng->cfg;
     const uint32_t block = (uint32_t)c.block_threads;
     const uint32_t tph = c.threads_per_heap > 0 ? (uint32_t)c.threads_per_heap : 4u;
-    const uint32_t H = std::max(1u, block / std::min(tph, block));
-    const uint32_t nblocks = (plain_heaps<GridProblem>(c) + H - 1) / H;
+    uint32_t H, nblocks;
+    plain_shape<GridProblem>(eng, block, tph, &H, &nblocks);
     int max_active = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&max_active, (const void *)k_round_floor,
                                                                   (int)block, 0);
@@ -1164,7 +1196,7 @@ int32_t uastar_puzzle_solve(uastar_engine *eng, int32_t n, const uint8_t *tiles,
     out->expanded = (int64_t)st.expanded;
     out->generated = (int64_t)st.generated;
     out->pushed = (int64_t)st.pushed;
-    out->rounds = (int64_t)st.round;
+    out->rounds = (int64_t)st.steps;
     out->table_used = (int64_t)st.inserted;
     out->kernel_ms = po.kernel_ms;
     out->table_grows = po.grows;
@@ -1176,22 +1208,12 @@ int32_t uastar_puzzle_solve(uastar_engine *eng, int32_t n, const uint8_t *tiles,
             std::vector<Key128> keys;
             rc = walk_keys_wide(eng, st.goal_slot, 4096, &keys);
             if (rc) return out->status = rc;
-            for (const Key128 &k : keys) {
-                int b = 24;
-                for (int c = 0; c < 24; ++c)
-                    if (PuzzleProblem<5>::field(k, c) == 0) b = c;
-                blanks.push_back(b);
-            }
+            for (const Key128 &k : keys) blanks.push_back((int)PuzzleProblem<5>::cell(k, 0));
         } else {
             std::vector<uint64_t> keys;
             rc = walk_keys(eng, st.goal_slot, 4096, &keys, PuzzleProblem<4>::kLink);
             if (rc) return out->status = rc;
-            for (uint64_t k : keys) {
-                int b = -1;
-                for (int c = 0; c < n * n; ++c)
-                    if (((k >> (4 * c)) & 15) == 0) b = c;
-                blanks.push_back(b);
-            }
+            for (uint64_t k : keys) blanks.push_back(key_blank(k));
         }
         for (size_t i = 1; i < blanks.size(); ++i) {
             const int d = blanks[i] - blanks[i - 1];

@@ -44,12 +44,15 @@ struct DevBuf {
     template <class T> T *as() const { return static_cast<T *>(p); }
 };
 
-// A 3x3 / 4x4 board packed as the search's 64-bit key (cell c in bits 4c..4c+3).
+// A 3x3 / 4x4 board as the search's 64-bit key: the cell of tile t in bits
+// 4t..4t+3, the nibbles past the last tile all ones (PuzzleProblem).
 inline uint64_t pack_board(int n, const uint8_t *tiles) {
-    uint64_t k = 0;
-    for (int i = 0; i < n * n; ++i) k |= (uint64_t)(tiles[i] & 15) << (4 * i);
+    uint64_t k = n * n < 16 ? ~0ull << (4 * n * n) : 0ull;
+    for (int i = 0; i < n * n; ++i) k |= (uint64_t)i << (4 * (tiles[i] & 15));
     return k;
 }
+// Blank cell of such a key.
+inline int key_blank(uint64_t key) { return (int)(key & 15u); }
 
 // Solvability of a valid board: the goal has no inversions and the blank in
 // row n-1.  A horizontal move keeps the inversion parity; a vertical move

@@ -32,7 +32,7 @@ enum : uint32_t {
 // One dedup-table slot: exactly one 32-byte sector, so a probe, the g update
 // and the pop-time read of a node each touch a single sector.
 struct __align__(32) Slot {
-    unsigned long long key;  // state key (grid cell id / packed board); kEmptyKey = free
+    unsigned long long key;  // state key (grid cell id / the cells of a board's tiles); kEmptyKey = free
     unsigned long long g;    // cost from the start (problem-specific packing)
     uint32_t aux;            // problem data (puzzle: PDB parts and last move)
     uint32_t prev;           // parent slot, kNone for the root
@@ -131,9 +131,14 @@ struct __align__(16) TeamState {
     uint32_t pad0_;
     uint32_t quit[3];                 // the round ended past the search's time slice (SearchMem::deadline_ns)
     uint32_t pad1_;
+    uint32_t pass[3];                 // most continuation passes a warp made in the round
+    uint32_t pad2_;
+    uint32_t pops[3];                 // entries popped in the round
+    uint32_t bound;                   // (float) the next round's bound on f (SearchMem::slack)
     // totals, stored by CTA 0 when the search stops or pauses
     unsigned long long goal_best;     // best goal f popped so far
     unsigned long long round;         // rounds completed
+    unsigned long long steps;         // expansion steps: one per round and one per continuation pass
     unsigned long long inserted;      // dedup slots in use
     unsigned long long expanded, generated, pushed;
     uint32_t goal_slot;
@@ -150,6 +155,7 @@ __host__ __device__ inline void team_state_init(TeamState *s) {
     unsigned char *b = reinterpret_cast<unsigned char *>(s);
     for (unsigned i = 0; i < sizeof(TeamState); ++i) b[i] = 0;
     for (int i = 0; i < 3; ++i) s->round_min[i] = s->goal_min[i] = kInfCost;
+    s->bound = 0x7f800000u;  // +infinity
     s->goal_best = kInfCost;
     s->goal_slot = kNone;
     s->status = ST_RUNNING;
@@ -194,34 +200,12 @@ __host__ __device__ __forceinline__ uint64_t mix64(uint64_t k) {
 __host__ __device__ __forceinline__ uint64_t key_hash(uint64_t k) { return mix64(k); }
 __host__ __device__ __forceinline__ uint64_t key_hash(const Key128 &k) { return mix64(k.lo ^ mix64(k.hi)); }
 
-enum : int { FIND_FOUND = 0, FIND_INSERTED = 1, FIND_FULL = 2 };
-
-// Open addressing with linear probing over 32-byte slots.  A free slot is
-// claimed with atomicCAS on its key; the winner of the race owns it and every
-// other writer of the same key sees the key on its retry.
-__device__ __forceinline__ int find_or_insert(Slot *tab, uint64_t mask, uint64_t key,
-                                              uint32_t max_probe, uint32_t *slot_out) {
-    uint64_t h = mix64(key) & mask;
-    for (uint32_t i = 0; i < max_probe; ++i) {
-        unsigned long long k = ldcg_u64(&tab[h].key);
-        if (k == key) {
-            *slot_out = (uint32_t)h;
-            return FIND_FOUND;
-        }
-        if (k == kEmptyKey) {
-            unsigned long long old = atomicCAS(&tab[h].key, kEmptyKey, (unsigned long long)key);
-            if (old == kEmptyKey) {
-                *slot_out = (uint32_t)h;
-                return FIND_INSERTED;
-            }
-            if (old == key) {
-                *slot_out = (uint32_t)h;
-                return FIND_FOUND;
-            }
-        }
-        h = (h + 1) & mask;
-    }
-    return FIND_FULL;
+// Probe order of the dedup table: the four slots of the home slot's 128-byte
+// line, from the home slot round, then the following lines from their first
+// slot.  A new key takes the first free slot in this order (slots are never
+// freed), so a search for it may stop at the first free one.
+__device__ __forceinline__ uint64_t probe_slot(uint64_t home, uint32_t i, uint64_t mask) {
+    return i < 4 ? (home & ~3ull) | ((home + i) & 3ull) : ((home & ~3ull) + i) & mask;
 }
 
 // ------------------------------------------------------- warp helpers ---
@@ -245,8 +229,10 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 // another CTA has flagged an error, it records ST_TIMEOUT (first error wins)
 // and leaves; the caller checks the error word after every barrier, so all
 // CTAs stop together at the next one.
+// `then` runs on thread 0 between its wait and the CTA's release.
+template <class F>
 __device__ __forceinline__ void grid_barrier(uint32_t *counter, uint32_t nblocks, uint32_t &epoch,
-                                             uint32_t *err, uint64_t timeout_ns) {
+                                             uint32_t *err, uint64_t timeout_ns, F &&then) {
     __syncthreads();
     if (threadIdx.x == 0) {
         epoch += 1;
@@ -267,6 +253,7 @@ __device__ __forceinline__ void grid_barrier(uint32_t *counter, uint32_t nblocks
         }
         // the acquire load that saw the last arrival orders this thread after
         // every CTA's release; the CTA barrier below carries that to the rest
+        then();
     }
     __syncthreads();
 }

@@ -29,17 +29,19 @@ __global__ void k_grow_move(const Slot *src, uint64_t n, Slot *dst, uint64_t mas
         uint64_t h;
         if constexpr (Wide) {
             const Key128 k{key, ((unsigned long long)a.w << 32) | a.z};
-            h = key_hash(k) & mask;
-            for (uint64_t probe = 0; probe <= mask; ++probe) {
+            const uint64_t home = key_hash(k) & mask;
+            h = home;
+            for (uint32_t probe = 1; probe <= mask; ++probe) {
                 const KeyG old = cas128(dst + h, KeyG{kEmptyKey, kEmptyKey}, KeyG{k.lo, k.hi});
                 if (old.key == kEmptyKey && old.g == kEmptyKey) break;
-                h = (h + 1) & mask;
+                h = probe_slot(home, probe, mask);
             }
         } else {
-            h = mix64(PrevInKey ? key & 0xffffffffull : key) & mask;
-            for (uint64_t probe = 0; probe <= mask; ++probe) {
+            const uint64_t home = mix64(PrevInKey ? key & 0xffffffffull : key) & mask;
+            h = home;
+            for (uint32_t probe = 1; probe <= mask; ++probe) {
                 if (atomicCAS(&dst[h].key, kEmptyKey, key) == kEmptyKey) break;
-                h = (h + 1) & mask;
+                h = probe_slot(home, probe, mask);
             }
         }
         uint4 *d = reinterpret_cast<uint4 *>(dst + h);

@@ -17,6 +17,13 @@
 
 namespace uastar {
 
+// How far a whole-GPU search of k heaps expands beyond its pops
+// (SearchMem::cont, cont_pops and slack).
+struct Expansion {
+    uint32_t cont, cont_pops;
+    float slack;
+};
+
 // ----------------------------------------------------------------- grid ---
 struct __align__(16) GridEntry {
     uint32_t fa, fb;  // f = fa + fb*sqrt(2)
@@ -51,11 +58,30 @@ struct GridProblem : NarrowSlots {
     __device__ static uint32_t slot_prev(const Slot *s) { return (uint32_t)(__ldcg(&s->key) >> 32); }
     __device__ static void set_link(Slot *, uint32_t, uint32_t) {}  // the link lives in the key word
 
+    struct Succ {  // see succ_begin
+        uint64_t key, g, f;
+    };
     const uint32_t *bm;  // bitmap as 32-bit words (same bytes as the uint64 words)
     int32_t H, W;
     int32_t sx, sy, ex, ey;
+    uint64_t w_inv;  // row_inverse(W)
+
+    // c / W as one widening multiply: w_inv = ceil(2^64 / W) makes
+    // floor(c * w_inv / 2^64) exact for every c < 2^32 (w_inv * W exceeds
+    // 2^64 by less than W, so the product by less than c / 2^64 < 1 / W);
+    // 0 stands for 2^64 (W = 1).
+    __host__ __device__ static uint64_t row_inverse(int32_t W) {
+        return W == 1 ? 0ull : ~0ull / (uint64_t)W + 1ull;
+    }
+    __device__ __forceinline__ uint32_t row_of(uint32_t c) const {
+        return w_inv ? (uint32_t)__umul64hi((uint64_t)c, w_inv) : c;
+    }
 
     __device__ static int cost_cmp(uint64_t a, uint64_t b) { return grid_cost_cmp(a, b); }
+    // a cost as one number, to place the round's bound (no exact test uses it)
+    __device__ static float cost_val(uint64_t c) {
+        return (float)(uint32_t)(c >> 32) + 1.41421356f * (float)(uint32_t)c;
+    }
 
     __device__ __forceinline__ bool open(int64_t id) const {
         return (__ldg(bm + (id >> 5)) >> (id & 31)) & 1u;
@@ -98,7 +124,7 @@ struct GridProblem : NarrowSlots {
     // distances to the goal, h = min(dx,dy)*sqrt2 + |dx-dy| — as a pair.
     __device__ __forceinline__ uint64_t h_of(uint64_t key) const {
         const uint32_t c = (uint32_t)key;  // H*W < 2^32 is checked on the host
-        const int x = (int)(c / (uint32_t)W), y = (int)(c - (uint32_t)x * (uint32_t)W);
+        const int x = (int)row_of(c), y = (int)(c - (uint32_t)x * (uint32_t)W);
         const int dx = abs(x - ex), dy = abs(y - ey);
         const int mn = min(dx, dy), mx = max(dx, dy);
         return ((uint64_t)(mx - mn) << 32) | (uint64_t)mn;
@@ -110,30 +136,47 @@ struct GridProblem : NarrowSlots {
     // Open bits of the cells (r, y-1), (r, y), (r, y+1) as bits 0..2 (0 for a
     // row or column outside the grid).  Two 32-bit words cover the three
     // cells, and their addresses depend on the cell alone, so the three rows
-    // of a node are read in one round trip of independent loads.
-    __device__ __forceinline__ uint32_t row3(int r, int y) const {
-        if (r < 0 || r >= H) return 0;
+    // of a node are read in one round trip of independent loads (look_begin)
+    // and taken apart later (look_rows).
+    struct Look {
+        uint64_t v[3];
+    };
+    __device__ __forceinline__ uint64_t row_words(int r, int y) const {
         const int64_t c0 = (int64_t)r * W + y - 1;  // cell (r, y-1); -1 only for (0, 0)
         const uint64_t lo = c0 < 0 ? 0 : (uint64_t)c0;
         const uint64_t wlast = ((uint64_t)(uint32_t)H * (uint32_t)W + 63) / 64 * 2 - 1;  // last 32-bit word
         const uint64_t w0 = lo >> 5, w1 = w0 + 1 <= wlast ? w0 + 1 : wlast;
-        const uint64_t v = (uint64_t)__ldg(bm + w0) | ((uint64_t)__ldg(bm + w1) << 32);
+        return (uint64_t)__ldg(bm + w0) | ((uint64_t)__ldg(bm + w1) << 32);
+    }
+    __device__ __forceinline__ uint32_t row_bits(uint64_t v, int r, int y) const {
+        if (r < 0 || r >= H) return 0;
+        const int64_t c0 = (int64_t)r * W + y - 1;
+        const uint64_t lo = c0 < 0 ? 0 : (uint64_t)c0;
         uint32_t bits = (uint32_t)(v >> (lo & 31u)) & 7u;
         if (c0 < 0) bits = (bits << 1) & 7u;  // the window starts one cell before the grid
         if (y == 0) bits &= ~1u;              // (r, -1) is no cell
         if (y == W - 1) bits &= ~4u;          // (r, W) is no cell (the next row's first)
         return bits;
     }
+    __device__ __forceinline__ void look_begin(uint64_t key, Look &k) const {
+        const uint32_t c = (uint32_t)key;
+        const int x = (int)row_of(c), y = (int)(c - (uint32_t)x * (uint32_t)W);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const int r = x - 1 + i;
+            k.v[i] = r < 0 || r >= H ? 0 : row_words(r, y);
+        }
+    }
 
-    // Valid moves of a popped cell, bit i = direction i (4 straight, then 4
+    // Valid moves of a cell, bit i = direction i (4 straight, then 4
     // diagonal; src/utils.hpp:120-122).  Only an open cell moves
     // (CPU-solver.cpp:98-100).  A move into a blocked cell is legal in the
     // reference but such a cell has no out-moves, so it is generated only
     // when it is the goal: no path cost changes.
-    __device__ uint32_t moves(uint64_t key, uint32_t) const {
+    __device__ __forceinline__ uint32_t rows_moves(uint64_t key, const Look &k) const {
         const uint32_t c = (uint32_t)key;
-        const int x = (int)(c / (uint32_t)W), y = (int)(c - (uint32_t)x * (uint32_t)W);
-        const uint32_t rows[3] = {row3(x - 1, y), row3(x, y), row3(x + 1, y)};
+        const int x = (int)row_of(c), y = (int)(c - (uint32_t)x * (uint32_t)W);
+        const uint32_t rows[3] = {row_bits(k.v[0], x - 1, y), row_bits(k.v[1], x, y), row_bits(k.v[2], x + 1, y)};
         if (!(rows[1] & 2u)) return 0;
         uint32_t m = 0;
 #pragma unroll
@@ -142,6 +185,32 @@ struct GridProblem : NarrowSlots {
             const bool goal = x + dx == ex && y + dy == ey;
             if (((rows[dx + 1] >> (dy + 1)) & 1u) || goal) m |= 1u << i;
         }
+        return m;
+    }
+    __device__ __forceinline__ uint32_t moves(uint64_t key, uint32_t) const {
+        Look k;
+        look_begin(key, k);
+        return rows_moves(key, k);
+    }
+    // Three passes a round, within 1/64 of the straight distance between the
+    // query's ends, 1 to 16.  Measured on 20000^2 (distance 28283): slack 4 /
+    // 8 / 16 / 32: 272 / 224 / 215 / 277 ms (narrow: more rounds; wide: every
+    // state expanded again), passes 2 / 3 / 4 / 5 at 8: 238 / 224 / 220 / 234;
+    // six queries on 1537 x 2049: 33-35 ms throughout; 61 x 67 (distance 84):
+    // slack 1 0.21 ms, 8 0.27, 32 0.32.
+    __host__ __device__ Expansion expansion(uint32_t) const {
+        const int dx = sx < ex ? ex - sx : sx - ex, dy = sy < ey ? ey - sy : sy - ey;
+        const int mn = dx < dy ? dx : dy, mx = dx < dy ? dy : dx;
+        const float slack = ((float)mx + 0.41421356f * (float)mn) / 64.f;
+        return Expansion{3u, ~0u, slack < 1.f ? 1.f : slack > 16.f ? 16.f : slack};
+    }
+    // Continuation (ga_search): whether this successor is within the bound, and
+    // the moves of one that is, looked at in look_begin; naux names its
+    // incoming move (entry_moves).
+    __device__ __forceinline__ bool peek(const Succ &s, float bound) const { return cost_val(s.f) <= bound; }
+    __device__ __forceinline__ uint32_t look_moves(uint64_t key, uint32_t naux, const Look &k) const {
+        uint32_t m = rows_moves(key, k);
+        if (dirs()) m &= ~pruned(naux >> kCellBits);
         return m;
     }
     __device__ __forceinline__ static int c_dx(int i) {
@@ -153,7 +222,7 @@ struct GridProblem : NarrowSlots {
     __device__ void apply(uint64_t key, uint64_t g, uint32_t, int mv, uint64_t &nkey,
                           uint64_t &ng, uint32_t &naux, uint64_t &nf) const {
         const uint32_t c = (uint32_t)key;
-        const int x = (int)(c / (uint32_t)W), y = (int)(c - (uint32_t)x * (uint32_t)W);
+        const int x = (int)row_of(c), y = (int)(c - (uint32_t)x * (uint32_t)W);
         nkey = (uint64_t)(x + c_dx(mv)) * W + (uint64_t)(y + c_dy(mv));
         ng = g + (mv < 4 ? (1ull << 32) : 1ull);
         naux = in_aux(nkey, mv);
@@ -162,9 +231,6 @@ struct GridProblem : NarrowSlots {
     // Successor in two steps (the puzzle's second step waits on a database
     // load that is issued in the first, so that it overlaps the table CAS);
     // for grids everything is register arithmetic in the first.
-    struct Succ {
-        uint64_t key, g, f;
-    };
     __device__ __forceinline__ void succ_begin(uint64_t key, uint64_t g, uint32_t aux, int mv, Succ &s) const {
         uint32_t naux;
         apply(key, g, aux, mv, s.key, s.g, naux, s.f);
@@ -269,6 +335,13 @@ template <int N> __host__ __device__ constexpr int pattern_of_tile(int t) {
     return -1;
 }
 
+// the pattern of every tile, 2 bits per tile
+template <int N> __host__ __device__ constexpr uint64_t pattern_bits() {
+    uint64_t m = 0;
+    for (int t = 1; t < N * N; ++t) m |= (uint64_t)pattern_of_tile<N>(t) << (2 * t);
+    return m;
+}
+
 template <int N> struct PuzzleProblem : NarrowSlots {
     using Entry = PuzzleEntry;
     static constexpr int kMoves = 4;
@@ -287,40 +360,52 @@ template <int N> struct PuzzleProblem : NarrowSlots {
     __device__ static uint32_t slot_prev(const Slot *s) { return (uint32_t)__ldcg(&s->g); }
     __device__ static void set_link(Slot *s, uint32_t, uint32_t aux) { s->aux = aux & 0xffffu; }
 
+    // The key is the board's inverse: nibble t = cell of tile t (tile 0 = the
+    // blank), nibbles past the last tile all ones (no cell has that number).
+    // Ranks read tiles' cells, so a successor's rank needs no inversion of its
+    // board, and a move swaps two nibbles (two tiles trade cells).
+    static constexpr uint64_t kPad = NN < 16 ? (~0ull << (4 * (NN < 16 ? NN : 0))) : 0ull;
+
     const uint8_t *pdb;   // concatenated tables
-    uint64_t start;       // packed board: cell i at bits 4i
+    uint64_t start;
     uint64_t goal;
 
     __device__ static int cost_cmp(uint64_t a, uint64_t b) { return a < b ? -1 : (a > b ? 1 : 0); }
+    __device__ static float cost_val(uint64_t c) { return (float)c; }
 
     __host__ __device__ static uint64_t goal_key() {
-        uint64_t k = 0;
-        for (int i = 0; i < NN; ++i) k |= (uint64_t)((i + 1) % NN) << (4 * i);
+        uint64_t k = kPad | (uint64_t)(NN - 1);
+        for (int t = 1; t < NN; ++t) k |= (uint64_t)(t - 1) << (4 * t);
         return k;
     }
-    // Inverse permutation: nibble t = cell of tile t.
-    __device__ __forceinline__ static uint64_t inverse(uint64_t key) {
-        uint64_t inv = 0;
+    // Rank of pattern p's tiles (the reference's mixed-radix code in Horner
+    // form: digit j counts the cells below tile j's that no earlier tile of
+    // the pattern holds).  Both patterns of the 4x4 board take the same
+    // instructions, each tile's cell selected by p: lanes of a warp move tiles
+    // of both, and the two ranks in diverged branches would add up.
+    __device__ __forceinline__ static uint32_t rank(int p, uint64_t key) {
+        constexpr int K = PuzzlePatterns<N>::count(0);
+        uint32_t used = 0, code = 0, shorter = 0;
 #pragma unroll
-        for (int i = 0; i < NN; ++i) inv |= (uint64_t)i << (4 * ((key >> (4 * i)) & 15));
-        return inv;
-    }
-    template <int P> __device__ __forceinline__ static uint32_t rank(uint64_t inv) {
-        uint32_t used = 0, code = 0;
-#pragma unroll
-        for (int j = 0; j < PuzzlePatterns<N>::count(P); ++j) {
-            const uint32_t pos = (uint32_t)(inv >> (4 * PuzzlePatterns<N>::tile(P, j))) & 15u;
-            const uint32_t v = pos - __popc(used & ((1u << pos) - 1u));
-            code += v * pattern_mult<N>(P, j + 1);
+        for (int j = 0; j < K; ++j) {
+            uint32_t pos = (uint32_t)(key >> (4 * PuzzlePatterns<N>::tile(0, j))) & 15u;
+            if constexpr (PuzzlePatterns<N>::kNum > 1) {
+                if (j < PuzzlePatterns<N>::count(1)) {
+                    const uint32_t pos1 = (uint32_t)(key >> (4 * PuzzlePatterns<N>::tile(1, j))) & 15u;
+                    pos = p ? pos1 : pos;
+                }
+            }
+            code = code * (uint32_t)(NN - j) + pos - __popc(used & ((1u << pos) - 1u));
             used |= 1u << pos;
+            if constexpr (PuzzlePatterns<N>::kNum > 1)
+                if (j + 1 == PuzzlePatterns<N>::count(1)) shorter = code;
         }
-        return code;
+        return PuzzlePatterns<N>::kNum > 1 && p ? shorter : code;
     }
-    __device__ __forceinline__ uint32_t part(int p, uint64_t inv) const {
-        if (p == 0) return __ldg(pdb + PuzzlePatterns<N>::offset(0) + rank<0>(inv));
-        if constexpr (PuzzlePatterns<N>::kNum > 1)
-            return __ldg(pdb + PuzzlePatterns<N>::offset(1) + rank<1>(inv));
-        return 0;
+    __device__ __forceinline__ uint32_t part(int p, uint64_t key) const {
+        uint32_t off = 0;
+        if constexpr (PuzzlePatterns<N>::kNum > 1) off = p ? (uint32_t)PuzzlePatterns<N>::offset(1) : 0u;
+        return __ldg(pdb + (off + rank(p, key)));
     }
     // aux = part0 | part1 << 8 | (last move + 1) << 16
     static constexpr uint32_t kLastMoveShift = 16;
@@ -328,19 +413,20 @@ template <int N> struct PuzzleProblem : NarrowSlots {
 
     __device__ uint64_t start_key() const { return start; }
     __device__ uint32_t start_aux() const {
-        const uint64_t inv = inverse(start);
-        uint32_t a = part(0, inv);
-        if (PuzzlePatterns<N>::kNum > 1) a |= part(1, inv) << 8;
+        uint32_t a = part(0, start);
+        if (PuzzlePatterns<N>::kNum > 1) a |= part(1, start) << 8;
         return a;
     }
     __device__ bool is_goal(uint64_t key) const { return key == goal; }
     __device__ __forceinline__ uint64_t f_of(uint64_t, uint64_t g, uint32_t aux) const {
         return g + hsum(aux);
     }
-    __device__ __forceinline__ static int blank(uint64_t key) {
-        constexpr uint64_t kPad = NN < 16 ? (~0ull << (4 * (NN < 16 ? NN : 0))) : 0ull;
-        uint64_t z = ~(key | kPad);
-        z = z & (z >> 1) & (z >> 2) & (z >> 3) & 0x1111111111111111ull;
+    __device__ __forceinline__ static int blank(uint64_t key) { return (int)(key & 15u); }
+    // The tile on cell q: the one nibble equal to q (lowest zero nibble of the
+    // difference; the test is exact up to the first one).
+    __device__ __forceinline__ static int tile_on(uint64_t key, int q) {
+        const uint64_t x = key ^ ((uint64_t)q * 0x1111111111111111ull);
+        const uint64_t z = (x - 0x1111111111111111ull) & ~x & 0x8888888888888888ull;
         return (__ffsll((long long)z) - 1) >> 2;
     }
     // Blank moves 0..3 = DX/DY[0..3] of src/utils.hpp:120-121.  The move that
@@ -357,22 +443,6 @@ template <int N> struct PuzzleProblem : NarrowSlots {
         if (last) m &= ~(1u << ((last - 1) ^ 1));
         return m;
     }
-    __device__ void apply(uint64_t key, uint64_t g, uint32_t aux, int mv, uint64_t &nkey,
-                          uint64_t &ng, uint32_t &naux, uint64_t &nf) const {
-        const int b = blank(key);
-        const int q = b + (mv == 0 ? N : mv == 1 ? -N : mv == 2 ? 1 : -1);
-        const uint64_t t = (key >> (4 * q)) & 15;
-        nkey = (key & ~(15ull << (4 * q))) | (t << (4 * b));
-        const uint64_t inv = inverse(nkey);
-        uint32_t a = aux & 0xffffu;
-        if (pattern_of_tile<N>((int)t) == 0)
-            a = (a & 0xff00u) | part(0, inv);
-        else
-            a = (a & 0x00ffu) | (part(1, inv) << 8);
-        naux = a | ((uint32_t)(mv + 1) << 16);
-        ng = g + 1;
-        nf = ng + hsum(naux);
-    }
     // Two-step successor (see GridProblem::Succ): the first step computes the
     // board and issues the load of the moved tile's pattern entry, the second
     // (after the table CAS) folds it into aux and f.
@@ -381,14 +451,16 @@ template <int N> struct PuzzleProblem : NarrowSlots {
         uint32_t part;  // the loaded pattern entry
         uint32_t which; // its pattern
     };
+    static constexpr uint64_t kPatternOf = pattern_bits<N>();
     __device__ __forceinline__ void succ_begin(uint64_t key, uint64_t g, uint32_t, int mv, Succ &s) const {
         const int b = blank(key);
         const int q = b + (mv == 0 ? N : mv == 1 ? -N : mv == 2 ? 1 : -1);
-        const uint64_t t = (key >> (4 * q)) & 15;
-        s.key = (key & ~(15ull << (4 * q))) | (t << (4 * b));
+        const int t = tile_on(key, q);
+        const uint64_t swap = (uint64_t)(b ^ q);  // tile t and the blank trade cells
+        s.key = key ^ swap ^ (swap << (4 * t));
         s.g = g + 1;
-        s.which = (uint32_t)pattern_of_tile<N>((int)t);
-        s.part = part((int)s.which, inverse(s.key));
+        s.which = (uint32_t)(kPatternOf >> (2 * t)) & 3u;
+        s.part = part((int)s.which, s.key);
     }
     __device__ __forceinline__ void succ_end(const Succ &s, uint32_t aux, int mv, uint32_t &naux,
                                              uint64_t &nf) const {
@@ -399,6 +471,25 @@ template <int N> struct PuzzleProblem : NarrowSlots {
             a = (a & 0x00ffu) | (s.part << 8);
         naux = a | ((uint32_t)(mv + 1) << 16);
         nf = s.g + hsum(naux);
+    }
+    // An 8-puzzle's search never fills the heaps: many passes, least f first
+    // (four boards: 0.70 ms without, 0.44 / 0.36 / 0.31 with 1 / 2 / 4 passes).
+    // A 15-puzzle does within ~25 rounds, and then a pass more is a longer round
+    // of the same expansions (60-move board: 6.2 ms without, 7.5 with two
+    // throughout, 6.3 with two while less than a quarter of the heaps pop); a
+    // slack of two f levels (4), since a strict order leaves most heaps idle
+    // (eight boards 16.3 ms against 19.0 with the least f only).
+    __host__ __device__ Expansion expansion(uint32_t k) const {
+        return N == 3 ? Expansion{4u, ~0u, 0.5f} : Expansion{2u, k / 4u, 4.f};
+    }
+    // Continuation (see GridProblem): f is known only once the pattern entry
+    // has arrived (ga_search tests it then), and the moves follow from the
+    // board alone.
+    struct Look {};
+    __device__ __forceinline__ bool peek(const Succ &, float) const { return true; }
+    __device__ __forceinline__ void look_begin(const uint64_t &, Look &) const {}
+    __device__ __forceinline__ uint32_t look_moves(const uint64_t & key, uint32_t naux, const Look &) const {
+        return moves(key, naux);
     }
     static constexpr bool kEntryKey = false;
     __device__ __forceinline__ Entry make_entry(uint64_t f, uint64_t g, uint32_t slot, uint32_t) const {
@@ -429,11 +520,11 @@ template <int N> struct PuzzleProblem : NarrowSlots {
 };
 
 // ------------------------------------------------------- 24-puzzle ---
-// 5x5 board, 128-bit key: cells 0..11 in `lo` and 12..23 in `hi`, 5 bits
-// each; cell 24 is implied (the tiles 0..24 sum to 300), so every state has
-// one key and bits 60..63 of both words stay zero (the all-ones empty key is
-// never a board).  aux = the four pattern parts, 7 bits each, | (last move +
-// 1) << 28.
+// 5x5 board, 128-bit key: the cells of tiles 0 (the blank) .. 11 in `lo` and
+// 12 .. 23 in `hi`, 5 bits each; tile 24's cell is implied (the cells sum to
+// 300), so every state has one key and bits 60..63 of both words stay zero
+// (the all-ones empty key is never a board).  aux = the four pattern parts, 7
+// bits each, | (last move + 1) << 28.
 template <> struct PuzzleProblem<5> : WideSlots {
     using Entry = PuzzleEntry;
     static constexpr int kMoves = 4;
@@ -446,75 +537,66 @@ template <> struct PuzzleProblem<5> : WideSlots {
     Key128 goal;
 
     __device__ static int cost_cmp(uint64_t a, uint64_t b) { return a < b ? -1 : (a > b ? 1 : 0); }
+    __device__ static float cost_val(uint64_t c) { return (float)c; }
 
-    __host__ __device__ static uint32_t field(const Key128 &k, int i) {
-        if (i < 12) return (uint32_t)(k.lo >> (5 * i)) & 31u;
-        if (i < 24) return (uint32_t)(k.hi >> (5 * (i - 12))) & 31u;
-        uint32_t sum = 0;
-        for (int c = 0; c < 12; ++c) sum += (uint32_t)(k.lo >> (5 * c)) & 31u;
-        for (int c = 0; c < 12; ++c) sum += (uint32_t)(k.hi >> (5 * c)) & 31u;
-        return 300u - sum;
+    // sum of the 12 fields of a word
+    __host__ __device__ static uint32_t field_sum(uint64_t w) {
+        constexpr uint64_t even = 0x007c1f07c1f07c1full;  // fields 0, 2, .. 10
+        const uint64_t s = (w & even) + ((w >> 5) & even);  // six sums, 10 bits apart
+        const uint64_t t = s + (s >> 30);                   // three of them
+        return (uint32_t)((t & 1023u) + (t >> 10 & 1023u) + (t >> 20 & 1023u));
     }
-    __host__ __device__ static void set_field(Key128 &k, int i, uint32_t v) {
-        if (i < 12)
-            k.lo = (k.lo & ~(31ull << (5 * i))) | ((uint64_t)v << (5 * i));
-        else if (i < 24)
-            k.hi = (k.hi & ~(31ull << (5 * (i - 12)))) | ((uint64_t)v << (5 * (i - 12)));
-        // cell 24 is implied
+    // cell of tile t
+    __host__ __device__ static uint32_t cell(const Key128 &k, int t) {
+        if (t < 12) return (uint32_t)(k.lo >> (5 * t)) & 31u;
+        if (t < 24) return (uint32_t)(k.hi >> (5 * (t - 12))) & 31u;
+        return 300u - field_sum(k.lo) - field_sum(k.hi);
     }
     __host__ __device__ static Key128 pack(const uint8_t *tiles) {
         Key128 k{0, 0};
-        for (int i = 0; i < 24; ++i) set_field(k, i, tiles[i]);
+        for (int i = 0; i < 25; ++i) {
+            const int t = tiles[i];
+            if (t < 12)
+                k.lo |= (uint64_t)i << (5 * t);
+            else if (t < 24)
+                k.hi |= (uint64_t)i << (5 * (t - 12));
+            // tile 24 is implied
+        }
         return k;
     }
     __host__ __device__ static Key128 goal_key() {
-        Key128 k{0, 0};
-        for (int i = 0; i < 24; ++i) set_field(k, i, (uint32_t)(i + 1));
-        return k;
+        uint8_t tiles[25] = {};
+        for (int i = 0; i < 24; ++i) tiles[i] = (uint8_t)(i + 1);
+        return pack(tiles);
     }
-    // index of the zero field of a 60-bit word of 5-bit fields (12 if none)
-    __device__ __forceinline__ static int zero_field(uint64_t w) {
-        const uint64_t t = w | (w >> 1) | (w >> 2) | (w >> 3) | (w >> 4);
-        const uint64_t z = ~t & kFieldLow;
+    __device__ __forceinline__ static int blank(const Key128 &k) { return (int)((uint32_t)k.lo & 31u); }
+    // index of the field of a 60-bit word equal to q (12 if none)
+    __device__ __forceinline__ static int field_of(uint64_t w, int q) {
+        const uint64_t x = w ^ ((uint64_t)q * kFieldLow);
+        const uint64_t z = (x - kFieldLow) & ~x & (kFieldLow << 4);
         return z ? (__ffsll((long long)z) - 1) / 5 : 12;
     }
-    __device__ __forceinline__ static int blank(const Key128 &k) {
-        const int a = zero_field(k.lo);
-        if (a < 12) return a;
-        const int b = zero_field(k.hi);
-        return b < 12 ? 12 + b : 24;
+    __device__ __forceinline__ static int tile_on(const Key128 &k, int q) {
+        const int a = field_of(k.lo, q);
+        return a < 12 ? a : 12 + field_of(k.hi, q);  // 24 if neither word names the cell
     }
-    // cell of each tile, 5 bits per tile, in a 128-bit word
-    __device__ __forceinline__ static unsigned __int128 inverse(const Key128 &k) {
-        unsigned __int128 inv = 0;
-        uint32_t sum = 0;
-#pragma unroll
-        for (int i = 0; i < 24; ++i) {
-            const uint32_t t = i < 12 ? (uint32_t)(k.lo >> (5 * i)) & 31u : (uint32_t)(k.hi >> (5 * (i - 12))) & 31u;
-            sum += t;
-            inv |= (unsigned __int128)i << (5 * t);
-        }
-        inv |= (unsigned __int128)24 << (5 * (300u - sum));
-        return inv;
-    }
-    template <int P> __device__ __forceinline__ static uint32_t rank(unsigned __int128 inv) {
+    // Rank of pattern p's six tiles (see PuzzleProblem::rank); the tile's cell
+    // is selected by p, so that the lanes of a warp rank their four patterns
+    // together.
+    __device__ __forceinline__ static uint32_t rank(int p, const Key128 &k) {
         uint32_t used = 0, code = 0;
 #pragma unroll
         for (int j = 0; j < 6; ++j) {
-            const uint32_t pos = (uint32_t)(inv >> (5 * PuzzlePatterns<5>::tile(P, j))) & 31u;
-            const uint32_t v = pos - __popc(used & ((1u << pos) - 1u));
-            code += v * pattern_mult<5>(P, j + 1);
+            const uint32_t c0 = cell(k, PuzzlePatterns<5>::tile(0, j)), c1 = cell(k, PuzzlePatterns<5>::tile(1, j));
+            const uint32_t c2 = cell(k, PuzzlePatterns<5>::tile(2, j)), c3 = cell(k, PuzzlePatterns<5>::tile(3, j));
+            const uint32_t pos = p < 2 ? (p == 0 ? c0 : c1) : (p == 2 ? c2 : c3);
+            code = code * (uint32_t)(NN - j) + pos - __popc(used & ((1u << pos) - 1u));
             used |= 1u << pos;
         }
         return code;
     }
-    __device__ __forceinline__ uint32_t part(int p, unsigned __int128 inv) const {
-        switch (p) {
-        case 0: return __ldg(pdb + PuzzlePatterns<5>::offset(0) + rank<0>(inv));
-        case 1: return __ldg(pdb + PuzzlePatterns<5>::offset(1) + rank<1>(inv));
-        case 2: return __ldg(pdb + PuzzlePatterns<5>::offset(2) + rank<2>(inv));
-        default: return __ldg(pdb + PuzzlePatterns<5>::offset(3) + rank<3>(inv));
-        }
+    __device__ __forceinline__ uint32_t part(int p, const Key128 &k) const {
+        return __ldg(pdb + ((uint32_t)p * (uint32_t)PuzzlePatterns<5>::offset(1) + rank(p, k)));
     }
     // aux = four 7-bit pattern parts | (last move + 1) << 28
     static constexpr uint32_t kLastMoveShift = 28;
@@ -524,8 +606,7 @@ template <> struct PuzzleProblem<5> : WideSlots {
 
     __device__ Key128 start_key() const { return start; }
     __device__ uint32_t start_aux() const {
-        const unsigned __int128 inv = inverse(start);
-        return part(0, inv) | part(1, inv) << 7 | part(2, inv) << 14 | part(3, inv) << 21;
+        return part(0, start) | part(1, start) << 7 | part(2, start) << 14 | part(3, start) << 21;
     }
     __device__ bool is_goal(const Key128 &k) const { return k.lo == goal.lo && k.hi == goal.hi; }
     __device__ __forceinline__ uint64_t f_of(const Key128 &, uint64_t g, uint32_t aux) const { return g + hsum(aux); }
@@ -547,16 +628,17 @@ template <> struct PuzzleProblem<5> : WideSlots {
         uint32_t part;   // the moved tile's pattern entry
         uint32_t which;  // its pattern
     };
+    static constexpr uint64_t kPatternOf = pattern_bits<5>();
     __device__ __forceinline__ void succ_begin(const Key128 &key, uint64_t g, uint32_t, int mv, Succ &s) const {
         const int b = blank(key);
         const int q = b + (mv == 0 ? N : mv == 1 ? -N : mv == 2 ? 1 : -1);
-        const uint32_t t = field(key, q);
-        s.key = key;
-        set_field(s.key, b, t);
-        set_field(s.key, q, 0);
+        const int t = tile_on(key, q);
+        const uint64_t swap = (uint64_t)(b ^ q);  // tile t and the blank trade cells
+        s.key.lo = key.lo ^ swap ^ (t < 12 ? swap << (5 * t) : 0ull);
+        s.key.hi = key.hi ^ (t >= 12 && t < 24 ? swap << (5 * (t - 12)) : 0ull);
         s.g = g + 1;
-        s.which = (uint32_t)pattern_of_tile<5>((int)t);
-        s.part = part((int)s.which, inverse(s.key));
+        s.which = (uint32_t)(kPatternOf >> (2 * t)) & 3u;
+        s.part = part((int)s.which, s.key);
     }
     __device__ __forceinline__ void succ_end(const Succ &s, uint32_t aux, int mv, uint32_t &naux,
                                              uint64_t &nf) const {
@@ -564,6 +646,17 @@ template <> struct PuzzleProblem<5> : WideSlots {
         uint32_t a = (aux & 0x0fffffffu & ~(127u << sh)) | (s.part << sh);
         naux = a | ((uint32_t)(mv + 1) << 28);
         nf = s.g + hsum(naux);
+    }
+    // (three boards of 60 random moves: 1.51 ms without, 1.09 ms)
+    __host__ __device__ Expansion expansion(uint32_t k) const { return Expansion{2u, k / 4u, 4.f}; }
+    // Continuation (see GridProblem): f is known only once the pattern entry
+    // has arrived (ga_search tests it then), and the moves follow from the
+    // board alone.
+    struct Look {};
+    __device__ __forceinline__ bool peek(const Succ &, float) const { return true; }
+    __device__ __forceinline__ void look_begin(const Key128 &, Look &) const {}
+    __device__ __forceinline__ uint32_t look_moves(const Key128 & key, uint32_t naux, const Look &) const {
+        return moves(key, naux);
     }
     static constexpr bool kEntryKey = false;
     __device__ __forceinline__ Entry make_entry(uint64_t f, uint64_t g, uint32_t slot, uint32_t) const {

@@ -6,21 +6,26 @@
 // H threads are their owners, T / H threads per heap), so the team has
 // k = C * H heaps.  A round is:
 //
-//   phase 1  each heap owner pops its heap's minimum; the round's minimum
-//            popped f is reduced (warp shuffles, one CAS per warp); stale
-//            entries (f no longer matching the node's g) are dropped; a goal
-//            pop lowers goal_best; every other pop is expanded.  The CTA then
-//            spreads the successors of its H pops over all T threads; each
-//            thread relaxes its successor in the open-addressed dedup table
-//            with one 16-byte CAS on (key, g): it either claims an empty slot
-//            with its g, or learns the slot's g and lowers it with a CAS loop.
-//            Only a strict improvement makes the successor a candidate, so
-//            among equal-g writers of one slot in a round exactly one
-//            candidate carries the final g.
-//   barrier  then a uniform decision: stop when the best goal f popped so
-//            far <= the round's minimum popped f (the GA* optimality test of
-//            the reference, src/pathway/GPU-solver.cu:219-243), fail when
-//            nothing was popped.
+//   phase 1  each heap owner looks at its heap's minimum; the round's minimum
+//            f is reduced (warp shuffles, one CAS per CTA).  A minimum at or
+//            below the round's bound, and below the best goal f, is popped;
+//            stale entries (f no longer matching the node's g) are dropped; a
+//            goal pop lowers goal_best; every other pop is expanded.  The CTA
+//            then spreads the successors of its pops over the relaxer threads;
+//            each thread relaxes its successor in the open-addressed dedup
+//            table with one 16-byte CAS on (key, g): it either claims an empty
+//            slot with its g, or learns the slot's g and lowers it with a CAS
+//            loop.  Only a strict improvement makes the successor a candidate,
+//            so among equal-g writers of one slot in a round exactly one
+//            candidate carries the final g.  A successor that improved its
+//            slot within the bound is not sent through a heap at all but
+//            expanded by the same warp at once (continuation), for up to
+//            m.cont passes.
+//   barrier  then a uniform decision: stop when the best goal f so far <=
+//            the round's minimum open f (the GA* optimality test of the
+//            reference, src/pathway/GPU-solver.cu:219-243; every entry made in
+//            the round descends from one at or above that minimum), fail when
+//            nothing is open.
 //   phase 2  CTA c takes the candidates of CTA (c + round) mod C's region
 //            (the successors of that CTA's pops); its threads check them in
 //            parallel (a candidate is the slot's winner iff the slot's g
@@ -39,6 +44,19 @@
 //
 // Heaps are CTA-private, so the top levels of every heap live in shared
 // memory (a pop touches global memory only below them).
+//
+// Continuation and bound.  A round costs a pop (record read), a relax, a
+// barrier, the decision and the staging in series, 8 us with everything in L2
+// and 14 us on the 20000^2 grid, and without continuation it advances a path
+// by one step: the number of rounds was the path length (22 293 cells: 24.7 k
+// rounds).  A continuation pass is one relax with the successor's neighbourhood
+// read beside it, 2-4 us, so a round of R passes advances a path by up to R + 1
+// steps.  The bound (the last round's minimum + m.slack) keeps the pops and
+// passes near the frontier's least f: unbounded, every state of that grid was
+// expanded 3.6 times (160 M expansions of 43 M states; within 16 of the
+// minimum 86 M).
+// Search kernel, before -> after (8192 heaps): 20000^2 grid 356 -> 194 ms,
+// 61 x 67 grid 0.51 -> 0.23 ms; four 8-puzzles 0.81 -> 0.31 ms.
 //
 // This replaces the reference's per-round kExtractExpand -> host copy ->
 // MergesortPairs -> kAssign -> host copy -> kDeduplicate -> kHeapInsert
@@ -85,6 +103,20 @@ template <class E> struct SearchMem {
     // wait for the staging only.  Needs SearchSmem<P>::bytes_split shared
     // memory.  0 = one barrier for all threads.
     uint32_t split = 0;
+    // Continuation passes of a round at most (0: every improved successor goes
+    // through the heaps), taken only while at most cont_pops entries were
+    // popped in the last round: where more heaps than that have work, the
+    // relaxers are busy without them.
+    uint32_t cont = 0;
+    uint32_t cont_pops = ~0u;
+    // A round pops and continues only nodes with f <= the last round's minimum
+    // + slack (0: no bound).
+    float slack = 0.f;
+    __host__ __device__ void set(const Expansion &x) {
+        cont = x.cont;
+        cont_pops = x.cont_pops;
+        slack = x.slack;
+    }
     // Sort-based dedup (ga_search<.., true>): every round's successors are
     // radix-sorted by key and each key's minimum-g record is relaxed once.
     unsigned long long *sort_buf = nullptr;  // 2 x C * H * kMoves pairs
@@ -106,12 +138,15 @@ __device__ __forceinline__ void named_arrive(uint32_t id, uint32_t n) {
 }
 
 // ------------------------------------------------------------------ teams ---
+// sync(then): the team barrier; thread 0 of each CTA runs `then` once it is
+// complete, before the CTA's other threads go on.
 // Split rounds (SearchMem::split) need the team barrier in two halves:
 // early_arrive() by the owner warps (no wait), relaxers_sync() by the
 // relaxer warps (arrive and wait), late_wait() by the owner warps after
 // their chores.  The grid team has no split form.
 struct GridTeam {
     static constexpr bool kSplit = false;
+    static constexpr bool kBeside = true;
     __device__ void early_arrive() {}  // (no split form: never called)
     __device__ void relaxers_sync(uint32_t) {}
     __device__ void late_wait() {}
@@ -120,7 +155,10 @@ struct GridTeam {
     uint64_t timeout_ns;
     __device__ uint32_t cta() const { return blockIdx.x; }
     __device__ uint32_t ctas() const { return gridDim.x; }
-    __device__ void sync() { grid_barrier(&st->barrier, gridDim.x, epoch, &st->error, timeout_ns); }
+    __device__ void sync() { sync([] {}); }
+    template <class F> __device__ void sync(F &&then) {
+        grid_barrier(&st->barrier, gridDim.x, epoch, &st->error, timeout_ns, then);
+    }
     __device__ uint64_t rd64(const unsigned long long *p) const { return ldcg_u64(p); }
     __device__ uint32_t rd32(const uint32_t *p) const { return ldcg_u32(p); }
 };
@@ -133,6 +171,7 @@ struct GridTeam {
 // ones included, so no separate fence is needed.
 struct ClusterTeam {
     static constexpr bool kSplit = true;
+    static constexpr bool kBeside = false;
     TeamState *st;  // global memory
     __device__ uint32_t cta() const {
         uint32_t r;
@@ -147,6 +186,11 @@ struct ClusterTeam {
     __device__ void sync() {
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
+    template <class F> __device__ void sync(F &&then) {
+        sync();
+        if (threadIdx.x == 0) then();
+        __syncthreads();
+    }
     // split halves: the cluster barrier's own arrive and wait, in the forms
     // that a diverged warp may execute
     __device__ void early_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
@@ -160,10 +204,16 @@ struct ClusterTeam {
 
 struct BlockTeam {
     static constexpr bool kSplit = true;
+    static constexpr bool kBeside = false;
     TeamState *st;  // shared memory
     __device__ uint32_t cta() const { return 0; }
     __device__ uint32_t ctas() const { return 1; }
     __device__ void sync() { __syncthreads(); }
+    template <class F> __device__ void sync(F &&then) {
+        __syncthreads();
+        if (threadIdx.x == 0) then();
+        __syncthreads();
+    }
     // split halves: named barrier 1 over the whole CTA, owners arriving early
     __device__ void early_arrive() { named_arrive(1, blockDim.x); }
     __device__ void relaxers_sync(uint32_t n) { named_sync(1, n); }
@@ -533,10 +583,16 @@ __device__ __forceinline__ KeyG cas128(Slot *s, KeyG cmp, KeyG val) {
 // probe limit was reached.
 enum : int { RELAX_NONE = 0, RELAX_IMPROVED = 1, RELAX_CLAIMED = 2, RELAX_INSERTED = 3, RELAX_FULL = 4 };
 
-// Find-or-insert `key` and lower its g to `g` in one pass.  The home slot is
-// tried with a single 16-byte CAS that either claims it empty with (key, g)
-// or returns what it holds; later probe steps read first and only CAS a slot
-// that is empty or holds the key.  Returns RELAX_INSERTED (new slot, g set),
+// Find-or-insert `key` and lower its g to `g` in one pass (the probe order is
+// probe_slot's).  The first turn tries the home slot with one 16-byte CAS,
+// which claims it empty with (key, g) or returns what it holds, and reads the
+// other three slots of its 128-byte line beside it; so a claim takes one memory
+// trip, an improvement or a collision two.  The lanes of a warp take their
+// turns together, whatever each one's next access is (the trips would add up
+// in diverged branches).  A turn under the load of a round is ~2.5 k cycles
+// and a warp waits for its slowest lane, so the number of turns is the relax
+// phase: with a look at the line as a turn of its own a warp took 3-4 turns, up
+// to 16 near half load.  Returns RELAX_INSERTED (new slot, g set),
 // RELAX_IMPROVED (existing slot, g strictly lowered), RELAX_NONE (existing
 // slot, g not better) or RELAX_FULL (probe limit).
 //
@@ -553,62 +609,63 @@ template <class P> __device__ __forceinline__ bool key_match(uint64_t word, uint
         return word == key;
 }
 
-template <class P>
-__device__ __forceinline__ int relax_at(Slot *tab, uint64_t h, KeyG cur, uint64_t word, uint64_t g,
-                                        uint64_t gw, uint32_t *slot_out) {
-    // the slot holds the key: lower g (and, with the link in the key or g
-    // word, set the link with it)
-    *slot_out = (uint32_t)h;
-    while (P::cost_cmp(g, P::word_g(cur.g)) < 0) {
-        const KeyG old = cas128(tab + h, cur, KeyG{P::kPrevInKey ? word : cur.key, gw});
-        if (old.key == cur.key && old.g == cur.g) return RELAX_IMPROVED;
-        cur = old;
-    }
-    return RELAX_NONE;
-}
-
-template <class P>
+template <class P, bool kBeside = true>
 __device__ __forceinline__ int relax(Slot *tab, uint64_t mask, uint32_t max_probe, uint64_t key, uint64_t g,
                                      uint32_t prev, uint32_t *slot_out, int mv = -1) {
-    // Linear probing.  The home slot is tried with one 16-byte CAS; past it
-    // the probe reads the rest of the home slot's 128-byte line (4 slots) and
-    // then whole lines, one dependent load per line.
-    const uint64_t word = P::kPrevInKey ? (key | (uint64_t)prev << 32) : key;
-    const uint64_t gw = P::g_word(g, prev, mv);
-    uint64_t h = mix64(key) & mask;
-    const KeyG empty{kEmptyKey, kInfCost};
-    KeyG cur = cas128(tab + h, empty, KeyG{word, gw});
-    if (cur.key == kEmptyKey) {
-        *slot_out = (uint32_t)h;
-        return RELAX_INSERTED;
-    }
-    if (key_match<P>(cur.key, key)) return relax_at<P>(tab, h, cur, word, g, gw, slot_out);
-    uint32_t probed = 1;
-    h = (h + 1) & mask;
-    while (probed < max_probe) {
-        // slots h .. end of h's line (the table is line-aligned, mask >= 3)
-        const uint32_t n = 4u - (uint32_t)(h & 3u);
+    const KeyG mine{P::kPrevInKey ? (key | (uint64_t)prev << 32) : key, P::g_word(g, prev, mv)};
+    const uint64_t home = mix64(key) & mask;
+    uint64_t h = home;              // the slot at probe index i
+    uint32_t i = 0;
+    KeyG cur{kEmptyKey, kInfCost};  // what the CAS expects there
+    bool cas = true, look = kBeside;  // this turn's accesses: CAS slot h; read the slots i (+ 1 with a CAS) .. end of line
+    for (;;) {
+        const uint32_t from = i + (cas ? 1u : 0u), n = look ? 4u - (i & 3u) - (cas ? 1u : 0u) : 0u;
         ulonglong2 v[4];
 #pragma unroll
         for (uint32_t q = 0; q < 4; ++q)
-            if (q < n) v[q] = __ldcg(reinterpret_cast<const ulonglong2 *>(tab + h + q));
-        for (uint32_t q = 0; q < n; ++q) {
-            const uint64_t hq = h + q;
-            if (key_match<P>(v[q].x, key)) return relax_at<P>(tab, hq, KeyG{v[q].x, v[q].y}, word, g, gw, slot_out);
-            if (v[q].x == kEmptyKey) {
-                cur = cas128(tab + hq, empty, KeyG{word, gw});
-                if (cur.key == kEmptyKey) {
-                    *slot_out = (uint32_t)hq;
-                    return RELAX_INSERTED;
-                }
-                if (key_match<P>(cur.key, key)) return relax_at<P>(tab, hq, cur, word, g, gw, slot_out);
-                // another key took it: keep probing
+            if (q < n) v[q] = __ldcg(reinterpret_cast<const ulonglong2 *>(tab + probe_slot(home, from + q, mask)));
+        KeyG old = cur;
+        if (cas) {
+            old = cas128(tab + h, cur, mine);
+            if (old.key == cur.key && old.g == cur.g) {
+                *slot_out = (uint32_t)h;
+                return old.key == kEmptyKey ? RELAX_INSERTED : RELAX_IMPROVED;
             }
         }
-        probed += n;
-        h = (h + n) & mask;
+        if (cas && key_match<P>(old.key, key)) {
+            cur = old;
+            look = false;
+        } else if (look) {
+            // the first of the slots read that holds the key or is free
+            uint32_t at = n;
+#pragma unroll
+            for (uint32_t q = 4; q-- > 0;)
+                if (q < n && (v[q].x == kEmptyKey || key_match<P>(v[q].x, key))) {
+                    at = q;
+                    cur = KeyG{v[q].x, v[q].y};
+                }
+            i = from + at;
+            if (at == n) {  // none: the next line
+                if (i >= max_probe) return RELAX_FULL;
+                cas = false;
+                continue;
+            }
+            h = probe_slot(home, i, mask);
+            cas = true;
+            look = false;
+        } else {
+            // another key holds the slot: look on behind it
+            i += 1;
+            if (i >= max_probe) return RELAX_FULL;
+            cas = false;
+            look = true;
+            continue;
+        }
+        if (cur.key != kEmptyKey && P::cost_cmp(g, P::word_g(cur.g)) >= 0) {
+            *slot_out = (uint32_t)h;
+            return RELAX_NONE;
+        }
     }
-    return RELAX_FULL;
 }
 
 // Wide keys: find-or-claim the 16-byte key with one 16-byte CAS per probed
@@ -617,9 +674,10 @@ __device__ __forceinline__ int relax(Slot *tab, uint64_t mask, uint32_t max_prob
 template <class P>
 __device__ __forceinline__ int relax_wide(Slot *tab, uint64_t mask, uint32_t max_probe, const Key128 &key,
                                           uint64_t g, uint32_t *slot_out) {
-    uint64_t h = key_hash(key) & mask;
+    const uint64_t home = key_hash(key) & mask;
     const KeyG empty{kEmptyKey, kEmptyKey};
     for (uint32_t probe = 0; probe < max_probe; ++probe) {
+        const uint64_t h = probe_slot(home, probe, mask);
         const KeyG cur = cas128(tab + h, empty, KeyG{key.lo, key.hi});
         const bool claimed = cur.key == kEmptyKey && cur.g == kEmptyKey;
         if (claimed || (cur.key == key.lo && cur.g == key.hi)) {
@@ -633,18 +691,17 @@ __device__ __forceinline__ int relax_wide(Slot *tab, uint64_t mask, uint32_t max
             }
             return claimed ? RELAX_CLAIMED : RELAX_NONE;
         }
-        h = (h + 1) & mask;
     }
     return RELAX_FULL;
 }
 
-template <class P>
+template <class P, bool kBeside = true>
 __device__ __forceinline__ int relax_key(Slot *tab, uint64_t mask, uint32_t max_probe, const typename P::Key &key,
                                          uint64_t g, uint32_t prev, uint32_t *slot_out, int mv = -1) {
     if constexpr (P::kWide)
         return relax_wide<P>(tab, mask, max_probe, key, g, slot_out);
     else
-        return relax<P>(tab, mask, max_probe, key, g, prev, slot_out, mv);
+        return relax<P, kBeside>(tab, mask, max_probe, key, g, prev, slot_out, mv);
 }
 
 __device__ __forceinline__ Cand load_cand(const Cand *p) {
@@ -660,7 +717,35 @@ __device__ __forceinline__ Cand load_cand(const Cand *p) {
     return c;
 }
 
+// Position of the n-th (from 0) set bit of a move mask (n < its set bits).
+__device__ __forceinline__ int nth_bit(uint32_t mask, uint32_t n) {
+    for (; n; --n) mask &= mask - 1u;
+    return __ffs((int)mask) - 1;
+}
+
+__device__ __forceinline__ uint64_t shfl_key(uint64_t v, int src) { return shfl64(v, src); }
+__device__ __forceinline__ Key128 shfl_key(const Key128 &v, int src) {
+    return Key128{shfl64(v.lo, src), shfl64(v.hi, src)};
+}
+
 // Shared-memory layout of one CTA of a search team.
+// A CTA's copy of the search's totals and of the last decision, kept by the
+// one thread that takes the decisions (ga_search) and read by the others.
+struct RoundState {
+    unsigned long long gbest;      // best goal f over the decided rounds
+    unsigned long long inserted;   // slots in use after them
+    unsigned long long rounds;     // their number
+    unsigned long long steps;      // expansion steps: rounds and their continuation passes
+    unsigned long long stop_at;    // the launch's round budget ends here
+    unsigned long long expanded, generated, pushed;  // this CTA, this launch
+    float bound;                   // the round's bound on f (SearchMem::slack)
+    uint32_t cont;                 // its continuation passes at most
+    uint32_t status, pause;        // the last decision
+    uint32_t nshare;               // candidates in this CTA's share
+    uint32_t pad;
+};
+static_assert(sizeof(RoundState) == 88, "22 words of the scratch");
+
 template <class Key> struct PopInfo {
     Key key;
     unsigned long long g;
@@ -705,11 +790,11 @@ template <class P> struct SearchSmem {
     static __host__ __device__ size_t scratch_offset(uint32_t H, uint32_t L) {
         return (buf_offset(H, L) + (size_t)H * kBufStride * sizeof(E) + 15) & ~(size_t)15;
     }
-    // warp totals of the block scans, this CTA's round counters, then the
-    // owner warps' minimum popped f (16 x 8 bytes)
-    static constexpr uint32_t kScratchWords = 72;
+    // warp totals of the block scans, this CTA's round counters, the owner
+    // warps' minimum f and pops, and the RoundState; then two words per owner
+    static constexpr uint32_t kScratchWords = 114;
     static __host__ __device__ size_t bytes(uint32_t H, uint32_t L) {
-        return scratch_offset(H, L) + 4 * kScratchWords;
+        return scratch_offset(H, L) + 4 * (kScratchWords + 2 * (size_t)H);
     }
     // the sort-based dedup's shared memory follows (T threads per CTA); or,
     // with split rounds, the push staging (the sift scratch is busy then)
@@ -771,42 +856,65 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                               unsigned char *smem, uint64_t budget) {
     static_assert(!kSort || (!P::kWide && P::kPrevInKey), "sorted dedup: 32-bit keys with the link in the key word");
     using E = typename P::Entry;
-    TeamState *st = team.st;
+    using Key = typename P::Key;
+    using S = SearchSmem<P>;
+    TeamState *const st = team.st;
     const uint32_t T = blockDim.x, tid = threadIdx.x, lane = tid & 31u;
     const uint32_t C = team.ctas(), cta = team.cta();
     const bool owner = tid < H;
-    const uint32_t myh = cta * H + tid;  // global heap index (valid when owner)
     const uint32_t L = m.L, topn = (1u << L) - 1;
     const uint32_t owner_warps = (H + 31u) / 32u;
     // Warps past the owners relax successors while the owners refill their
-    // heaps' root holes; with no such warps, everyone relaxes first.
+    // heaps' root holes; with no such warps, everyone does both.
     const uint32_t rfirst = T > owner_warps * 32u ? owner_warps * 32u : 0u;
     const uint32_t rthreads = T - rfirst;
     const bool relaxer = tid >= rfirst;
     // split rounds (SearchMem::split), uniform over the team
     bool split = false;
     if constexpr (Team::kSplit && !kSort) split = m.split != 0 && rfirst > 0;
+    // the thread that publishes the CTA's round and takes its decision
+    const bool lead = tid == (split ? rfirst : 0u);
 
-    using Key = typename P::Key;
-    PopInfo<Key> *pop = reinterpret_cast<PopInfo<Key> *>(smem);
-    E *tops = reinterpret_cast<E *>(smem + SearchSmem<P>::tops_offset(H));
-    E *scr = reinterpret_cast<E *>(smem + SearchSmem<P>::scr_offset(H, L));
-    uint32_t *scratch = reinterpret_cast<uint32_t *>(smem + SearchSmem<P>::scratch_offset(H, L));
+    // Shared memory.  What an owner keeps between its phases (heap size,
+    // buffer fill) and what the round decides live there too: held in
+    // registers across the relax phase they made the kernels of the CTA and
+    // cluster teams spill.
+    PopInfo<Key> *const pop = reinterpret_cast<PopInfo<Key> *>(smem);
+    E *const scr = reinterpret_cast<E *>(smem + S::scr_offset(H, L));
+    uint32_t *const scratch = reinterpret_cast<uint32_t *>(smem + S::scratch_offset(H, L));
+    uint32_t *const s_hs = scratch + S::kScratchWords;  // heap sizes
+    uint32_t *const s_bn = s_hs + H;                    // entries in the insertion buffers
+    uint32_t *const s_cnt = scratch + 36;    // this CTA's candidates this round
+    uint32_t *const s_ins = scratch + 37;    // dedup slots it claimed this round
+    uint32_t *const s_ins2 = scratch + 38;   // (kSort) slots claimed after the sort
+    uint32_t *const s_room = scratch + 39;   // candidate room taken by continued nodes' successors
+    unsigned long long *const wmins = reinterpret_cast<unsigned long long *>(scratch + 40);  // per owner warp (16)
+    uint32_t *const s_pass = scratch + 72;   // continuation passes this CTA made this round
+    uint32_t *const wtook = scratch + 73;    // entries popped, per owner warp (16)
+    uint32_t *const s_stat = scratch + 89;   // expanded, generated, pushed since the last publish
+    RoundState *const rs = reinterpret_cast<RoundState *>(scratch + 92);
+    uint32_t *const ssm = reinterpret_cast<uint32_t *>(smem + S::sort_offset(H, L));
 
-    E *const gblock = m.heaps + (size_t)(owner ? myh : 0) * m.stride;  // saved top, then bricks
-    BrickHeap<P> myheap{gblock + top_reserve<P>(L), tops + (size_t)(owner ? tid : 0) * SearchSmem<P>::top_stride(L),
-                        scr + (size_t)(owner ? tid : 0) * SearchSmem<P>::kScrStride, L};
+    // An owner's heap: its saved top, then bricks, in global memory.
+    const uint32_t myh = cta * H + (owner ? tid : 0u);
+    const auto heap_block = [&]() { return m.heaps + (size_t)myh * m.stride; };
+    const auto heap_of = [&]() {
+        const uint32_t t = owner ? tid : 0u;
+        return BrickHeap<P>{heap_block() + top_reserve<P>(L),
+                            reinterpret_cast<E *>(smem + S::tops_offset(H)) + (size_t)t * S::top_stride(L),
+                            scr + (size_t)t * S::kScrStride, L};
+    };
     // The heap's insertion buffer: an unordered list of up to kBuf entries in
     // shared memory in front of the heap.  The push phase only appends to it;
     // a pop takes the smaller of the heap's root and the buffer's minimum;
     // the owner moves entries from the buffer into the heap in the relax
     // phase (drain), off the round's critical path, keeping room for the next
     // push phase.  The heap and the buffer together are the priority queue.
-    constexpr uint32_t kBuf = SearchSmem<P>::kBuf;
-    E *const ibuf =
-        reinterpret_cast<E *>(smem + SearchSmem<P>::buf_offset(H, L)) + (size_t)(owner ? tid : 0) * SearchSmem<P>::kBufStride;
-    uint32_t bn = 0;  // entries in ibuf (owner; empty whenever the search is parked)
-    uint64_t nE = 0, nS = 0, nP = 0;
+    // (Empty whenever the search is parked.)
+    constexpr uint32_t kBuf = S::kBuf;
+    const auto buf_of = [&]() {
+        return reinterpret_cast<E *>(smem + S::buf_offset(H, L)) + (size_t)(owner ? tid : 0u) * S::kBufStride;
+    };
 
     // Every thread reads `started` before the team's rank 0 may set it below,
     // so that all take the same branch (and the same number of barriers).
@@ -822,7 +930,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             } else {
                 P::set_link(m.tab + s0, kNone, aux0);
                 uint32_t sz = 0;
-                heap_push<P>(myheap, sz, prob.make_entry(prob.f_of(key0, 0, aux0), 0, s0, aux0));
+                heap_push<P>(heap_of(), sz, prob.make_entry(prob.f_of(key0, 0, aux0), 0, s0, aux0));
                 m.heap_size[myh] = sz;
                 st->inserted = 1;
             }
@@ -831,27 +939,45 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
         team.sync();
     } else if (owner) {
         // resuming: bring the shared top of this heap back from global memory
+        const BrickHeap<P> h = heap_of();
+        const E *const gblock = heap_block();
         const uint32_t sz = ldcg_u32(&m.heap_size[myh]);
-        for (uint32_t i = 1; i <= topn && i <= sz; ++i) myheap.s[i] = P::load(gblock + i);
+        for (uint32_t i = 1; i <= topn && i <= sz; ++i) h.s[i] = P::load(gblock + i);
+    }
+    if (owner) {
+        s_hs[tid] = ldcg_u32(&m.heap_size[myh]);
+        s_bn[tid] = 0;
+    }
+    const uint64_t round0 = team.rd64(&st->round);
+    uint32_t base = team.rd32(&st->base);
+    // round number modulo 3 (team fields), modulo 2 (candidate buffers), and
+    // the CTA whose region this one takes in the push phase
+    uint32_t r3 = (uint32_t)(round0 % 3), par = (uint32_t)(round0 & 1), src = (uint32_t)((cta + round0) % C);
+    // Continuation passes left before the limit on expansion steps.
+    const auto passes = [&](uint64_t steps) {
+        const uint64_t left = m.max_rounds > steps ? m.max_rounds - steps : 1;
+        return left - 1 < m.cont ? (uint32_t)(left - 1) : m.cont;
+    };
+    if (lead) {
+        rs->gbest = team.rd64(&st->goal_best);
+        rs->inserted = team.rd64(&st->inserted);
+        rs->rounds = round0;
+        rs->steps = team.rd64(&st->steps);
+        rs->stop_at = budget < ~round0 ? round0 + budget : ~0ull;
+        rs->expanded = rs->generated = rs->pushed = 0;
+        rs->bound = __uint_as_float(team.rd32(&st->bound));
+        rs->cont = passes(rs->steps);
+        rs->status = ST_RUNNING;
+        s_stat[0] = s_stat[1] = s_stat[2] = 0;
     }
     __syncthreads();
 
-    uint32_t base = team.rd32(&st->base);
-    uint64_t round = team.rd64(&st->round);
-    uint64_t gbest = team.rd64(&st->goal_best);     // best goal f over the decided rounds
-    uint64_t ins_total = team.rd64(&st->inserted);  // slots in use after the decided rounds
-    uint32_t status = ST_RUNNING;
-    uint32_t hs = owner ? ldcg_u32(&m.heap_size[myh]) : 0;  // this owner's heap size (private)
     // Candidates: two buffers by round parity (a CTA may append round r + 1's
     // while another still reads round r's), each one region per CTA (its
     // header record holds the count), so a relaxing warp claims room with a
     // shared-memory atomic and the CTA publishes one count per round.
     const uint64_t RR = cand_region_records<P>(H);
-    uint32_t *const s_cnt = scratch + 36;  // this CTA's candidates this round
-    uint32_t *const s_ins = scratch + 37;  // dedup slots it claimed this round
-    uint32_t *const s_ins2 = scratch + 38;  // (kSort) slots claimed after the sort
-    uint32_t *const ssm = reinterpret_cast<uint32_t *>(smem + SearchSmem<P>::sort_offset(H, L));
-    unsigned long long *const wmins = reinterpret_cast<unsigned long long *>(scratch + 40);  // per owner warp
+    const auto region = [&](uint32_t c) { return m.cand + ((size_t)par * C + c) * RR; };
     // Push-phase staging: one entry per candidate of this CTA's share (at most
     // H * kMoves), then the C + 1 region offsets of the round's candidates
     // (the host keeps C < 32 H); it reuses the sift-down scratch, idle then.
@@ -859,35 +985,52 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
     // With split rounds the owners may still be sifting while the relaxers
     // stage, so the staging has its own room after the CTA's other shared
     // memory (bytes_split).
-    E *const stage =
-        split ? reinterpret_cast<E *>(smem + SearchSmem<P>::sort_offset(H, L)) : scr;
+    E *const stage = split ? reinterpret_cast<E *>(smem + S::sort_offset(H, L)) : scr;
     uint32_t *const roff = reinterpret_cast<uint32_t *>(scr + (size_t)H * P::kMoves);
+    uint32_t status = ST_RUNNING;
 
-    for (uint64_t it = 0;; ++it) {
-        const uint32_t r3 = (uint32_t)(round % 3);
-        Cand *const half = m.cand + (size_t)(round & 1) * C * RR;
-        Cand *const myreg = half + (size_t)cta * RR + 1;
+    for (;;) {
         if (tid == 0) {
             *s_cnt = 0;
             *s_ins = 0;
             *s_ins2 = 0;
+            *s_room = 0;
+            *s_pass = 0;
         }
 
         // ------------------------------------------------ phase 1: pop ---
-        // The owner takes the root now and refills the hole later in the
-        // round (pending_sift), off the path to the successors.
+        // The owner takes the root now and refills the hole in its chores,
+        // off the path to the successors.
         bool pending_sift = false, have_last = false;
         E last;
+        uint32_t hs = 0, bn = 0;
         if (tid < owner_warps * 32u) {
+            const BrickHeap<P> myheap = heap_of();
+            E *const ibuf = buf_of();
+            if (owner) {
+                hs = s_hs[tid];
+                bn = s_bn[tid];
+            }
             E e;
-            uint32_t mv = 0;
-            const bool have = owner && (hs > 0 || bn > 0);
+            uint32_t mv = 0, bi = 0;
+            bool have = hs > 0 || bn > 0, from_heap = false;
             if (have) {
-                uint32_t bi = 0;
                 for (uint32_t j = 1; j < bn; ++j)
                     if (P::less(ibuf[j], ibuf[bi])) bi = j;
-                if (hs > 0 && (bn == 0 || !P::less(ibuf[bi], myheap.s[1]))) {
-                    e = myheap.s[1];
+                from_heap = hs > 0 && (bn == 0 || !P::less(ibuf[bi], myheap.s[1]));
+                e = from_heap ? myheap.s[1] : ibuf[bi];
+            }
+            const uint64_t ecost = have ? P::entry_cost(e) : kInfCost;
+            const uint64_t wmin = warp_min_cost<P>(ecost);
+            if (lane == 0) wmins[tid >> 5] = wmin;  // the CTA's minimum goes out once, below
+            // the heap's minimum stays where it is if it is above the round's
+            // bound (or cannot beat the goal found so far)
+            have = have && P::cost_val(ecost) <= rs->bound && P::cost_cmp(ecost, rs->gbest) < 0;
+            const uint32_t took = __ballot_sync(kFull, have);
+            if (lane == 0) wtook[tid >> 5] = (uint32_t)__popc(took);
+            bool expands = false;
+            if (have) {
+                if (from_heap) {
                     // the heap's last entry refills the root unless the
                     // buffer has a run to drain (below), whose least entry
                     // refills it instead
@@ -898,15 +1041,9 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                     hs -= 1;
                     pending_sift = hs > 0;
                 } else {
-                    e = ibuf[bi];
                     ibuf[bi] = ibuf[bn - 1];
                     bn -= 1;
                 }
-            }
-            const uint64_t ecost = have ? P::entry_cost(e) : kInfCost;
-            const uint64_t wmin = warp_min_cost<P>(ecost);
-            if (lane == 0) wmins[tid >> 5] = wmin;  // the CTA's minimum goes out once, below
-            if (have) {
                 Key key;
                 uint64_t g;
                 uint32_t aux;
@@ -922,7 +1059,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                     atomic_min_cost<P>(&st->goal_min[r3], fcur);
                     st->goal_slot = e.slot;  // every goal pop names the same slot
                 } else {
-                    ++nE;
+                    expands = true;
                     if constexpr (P::kEntryKey)
                         mv = mv_pre;
                     else
@@ -933,6 +1070,8 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                     pop[tid].slot = e.slot;
                 }
             }
+            const uint32_t nexp = __ballot_sync(kFull, expands);
+            if (lane == 0 && nexp) atomicAdd(&s_stat[0], (uint32_t)__popc(nexp));
             // exclusive prefix of successor counts: within the warp here,
             // warp offsets added after the barrier
             const uint32_t cnt = __popc(mv);
@@ -949,7 +1088,8 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             if (lane == 31) scratch[2 + (tid >> 5)] = incl;
         }
         __syncthreads();
-        uint64_t cmin = kInfCost;  // the CTA's minimum popped f (thread 0)
+        uint64_t cmin = kInfCost;  // the CTA's minimum open f (thread 0)
+        uint32_t ctook = 0;
         if (tid == 0) {
             uint32_t acc = 0;
             for (uint32_t w = 0; w < owner_warps; ++w) {
@@ -957,6 +1097,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                 scratch[2 + w] = acc;
                 acc += t;
                 if (P::cost_cmp(wmins[w], cmin) < 0) cmin = wmins[w];
+                ctook += wtook[w];
             }
             scratch[0] = acc;
         }
@@ -966,100 +1107,104 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
         __syncthreads();
         // into the team's round minimum, off the pop's path (before the barrier)
         if (tid == 0 && cmin != kInfCost) atomic_min_cost<P>(&st->round_min[r3], cmin);
+        if (tid == 0 && ctook) atomicAdd(&st->pops[r3], ctook);
 
         // ------------------ phase 1: relax successors / refill heap roots ---
         // Owner chores of the round, while the other warps relax: refill the
         // root hole, then drain the insertion buffer down to kBuf - kMoves
-        // entries (room for this round's pushes).
-        // The buffer's run to drain (its largest entries: the small ones are
-        // popped soon), down to room for this round's pushes.  An overflow
-        // stops the search at this round's decision, so it is reported before
-        // the owner arrives at the team barrier.
-        uint32_t run = 0;
-        if (owner) {
-            run = bn > kBuf - P::kMoves ? bn - (kBuf - P::kMoves) : 0u;
-            if (hs + run > m.hcap) {
-                set_error(&st->err[r3], ST_HEAP_OVERFLOW);
-                run = m.hcap > hs ? m.hcap - hs : 0u;
-            }
-        }
-        const auto chores = [&]() {
-            // the run to the buffer's end, its largest entry last
-            for (uint32_t q = 0; q < run; ++q) {
-                const uint32_t end = bn - 1 - q;
-                uint32_t bx = 0;
-                for (uint32_t j = 1; j <= end; ++j)
-                    if (P::less(ibuf[bx], ibuf[j])) bx = j;
-                const E e = ibuf[bx];
-                ibuf[bx] = ibuf[end];
-                ibuf[end] = e;
-            }
-            // A root taken from the heap is refilled by the run's least entry
-            // (heapreplace): one sift-down serves the pop and one push, and
-            // the heap's last entry stays where it is.  Without a run the
-            // last entry refills it.
-            const bool replace = pending_sift && run > 0;
-            E top = last;
-            if (replace) {
-                top = ibuf[bn - run];
-                hs += 1;
-            } else if (pending_sift && !have_last) {
-                top = myheap.ld(hs + 1);  // (a run cut short by an overflow)
-            }
-            const uint32_t rest = run - (replace ? 1u : 0u);
-            // the rest's bottom brick is read while the sift-down runs (a
-            // fresh bottom brick, at depth 0, needs no read)
-            uint32_t pre = 0;
-            if (rest && hs + 1 > topn) {
-                uint32_t d;
-                const uint32_t root = myheap.brick_root(hs + 1, &d);
-                if (d > 0) {
-                    myheap.fetch_async(root, 2);
-                    pre = root;
+        // entries (room for this round's pushes).  In split rounds the owner
+        // warps arrive at the team barrier first.
+        if (tid < owner_warps * 32u) {
+            // The buffer's run to drain (its largest entries: the small ones
+            // are popped soon), down to room for this round's pushes.  An
+            // overflow stops the search at this round's decision, so it is
+            // reported before the owner arrives at the team barrier.
+            uint32_t run = 0;
+            if (owner) {
+                run = bn > kBuf - P::kMoves ? bn - (kBuf - P::kMoves) : 0u;
+                if (hs + run > m.hcap) {
+                    set_error(&st->err[r3], ST_HEAP_OVERFLOW);
+                    run = m.hcap > hs ? m.hcap - hs : 0u;
                 }
             }
-            if (pending_sift) {
-                const uint32_t fin = heap_sift_down<P>(myheap, hs, top);
-                // the sift wrote into that brick: its copy is stale
-                if (pre && fin > topn && myheap.brick_root(fin) == pre) {
-                    cp_async_wait_all();
-                    pre = 0;
+            if (split) team.early_arrive();
+            if (owner) {
+                const BrickHeap<P> myheap = heap_of();
+                E *const ibuf = buf_of();
+                // the run to the buffer's end, its largest entry last
+                for (uint32_t q = 0; q < run; ++q) {
+                    const uint32_t end = bn - 1 - q;
+                    uint32_t bx = 0;
+                    for (uint32_t j = 1; j <= end; ++j)
+                        if (P::less(ibuf[bx], ibuf[j])) bx = j;
+                    const E e = ibuf[bx];
+                    ibuf[bx] = ibuf[end];
+                    ibuf[end] = e;
                 }
-            }
-            if (pre) cp_async_wait_all();
-            if (rest) heap_push_run<P>(myheap, hs, ibuf + (bn - rest), rest, pre);
-            bn -= run;
-        };
-        if (split) {
-            // owner warps: arrive at the team barrier now, refill the heaps,
-            // then wait for the staging (below)
-            if (!relaxer) {
-                team.early_arrive();
-                if (owner) chores();
-            }
-        } else if (rfirst > 0 && owner) {
-            chores();
-        }
-        if constexpr (kSort) {
-            // every successor's record, at its number in the CTA's list
-            if (relaxer) {
-                for (uint32_t j = tid - rfirst; j < total; j += rthreads) {
-                    uint32_t lo = 0, hi = H - 1;
-                    while (lo < hi) {
-                        const uint32_t mid = (lo + hi + 1) >> 1;
-                        if (pop[mid].excl <= j)
-                            lo = mid;
-                        else
-                            hi = mid - 1;
+                // A root taken from the heap is refilled by the run's least
+                // entry (heapreplace): one sift-down serves the pop and one
+                // push, and the heap's last entry stays where it is.  Without
+                // a run the last entry refills it.
+                const bool replace = pending_sift && run > 0;
+                E top = last;
+                if (replace) {
+                    top = ibuf[bn - run];
+                    hs += 1;
+                } else if (pending_sift && !have_last) {
+                    top = myheap.ld(hs + 1);  // (a run cut short by an overflow)
+                }
+                const uint32_t rest = run - (replace ? 1u : 0u);
+                // the rest's bottom brick is read while the sift-down runs (a
+                // fresh bottom brick, at depth 0, needs no read)
+                uint32_t pre = 0;
+                if (rest && hs + 1 > topn) {
+                    uint32_t d;
+                    const uint32_t root = myheap.brick_root(hs + 1, &d);
+                    if (d > 0) {
+                        myheap.fetch_async(root, 2);
+                        pre = root;
                     }
-                    const PopInfo<Key> &pi = pop[lo];
-                    const int move = (int)__fns(pi.mask, 0, (int)(j - pi.excl) + 1);
+                }
+                if (pending_sift) {
+                    const uint32_t fin = heap_sift_down<P>(myheap, hs, top);
+                    // the sift wrote into that brick: its copy is stale
+                    if (pre && fin > topn && myheap.brick_root(fin) == pre) {
+                        cp_async_wait_all();
+                        pre = 0;
+                    }
+                }
+                if (pre) cp_async_wait_all();
+                if (rest) heap_push_run<P>(myheap, hs, ibuf + (bn - rest), rest, pre);
+                s_hs[tid] = hs;
+                s_bn[tid] = bn - run;
+            }
+        }
+        if (relaxer) {
+            Cand *const myreg = region(cta) + 1;
+            const uint32_t rt = tid - rfirst;
+            // source pop of the CTA's successor j = largest h with excl[h] <= j
+            // (it has a successor)
+            const auto source = [&](uint32_t j) -> const PopInfo<Key> & {
+                uint32_t lo = 0, hi = H - 1;
+                while (lo < hi) {
+                    const uint32_t mid = (lo + hi + 1) >> 1;
+                    if (pop[mid].excl <= j)
+                        lo = mid;
+                    else
+                        hi = mid - 1;
+                }
+                return pop[lo];
+            };
+            if constexpr (kSort) {
+                // every successor's record, at its number in the CTA's list
+                for (uint32_t j = rt; j < total; j += rthreads) {
+                    const PopInfo<Key> &pi = source(j);
+                    const int move = nth_bit(pi.mask, j - pi.excl);
                     typename P::Succ sc;
                     prob.succ_begin(pi.key, pi.g, pi.aux, move, sc);
                     uint32_t naux;
                     uint64_t nf;
                     prob.succ_end(sc, pi.aux, move, naux, nf);
-                    ++nS;
                     Cand c;
                     c.slot = (uint32_t)sc.key;
                     c.parent = pi.slot;
@@ -1069,83 +1214,200 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                     c.pad = 0;
                     myreg[j] = c;
                 }
-            }
-        } else if (relaxer) {  // (not kSort)
-            const uint32_t rt = tid - rfirst;
-            for (uint32_t b0 = 0; b0 < total; b0 += rthreads) {
-                const uint32_t j = b0 + rt;
-                bool improved = false, inserted = false;
-                uint32_t nslot = 0, naux = 0, oslot = 0;
-                uint64_t ng = 0, nf = 0;
-                if (j < total) {
-                    // source pop = largest h with excl[h] <= j (it has a successor)
-                    uint32_t lo = 0, hi = H - 1;
-                    while (lo < hi) {
-                        const uint32_t mid = (lo + hi + 1) >> 1;
-                        if (pop[mid].excl <= j)
-                            lo = mid;
-                        else
-                            hi = mid - 1;
+                if (rt == 0) atomicAdd(&s_stat[1], total);
+            } else {
+                // Continuation (see the head of this file): the warp's next pass
+                // takes the successors of this pass's continued nodes, at most one
+                // per lane.
+                uint32_t deepest = 0;
+                for (uint32_t b0 = 0; b0 < total; b0 += rthreads) {
+                    const uint32_t j = b0 + rt;
+                    bool act = j < total;
+                    // the node this lane expands by one move
+                    Key pkey{};
+                    uint64_t pg = 0;
+                    uint32_t paux = 0, oslot = 0;
+                    int move = 0;
+                    if (act) {
+                        const PopInfo<Key> &pi = source(j);
+                        move = nth_bit(pi.mask, j - pi.excl);
+                        oslot = pi.slot;
+                        pkey = pi.key;
+                        pg = pi.g;
+                        paux = pi.aux;
                     }
-                    const PopInfo<Key> &pi = pop[lo];
-                    const int move = (int)__fns(pi.mask, 0, (int)(j - pi.excl) + 1);
-                    oslot = pi.slot;
-                    typename P::Succ sc;
-                    prob.succ_begin(pi.key, pi.g, pi.aux, move, sc);
-                    ng = sc.g;
-                    ++nS;
-                    const int r = relax_key<P>(m.tab, m.mask, m.max_probe, sc.key, sc.g, oslot, &nslot, move);
-                    prob.succ_end(sc, pi.aux, move, naux, nf);
-                    if (r == RELAX_FULL) {
-                        set_error(&st->err[r3], ST_HASH_FULL);
-                    } else {
-                        inserted = (r & RELAX_CLAIMED) != 0;
-                        improved = (r & RELAX_IMPROVED) != 0;
-                        // (link in the g word: the claimer stores the node's
-                        // pattern parts, the same for every writer of the key)
-                        if constexpr (P::kLink == LINK_IN_G)
-                            if (inserted) P::set_link(m.tab + nslot, oslot, naux);
+                    for (uint32_t pass = 0;; ++pass) {
+                        bool improved = false, inserted = false, goal = false;
+                        uint32_t nslot = 0, naux = 0, mask = 0;
+                        uint64_t nf = 0;
+                        typename P::Succ sc{};
+                        bool cand = false;  // improved within the bound: may be continued
+                        const uint32_t acts = __ballot_sync(kFull, act);
+                        if (lane == 0) atomicAdd(&s_stat[1], (uint32_t)__popc(acts));
+                        if (act) {
+                            prob.succ_begin(pkey, pg, paux, move, sc);
+                            // the successor's neighbourhood is read beside the CAS
+                            typename P::Look look;
+                            const bool peek = pass < rs->cont && prob.peek(sc, rs->bound);
+                            if (peek) prob.look_begin(sc.key, look);
+                            const int r =
+                                relax_key<P, Team::kBeside>(m.tab, m.mask, m.max_probe, sc.key, sc.g, oslot, &nslot, move);
+                            prob.succ_end(sc, paux, move, naux, nf);
+                            if (r == RELAX_FULL) {
+                                set_error(&st->err[r3], ST_HASH_FULL);
+                            } else {
+                                inserted = (r & RELAX_CLAIMED) != 0;
+                                improved = (r & RELAX_IMPROVED) != 0;
+                                // (link in the g word: the claimer stores the node's
+                                // pattern parts, the same for every writer of the key)
+                                if constexpr (P::kLink == LINK_IN_G)
+                                    if (inserted) P::set_link(m.tab + nslot, oslot, naux);
+                            }
+                            if (improved) {
+                                goal = prob.is_goal(sc.key);
+                                cand = peek && !goal && P::cost_val(nf) <= rs->bound && P::cost_cmp(nf, rs->gbest) < 0;
+                                if (cand) mask = prob.look_moves(sc.key, naux, look);
+                                if constexpr (P::kLink != LINK_FIELD) {
+                                    // the goal's link is in place: the decision
+                                    // may take it this round, no pop needed
+                                    if (goal) {
+                                        atomic_min_cost<P>(&st->goal_min[r3], nf);
+                                        st->goal_slot = nslot;
+                                    }
+                                } else {
+                                    goal = false;  // (popped: its link is written in the push phase)
+                                }
+                            }
+                        }
+                        const uint32_t ib = __ballot_sync(kFull, inserted);
+                        if (ib && lane == (uint32_t)(__ffs(ib) - 1)) atomicAdd(s_ins, (uint32_t)__popc(ib));
+                        // nodes to continue: as many (in lane order) as have at
+                        // most 32 successors together, if the CTA's candidate
+                        // region has room for all of those beside the pops'
+                        uint32_t n_next = 0, incl = 0;
+                        bool go = false;
+                        if (__any_sync(kFull, cand)) {
+                            incl = (uint32_t)__popc(mask);
+#pragma unroll
+                            for (int o = 1; o < 32; o <<= 1) {
+                                const uint32_t t = __shfl_up_sync(kFull, incl, o);
+                                if (lane >= (uint32_t)o) incl += t;
+                            }
+                            go = cand && incl <= 32u;
+                            n_next = __reduce_max_sync(kFull, go ? incl : 0u);
+                            // (wide keys: a continued node keeps a record, for its link)
+                            uint32_t need = n_next;
+                            if constexpr (P::kLink == LINK_FIELD) need += (uint32_t)__popc(__ballot_sync(kFull, go));
+                            uint32_t ok = 1;
+                            if (lane == 0 && need && atomicAdd(s_room, need) + need > H * P::kMoves - total) {
+                                atomicSub(s_room, need);
+                                ok = 0;
+                            }
+                            if (!__shfl_sync(kFull, ok, 0)) {
+                                go = false;
+                                n_next = 0;
+                            }
+                            const uint32_t gos = __ballot_sync(kFull, go);
+                            if (lane == 0 && gos) atomicAdd(&s_stat[0], (uint32_t)__popc(gos));
+                        }
+                        const bool rec = improved && ((!go && !goal) || P::kLink == LINK_FIELD);
+                        const uint32_t bal = __ballot_sync(kFull, rec);
+                        if (bal) {
+                            const uint32_t leader = (uint32_t)(__ffs(bal) - 1);
+                            uint32_t cbase = 0;
+                            if (lane == leader) cbase = atomicAdd(s_cnt, (uint32_t)__popc(bal));
+                            cbase = __shfl_sync(kFull, cbase, leader);
+                            if (rec) {
+                                Cand c;
+                                c.slot = nslot;
+                                c.parent = oslot;
+                                c.g = sc.g;
+                                c.f = nf;
+                                c.aux = naux;
+                                c.pad = go ? 1u : 0u;
+                                myreg[cbase + __popc(bal & lanemask_lt())] = c;
+                            }
+                        }
+                        if (n_next == 0) break;
+                        deepest = max(deepest, pass + 1);
+                        // successor `lane` of the continued nodes: the first lane
+                        // whose inclusive count exceeds it
+                        uint32_t from = 0;
+#pragma unroll
+                        for (uint32_t q = 16; q; q >>= 1)
+                            if (__shfl_sync(kFull, incl, (int)(from + q - 1)) <= lane) from += q;
+                        act = lane < n_next;
+                        pkey = shfl_key(sc.key, (int)from);
+                        pg = shfl64(sc.g, (int)from);
+                        paux = __shfl_sync(kFull, naux, (int)from);
+                        oslot = __shfl_sync(kFull, nslot, (int)from);
+                        const uint32_t smask = __shfl_sync(kFull, mask, (int)from);
+                        const uint32_t sincl = __shfl_sync(kFull, incl, (int)from);
+                        move = act ? nth_bit(smask, lane - (sincl - (uint32_t)__popc(smask))) : 0;
                     }
                 }
-                const uint32_t ib = __ballot_sync(kFull, inserted);
-                if (ib && lane == (uint32_t)(__ffs(ib) - 1)) atomicAdd(s_ins, (uint32_t)__popc(ib));
-                const uint32_t bal = __ballot_sync(kFull, improved);
-                if (bal) {
-                    const uint32_t leader = (uint32_t)(__ffs(bal) - 1);
-                    uint32_t cbase = 0;
-                    if (lane == leader) cbase = atomicAdd(s_cnt, (uint32_t)__popc(bal));
-                    cbase = __shfl_sync(kFull, cbase, leader);
-                    if (improved) {
-                        Cand c;
-                        c.slot = nslot;
-                        c.parent = oslot;
-                        c.g = ng;
-                        c.f = nf;
-                        c.aux = naux;
-                        c.pad = 0;
-                        myreg[cbase + __popc(bal & lanemask_lt())] = c;
-                    }
-                }
+                if (deepest && lane == 0) atomicMax(s_pass, deepest);
             }
         }
-        if (rfirst == 0 && owner) chores();
 
         // publish this CTA's round: its candidate count and claimed slots
         const auto publish = [&]() {
-            half[(size_t)cta * RR].slot = kSort ? total : *s_cnt;
+            region(cta)->slot = kSort ? total : *s_cnt;
             if (*s_ins) atomicAdd(&st->ins[r3], (unsigned long long)*s_ins);
+            if (*s_pass) atomicMax(&st->pass[r3], *s_pass);
             // the time slice is read by one thread of the team, so that all
             // threads take the same decision
             if (cta == 0 && m.deadline_ns) st->quit[r3] = globaltimer_ns() >= m.deadline_ns ? 1u : 0u;
         };
+        // The decision, taken by one thread of each CTA once the barrier is
+        // complete and handed to the others in shared memory: the same words
+        // read by every thread of the team queue up at one L2 slice (1.6 us a
+        // round with 32768 threads).  They were written before the barrier
+        // and are not written again before every CTA has read them (see
+        // TeamState), so all CTAs decide alike.
+        const auto decide = [&]() {
+            const uint64_t rmin = team.rd64(&st->round_min[r3]), gmin = team.rd64(&st->goal_min[r3]);
+            const uint64_t ins = team.rd64(&st->ins[r3]);
+            const uint32_t e1 = team.rd32(&st->err[r3]), e2 = team.rd32(&st->error);
+            const uint32_t quit = team.rd32(&st->quit[r3]), pass = team.rd32(&st->pass[r3]);
+            const uint32_t pops = team.rd32(&st->pops[r3]);
+            // the one region this CTA takes in the push phase
+            rs->nshare = kSort ? 0u : ldcg_u32(&region(src)->slot);
+            uint64_t gbest = rs->gbest;
+            if (P::cost_cmp(gmin, gbest) < 0) rs->gbest = gbest = gmin;
+            const uint64_t inserted = rs->inserted += ins;
+            const uint64_t steps = rs->steps += 1 + pass;
+            const uint64_t rounds = rs->rounds += 1;
+            uint32_t err = e1 ? e1 : e2;
+            if (!err && inserted > m.max_inserted) err = ST_HASH_FULL;
+            uint32_t s = ST_RUNNING;
+            if (err)
+                s = err;
+            else if (gbest != kInfCost && P::cost_cmp(gbest, rmin) <= 0)
+                s = ST_OK;
+            else if (rmin == kInfCost)
+                s = ST_NO_SOLUTION;
+            else if (steps >= m.max_rounds)
+                s = ST_ITER_LIMIT;
+            rs->status = s;
+            rs->pause = inserted > m.grow_at || (m.deadline_ns && quit) || rounds >= rs->stop_at;
+            if (m.slack > 0.f && rmin != kInfCost) rs->bound = P::cost_val(rmin) + m.slack;
+            rs->cont = pops > m.cont_pops ? 0u : passes(steps);
+            rs->expanded += s_stat[0];
+            rs->generated += s_stat[1];
+            rs->pushed += s_stat[2];
+            s_stat[0] = s_stat[1] = s_stat[2] = 0;
+        };
         if (!split) {
             __syncthreads();
-            if (tid == 0) publish();
-            team.sync();
+            if (lead) publish();
+            team.sync(decide);
         } else if (relaxer) {
             named_sync(2, rthreads);  // every relaxer's counts are in
-            if (tid == rfirst) publish();
+            if (lead) publish();
             team.relaxers_sync(T);
+            if (lead) decide();
+            named_sync(2, rthreads);
         } else {
             // Owner warps, chores done: the relaxers arrive at barrier 3 once
             // they have decided and staged the pushes (or stopped); then the
@@ -1153,35 +1415,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             named_sync(3, T);
             team.late_wait();
         }
-
-        // -------------------------------------------------- decision ---
-        // Every value read here was written before the barrier above and is
-        // not written again before every CTA has read it (see TeamState), so
-        // all threads decide alike.
-        // the push phase's region counts, read beside the decision's words:
-        // the one region this CTA takes, or (kSort) every region
-        const uint32_t src = (uint32_t)((cta + round) % C);
-        const uint32_t per = (C + T - 1) / T, rb = tid * per, re = min(rb + per, C);
-        const uint32_t pre0 = kSort ? (rb < re ? ldcg_u32(&half[(size_t)rb * RR].slot) : 0u)
-                                    : ldcg_u32(&half[(size_t)src * RR].slot);
-        const uint32_t pre1 = kSort && rb + 1 < re ? ldcg_u32(&half[(size_t)(rb + 1) * RR].slot) : 0u;
-        const uint64_t rmin = team.rd64(&st->round_min[r3]);
-        const uint64_t gmin = team.rd64(&st->goal_min[r3]);
-        if (P::cost_cmp(gmin, gbest) < 0) gbest = gmin;
-        uint32_t err = team.rd32(&st->err[r3]);
-        if (!err) err = team.rd32(&st->error);
-        ins_total += team.rd64(&st->ins[r3]);
-        if (!err && ins_total > m.max_inserted) err = ST_HASH_FULL;
-        const bool pause = ins_total > m.grow_at || (m.deadline_ns && team.rd32(&st->quit[r3]));
-        round += 1;
-        if (err)
-            status = err;
-        else if (gbest != kInfCost && P::cost_cmp(gbest, rmin) <= 0)
-            status = ST_OK;
-        else if (rmin == kInfCost)
-            status = ST_NO_SOLUTION;
-        else if (round >= m.max_rounds)
-            status = ST_ITER_LIMIT;
+        status = rs->status;
         if (status != ST_RUNNING) {
             if (split && relaxer) named_arrive(3, T);  // the owner warps wait there
             break;
@@ -1189,12 +1423,14 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
 
         // ---------------------------------------------------- phase 2 ---
         if (cta == 0 && tid == 0) {
-            const uint32_t a = (r3 + 2) % 3;  // the round after next
+            const uint32_t a = r3 == 0 ? 2u : r3 - 1u;  // the round after next
             st->round_min[a] = kInfCost;
             st->goal_min[a] = kInfCost;
             st->ins[a] = 0;
             st->err[a] = 0;
             st->quit[a] = 0;
+            st->pass[a] = 0;
+            st->pops[a] = 0;
         }
         // This CTA's share of the round's candidates is the whole region of
         // CTA (c + round) mod C: the successors of that CTA's H pops, a
@@ -1203,13 +1439,14 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
         // part of the share: a candidate is the slot's winner iff the slot's
         // g still equals its g; winners write prev/aux and are staged for
         // their heap's owner.
-        uint32_t nshare = pre0;
+        uint32_t nshare = rs->nshare;
         if constexpr (kSort) {
             // The round's candidates are numbered region by region: offsets of
             // the C regions (each thread sums `per` consecutive regions' counts).
+            const uint32_t per = (C + T - 1) / T, rb = tid * per, re = min(rb + per, C);
             uint32_t mine = 0;
             for (uint32_t r = rb; r < re; ++r) {
-                const uint32_t n = r == rb ? pre0 : r == rb + 1 ? pre1 : ldcg_u32(&half[(size_t)r * RR].slot);
+                const uint32_t n = ldcg_u32(&region(r)->slot);
                 roff[r] = n;
                 mine += n;
             }
@@ -1232,7 +1469,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                     else
                         hi = mid - 1;
                 }
-                return half + (size_t)lo * RR + 1 + (i - roff[lo]);
+                return region(lo) + 1 + (i - roff[lo]);
             };
             // Sort the round's successors by key, then CTA c takes the sorted
             // positions c, c + C, ...; a position that starts a key's run
@@ -1241,7 +1478,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             const unsigned long long *sorted = team_radix_sort<P::kMoves>(
                 team, ncand, m.sort_bits, [&](uint32_t i) { return ldcg_u32(&rec(i)->slot); }, m.sort_buf,
                 m.sort_buf + nmax, m.sort_hist, ssm, &st->error);
-            const uint32_t nxt = (r3 + 1) % 3;  // claims count toward the next round's decision
+            const uint32_t nxt = r3 == 2 ? 0u : r3 + 1u;  // claims count toward the next round's decision
             uint32_t claimed = 0;
             for (uint32_t q = tid; q < nshare; q += T) {
                 const uint32_t p = cta + C * q;
@@ -1274,7 +1511,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             __syncthreads();
             if (tid == 0 && *s_ins2) atomicAdd(&st->ins[nxt], (unsigned long long)*s_ins2);
         }
-        const Cand *const sreg = half + (size_t)src * RR + 1;
+        const Cand *const sreg = region(src) + 1;
         // (split rounds: the relaxers stage, the owner warps are waiting)
         const uint32_t q0 = split ? tid - rfirst : tid, qstep = split ? rthreads : T;
         const uint32_t nstage = kSort || (split && !relaxer) ? 0u : nshare;
@@ -1286,6 +1523,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                     P::set_link(m.tab + c.slot, c.parent, c.aux);
                 else
                     e.slot = kNone;  // lost to a better writer
+                if (c.pad) e.slot = kNone;  // continued: already expanded, only its link was due
             }
             // (link in the key or g word: every candidate is pushed; one that
             // lost to a better writer of the round is a stale entry, dropped
@@ -1300,23 +1538,37 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
         // The share is dealt round-robin over the CTA's heaps (at most
         // kMoves per heap: the share is at most H * kMoves) into their
         // insertion buffers, which the relax phase left with room for kMoves.
-        if (owner) {
-            for (uint32_t q = (tid + base) % H; q < nshare; q += H) {
-                const E e = stage[q];
-                if (e.slot == kNone) continue;
-                ibuf[bn++] = e;
-                ++nP;
+        if (tid < owner_warps * 32u) {
+            uint32_t npush = 0;
+            if (owner) {
+                E *const ibuf = buf_of();
+                uint32_t n = s_bn[tid];
+                for (uint32_t q = (tid + base) % H; q < nshare; q += H) {
+                    const E e = stage[q];
+                    if (e.slot == kNone) continue;
+                    ibuf[n++] = e;
+                    ++npush;
+                }
+                s_bn[tid] = n;
             }
+            npush = __reduce_add_sync(kFull, npush);
+            if (lane == 0 && npush) atomicAdd(&s_stat[2], npush);
         }
-        base = (uint32_t)(((uint64_t)base + nshare) % H);
-        if (pause || it + 1 >= budget) break;
+        base = (base + nshare) % H;
+        r3 = r3 == 2 ? 0u : r3 + 1u;
+        par ^= 1u;
+        src = src + 1u == C ? 0u : src + 1u;
+        if (rs->pause) break;
     }
 
     // Persist the resumable state: the buffers go into the heaps, then the
     // sizes and the shared tops.  (The pushes use the sift scratch, which
     // the last push phase's staging shares: wait for every owner first.)
     __syncthreads();
-    if (owner && status == ST_RUNNING) {
+    if (owner) {
+        const BrickHeap<P> myheap = heap_of();
+        E *const ibuf = buf_of(), *const gblock = heap_block();
+        uint32_t hs = s_hs[tid], bn = status == ST_RUNNING ? s_bn[tid] : 0u;
         while (bn > 0) {
             if (hs + 1 > m.hcap) {
                 set_error(&st->error, ST_HEAP_OVERFLOW);  // reported by the next decision
@@ -1324,29 +1576,22 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             }
             heap_push<P>(myheap, hs, ibuf[--bn]);
         }
-    }
-    if (owner) {
         m.heap_size[myh] = hs;
         for (uint32_t i = 1; i <= topn && i <= hs; ++i) P::store(gblock + i, myheap.s[i]);
     }
-    if (cta == 0 && tid == 0) {
-        st->round = round;
-        st->base = base;
-        st->goal_best = gbest;
-        st->inserted = ins_total;
-        if (status != ST_RUNNING) st->status = status;
-    }
-    // Flush statistics: one atomic per warp.
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        nE += __shfl_xor_sync(kFull, (unsigned long long)nE, o);
-        nS += __shfl_xor_sync(kFull, (unsigned long long)nS, o);
-        nP += __shfl_xor_sync(kFull, (unsigned long long)nP, o);
-    }
-    if (lane == 0) {
-        atomicAdd(&st->expanded, (unsigned long long)nE);
-        atomicAdd(&st->generated, (unsigned long long)nS);
-        atomicAdd(&st->pushed, (unsigned long long)nP);
+    if (lead) {
+        if (cta == 0) {
+            st->round = rs->rounds;
+            st->steps = rs->steps;
+            st->bound = __float_as_uint(rs->bound);
+            st->base = base;
+            st->goal_best = rs->gbest;
+            st->inserted = rs->inserted;
+            if (status != ST_RUNNING) st->status = status;
+        }
+        atomicAdd(&st->expanded, rs->expanded + s_stat[0]);
+        atomicAdd(&st->generated, rs->generated + s_stat[1]);
+        atomicAdd(&st->pushed, rs->pushed + s_stat[2]);
     }
     return status;
 }

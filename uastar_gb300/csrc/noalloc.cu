@@ -105,7 +105,7 @@ __global__ void k_noalloc_finish(const unsigned char *scratch, int32_t *path, in
         r.status = (int32_t)__ldcg(&st->status);
         r.expanded = (int64_t)__ldcg(&st->expanded);
         r.generated = (int64_t)__ldcg(&st->generated);
-        r.rounds = (int64_t)__ldcg(&st->round);
+        r.rounds = (int64_t)__ldcg(&st->steps);
         long long n = 0;
         if (r.status == ST_OK) {
             const unsigned long long gbest = __ldcg(&st->goal_best);
@@ -182,6 +182,7 @@ extern "C" int32_t uastar_grid_solve_noalloc(const uint64_t *d_words, int32_t H,
     prob.sy = sy;
     prob.ex = ex;
     prob.ey = ey;
+    prob.w_inv = GridProblem::row_inverse(prob.W);
     SearchMem<GridEntry> m;
     m.tab = reinterpret_cast<Slot *>(scratch + kOffTable);
     m.mask = kTableSlots - 1;
@@ -194,6 +195,7 @@ extern "C" int32_t uastar_grid_solve_noalloc(const uint64_t *d_words, int32_t H,
     m.heap_size = reinterpret_cast<uint32_t *>(scratch + kOffSizes);
     m.cand = reinterpret_cast<Cand *>(scratch + kOffCand);
     m.max_rounds = 1ull << 31;
+    m.set(prob.expansion(kHeaps));
     TeamState *st = reinterpret_cast<TeamState *>(scratch + kOffState);
     uint64_t timeout_ns = 10ull * 1000000000ull;  // bound on every team-barrier wait (UASTAR_TIMEOUT)
     void *args[] = {&prob, &m, &st, &timeout_ns};
