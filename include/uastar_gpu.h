@@ -266,8 +266,8 @@ typedef struct {
     double load_factor;           /* target dedup-partition load (0 -> 0.5; uastar_autotune picks one) */
     int32_t ctas;                 /* persistent CTAs (0 -> all SMs x occupancy) */
     int32_t use_graph;            /* launch through a captured CUDA graph (default 1) */
-    int32_t tier1_rounds;         /* round budget of a single-CTA team (0 -> 2048) */
-    int32_t tier2_puzzle_rounds;  /* round budget of a puzzle on a cluster team (0 -> 16384) */
+    int32_t tier1_rounds;         /* budget of a single-CTA team, in expansion steps (0 -> 2048) */
+    int32_t tier2_puzzle_rounds;  /* the same of a puzzle on a cluster team (0 -> 16384) */
     int32_t cluster_size;         /* CTAs per cluster team (0 -> 8; 2..16) */
     int32_t reserved;
 } uastar_batch_config;
@@ -288,11 +288,13 @@ typedef struct {
 
 /* Solve `count` instances of mixed kinds with persistent launches: in the
  * first wave each CTA takes instances from a device work queue and runs GA*
- * on one with its own heap slice and dedup partition, under a round budget
- * (tier1_rounds); grids above 2048^2 and the instances that ran out of rounds
- * or space go to a second wave of 8-CTA cluster teams with 16x the
+ * on one with its own heap slice and dedup partition, under a budget of
+ * expansion steps (tier1_rounds); grids above 2048^2 and the instances that ran
+ * out of steps or space go to a second wave of 8-CTA cluster teams with 16x the
  * partition (puzzles under tier2_puzzle_rounds), and what fails there is
- * solved by the plain engine, one instance at a time.  No counterpart in the
+ * solved by the plain engine, one instance at a time.  The last instances of a
+ * wave (few enough to leave most of the GPU idle) move on without using up
+ * their budget.  No counterpart in the
  * reference, which solves one instance per process through
  * GPUPathwaySolver / GPUPuzzleSolver. */
 int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int32_t count,
@@ -320,7 +322,7 @@ typedef struct {
                                  its latency; more pops per round shorten it) */
     int32_t heap_capacity;    /* entries per heap of a CTA slot (0 -> 16383, 4095 where the budget's
                                  heap share cannot hold one slot of those; 4x on overflow) */
-    int32_t rounds_per_quantum; /* cap on GA* rounds per persistent-kernel launch (0 -> 65536 with
+    int32_t rounds_per_quantum; /* cap on expansion steps per persistent-kernel launch (0 -> 65536 with
                                    a time slice, 256 without) */
     double load_factor;
     int32_t cluster_slots;    /* cap on 8-CTA slots for requests whose search outgrows one CTA

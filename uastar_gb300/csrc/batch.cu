@@ -48,7 +48,7 @@ struct InstDesc {
     uint64_t heap_off;    // serving: byte offset of this request's heap slice
     uint32_t heap_stride; // serving: entries per heap of that slice
     uint32_t heap_hcap;   // serving: maximum heap size
-    uint64_t budget;      // batch: rounds before the instance gives up its team (0: the launch's)
+    uint64_t budget;      // batch: expansion steps before the instance gives up its team (0: the launch's)
     uint64_t key_off;     // batch: first path key of this instance in the key buffer
     uint64_t key_cap;     // batch: room for path keys
     uint64_t grow_at;     // serving: pause the search when it has claimed this many slots (0: never)
@@ -83,10 +83,12 @@ struct BatchArgs {
     TeamState *cstates;    // cluster teams: per cluster team state
     uint32_t *cnext;       // cluster teams: instance index broadcast per cluster
     double max_load;
-    uint64_t budget;       // rounds per call (serving quantum) or ~0
+    uint64_t budget;       // expansion steps per call (serving quantum) or ~0
     int serving;           // 1: CTA b serves slot b; 0: work queue
     uint64_t region_slots; // batch: dedup region of each team (reused by the instances it takes)
     uint64_t quantum_ns;   // serving: time slice of the launch, from each team's start (0: rounds only)
+    uint32_t *idle;        // batch: teams that found the queue empty (SearchMem::idle)
+    uint32_t idle_min, yield_steps;
     uint64_t walk_inline;  // serving: paths of more cells are walked after the quantum (0: all inline)
     unsigned long long *keys;  // batch: path keys of solved instances
 };
@@ -175,6 +177,9 @@ __device__ uint32_t run_instance(const BatchArgs &a, const InstDesc &d, Team &te
             m.grow_at = d.grow_at ? d.grow_at : ~0ull;
             m.deadline_ns = deadline_ns;
             m.split = grid ? a.split_grid : a.split_puzzle;
+            m.idle = a.idle;
+            m.idle_min = a.idle_min;
+            m.yield_steps = a.yield_steps;
             m.sort_buf = nullptr;
             m.sort_hist = nullptr;
             m.sort_bits = 0;
@@ -237,7 +242,10 @@ __global__ void __launch_bounds__(512, 1) k_batch(BatchArgs a) {
         }
         __syncthreads();
         const uint32_t i = s_next;
-        if (i >= a.count) break;
+        if (i >= a.count) {
+            if (a.idle && threadIdx.x == 0) atomicAdd(a.idle, 1u);
+            break;
+        }
         const InstDesc d = a.descs[i];
         if (a.serving && d.kind == 0) break;  // empty serving slot
         const unsigned long long t_start = globaltimer_ns();
@@ -330,7 +338,10 @@ __global__ void __launch_bounds__(512, 1) k_batch_cluster(BatchArgs a) {
             team.sync();
             i = ldcg_u32(&a.cnext[cid]);
         }
-        if (i >= a.count) break;
+        if (i >= a.count) {
+            if (a.idle && crank == 0 && threadIdx.x == 0) atomicAdd(a.idle, 1u);
+            break;
+        }
         const InstDesc d = a.descs[i];
         if (a.serving && d.kind == 0) break;  // empty slot
         if (a.serving) heaps = a.heaps + d.heap_off;
@@ -588,11 +599,13 @@ int32_t resolve_geometry(uastar_engine *eng, const uastar_batch_config *cfg, Bat
 // Each team (CTA or cluster) owns one dedup region, sized for the largest
 // partition of the wave and reused by every instance the team takes, so the
 // wave's table memory is teams x region, not the sum over instances.
-// `puzzle_budget` (0: none) is a round budget for puzzle instances only.
+// `budget` and `puzzle_budget` (0: none; puzzle instances only) count expansion
+// steps.  Once no more than `keep` instances are left running, those that have
+// made yield_steps steps return unfinished as if out of budget.
 int32_t run_wave(uastar_engine *eng, const uastar_instance *insts, const std::vector<int> &idx,
                  const BatchGeometry &g, const std::vector<int> &space_mult, bool use_graph, uint64_t budget,
-                 uint64_t puzzle_budget, uastar_instance_result *results, uastar_batch_stats *stats,
-                 std::vector<int> *retry) {
+                 uint64_t puzzle_budget, int keep, uint32_t yield_steps, uastar_instance_result *results,
+                 uastar_batch_stats *stats, std::vector<int> *retry) {
     cudaError_t e;
     const int cnt = (int)idx.size();
     // plan: order largest estimate first (longest-processing-time first)
@@ -702,6 +715,10 @@ int32_t run_wave(uastar_engine *eng, const uastar_instance *insts, const std::ve
     a.budget = budget;
     a.region_slots = region_slots;
     a.keys = eng->b_walk.as<unsigned long long>();
+    // the last `keep` running instances give up their teams
+    a.idle = a.queue + 1;
+    a.idle_min = (uint32_t)std::max(0, teams - keep);
+    a.yield_steps = yield_steps;
     int ctas = std::min(g.ctas, cnt);
     cudaLaunchConfig_t lc = {};
     cudaLaunchAttribute lat[1];
@@ -731,7 +748,7 @@ int32_t run_wave(uastar_engine *eng, const uastar_instance *insts, const std::ve
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     auto enqueue = [&]() {
-        cudaMemsetAsync(eng->b_queue.p, 0, 4, eng->stream);
+        cudaMemsetAsync(eng->b_queue.p, 0, 8, eng->stream);
         if (g.csize > 0)
             cudaLaunchKernelEx(&lc, k_batch_cluster, a);
         else
@@ -926,10 +943,24 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
         else
             tier1.push_back(i);
     }
+    // A tier's last instances are better off with more of the GPU each, although
+    // they start over there: with most of a wave's teams idle, one puzzle that
+    // holds its cluster for 200-330 ms is solved by the whole GPU in 14.  So a
+    // single-CTA wave gives up what is left once two instances per cluster
+    // team remain (after 256 steps: the small ones finish), a cluster wave
+    // once an eighth of its teams is busy (after 1024).  Eight batches of 16
+    // to 400 instances: 1092 ms without, 605 with the second rule (2 / 4 / 8 /
+    // 16 of 36 teams: 710 / 605 / 603 / 756), 536 with both (18 / 36 / 72 / 150
+    // instances: 583 / 574 / 536 / 539).
+    BatchGeometry gc = g;
+    rc = resolve_cluster_geometry(eng, cfg && cfg->cluster_size >= 2 && cfg->cluster_size <= 16 ? cfg->cluster_size : 8,
+                                  &gc);
+    const int clusters = rc ? 0 : gc.ctas / gc.csize;
+    const int32_t cluster_rc = rc;
     if (!tier1.empty()) {
         std::vector<int> m(tier1.size(), 1);
         const uint64_t b1 = cfg && cfg->tier1_rounds > 0 ? (uint64_t)cfg->tier1_rounds : 2048;
-        rc = run_wave(eng, insts, tier1, g, m, use_graph, b1, 0, results, stats, &retry);
+        rc = run_wave(eng, insts, tier1, g, m, use_graph, b1, 0, 2 * clusters, 256, results, stats, &retry);
         if (rc) return rc;
         // running out of rounds proves an instance large just as an overflow does
         for (int i : retry) {
@@ -939,13 +970,10 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
     }
     todo.clear();
     if (!tier2.empty()) {
-        BatchGeometry gc = g;
+        if (cluster_rc) return cluster_rc;
         bool heap_over = false;
         for (int i : tier2) heap_over |= results[i].status == UASTAR_HEAP_OVERFLOW;
         if (heap_over) gc.set_capacity(g.want * 16 + 15);
-        const int csize = cfg && cfg->cluster_size >= 2 && cfg->cluster_size <= 16 ? cfg->cluster_size : 8;
-        rc = resolve_cluster_geometry(eng, csize, &gc);
-        if (rc) return rc;
         std::vector<int> m(tier2.size());
         for (size_t j = 0; j < tier2.size(); ++j) m[j] = mult[tier2[j]] * 2;
         retry.clear();
@@ -954,7 +982,8 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
         // Grids do not: their rounds are bounded by the path length, which
         // costs a cluster no more rounds than the whole GPU.
         const uint64_t b2 = cfg && cfg->tier2_puzzle_rounds > 0 ? (uint64_t)cfg->tier2_puzzle_rounds : 16384;
-        rc = run_wave(eng, insts, tier2, gc, m, use_graph, ~0ull, b2, results, stats, &retry);
+        rc = run_wave(eng, insts, tier2, gc, m, use_graph, ~0ull, b2, std::max(1, clusters / 8), 1024, results, stats,
+                      &retry);
         if (rc) return rc;
         todo = retry;
     }

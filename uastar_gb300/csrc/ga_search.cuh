@@ -96,6 +96,11 @@ template <class E> struct SearchMem {
     // 0 = none.  The serving loop's quanta end on it, so that every resident
     // search runs for the same time rather than the same number of rounds.
     uint64_t deadline_ns = 0;
+    // Yielding: the search also pauses once *idle (teams of the launch that have
+    // run out of instances) reaches idle_min and it has made yield_steps
+    // expansion steps; looked at every 32nd round.  nullptr = never.
+    const uint32_t *idle = nullptr;
+    uint32_t idle_min = 0, yield_steps = 0;
     // Split rounds (CTA and cluster teams, table-minimum dedup, separate
     // owner warps): the heap owners arrive at the team barrier as soon as
     // their pops are published and refill their heaps while the relaxers
@@ -736,7 +741,7 @@ struct RoundState {
     unsigned long long inserted;   // slots in use after them
     unsigned long long rounds;     // their number
     unsigned long long steps;      // expansion steps: rounds and their continuation passes
-    unsigned long long stop_at;    // the launch's round budget ends here
+    unsigned long long stop_at;    // the launch's budget of steps ends here
     unsigned long long expanded, generated, pushed;  // this CTA, this launch
     float bound;                   // the round's bound on f (SearchMem::slack)
     uint32_t cont;                 // its continuation passes at most
@@ -837,7 +842,7 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *scratc
 }
 
 // ------------------------------------------------------------ the search ---
-// Runs up to `budget` rounds (resumable: state lives in TeamState, the heaps
+// Runs up to `budget` expansion steps (to the end of the round that makes the last) (resumable: state lives in TeamState, the heaps
 // and the table).  Returns ST_RUNNING if the budget ran out first or the
 // table passed m.grow_at, else the final status.  Every thread of every CTA of the team must call it with the
 // same H (heaps per CTA, 1 <= H <= blockDim.x); `smem` points at
@@ -963,7 +968,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
         rs->inserted = team.rd64(&st->inserted);
         rs->rounds = round0;
         rs->steps = team.rd64(&st->steps);
-        rs->stop_at = budget < ~round0 ? round0 + budget : ~0ull;
+        rs->stop_at = budget < ~rs->steps ? rs->steps + budget : ~0ull;
         rs->expanded = rs->generated = rs->pushed = 0;
         rs->bound = __uint_as_float(team.rd32(&st->bound));
         rs->cont = passes(rs->steps);
@@ -1358,6 +1363,8 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             // the time slice is read by one thread of the team, so that all
             // threads take the same decision
             if (cta == 0 && m.deadline_ns) st->quit[r3] = globaltimer_ns() >= m.deadline_ns ? 1u : 0u;
+            if (cta == 0 && m.idle && (rs->rounds & 31u) == 31u && rs->steps >= m.yield_steps)
+                st->quit[r3] = ldcg_u32(m.idle) >= m.idle_min ? 1u : 0u;
         };
         // The decision, taken by one thread of each CTA once the barrier is
         // complete and handed to the others in shared memory: the same words
@@ -1377,7 +1384,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             if (P::cost_cmp(gmin, gbest) < 0) rs->gbest = gbest = gmin;
             const uint64_t inserted = rs->inserted += ins;
             const uint64_t steps = rs->steps += 1 + pass;
-            const uint64_t rounds = rs->rounds += 1;
+            rs->rounds += 1;
             uint32_t err = e1 ? e1 : e2;
             if (!err && inserted > m.max_inserted) err = ST_HASH_FULL;
             uint32_t s = ST_RUNNING;
@@ -1390,7 +1397,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             else if (steps >= m.max_rounds)
                 s = ST_ITER_LIMIT;
             rs->status = s;
-            rs->pause = inserted > m.grow_at || (m.deadline_ns && quit) || rounds >= rs->stop_at;
+            rs->pause = inserted > m.grow_at || quit || steps >= rs->stop_at;
             if (m.slack > 0.f && rmin != kInfCost) rs->bound = P::cost_val(rmin) + m.slack;
             rs->cont = pops > m.cont_pops ? 0u : passes(steps);
             rs->expanded += s_stat[0];
