@@ -24,72 +24,130 @@ using namespace uastar;
 namespace uastar {
 
 // One BFS level: every entry equal to d expands; unreached neighbours get d+1.
-// Threads scan 16 entries each (one 16-byte load), so the level scan runs at
-// streaming bandwidth and only the expansions make random accesses.  Racing
-// writers of a neighbour all store the same value.
+// A warp scans 512 entries at a time (16 per lane, one 16-byte load), so the
+// level scan runs at streaming bandwidth; the ranks that match go to a queue
+// in shared memory, and the warp expands them 32 at a time.  (Expanded where
+// they are found, in a branch per entry, a warp ran one match at a time:
+// neighbouring ranks lie on ~20 different levels.)  Racing writers of a
+// neighbour all store the same value.
+//
+// A neighbour's rank follows from the entry's own.  Tile j's digit counts the
+// cells below its cell that no earlier tile holds.  Moved one cell sideways it
+// passes no other tile: the rank moves by its multiplier.  Moved one row it
+// passes the N - 1 cells between: its digit moves by N less the earlier tiles
+// among them, and the digit of each later tile among them by one the same way.
+//
+// 7-8 tables of the 4x4 board (577 MB): 371 -> 37.4 ms, 5x5 (510 MB): 240 ->
+// 42.6 ms, 3x3: 1.5 -> 0.65 ms.  What is left is L1: ~12 single-byte gathers per
+// entry, two in three of them a line apart (52 ms with each gather waiting for
+// the one before).
 template <int N, int P>
 __global__ void __launch_bounds__(256) k_pdb_level(uint8_t *table, uint64_t size, uint32_t d,
                                                    uint32_t *changed) {
     constexpr int NN = N * N;
     constexpr int K = PuzzlePatterns<N>::count(P);
-    const uint64_t chunks = (size + 15) / 16;
+    constexpr uint32_t kScan = 512;  // entries of a warp's scan step
+    __shared__ uint32_t queue[8][kScan + 32];
+    // a level after one that changed nothing has nothing to do
+    if (d > 0 && !__ldcg(changed + d - 1)) return;
+    uint32_t *const q = queue[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t n = 0;  // entries waiting in q (warp-uniform)
     bool any = false;
-    for (uint64_t cidx = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; cidx < chunks;
-         cidx += (uint64_t)gridDim.x * blockDim.x) {
-        uint4 v;
-        const uint64_t r0 = cidx * 16;
+
+    const auto expand = [&](uint32_t rank) {
+        // decode rank -> cells of the K tracked tiles: digit j picks the
+        // digit-th free cell
+        uint32_t code = rank, used = 0;
+        uint32_t pos[K];
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            constexpr uint32_t kAll = NN < 32 ? (1u << NN) - 1u : ~0u;
+            const uint32_t m = pattern_mult<N>(P, j + 1);
+            uint32_t v = code / m, cell = 0, f = ~used & kAll;
+            code -= v * m;
+#pragma unroll
+            for (int w = 16; w; w >>= 1) {  // the v-th set bit of f, by halves
+                if (w >= NN) continue;
+                const uint32_t low = __popc(f & ((1u << w) - 1u));
+                if (v >= low) {
+                    v -= low;
+                    f >>= w;
+                    cell += w;
+                }
+            }
+            pos[j] = cell;
+            used |= 1u << cell;
+        }
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            const uint32_t c = pos[j], y = c % N;
+            const uint32_t mj = pattern_mult<N>(P, j + 1);
+            // rank change of tile j's move one row up or down, from the tiles
+            // on the cells passed
+            uint32_t down = (uint32_t)N * mj, up = (uint32_t)N * mj;
+#pragma unroll
+            for (int t = 0; t < K; ++t) {
+                if (t == j) continue;
+                const uint32_t w = t < j ? 0u - mj : pattern_mult<N>(P, t + 1);
+                if (pos[t] - c - 1u < (uint32_t)(N - 1)) down += w;
+                if (c - pos[t] - 1u < (uint32_t)(N - 1)) up += w;
+            }
+            const bool ok[4] = {c + N < NN && !(used >> (c + N) & 1u), c >= N && !(used >> (c >= N ? c - N : 0u) & 1u),
+                                y + 1 < N && !(used >> (c + 1) & 1u), y > 0 && !(used >> (y > 0 ? c - 1 : 0u) & 1u)};
+            const uint32_t r[4] = {rank + down, rank - up, rank + mj, rank - mj};
+            // the four reads in flight together; through L1, where a stale
+            // 0xFF only repeats a store of the same value
+            uint8_t old[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) old[k] = ok[k] ? __ldca(table + r[k]) : 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (old[k] == 0xFF) {
+                    table[r[k]] = (uint8_t)(d + 1);
+                    any = true;
+                }
+        }
+    };
+
+    const uint64_t step = (uint64_t)gridDim.x * 8u * kScan;
+    const uint32_t d4 = d * 0x01010101u;
+    for (uint64_t base = ((uint64_t)blockIdx.x * 8u + (threadIdx.x >> 5)) * kScan; base < size; base += step) {
+        const uint64_t r0 = base + lane * 16u;
+        uint4 v = make_uint4(~0u, ~0u, ~0u, ~0u);  // (no level is 255)
         if (r0 + 16 <= size) {
             v = __ldcg(reinterpret_cast<const uint4 *>(table + r0));
-        } else {
+        } else if (r0 < size) {
             uint8_t tmp[16];
             for (int i = 0; i < 16; ++i) tmp[i] = r0 + i < size ? __ldcg(table + r0 + i) : 0xFF;
             memcpy(&v, tmp, 16);
         }
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll 1
-        for (int i = 0; i < 16; ++i) {
-            if (((w[i >> 2] >> (8 * (i & 3))) & 0xFFu) != d) continue;
-            // decode rank -> cells of the K tracked tiles
-            uint64_t code = r0 + i;
-            uint32_t pos[K];
-            uint32_t used = 0;
+        // one bit per matching entry: entry 4 a + b of the lane at bit 8 b + a
+        uint32_t hits = (__vcmpeq4(v.x, d4) & 0x01010101u) | (__vcmpeq4(v.y, d4) & 0x02020202u) |
+                        (__vcmpeq4(v.z, d4) & 0x04040404u) | (__vcmpeq4(v.w, d4) & 0x08080808u);
+        const uint32_t mine = __popc(hits);
+        uint32_t incl = mine;
 #pragma unroll
-            for (int j = 0; j < K; ++j) {
-                const uint32_t m = pattern_mult<N>(P, j + 1);
-                const uint32_t vj = (uint32_t)(code / m);
-                code -= (uint64_t)vj * m;
-                const uint32_t cell = __fns(~used, 0, (int)vj + 1);
-                pos[j] = cell;
-                used |= 1u << cell;
-            }
-            // every tracked tile, every direction
-#pragma unroll
-            for (int j = 0; j < K; ++j) {
-                const int c = (int)pos[j], cx = c / N, cy = c % N;
-#pragma unroll
-                for (int dir = 0; dir < 4; ++dir) {
-                    const int nx = cx + (dir == 0 ? 1 : dir == 1 ? -1 : 0);
-                    const int ny = cy + (dir == 2 ? 1 : dir == 3 ? -1 : 0);
-                    if (nx < 0 || nx >= N || ny < 0 || ny >= N) continue;
-                    const uint32_t q = (uint32_t)(nx * N + ny);
-                    if (used >> q & 1u) continue;
-                    uint32_t u2 = 0, r = 0;
-#pragma unroll
-                    for (int t = 0; t < K; ++t) {
-                        const uint32_t p = t == j ? q : pos[t];
-                        r += (p - __popc(u2 & ((1u << p) - 1u))) * pattern_mult<N>(P, t + 1);
-                        u2 |= 1u << p;
-                    }
-                    if (__ldcg(table + r) == 0xFF) {
-                        table[r] = (uint8_t)(d + 1);
-                        any = true;
-                    }
-                }
-            }
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(kFull, incl, o);
+            if (lane >= (uint32_t)o) incl += t;
         }
+        uint32_t at = n + incl - mine;
+        n += __shfl_sync(kFull, incl, 31);
+        while (hits) {
+            const uint32_t b = __ffs((int)hits) - 1;
+            hits &= hits - 1u;
+            q[at++] = (uint32_t)r0 + ((b & 7u) << 2) + (b >> 3);
+        }
+        __syncwarp();
+        while (n >= 32) {
+            n -= 32;
+            expand(q[n + lane]);
+        }
+        __syncwarp();
     }
-    if (__syncthreads_or(any) && threadIdx.x == 0) *changed = 1u;
-    (void)NN;
+    if (lane < n) expand(q[lane]);
+    if (__any_sync(kFull, any) && lane == 0) changed[d] = 1u;
 }
 
 __global__ void k_pdb_set(uint8_t *table, uint64_t idx) { table[idx] = 0; }
@@ -174,22 +232,27 @@ int32_t build_one(uastar_engine *eng, uint8_t *table, uint64_t size, uint64_t go
     if ((e = cudaMemsetAsync(table, 0xFF, size, eng->stream)) != cudaSuccess) return fail_cuda(eng, e, "pdb clear");
     k_pdb_set<<<1, 1, 0, eng->stream>>>(table, goal);
     eng->launches++;
+    // one flag per level; the host looks at them every kLevels levels (a level
+    // past the last returns at once), so the launches queue up behind each other
+    constexpr uint32_t kLevels = 16, kMax = 254;
     uastar::DevBuf flag;
-    if ((e = flag.ensure(64)) != cudaSuccess) return fail_cuda(eng, e, "pdb flag");
+    if ((e = flag.ensure((kMax + kLevels) * 4)) != cudaSuccess) return fail_cuda(eng, e, "pdb flag");
     uint32_t *d_changed = flag.as<uint32_t>();
     uint32_t *h_changed = nullptr;
     if ((e = cudaMallocHost(&h_changed, sizeof(uint32_t))) != cudaSuccess) {
         flag.release();
         return fail_cuda(eng, e, "pdb host flag");
     }
-    const uint64_t chunks = (size + 15) / 16;
-    const int blocks = (int)std::min<uint64_t>((chunks + 255) / 256, (uint64_t)eng->sms * 16);
+    cudaMemsetAsync(d_changed, 0, (kMax + kLevels) * 4, eng->stream);
+    const uint64_t warps = (size + 511) / 512;
+    const int blocks = (int)std::min<uint64_t>((warps + 7) / 8, (uint64_t)eng->sms * 16);
     int32_t rc = UASTAR_OK;
-    for (uint32_t d = 0; d < 254; ++d) {
-        cudaMemsetAsync(d_changed, 0, 4, eng->stream);
-        k_pdb_level<N, P><<<blocks, 256, 0, eng->stream>>>(table, size, d, d_changed);
-        eng->launches++;
-        cudaMemcpyAsync(h_changed, d_changed, 4, cudaMemcpyDeviceToHost, eng->stream);
+    for (uint32_t d = 0; d < kMax;) {
+        for (uint32_t q = 0; q < kLevels && d < kMax; ++q, ++d) {
+            k_pdb_level<N, P><<<blocks, 256, 0, eng->stream>>>(table, size, d, d_changed);
+            eng->launches++;
+        }
+        cudaMemcpyAsync(h_changed, d_changed + d - 1, 4, cudaMemcpyDeviceToHost, eng->stream);
         if ((e = cudaStreamSynchronize(eng->stream)) != cudaSuccess) {
             rc = fail_cuda(eng, e, "pdb level");
             break;
