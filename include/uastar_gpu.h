@@ -330,7 +330,8 @@ typedef struct {
     int32_t quantum_us;       /* time slice of a persistent-kernel launch: every resident search
                                  runs rounds until this many microseconds have passed since the
                                  launch began, so that fast and slow searches share the GPU's time
-                                 rather than a round count (0 -> 8000; < 0 -> none, rounds only) */
+                                 rather than a round count (0 -> 8000, 2000 while nothing waits and at most
+                                 half of the GPU is taken; < 0 -> none, rounds only) */
 } uastar_serve_config;
 
 typedef struct {

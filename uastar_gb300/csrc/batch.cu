@@ -1251,6 +1251,7 @@ struct ServeState {
     uastar_engine *eng = nullptr;
     uastar_serve_config cfg{};
     ServeTier tier[2];  // 0 = CTA slots, 1 = cluster slots
+    bool light = false; // nothing waits and at most half of the CTAs are taken
     int capacity = 0;   // co-resident CTAs shared by both tiers' resident requests
     uint64_t heap_bytes = 0;
     std::thread th;
@@ -1462,9 +1463,13 @@ static BatchArgs serve_args(ServeState *S, ServeTier &t) {
     // 8 ms by default: the first 4000 requests of the 20000-request stream at
     // 1000/s served at 193 / 225 / 231-257 / 252 / 250 solves/s with 2 / 4 /
     // 8 / 12 / 16 ms slices (a launch's fixed costs against the wait of a
-    // finished request for its slice's end).
+    // finished request for its slice's end).  2 ms under a light load, where a
+    // finished request waits for nobody else's work and a wide one moves to a
+    // cluster at the end of its first slice: bursts of 10 to 48 requests 76 /
+    // 36 / 76 / 154 / 115 / 205 / 42 ms with 8 ms slices, 52 / 15 / 53 / 141 /
+    // 104 / 192 / 20 with 4, 46 / 14 / 49 / 136 / 106 / 197 / 15 with 2.
     const bool sliced = S->cfg.quantum_us >= 0;
-    a.quantum_ns = sliced ? (uint64_t)(S->cfg.quantum_us > 0 ? S->cfg.quantum_us : 8000) * 1000ull : 0;
+    a.quantum_ns = sliced ? (uint64_t)(S->cfg.quantum_us > 0 ? S->cfg.quantum_us : S->light ? 2000 : 8000) * 1000ull : 0;
     // paths beyond 1024 cells (~0.5 ms of pointer chase) are walked after
     // the quantum, on the walk stream (serve_walk_issue)
     a.walk_inline = 1024;
@@ -1802,7 +1807,8 @@ static bool serve_migrate(ServeState *S, int q) {
 // overflows a cluster slot retries there with more.  A request that keeps its
 // CTA's heaps saturated (a wide frontier, which more heaps cover in fewer
 // rounds) moves to a cluster slot with its search state (serve_migrate) when
-// the GPU has spare CTAs and nothing waits (`spare`: latency), or once it has
+// the GPU has spare CTAs and nothing waits (`spare`: latency, so after 64
+// rounds; 1024 otherwise), or once it has
 // taken 4M expansions (a request that large would otherwise be the stream's
 // tail); other requests stay on one CTA, the most work per CTA.  A grid with
 // a thin frontier never moves: its rounds are bounded by its path length,
@@ -1830,7 +1836,7 @@ static void serve_retire(ServeState *S, ServeTier &t, std::deque<ServeReq> &to_l
             }
             // a wide frontier that has already taken 4M expansions (or any, when
             // the GPU has spare CTAs) moves to a cluster slot, search state and all
-            const bool saturated = o.rounds >= 1024 && (double)o.expanded >= 0.5 * t.geo.H * (double)o.rounds;
+            const bool saturated = o.rounds >= (spare ? 64u : 1024u) && (double)o.expanded >= 0.5 * t.geo.H * (double)o.rounds;
             if (!t.large && saturated && large.nslots > 0 && to_large.empty() && (spare || o.expanded >= 4000000ull)) {
                 if (serve_migrate(S, q)) continue;
                 if (S->loop_error) return;
@@ -2032,6 +2038,7 @@ static void serve_loop(ServeState *S) {
         //    does not leave, so launched apart the two kernels would take
         //    turns on the GPU instead of sharing it
         const bool idle = !small.inflight && !large.inflight;
+        S->light = pending.empty() && to_large.empty() && rs + 8 * rl <= S->capacity / 2;
         for (int ti = 1; ti >= 0 && idle; --ti) {
             ServeTier &t = S->tier[ti];
             if (!t.nslots || !t.resident()) continue;
