@@ -279,6 +279,12 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
     const uint32_t tph = c.threads_per_heap > 0 ? (uint32_t)c.threads_per_heap : 4u;
     uint32_t H, nblocks;
     plain_shape<P>(eng, block, tph, &H, &nblocks);
+    // A capped table much smaller than a round's successors would pause the
+    // search after every round: fewer heaps, so that it holds four rounds.
+    if (max_log2 > 0 && c.heaps <= 0) {
+        const double room = c.max_load * (double)(1ull << max_log2) / (4.0 * P::kMoves * H);
+        nblocks = std::max(1u, std::min(nblocks, (uint32_t)room));
+    }
     const uint32_t k = nblocks * H;
     int log2 = c.hash_log2_slots > 0 ? c.hash_log2_slots : log2_auto;
     if (log2 > 31) {
@@ -401,11 +407,14 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
             m.sort_bits = sort_bits;
         }
         // an auto-sized table grows in place (x4) when half full; at the cap
-        // the search pauses instead, two rounds' worth of inserts short of
-        // the load limit
+        // the search pauses instead, a round's worth of inserts short of the
+        // load limit (a round relaxes at most kMoves successors per heap)
         const bool auto_table = c.hash_log2_slots <= 0 || max_log2 > 0;
-        const uint64_t full_at = m.max_inserted > 4ull * k * P::kMoves ? m.max_inserted - 4ull * k * P::kMoves : 0;
-        auto pause_point = [&](uint64_t n) { return max_log2 > 0 && n >= (1ull << max_log2) ? full_at : n / 2; };
+        const uint64_t round_max = (uint64_t)k * P::kMoves;
+        const auto pause_point = [&](uint64_t n) -> uint64_t {
+            if (max_log2 <= 0 || n < (1ull << max_log2)) return n / 2;
+            return m.max_inserted > round_max ? m.max_inserted - round_max : 0ull;
+        };
         m.grow_at = auto_table ? pause_point(slots) : ~0ull;
         TeamState *st = eng->team.as<TeamState>();
         uint64_t timeout_ns = (uint64_t)(c.wait_timeout_s * 1e9);
@@ -430,9 +439,7 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
             if (max_log2 > 0 && m.mask + 1 >= (1ull << max_log2)) break;
             if (grow_table<P>(eng, m, k, st)) {
                 out->grows += 1;
-                const uint64_t n = m.mask + 1;
-                const uint64_t fa = m.max_inserted > 4ull * k * P::kMoves ? m.max_inserted - 4ull * k * P::kMoves : 0;
-                m.grow_at = max_log2 > 0 && n >= (1ull << max_log2) ? fa : n / 2;
+                m.grow_at = pause_point(m.mask + 1);
             } else {
                 m.grow_at = ~0ull;  // no room: carry on up to the load limit
                 if ((e = cudaMemsetAsync(&st->barrier, 0, sizeof(uint32_t), eng->stream)) != cudaSuccess)
@@ -710,89 +717,6 @@ void boards_to_moves(int n, const std::vector<std::vector<uint8_t>> &boards, std
 }
 
 // ---- exact phase of the memory-bounded mode: IDA* passes (ga_ida.cuh) ----
-// A board on the host: tiles, blank cell, the move that reached it (+1) and
-// the moves from the start (2 bits each, first lowest).
-struct HostBoard {
-    uint8_t b[25];
-    int8_t blank;
-    uint8_t last;
-    uint64_t prefix;
-};
-
-// Blank move mv (0..3 = (+1,0), (-1,0), (0,+1), (0,-1) in (row, column), the
-// reference's DX/DY) on an n x n board; false if it leaves the board.
-template <int N> bool host_blank_move(HostBoard &h, int mv) {
-    const int bx = h.blank / N, by = h.blank % N;
-    const int nx = bx + (mv == 0) - (mv == 1), ny = by + (mv == 2) - (mv == 3);
-    if (nx < 0 || nx >= N || ny < 0 || ny >= N) return false;
-    const int q = nx * N + ny;
-    h.b[h.blank] = h.b[q];
-    h.b[q] = 0;
-    h.blank = (int8_t)q;
-    return true;
-}
-
-template <int N> bool host_is_goal(const uint8_t *b) {
-    for (int i = 0; i < N * N; ++i)
-        if (b[i] != (i + 1) % (N * N)) return false;
-    return true;
-}
-
-// The start's search tree cut at the first depth with at least `want` nodes
-// (at most max_depth <= 32), without moves that undo the previous one (the
-// search prunes those too).  A goal met on the way ends the cut: every
-// shorter move sequence was enumerated before it, so its depth is optimal.
-template <int N>
-void ida_roots(const uint8_t *tiles, size_t want, int max_depth, std::vector<IdaRoot> *roots,
-               std::vector<int32_t> *goal_moves, bool *goal) {
-    std::vector<HostBoard> cur(1), next;
-    HostBoard &s0 = cur[0];
-    std::memset(&s0, 0, sizeof s0);
-    std::memcpy(s0.b, tiles, N * N);
-    for (int i = 0; i < N * N; ++i)
-        if (!tiles[i]) s0.blank = (int8_t)i;
-    *goal = host_is_goal<N>(tiles);
-    if (*goal) return;
-    for (int d = 0; d < max_depth && cur.size() < want; ++d) {
-        next.clear();
-        next.reserve(cur.size() * 3);
-        for (const HostBoard &h : cur)
-            for (int mv = 0; mv < 4; ++mv) {
-                if (h.last && mv == ((h.last - 1) ^ 1)) continue;
-                HostBoard m = h;
-                if (!host_blank_move<N>(m, mv)) continue;
-                m.last = (uint8_t)(mv + 1);
-                m.prefix = h.prefix | ((uint64_t)mv << (2 * d));
-                if (host_is_goal<N>(m.b)) {
-                    *goal = true;
-                    goal_moves->clear();
-                    for (int j = 0; j <= d; ++j) goal_moves->push_back((int32_t)((m.prefix >> (2 * j)) & 3));
-                    return;
-                }
-                next.push_back(m);
-            }
-        cur.swap(next);
-        if (cur.size() >= want || d + 1 >= max_depth) {
-            roots->resize(cur.size());
-            for (size_t i = 0; i < cur.size(); ++i) {
-                IdaRoot &r = (*roots)[i];
-                if constexpr (N == 5) {
-                    const Key128 k = PuzzleProblem<5>::pack(cur[i].b);
-                    r.lo = k.lo;
-                    r.hi = k.hi;
-                } else {
-                    r.lo = pack_board(N, cur[i].b);
-                    r.hi = 0;
-                }
-                r.g = (uint32_t)(d + 1);
-                r.last = cur[i].last;
-                r.prefix = cur[i].prefix;
-            }
-            return;
-        }
-    }
-}
-
 // IDA* passes from the lower bound lb up to the length ub of the solution
 // in hand, for at most budget_ms.  A pass that finds a goal writes the
 // optimal moves; one that completes without a goal raises out->lower_bound
@@ -802,43 +726,81 @@ int32_t ida_exact(uastar_engine *eng, const uint8_t *tiles, int32_t lb, int32_t 
                   std::vector<int32_t> *moves, uastar_bounded_result *out) {
     constexpr int kMaxDepth = N == 3 ? 48 : N == 4 ? 100 : 200;
     const double t0 = now_ms();
-    std::vector<IdaRoot> roots;
-    std::vector<int32_t> goal_moves;
-    bool goal = false;
-    ida_roots<N>(tiles, 1u << 18, 24, &roots, &goal_moves, &goal);
-    if (goal) {  // the cut met the goal first: that is the optimum
-        *moves = goal_moves;
-        out->lower_bound = (int32_t)goal_moves.size();
+    PuzzleProblem<N> prob;
+    prob.pdb = eng->pdb[N].as<uint8_t>();
+    prob.goal = PuzzleProblem<N>::goal_key();
+    if constexpr (N == 5)
+        prob.start = PuzzleProblem<5>::pack(tiles);
+    else
+        prob.start = pack_board(N, tiles);
+    if (prob.start_is_goal()) {
+        moves->clear();
+        out->lower_bound = 0;
         out->exact_optimal = 1;
         out->exact_ms = now_ms() - t0;
         return UASTAR_OK;
     }
-    const size_t head = (sizeof(IdaPass) + 255) & ~(size_t)255;
+    // pass state, cut state, the start, two levels of the cut
+    constexpr size_t kCutAt = (sizeof(IdaPass) + 255) & ~(size_t)255;
+    constexpr size_t kStartAt = (kCutAt + sizeof(IdaCut) + 255) & ~(size_t)255;
+    constexpr size_t kLevelAt = (kStartAt + sizeof(IdaRoot) + 255) & ~(size_t)255;
+    const size_t room = 4 * (size_t)kIdaRoots;  // a level's children
     cudaError_t e;
-    if ((e = eng->ida.ensure(head + roots.size() * sizeof(IdaRoot))) != cudaSuccess) return fail_cuda(eng, e, "alloc ida");
-    IdaPass *d_pass = eng->ida.as<IdaPass>();
-    IdaRoot *d_roots = reinterpret_cast<IdaRoot *>(eng->ida.as<unsigned char>() + head);
-    if ((e = cudaMemcpyAsync(d_roots, roots.data(), roots.size() * sizeof(IdaRoot), cudaMemcpyHostToDevice,
-                             eng->stream)) != cudaSuccess)
-        return fail_cuda(eng, e, "ida roots");
-    PuzzleProblem<N> prob;
-    prob.pdb = eng->pdb[N].as<uint8_t>();
-    prob.goal = PuzzleProblem<N>::goal_key();
-    prob.start = prob.goal;
+    if ((e = eng->ida.ensure(kLevelAt + 2 * room * sizeof(IdaRoot))) != cudaSuccess)
+        return fail_cuda(eng, e, "alloc ida");
+    unsigned char *const base = eng->ida.as<unsigned char>();
+    IdaPass *d_pass = reinterpret_cast<IdaPass *>(base);
+    IdaCut *d_cut = reinterpret_cast<IdaCut *>(base + kCutAt);
+    IdaRoot *d_start = reinterpret_cast<IdaRoot *>(base + kStartAt);
+    IdaRoot *const d_level[2] = {reinterpret_cast<IdaRoot *>(base + kLevelAt),
+                                 reinterpret_cast<IdaRoot *>(base + kLevelAt) + room};
+    k_ida_start<PuzzleProblem<N>><<<1, 1, 0, eng->stream>>>(prob, d_start);
+    eng->launches++;
     uint32_t t = (uint32_t)std::max(lb, 0);
     bool optimal = false;
     while (t < (uint32_t)ub) {
         const double left_ms = budget_ms - (now_ms() - t0);
         if (left_ms <= 0) break;
-        IdaPass init;
+        struct {
+            IdaPass pass;
+            IdaCut cut;
+        } init;
         std::memset(&init, 0, sizeof init);
-        init.min_exceed = ~0u;
-        if ((e = cudaMemcpyAsync(d_pass, &init, sizeof init, cudaMemcpyHostToDevice, eng->stream)) != cudaSuccess)
+        init.pass.min_exceed = init.cut.min_exceed = ~0u;
+        init.cut.count[0] = 1;
+        if ((e = cudaMemcpyAsync(d_pass, &init.pass, sizeof init.pass, cudaMemcpyHostToDevice, eng->stream)) !=
+                cudaSuccess ||
+            (e = cudaMemcpyAsync(d_cut, &init.cut, sizeof init.cut, cudaMemcpyHostToDevice, eng->stream)) != cudaSuccess)
             return fail_cuda(eng, e, "ida state");
+        for (uint32_t d = 0; d < kIdaCutDepth; ++d) {
+            k_ida_cut<PuzzleProblem<N>><<<std::max(1, eng->sms * 4), 256, 0, eng->stream>>>(
+                prob, d == 0 ? d_start : d_level[d & 1], d_level[(d + 1) & 1], d, t, d_cut);
+            eng->launches++;
+        }
+        IdaCut cut;
+        if ((e = cudaGetLastError()) != cudaSuccess) return fail_cuda(eng, e, "ida cut");
+        if ((e = cudaMemcpyAsync(&cut, d_cut, sizeof cut, cudaMemcpyDeviceToHost, eng->stream)) != cudaSuccess ||
+            (e = cudaStreamSynchronize(eng->stream)) != cudaSuccess)
+            return fail_cuda(eng, e, "ida cut");
+        uint32_t depth = 0;
+        while (depth < kIdaCutDepth && cut.count[depth + 1]) out->exact_nodes += cut.count[++depth];
+        if (cut.goal) {
+            out->exact_passes += 1;
+            moves->clear();
+            for (uint32_t q = 0; q < cut.goal; ++q) moves->push_back((int32_t)((cut.goal_prefix >> (2 * q)) & 3));
+            out->lower_bound = (int32_t)cut.goal;
+            optimal = true;
+            break;
+        }
+        const IdaRoot *const d_roots = d_level[depth & 1];
+        // (level `depth` is whole only if it is where the cut stopped; otherwise
+        // the tree below t ended within the cut)
+        const bool ended = depth < kIdaCutDepth && cut.count[depth] < kIdaRoots;
+        const uint32_t nroots = ended ? 0u : cut.count[depth];
         // threads read the device clock at their start: the pass ends
         // `left_ms` after it began
         k_ida_pass<PuzzleProblem<N>, kMaxDepth><<<std::max(1, eng->sms * 8), 128, 0, eng->stream>>>(
-            prob, d_roots, (uint32_t)roots.size(), t, d_pass, (unsigned long long)(left_ms * 1e6));
+            prob, d_roots, nroots, t, d_pass, (unsigned long long)(left_ms * 1e6));
         eng->launches++;
         if ((e = cudaGetLastError()) != cudaSuccess) return fail_cuda(eng, e, "ida launch");
         IdaPass res;
@@ -848,7 +810,11 @@ int32_t ida_exact(uastar_engine *eng, const uint8_t *tiles, int32_t lb, int32_t 
         out->exact_passes += 1;
         out->exact_nodes += (int64_t)res.nodes;
         if (res.found) {
-            const IdaRoot &r = roots[res.found_root];
+            IdaRoot r;
+            if ((e = cudaMemcpyAsync(&r, d_roots + res.found_root, sizeof r, cudaMemcpyDeviceToHost, eng->stream)) !=
+                    cudaSuccess ||
+                (e = cudaStreamSynchronize(eng->stream)) != cudaSuccess)
+                return fail_cuda(eng, e, "ida root");
             moves->clear();
             for (uint32_t j = 0; j < r.g; ++j) moves->push_back((int32_t)((r.prefix >> (2 * j)) & 3));
             for (uint32_t j = 0; j < res.found_len; ++j) moves->push_back((int32_t)res.moves[j]);
@@ -856,6 +822,7 @@ int32_t ida_exact(uastar_engine *eng, const uint8_t *tiles, int32_t lb, int32_t 
             optimal = true;
             break;
         }
+        res.min_exceed = std::min(res.min_exceed, cut.min_exceed);
         if (res.stopped) break;  // out of time (or a subtree deeper than the stack): t stays the bound
         if (res.min_exceed == ~0u) break;  // nothing cut off and no goal: cannot happen on a solvable board
         t = res.min_exceed;

@@ -2,15 +2,22 @@
 // puzzles: the exact phase of the memory-bounded mode.
 //
 // One pass searches every path whose f = g + h stays at or below a threshold
-// t, depth-first, with memory proportional to the depth only (no dedup
-// table).  The start's tree is cut at a fixed depth on the host into roots
-// (move sequences without immediate reversal, as the search itself prunes);
-// every thread takes roots from a queue and searches each one's subtree with
-// a stack of at most kMaxDepth levels in its own local memory.  A pass that
-// finds no goal proves the optimum above t and reports the least f it cut
-// off, the next threshold (Korf, "Depth-first iterative-deepening: an optimal
-// admissible tree search", 1985).  With an admissible h the first pass that
-// finds a goal finds an optimal solution.
+// t (no dedup table).  Its first moves are searched level by level (k_ida_cut;
+// move sequences without immediate reversal, as the search itself prunes)
+// until a level has enough nodes to go round; then threads take those roots
+// from a queue and search each one's subtree depth-first, with memory
+// proportional to the depth, a stack of at most kMaxDepth levels in the
+// thread's own local memory.  A pass that finds no goal proves the optimum
+// above t and reports the least f it cut off, the next threshold (Korf,
+// "Depth-first iterative-deepening: an optimal admissible tree search", 1985).
+// With an admissible h the first pass that finds a goal finds an optimal
+// solution.
+//
+// A pass lasts as long as its largest subtree (a chain of dependent pattern
+// reads per node), so the roots are many and near the leaves.  57-move
+// 15-puzzle, table capped at 2^18 slots: 189 ms with 2^18 roots of one depth
+// cut on the host (10 ms of them the cut), 162 / 86 / 64 with 2^18 / 2^20 / 2^21
+// cut here, 54 with 2^20 of a tree cut at the pass's threshold.
 #pragma once
 #include <cstdint>
 
@@ -19,14 +26,25 @@
 
 namespace uastar {
 
-// A root of the cut tree: its board (narrow keys use lo only), depth, the
-// move that reached it (+1, 0 for the start) and the moves from the start,
-// 2 bits each, first move in the lowest bits.
+// A root of the cut tree: its board (narrow keys use lo only), depth, aux word
+// (pattern parts and the move that reached it) and the moves from the start, 2
+// bits each, first move in the lowest bits.
 struct IdaRoot {
     unsigned long long lo, hi;
     uint32_t g;
-    uint32_t last;
+    uint32_t aux;
     unsigned long long prefix;
+};
+
+// The cut: the first depth with this many nodes, at most kIdaCutDepth (what a
+// prefix holds).
+constexpr uint32_t kIdaRoots = 1u << 20;
+constexpr uint32_t kIdaCutDepth = 32;
+struct IdaCut {
+    uint32_t count[kIdaCutDepth + 1];  // nodes per level; 0 past the last
+    uint32_t goal;                     // a goal's depth (0: none met)
+    uint32_t min_exceed;               // least f above the threshold
+    unsigned long long goal_prefix;    // the moves to the goal
 };
 
 constexpr uint32_t kIdaMaxMoves = 256;  // longest solution a pass records
@@ -48,6 +66,72 @@ template <class P> __device__ __forceinline__ typename P::Key ida_key(const IdaR
         return Key128{r.lo, r.hi};
     else
         return (uint64_t)r.lo;
+}
+
+// The start as the cut's first node.
+template <class P> __global__ void k_ida_start(P prob, IdaRoot *out) {
+    IdaRoot r;
+    if constexpr (P::kWide) {
+        r.lo = prob.start.lo;
+        r.hi = prob.start.hi;
+    } else {
+        r.lo = prob.start;
+        r.hi = 0;
+    }
+    r.g = 0;
+    r.aux = prob.start_aux();
+    r.prefix = 0;
+    *out = r;
+}
+
+// One level of the cut: the children of level d's nodes with f <= t, appended
+// to `out` in any order, unless level d is the last.
+template <class P>
+__global__ void __launch_bounds__(256) k_ida_cut(P prob, const IdaRoot *in, IdaRoot *out, uint32_t d, uint32_t t,
+                                                 IdaCut *cut) {
+    const uint32_t n = ldcg_u32(&cut->count[d]);
+    if (n == 0 || n >= kIdaRoots) return;
+    uint32_t minx = ~0u;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const IdaRoot r = in[i];
+        const typename P::Key key = ida_key<P>(r);
+        const uint32_t mask = prob.moves(key, r.aux);
+        typename P::Succ sc[4];
+        uint32_t naux[4], keep = 0;
+#pragma unroll
+        for (int mv = 0; mv < 4; ++mv) {
+            if (!(mask >> mv & 1u)) continue;
+            prob.succ_begin(key, d, r.aux, mv, sc[mv]);
+            uint64_t nf;
+            prob.succ_end(sc[mv], r.aux, mv, naux[mv], nf);
+            if (nf > t) {
+                minx = min(minx, (uint32_t)nf);
+                continue;
+            }
+            keep |= 1u << mv;
+            if (prob.is_goal(sc[mv].key) && atomicCAS(&cut->goal, 0u, d + 1) == 0u)
+                cut->goal_prefix = r.prefix | (unsigned long long)mv << (2 * d);
+        }
+        if (!keep) continue;
+        uint32_t at = atomicAdd(&cut->count[d + 1], (uint32_t)__popc(keep));
+#pragma unroll
+        for (int mv = 0; mv < 4; ++mv) {
+            if (!(keep >> mv & 1u)) continue;
+            IdaRoot c;
+            if constexpr (P::kWide) {
+                c.lo = sc[mv].key.lo;
+                c.hi = sc[mv].key.hi;
+            } else {
+                c.lo = sc[mv].key;
+                c.hi = 0;
+            }
+            c.g = d + 1;
+            c.aux = naux[mv];
+            c.prefix = r.prefix | (unsigned long long)mv << (2 * d);
+            out[at++] = c;
+        }
+    }
+    if (minx != ~0u) atomicMin(&cut->min_exceed, minx);
 }
 
 template <class P, int kMaxDepth>
@@ -72,18 +156,10 @@ __global__ void __launch_bounds__(128) k_ida_pass(P prob, const IdaRoot *roots, 
         const uint32_t i = atomicAdd(&out->next_root, 1u);
         if (i >= nroots) break;
         const IdaRoot r = roots[i];
-        P q = prob;
-        q.start = ida_key<P>(r);
-        const uint32_t a0 = q.start_aux() | (r.last << P::kLastMoveShift);
         const uint32_t g0 = r.g;
-        const uint32_t f0 = g0 + P::hsum(a0);
-        if (f0 > t) {
-            minx = min(minx, f0);
-            continue;
-        }
-        ks[0] = q.start;
-        as[0] = a0;
-        rem[0] = (uint8_t)prob.moves(ks[0], a0);
+        ks[0] = ida_key<P>(r);
+        as[0] = r.aux;
+        rem[0] = (uint8_t)prob.moves(ks[0], as[0]);
         int d = 0;
         while (d >= 0) {
             if (rem[d] == 0) {

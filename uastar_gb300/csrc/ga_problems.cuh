@@ -418,6 +418,7 @@ template <int N> struct PuzzleProblem : NarrowSlots {
         return a;
     }
     __device__ bool is_goal(uint64_t key) const { return key == goal; }
+    __host__ bool start_is_goal() const { return start == goal; }
     __device__ __forceinline__ uint64_t f_of(uint64_t, uint64_t g, uint32_t aux) const {
         return g + hsum(aux);
     }
@@ -609,6 +610,7 @@ template <> struct PuzzleProblem<5> : WideSlots {
         return part(0, start) | part(1, start) << 7 | part(2, start) << 14 | part(3, start) << 21;
     }
     __device__ bool is_goal(const Key128 &k) const { return k.lo == goal.lo && k.hi == goal.hi; }
+    __host__ bool start_is_goal() const { return start.lo == goal.lo && start.hi == goal.hi; }
     __device__ __forceinline__ uint64_t f_of(const Key128 &, uint64_t g, uint32_t aux) const { return g + hsum(aux); }
     // Blank moves 0..3 = DX/DY[0..3]; the move undoing the parent's is skipped.
     __device__ uint32_t moves(const Key128 &k, uint32_t aux) const {
