@@ -999,8 +999,8 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             *s_cnt = 0;
             *s_ins = 0;
             *s_ins2 = 0;
-            *s_room = 0;
             *s_pass = 0;
+            *s_room = 0;
         }
 
         // ------------------------------------------------ phase 1: pop ---
@@ -1077,8 +1077,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             }
             const uint32_t nexp = __ballot_sync(kFull, expands);
             if (lane == 0 && nexp) atomicAdd(&s_stat[0], (uint32_t)__popc(nexp));
-            // exclusive prefix of successor counts: within the warp here,
-            // warp offsets added after the barrier
+            // exclusive prefix of successor counts within the warp
             const uint32_t cnt = __popc(mv);
             uint32_t incl = cnt;
 #pragma unroll
@@ -1093,26 +1092,20 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             if (lane == 31) scratch[2 + (tid >> 5)] = incl;
         }
         __syncthreads();
-        uint64_t cmin = kInfCost;  // the CTA's minimum open f (thread 0)
-        uint32_t ctook = 0;
+        // the CTA's successors: warp by warp, each warp's in its pops' order
+        uint32_t total = 0;
+        for (uint32_t w = 0; w < owner_warps; ++w) total += scratch[2 + w];
         if (tid == 0) {
-            uint32_t acc = 0;
-            for (uint32_t w = 0; w < owner_warps; ++w) {
-                const uint32_t t = scratch[2 + w];
-                scratch[2 + w] = acc;
-                acc += t;
+            // into the team's round minimum, off the pop's path (before the barrier)
+            uint64_t cmin = wmins[0];
+            uint32_t ctook = wtook[0];
+            for (uint32_t w = 1; w < owner_warps; ++w) {
                 if (P::cost_cmp(wmins[w], cmin) < 0) cmin = wmins[w];
                 ctook += wtook[w];
             }
-            scratch[0] = acc;
+            if (cmin != kInfCost) atomic_min_cost<P>(&st->round_min[r3], cmin);
+            if (ctook) atomicAdd(&st->pops[r3], ctook);
         }
-        __syncthreads();
-        if (owner) pop[tid].excl += scratch[2 + (tid >> 5)];
-        const uint32_t total = scratch[0];
-        __syncthreads();
-        // into the team's round minimum, off the pop's path (before the barrier)
-        if (tid == 0 && cmin != kInfCost) atomic_min_cost<P>(&st->round_min[r3], cmin);
-        if (tid == 0 && ctook) atomicAdd(&st->pops[r3], ctook);
 
         // ------------------ phase 1: relax successors / refill heap roots ---
         // Owner chores of the round, while the other warps relax: refill the
@@ -1187,10 +1180,13 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
         if (relaxer) {
             Cand *const myreg = region(cta) + 1;
             const uint32_t rt = tid - rfirst;
-            // source pop of the CTA's successor j = largest h with excl[h] <= j
-            // (it has a successor)
-            const auto source = [&](uint32_t j) -> const PopInfo<Key> & {
-                uint32_t lo = 0, hi = H - 1;
+            // source pop of the CTA's successor j: its warp, then the largest h
+            // there with excl[h] <= j (it has a successor); j becomes the
+            // number of the successor among the pop's
+            const auto source = [&](uint32_t &j) -> const PopInfo<Key> & {
+                uint32_t w = 0;
+                for (; j >= scratch[2 + w]; ++w) j -= scratch[2 + w];
+                uint32_t lo = w * 32u, hi = min(lo + 31u, H - 1u);
                 while (lo < hi) {
                     const uint32_t mid = (lo + hi + 1) >> 1;
                     if (pop[mid].excl <= j)
@@ -1198,13 +1194,15 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                     else
                         hi = mid - 1;
                 }
+                j -= pop[lo].excl;
                 return pop[lo];
             };
             if constexpr (kSort) {
                 // every successor's record, at its number in the CTA's list
                 for (uint32_t j = rt; j < total; j += rthreads) {
-                    const PopInfo<Key> &pi = source(j);
-                    const int move = nth_bit(pi.mask, j - pi.excl);
+                    uint32_t q = j;
+                    const PopInfo<Key> &pi = source(q);
+                    const int move = nth_bit(pi.mask, q);
                     typename P::Succ sc;
                     prob.succ_begin(pi.key, pi.g, pi.aux, move, sc);
                     uint32_t naux;
@@ -1234,8 +1232,9 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                     uint32_t paux = 0, oslot = 0;
                     int move = 0;
                     if (act) {
-                        const PopInfo<Key> &pi = source(j);
-                        move = nth_bit(pi.mask, j - pi.excl);
+                        uint32_t q = j;
+                        const PopInfo<Key> &pi = source(q);
+                        move = nth_bit(pi.mask, q);
                         oslot = pi.slot;
                         pkey = pi.key;
                         pg = pi.g;
@@ -1288,7 +1287,9 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                         if (ib && lane == (uint32_t)(__ffs(ib) - 1)) atomicAdd(s_ins, (uint32_t)__popc(ib));
                         // nodes to continue: as many (in lane order) as have at
                         // most 32 successors together, if the CTA's candidate
-                        // region has room for all of those beside the pops'
+                        // region has room for all of those beside the pops' (a
+                        // share per warp left the long chains without: 31 k ->
+                        // 38 k steps on the 20000^2 grid)
                         uint32_t n_next = 0, incl = 0;
                         bool go = false;
                         if (__any_sync(kFull, cand)) {
