@@ -17,6 +17,7 @@
 #include "ga_search.cuh"
 #include "ga_grow.cuh"
 #include "ga_ida.cuh"
+#include "ga_walk.cuh"
 
 using namespace uastar;
 
@@ -28,6 +29,19 @@ __global__ void k_fill_ff(uint4 *p, size_t n16) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n16;
          i += (size_t)gridDim.x * blockDim.x)
         p[i] = v;
+}
+
+// A plain solve's memory before its first round: empty table and heaps, fresh
+// team state.  Bound by the table's bytes (8.6 GB: 1.29 ms, 6.7 TB/s); one launch
+// instead of a fill, a memset and a copy, and the walk queued behind the search
+// (run_plain), take four trips to the driver and one wait off a solve: 61 x 67
+// 340 -> 306 us, an 8-puzzle 134 -> 115 us.
+__global__ void k_plain_reset(uint4 *tab, size_t n16, uint32_t *heap_size, uint32_t k, TeamState *st) {
+    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    if (t == 0) team_state_init(st);
+    for (size_t i = t; i < k; i += step) heap_size[i] = 0;
+    const uint4 v = make_uint4(~0u, ~0u, ~0u, ~0u);
+    for (size_t i = t; i < n16; i += step) tab[i] = v;
 }
 
 template <class P, bool kSort = false>
@@ -109,35 +123,58 @@ __global__ void __launch_bounds__(512, 1) k_round_floor(TeamState *st, uint64_t 
 
 // Walk the prev chain from the goal slot (one thread: a pointer chase).
 // Writes keys goal -> start; *len = count, or cap + 1 when truncated.
-__global__ void k_walk(const Slot *tab, uint32_t goal_slot, unsigned long long *keys,
-                       uint64_t cap, unsigned long long *len, int link) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+__device__ void walk_boards_dev(const Slot *tab, uint32_t goal_slot, unsigned long long *keys, uint64_t cap,
+                                unsigned long long *len) {
     uint32_t s = goal_slot;
     uint64_t n = 0;
     while (s != kNone && n < cap) {
         uint64_t key;
         uint32_t prev;
-        slot_key_prev(tab + s, link, key, prev);
+        slot_key_prev(tab + s, PuzzleProblem<4>::kLink, key, prev);
         keys[n++] = key;
         s = prev;
     }
     *len = (s != kNone) ? cap + 1 : n;
 }
-
 // The same walk for 16-byte keys: two words (lo, hi) per board.
-__global__ void k_walk_wide(const Slot *tab, uint32_t goal_slot, unsigned long long *keys, uint64_t cap,
-                            unsigned long long *len) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+__device__ void walk_boards_dev(const WideSlot *tab, uint32_t goal_slot, unsigned long long *keys, uint64_t cap,
+                                unsigned long long *len) {
     uint32_t s = goal_slot;
     uint64_t n = 0;
     while (s != kNone && n < cap) {
-        const WideSlot *w = WideSlots::w(tab + s);
+        const WideSlot *w = tab + s;
         keys[2 * n] = __ldcg(&w->lo);
         keys[2 * n + 1] = __ldcg(&w->hi);
         ++n;
         s = __ldcg(&w->prev);
     }
     *len = (s != kNone) ? cap + 1 : n;
+}
+template <class S>
+__global__ void k_walk(const S *tab, uint32_t goal_slot, unsigned long long *keys, uint64_t cap,
+                       unsigned long long *len) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) walk_boards_dev(tab, goal_slot, keys, cap, len);
+}
+
+// The walk of a search that may have ended just before on the stream: nothing
+// unless it solved its problem.
+template <class S>
+__global__ void k_walk_solved(const S *tab, const TeamState *st, unsigned long long *keys, uint64_t cap,
+                              unsigned long long *len) {
+    if (blockIdx.x != 0 || threadIdx.x != 0 || ldcg_u32(&st->status) != ST_OK) return;
+    walk_boards_dev(tab, ldcg_u32(&st->goal_slot), keys, cap, len);
+}
+// The grid's (ga_walk.cuh); nothing either if the path has more than cap cells.
+__global__ void __launch_bounds__(1024) k_walk_grid_solved(GridProblem prob, const Slot *tab, uint64_t mask,
+                                                           const TeamState *st, int32_t *cells, uint64_t cap,
+                                                           unsigned long long *len) {
+    __shared__ GridWalkSmem s;
+    if (ldcg_u32(&st->status) != ST_OK) return;
+    const uint64_t g = ldcg_u64(&st->goal_best);
+    if ((g >> 32) + (g & 0xffffffffull) + 1 > cap) return;
+    const unsigned long long n = walk_grid(tab, mask, prob, ldcg_u32(&st->goal_slot), cap, s,
+                                           [&](unsigned long long i, uint32_t cell) { cells[i] = (int32_t)cell; });
+    if (threadIdx.x == 0) *len = n;
 }
 
 int32_t fill_ff_async(uastar_engine *eng, void *p, size_t bytes, cudaStream_t stream) {
@@ -196,7 +233,19 @@ struct PlainOut {
     int grows;         // in-place table growths
     SearchMem<PuzzleEntry> mem;  // the last attempt's memory (puzzle solves; used by the bounded mode)
     uint32_t k;        // heaps
+    // what the caller's tail had copied from behind the team state, in the
+    // engine's pinned buffer
+    const unsigned char *tail = nullptr;
 };
+
+// What follows the search of a plain solve on the stream: nothing.
+struct NoTail {
+    static constexpr size_t bytes = 0;
+    template <class M> void operator()(const M &, const TeamState *, unsigned char *) const {}
+};
+// Device and pinned buffer: the team state, then a tail's bytes.
+constexpr size_t kTailAt = 512;
+static_assert(sizeof(TeamState) <= kTailAt, "the tail starts behind the team state");
 
 // Run one instance with the whole GPU as the team.  Grows the dedup table /
 // heaps and retries when they overflow and were auto-sized.
@@ -270,9 +319,12 @@ bool grow_table(uastar_engine *eng, SearchMem<typename P::Entry> &m, uint32_t k,
 // max_log2 > 0 caps the dedup table at 2^max_log2 slots (the memory-bounded
 // mode): a search that fills it pauses near its load limit at a round
 // boundary and returns with status ST_RUNNING, its heaps and table intact.
-template <class P>
+// `tail` enqueues what is to run behind each search launch (a path walk that
+// looks at the team state itself) and its `bytes` come back with the state in
+// one copy, so that a solved search needs no second trip to the host.
+template <class P, class Tail = NoTail>
 int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t stride_auto,
-                  PlainOut *out, int max_log2 = 0) {
+                  PlainOut *out, int max_log2 = 0, const Tail &tail = Tail()) {
     using E = typename P::Entry;
     const uastar_config &c = eng->cfg;
     const uint32_t block = (uint32_t)c.block_threads;
@@ -361,19 +413,17 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
         if (e != cudaSuccess) return fail_cuda(eng, e, "alloc heaps");
         if ((e = eng->heap_size.ensure((size_t)k * 4)) != cudaSuccess) return fail_cuda(eng, e, "alloc heap sizes");
         if ((e = eng->cand.ensure(cand_b)) != cudaSuccess) return fail_cuda(eng, e, "alloc candidates");
-        if ((e = eng->team.ensure(sizeof(TeamState))) != cudaSuccess) return fail_cuda(eng, e, "alloc state");
+        if ((e = eng->team.ensure(kTailAt + tail.bytes)) != cudaSuccess) return fail_cuda(eng, e, "alloc state");
+        if ((e = eng->pin(kTailAt + tail.bytes)) != cudaSuccess) return fail_cuda(eng, e, "alloc host state");
         const uint64_t sort_n = (uint64_t)k * P::kMoves;  // a round's successors at most
         if (sorted && (e = eng->sortb.ensure(2 * sort_n * 8 + 256ull * (nblocks + 1) * 4)) != cudaSuccess)
             return fail_cuda(eng, e, "alloc sort buffers");
 
-        int32_t rc = fill_ff(eng, eng->tab.p, tab_b);
-        if (rc) return rc;
-        if ((e = cudaMemsetAsync(eng->heap_size.p, 0, (size_t)k * 4, eng->stream)) != cudaSuccess)
-            return fail_cuda(eng, e, "memset");
-        TeamState init = fresh_team_state();
-        if ((e = cudaMemcpyAsync(eng->team.p, &init, sizeof init, cudaMemcpyHostToDevice, eng->stream)) !=
-            cudaSuccess)
-            return fail_cuda(eng, e, "state upload");
+        TeamState *st = eng->team.as<TeamState>();
+        k_plain_reset<<<std::max(1, eng->sms * 8), 256, 0, eng->stream>>>(eng->tab.as<uint4>(), tab_b / 16,
+                                                                          eng->heap_size.as<uint32_t>(), k, st);
+        eng->launches++;
+        if ((e = cudaGetLastError()) != cudaSuccess) return fail_cuda(eng, e, "reset");
 
         SearchMem<E> m;
         m.tab = eng->tab.as<Slot>();
@@ -416,7 +466,6 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
             return m.max_inserted > round_max ? m.max_inserted - round_max : 0ull;
         };
         m.grow_at = auto_table ? pause_point(slots) : ~0ull;
-        TeamState *st = eng->team.as<TeamState>();
         uint64_t timeout_ns = (uint64_t)(c.wait_timeout_s * 1e9);
         P pr = prob;
         uint32_t h_arg = H;
@@ -427,10 +476,14 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
             if (e != cudaSuccess) return fail_cuda(eng, e, "cooperative launch");
             eng->launches++;
             cudaEventRecord(eng->ev1, eng->stream);
-            if ((e = cudaMemcpyAsync(&out->st, st, sizeof(TeamState), cudaMemcpyDeviceToHost, eng->stream)) !=
+            tail(m, st, eng->team.as<unsigned char>() + kTailAt);
+            if ((e = cudaGetLastError()) != cudaSuccess) return fail_cuda(eng, e, "walk launch");
+            if ((e = cudaMemcpyAsync(eng->h_pin, st, kTailAt + tail.bytes, cudaMemcpyDeviceToHost, eng->stream)) !=
                 cudaSuccess)
                 return fail_cuda(eng, e, "state download");
             if ((e = cudaStreamSynchronize(eng->stream)) != cudaSuccess) return fail_cuda(eng, e, "search");
+            std::memcpy(&out->st, eng->h_pin, sizeof(TeamState));
+            out->tail = eng->h_pin + kTailAt;
             float ms = 0;
             cudaEventElapsedTime(&ms, eng->ev0, eng->ev1);
             out->kernel_ms += ms;
@@ -471,72 +524,95 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
     return UASTAR_OK;
 }
 
-int32_t walk_keys(uastar_engine *eng, uint32_t goal_slot, uint64_t cap, std::vector<uint64_t> *keys, int link) {
-    cudaError_t e;
-    const size_t need = (size_t)cap * 8 + 64;
-    if ((e = eng->walk.ensure(need)) != cudaSuccess) return fail_cuda(eng, e, "alloc walk");
-    unsigned long long *d_keys = eng->walk.as<unsigned long long>();
-    unsigned long long *d_len = d_keys + cap;
-    k_walk<<<1, 32, 0, eng->stream>>>(eng->tab.as<Slot>(), goal_slot, d_keys, cap, d_len, link);
-    eng->launches++;
-    if ((e = cudaGetLastError()) != cudaSuccess) return fail_cuda(eng, e, "walk launch");
-    unsigned long long len = 0;
-    if (cap <= 8192) {
-        // short walks (puzzles): the whole buffer and its length in one copy
-        std::vector<uint64_t> all(cap + 1);
-        if ((e = cudaMemcpyAsync(all.data(), d_keys, (cap + 1) * 8, cudaMemcpyDeviceToHost, eng->stream)) !=
-                cudaSuccess ||
-            (e = cudaStreamSynchronize(eng->stream)) != cudaSuccess)
-            return fail_cuda(eng, e, "walk");
-        len = all[cap];
-        if (len > cap) {
-            eng->set_err("solution path longer than the walk buffer");
-            return UASTAR_ARENA_FULL;
-        }
-        keys->assign(all.begin(), all.begin() + (ptrdiff_t)len);
-        std::reverse(keys->begin(), keys->end());
-        return UASTAR_OK;
+// Tails (run_plain): the path's length, then its cells or boards, goal first.
+struct GridTail {
+    GridProblem prob;
+    uint64_t cap;
+    size_t bytes;
+    GridTail(const GridProblem &p, uint64_t c) : prob(p), cap(c), bytes(16 + (size_t)c * 4) {}
+    void operator()(const SearchMem<GridEntry> &m, const TeamState *st, unsigned char *at) const {
+        k_walk_grid_solved<<<1, 1024, 0, eng->stream>>>(prob, m.tab, m.mask, st, reinterpret_cast<int32_t *>(at + 16),
+                                                       cap, reinterpret_cast<unsigned long long *>(at));
+        eng->launches++;
     }
-    if ((e = cudaMemcpyAsync(&len, d_len, 8, cudaMemcpyDeviceToHost, eng->stream)) != cudaSuccess)
-        return fail_cuda(eng, e, "walk length");
-    if ((e = cudaStreamSynchronize(eng->stream)) != cudaSuccess) return fail_cuda(eng, e, "walk");
-    if (len > cap) {
+    uastar_engine *eng = nullptr;
+};
+template <int N> struct PuzzleTail {
+    static constexpr uint64_t cap = 256;  // boards
+    static constexpr size_t words = N == 5 ? 2 : 1;
+    static constexpr size_t bytes = 16 + cap * words * 8;
+    void operator()(const SearchMem<PuzzleEntry> &m, const TeamState *st, unsigned char *at) const {
+        auto *len = reinterpret_cast<unsigned long long *>(at), *boards = len + 2;
+        if constexpr (N == 5)
+            k_walk_solved<WideSlot><<<1, 32, 0, eng->stream>>>(eng->tab.as<WideSlot>(), st, boards, cap, len);
+        else
+            k_walk_solved<Slot><<<1, 32, 0, eng->stream>>>(m.tab, st, boards, cap, len);
+        eng->launches++;
+    }
+    uastar_engine *eng = nullptr;
+};
+
+// The path of a solved grid search whose tail had no room for it, goal first.
+int32_t walk_grid_long(uastar_engine *eng, const GridProblem &prob, uint64_t mask, uint64_t n, uint64_t cap,
+                       std::vector<int32_t> *cells) {
+    cudaError_t e;
+    if (n > cap) {
         eng->set_err("solution path longer than the walk buffer");
         return UASTAR_ARENA_FULL;
     }
-    keys->resize(len);
-    if (len && (e = cudaMemcpyAsync(keys->data(), d_keys, len * 8, cudaMemcpyDeviceToHost, eng->stream)) !=
-                   cudaSuccess)
-        return fail_cuda(eng, e, "walk keys");
-    if ((e = cudaStreamSynchronize(eng->stream)) != cudaSuccess) return fail_cuda(eng, e, "walk copy");
-    std::reverse(keys->begin(), keys->end());
+    if ((e = eng->walk.ensure(16 + (size_t)n * 4)) != cudaSuccess) return fail_cuda(eng, e, "alloc walk");
+    unsigned char *at = eng->walk.as<unsigned char>();
+    k_walk_grid_solved<<<1, 1024, 0, eng->stream>>>(prob, eng->tab.as<Slot>(), mask, eng->team.as<TeamState>(),
+                                                   reinterpret_cast<int32_t *>(at + 16), n,
+                                                   reinterpret_cast<unsigned long long *>(at));
+    eng->launches++;
+    if ((e = cudaGetLastError()) != cudaSuccess) return fail_cuda(eng, e, "walk launch");
+    unsigned long long len = 0;
+    cells->resize(n);
+    if ((e = cudaMemcpyAsync(&len, at, 8, cudaMemcpyDeviceToHost, eng->stream)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(cells->data(), at + 16, n * 4, cudaMemcpyDeviceToHost, eng->stream)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(eng->stream)) != cudaSuccess)
+        return fail_cuda(eng, e, "walk");
+    if (len != n) {
+        eng->set_err("solution path of another length than its cost");
+        return UASTAR_CUDA_ERROR;
+    }
     return UASTAR_OK;
 }
 
-// Boards goal -> start of a 16-byte-key search, reversed to start -> goal.
-int32_t walk_keys_wide(uastar_engine *eng, uint32_t goal_slot, uint64_t cap, std::vector<Key128> *keys) {
+// Boards start -> `slot` of a puzzle search's table, as key words (two per
+// board on 5x5).
+template <int N>
+int32_t walk_keys(uastar_engine *eng, uint32_t slot, std::vector<uint64_t> *keys) {
+    using T = PuzzleTail<N>;
+    constexpr uint64_t cap = 4096;
     cudaError_t e;
-    if ((e = eng->walk.ensure((size_t)cap * 16 + 64)) != cudaSuccess) return fail_cuda(eng, e, "alloc walk");
-    unsigned long long *d_keys = eng->walk.as<unsigned long long>();
-    unsigned long long *d_len = d_keys + 2 * cap;
-    k_walk_wide<<<1, 32, 0, eng->stream>>>(eng->tab.as<Slot>(), goal_slot, d_keys, cap, d_len);
+    if ((e = eng->walk.ensure(16 + cap * T::words * 8)) != cudaSuccess) return fail_cuda(eng, e, "alloc walk");
+    unsigned char *at = eng->walk.as<unsigned char>();
+    auto *len = reinterpret_cast<unsigned long long *>(at), *boards = len + 2;
+    if constexpr (N == 5)
+        k_walk<WideSlot><<<1, 32, 0, eng->stream>>>(eng->tab.as<WideSlot>(), slot, boards, cap, len);
+    else
+        k_walk<Slot><<<1, 32, 0, eng->stream>>>(eng->tab.as<Slot>(), slot, boards, cap, len);
     eng->launches++;
     if ((e = cudaGetLastError()) != cudaSuccess) return fail_cuda(eng, e, "walk launch");
-    unsigned long long len = 0;
-    if ((e = cudaMemcpyAsync(&len, d_len, 8, cudaMemcpyDeviceToHost, eng->stream)) != cudaSuccess)
-        return fail_cuda(eng, e, "walk length");
-    if ((e = cudaStreamSynchronize(eng->stream)) != cudaSuccess) return fail_cuda(eng, e, "walk");
-    if (len > cap) {
+    std::vector<uint64_t> all(2 + cap * T::words);
+    if ((e = cudaMemcpyAsync(all.data(), at, all.size() * 8, cudaMemcpyDeviceToHost, eng->stream)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(eng->stream)) != cudaSuccess)
+        return fail_cuda(eng, e, "walk");
+    if (all[0] > cap) {
         eng->set_err("solution path longer than the walk buffer");
         return UASTAR_ARENA_FULL;
     }
-    keys->resize(len);
-    if (len && (e = cudaMemcpyAsync(keys->data(), d_keys, len * 16, cudaMemcpyDeviceToHost, eng->stream)) !=
-                   cudaSuccess)
-        return fail_cuda(eng, e, "walk keys");
-    if ((e = cudaStreamSynchronize(eng->stream)) != cudaSuccess) return fail_cuda(eng, e, "walk copy");
-    std::reverse(keys->begin(), keys->end());
+    keys->clear();
+    for (uint64_t b = all[0]; b-- > 0;)
+        for (size_t w = 0; w < T::words; ++w) keys->push_back(all[2 + b * T::words + w]);
     return UASTAR_OK;
+}
+
+// Cell of the blank on the board at kw.
+template <int N> int board_blank(const uint64_t *kw) {
+    return N == 5 ? (int)PuzzleProblem<5>::cell(Key128{kw[0], N == 5 ? kw[1] : 0}, 0) : key_blank(kw[0]);
 }
 
 int32_t grid_load_impl(uastar_engine *eng, const uint64_t *words, int32_t H, int32_t W) {
@@ -586,8 +662,12 @@ int32_t grid_solve_impl(uastar_engine *eng, const uint64_t *host_words, int32_t 
     const int log2_auto = std::min(28, std::max(20, ceil_log2_u64(cells) - 1));
     const uint32_t per_heap =
         (uint32_t)std::min<uint64_t>(8192, std::max<uint64_t>(64, 4 * cells / plain_heaps<GridProblem>(eng->cfg)));
+    // room for the path beside the result: a few times the straight way
+    // across, at most 128 KB (a longer path is walked after it)
+    GridTail tail(prob, std::min<uint64_t>(32768, std::min<uint64_t>(cells, 2ull * ((uint64_t)H + W) + 256)));
+    tail.eng = eng;
     PlainOut po;
-    int32_t rc = run_plain(eng, prob, log2_auto, next_pow2_u32(per_heap), &po);
+    int32_t rc = run_plain(eng, prob, log2_auto, next_pow2_u32(per_heap), &po, 0, tail);
     if (rc) return out->status = rc;
     const TeamState &st = po.st;
     out->status = (int32_t)st.status;
@@ -609,15 +689,25 @@ int32_t grid_solve_impl(uastar_engine *eng, const uint64_t *host_words, int32_t 
         eng->lsy = sy;
         eng->lex = ex;
         eng->ley = ey;
-        // Path: walk prev pointers on the device, re-validate on the host.
-        std::vector<uint64_t> keys;
+        // Path: walked on the device (goal first), re-validated on the host.
+        const uint64_t n = (uint64_t)out->straight + (uint64_t)out->diagonal + 1;
         const uint64_t cap = std::min<uint64_t>(cells + 1, 1ull << 26);
-        rc = walk_keys(eng, st.goal_slot, cap, &keys, GridProblem::kLink);
-        if (rc) return out->status = rc;
-        eng->path.assign(keys.size(), 0);
-        for (size_t i = 0; i < keys.size(); ++i) eng->path[i] = (int32_t)keys[i];
+        std::vector<int32_t> far;
+        const int32_t *walked = reinterpret_cast<const int32_t *>(po.tail + 16);
+        unsigned long long got = 0;
+        std::memcpy(&got, po.tail, 8);
+        if (n > tail.cap) {
+            rc = walk_grid_long(eng, prob, po.slots - 1, n, cap, &far);
+            if (rc) return out->status = rc;
+            walked = far.data();
+        } else if (got != n) {
+            eng->set_err("solution path of another length than its cost");
+            return out->status = UASTAR_CUDA_ERROR;
+        }
+        eng->path.resize(n);
+        for (uint64_t i = 0; i < n; ++i) eng->path[i] = walked[n - 1 - i];
         eng->path_cached = true;
-        out->path_len = (int64_t)keys.size();
+        out->path_len = (int64_t)n;
         // float32 g accumulated along the path in order, as the reference's
         // CPU solver computes it (CPU-solver.cpp:105)
         {
@@ -659,46 +749,45 @@ bool board_ok(int n, const uint8_t *tiles) {
     return true;
 }
 
+// `keys`: the boards of the solution, start first (see walk_keys).
 template <int N>
-int32_t puzzle_solve_n(uastar_engine *eng, const uint8_t *tiles, PlainOut *po) {
+int32_t puzzle_solve_n(uastar_engine *eng, const uint8_t *tiles, PlainOut *po, std::vector<uint64_t> *keys) {
     PuzzleProblem<N> prob;
     prob.pdb = eng->pdb[N].as<uint8_t>();
-    prob.start = pack_board(N, tiles);
+    if constexpr (N == 5)
+        prob.start = PuzzleProblem<5>::pack(tiles);
+    else
+        prob.start = pack_board(N, tiles);
     prob.goal = PuzzleProblem<N>::goal_key();
-    const int log2_start = eng->puzzle_log2_start > 0 ? eng->puzzle_log2_start : (N == 3 ? 20 : 22);
-    return run_plain(eng, prob, log2_start, N == 3 ? 1024 : 16383, po);
-}
-
-// 5x5: 16-byte keys (PuzzleProblem<5>)
-template <>
-int32_t puzzle_solve_n<5>(uastar_engine *eng, const uint8_t *tiles, PlainOut *po) {
-    PuzzleProblem<5> prob;
-    prob.pdb = eng->pdb[5].as<uint8_t>();
-    prob.start = PuzzleProblem<5>::pack(tiles);
-    prob.goal = PuzzleProblem<5>::goal_key();
-    return run_plain(eng, prob, 22, 16383, po);
+    const int log2_start = N < 5 && eng->puzzle_log2_start > 0 ? eng->puzzle_log2_start : (N == 3 ? 20 : 22);
+    PuzzleTail<N> tail;
+    tail.eng = eng;
+    if (int32_t rc = run_plain(eng, prob, log2_start, N == 3 ? 1024 : 16383, po, 0, tail)) return rc;
+    if (po->st.status != ST_OK) return UASTAR_OK;
+    const uint64_t *t = reinterpret_cast<const uint64_t *>(po->tail);
+    if (t[0] > tail.cap) return walk_keys<N>(eng, po->st.goal_slot, keys);
+    keys->clear();
+    for (uint64_t b = t[0]; b-- > 0;)
+        for (size_t w = 0; w < tail.words; ++w) keys->push_back(t[2 + b * tail.words + w]);
+    return UASTAR_OK;
 }
 
 // Boards (tiles per cell) along the prev chain ending at `slot`, start first.
 template <int N>
 int32_t walk_boards(uastar_engine *eng, uint32_t slot, std::vector<std::vector<uint8_t>> *boards) {
     boards->clear();
-    if constexpr (N == 5) {
-        std::vector<Key128> keys;
-        if (int32_t rc = walk_keys_wide(eng, slot, 4096, &keys)) return rc;
-        for (const Key128 &k : keys) {
-            std::vector<uint8_t> b(25);
-            for (int t = 0; t < 25; ++t) b[PuzzleProblem<5>::cell(k, t)] = (uint8_t)t;
-            boards->push_back(b);
+    std::vector<uint64_t> keys;
+    if (int32_t rc = walk_keys<N>(eng, slot, &keys)) return rc;
+    constexpr size_t words = PuzzleTail<N>::words;
+    for (size_t i = 0; i < keys.size(); i += words) {
+        std::vector<uint8_t> b(N * N);
+        for (int t = 0; t < N * N; ++t) {
+            if constexpr (N == 5)
+                b[PuzzleProblem<5>::cell(Key128{keys[i], keys[i + 1]}, t)] = (uint8_t)t;
+            else
+                b[(keys[i] >> (4 * t)) & 15] = (uint8_t)t;
         }
-    } else {
-        std::vector<uint64_t> keys;
-        if (int32_t rc = walk_keys(eng, slot, 4096, &keys, PuzzleProblem<4>::kLink)) return rc;
-        for (uint64_t k : keys) {
-            std::vector<uint8_t> b(N * N);
-            for (int t = 0; t < N * N; ++t) b[(k >> (4 * t)) & 15] = (uint8_t)t;
-            boards->push_back(b);
-        }
+        boards->push_back(b);
     }
     return UASTAR_OK;
 }
@@ -962,8 +1051,9 @@ void uastar_destroy(uastar_engine *eng) {
                       &eng->tab_next, &eng->grow_map, &eng->sortb,
                       &eng->bitmap, &eng->b_desc, &eng->b_out, &eng->b_queue, &eng->b_bitmaps,
                       &eng->b_tab, &eng->b_heaps, &eng->b_hsize, &eng->b_cand, &eng->b_walk,
-                      &eng->b_walklen, &eng->b_cstate, &eng->b_cnext})
+                      &eng->b_walklen, &eng->b_cstate, &eng->b_cnext, &eng->ida})
         b->release();
+    if (eng->h_pin) cudaFreeHost(eng->h_pin);
     for (auto &b : eng->pdb) b.release();
     for (auto &kv : eng->b_graphs) cudaGraphExecDestroy(kv.second);
     if (eng->ev0) cudaEventDestroy(eng->ev0);
@@ -1154,9 +1244,10 @@ int32_t uastar_puzzle_solve(uastar_engine *eng, int32_t n, const uint8_t *tiles,
         return out->status;
     }
     PlainOut po;
-    int32_t rc = n == 3   ? puzzle_solve_n<3>(eng, tiles, &po)
-                 : n == 4 ? puzzle_solve_n<4>(eng, tiles, &po)
-                          : puzzle_solve_n<5>(eng, tiles, &po);
+    std::vector<uint64_t> keys;
+    int32_t rc = n == 3   ? puzzle_solve_n<3>(eng, tiles, &po, &keys)
+                 : n == 4 ? puzzle_solve_n<4>(eng, tiles, &po, &keys)
+                          : puzzle_solve_n<5>(eng, tiles, &po, &keys);
     if (rc) return out->status = rc;
     const TeamState &st = po.st;
     out->status = (int32_t)st.status;
@@ -1171,17 +1262,8 @@ int32_t uastar_puzzle_solve(uastar_engine *eng, int32_t n, const uint8_t *tiles,
         out->steps = (int32_t)st.goal_best;
         eng->path.clear();
         std::vector<int> blanks;  // blank cell of each board, start -> goal
-        if (n == 5) {
-            std::vector<Key128> keys;
-            rc = walk_keys_wide(eng, st.goal_slot, 4096, &keys);
-            if (rc) return out->status = rc;
-            for (const Key128 &k : keys) blanks.push_back((int)PuzzleProblem<5>::cell(k, 0));
-        } else {
-            std::vector<uint64_t> keys;
-            rc = walk_keys(eng, st.goal_slot, 4096, &keys, PuzzleProblem<4>::kLink);
-            if (rc) return out->status = rc;
-            for (uint64_t k : keys) blanks.push_back(key_blank(k));
-        }
+        for (size_t i = 0; i < keys.size(); i += n == 5 ? 2 : 1)
+            blanks.push_back(n == 5 ? board_blank<5>(&keys[i]) : board_blank<4>(&keys[i]));
         for (size_t i = 1; i < blanks.size(); ++i) {
             const int d = blanks[i] - blanks[i - 1];
             eng->path.push_back(d == n ? 0 : d == -n ? 1 : d == 1 ? 2 : 3);

@@ -95,6 +95,17 @@ struct uastar_engine {
     // already filled a cluster's partition or round budget
     int puzzle_log2_start = 0;
     uastar::DevBuf sortb;               // per-round successor sort (dedup = 1), uastar_sort_keys
+    unsigned char *h_pin = nullptr;     // pinned host mirror of `team` (a solve's state and path)
+    size_t h_pin_bytes = 0;
+    cudaError_t pin(size_t need) {
+        if (need <= h_pin_bytes) return cudaSuccess;
+        if (h_pin) cudaFreeHost(h_pin);
+        h_pin = nullptr;
+        h_pin_bytes = 0;
+        const cudaError_t e = cudaMallocHost(&h_pin, need);
+        if (e == cudaSuccess) h_pin_bytes = need;
+        return e;
+    }
     uastar::DevBuf ida;                 // memory-bounded mode: IDA* roots and pass state
     // launch-configuration queries of the plain engine, made once per shape:
     // the dynamic shared memory limit set per kernel, and co-resident CTAs

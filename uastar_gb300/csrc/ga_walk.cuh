@@ -1,0 +1,130 @@
+// Reading a path out of a finished grid search: the prev chain from the goal
+// to the start, by one CTA.
+//
+// Followed link by link, the chain is one dependent table read per cell (0.44 us
+// each, 9.8 ms on the 20000^2 grid's 22 293 cells).  But the next cell is one of
+// the eight neighbours, so the CTA looks up a whole window of cells around the
+// current one at once (each by its own hash), finds every cell's parent among
+// its neighbours in shared memory, and one thread then follows the chain there
+// until it leaves the window.  The window lies on the side of the start, so a
+// path that makes its way there stays in it for ~27 cells, at the price of
+// about two memory trips.  Bound by these trips and the chain in shared memory
+// (45 cycles a cell).  Walks of 1000^2, 700 x 1021 and 20000^2 cells: 490 -> 153,
+// 390 -> 116 and 9800 -> 3130 us.  Windows 64 wide took 215 us at 1000^2 where
+// these, not yet trimmed, took 170: four times the look-ups, half of them for
+// nothing.
+#pragma once
+#include <cstdint>
+
+#include "ga_device.cuh"
+#include "ga_problems.cuh"
+
+namespace uastar {
+
+struct GridWalkSmem {
+    static constexpr uint32_t kSide = 32, kCells = kSide * kSide;
+    static constexpr uint32_t kAhead = kSide - 5;  // cells of the window towards the start
+    static constexpr uint16_t kOut = 0xFFFF, kEnd = 0xFFFE;
+    uint32_t slot[kCells], prev[kCells];  // the cell's slot (kNone: not in the table) and its parent's
+    uint16_t next[kCells];                // its parent's place in the window, kOut or kEnd
+    uint16_t chain[kCells];               // the chain's places in the window, from its first cell on
+    uint32_t links;                       // cells of it before the last
+    uint16_t last;                        // the last one's next: kOut or kEnd
+};
+
+// Slot and parent slot of a cell; kNone if the table does not hold it.  Most
+// cells are in their home slot or have it free: the other three of a line are
+// read only for the rest (each is a memory sector of its own).
+__device__ __forceinline__ void find_cell(const Slot *tab, uint64_t mask, uint32_t cell, uint32_t &slot,
+                                          uint32_t &prev) {
+    const uint64_t home = mix64(cell) & mask;
+    slot = prev = kNone;
+    for (uint64_t i = 0; i <= mask; ++i) {
+        const uint64_t at = probe_slot(home, i, mask);
+        const unsigned long long w = __ldcg(&tab[at].key);
+        if (w == kEmptyKey) return;
+        if ((uint32_t)w == cell) {
+            slot = (uint32_t)at;
+            prev = (uint32_t)(w >> 32);
+            return;
+        }
+    }
+}
+
+// Calls store(i, cell) for the i-th cell of the chain from `goal_slot`, at most
+// `cap` of them, each on some thread of the first warp; returns their number,
+// or cap + 1 if the chain is longer.  All threads of the CTA call it and get
+// the result.
+template <class Store>
+__device__ unsigned long long walk_grid(const Slot *tab, uint64_t mask, const GridProblem &prob, uint32_t goal_slot,
+                                        uint64_t cap, GridWalkSmem &s, Store &&store) {
+    constexpr int kSide = (int)GridWalkSmem::kSide;
+    constexpr uint32_t kCells = GridWalkSmem::kCells;
+    const uint32_t tid = threadIdx.x, T = blockDim.x;
+    const uint32_t goal = (uint32_t)__ldcg(&tab[goal_slot].key);
+    int cx = (int)prob.row_of(goal), cy = (int)(goal - (uint32_t)cx * (uint32_t)prob.W);
+    // n cells lie before (cx, cy), the first of the window's part of the chain
+    for (unsigned long long n = 0;;) {
+        const auto first = [](int at, int to) {
+            return at - (to < at ? (int)GridWalkSmem::kAhead : to > at ? kSide - 1 - (int)GridWalkSmem::kAhead : kSide / 2);
+        };
+        const int x0 = first(cx, prob.sx), y0 = first(cy, prob.sy);
+        for (uint32_t w = tid; w < kCells; w += T) {
+            const int x = x0 + (int)(w / kSide), y = y0 + (int)(w % kSide);
+            uint32_t slot = kNone, prev = kNone;
+            if (x >= 0 && x < prob.H && y >= 0 && y < prob.W)
+                find_cell(tab, mask, (uint32_t)x * (uint32_t)prob.W + (uint32_t)y, slot, prev);
+            s.slot[w] = slot;
+            s.prev[w] = prev;
+        }
+        __syncthreads();
+        for (uint32_t w = tid; w < kCells; w += T) {
+            const uint32_t prev = s.prev[w];
+            uint16_t to = prev == kNone ? GridWalkSmem::kEnd : GridWalkSmem::kOut;
+            if (prev != kNone) {
+                const int lx = (int)(w / kSide), ly = (int)(w % kSide);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int px = lx + GridProblem::c_dx(i), py = ly + GridProblem::c_dy(i);
+                    if (px < 0 || px >= kSide || py < 0 || py >= kSide) continue;
+                    if (s.slot[px * kSide + py] == prev) to = (uint16_t)(px * kSide + py);
+                }
+            }
+            s.next[w] = to;
+        }
+        __syncthreads();
+        if (tid < 32) {
+            if (tid == 0) {
+                uint32_t at = (uint32_t)((cx - x0) * kSide + (cy - y0)), k = 0;
+                for (;;) {
+                    s.chain[k] = (uint16_t)at;
+                    const uint32_t to = s.next[at];
+                    if (to >= kCells || k + 1 >= kCells) {  // (a chain visits no cell twice)
+                        s.last = (uint16_t)to;
+                        break;
+                    }
+                    ++k;
+                    at = to;
+                }
+                s.links = k;
+            }
+            __syncwarp();
+            // the last cell of a chain that leaves the window is the first of
+            // the next one's, which has its whole neighbourhood
+            const uint32_t links = s.links + (s.last == GridWalkSmem::kEnd ? 1u : 0u);
+            for (uint32_t k = tid; k < links && n + k < cap; k += 32) {
+                const uint32_t at = s.chain[k];
+                store(n + k, (uint32_t)((x0 + (int)(at / kSide)) * prob.W + y0 + (int)(at % kSide)));
+            }
+        }
+        __syncthreads();
+        const uint32_t links = s.links, at = s.chain[links];
+        n += links;
+        if (s.last == GridWalkSmem::kEnd) return n + 1 <= cap ? n + 1 : cap + 1;
+        if (n >= cap || links == 0) return cap + 1;
+        cx = x0 + (int)(at / kSide);
+        cy = y0 + (int)(at % kSide);
+    }
+}
+
+}  // namespace uastar

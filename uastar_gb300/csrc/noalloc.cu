@@ -38,6 +38,7 @@
 #include "ga_device.cuh"
 #include "ga_problems.cuh"
 #include "ga_search.cuh"
+#include "ga_walk.cuh"
 
 using namespace uastar;
 
@@ -92,44 +93,38 @@ __global__ void __launch_bounds__(kBlock, 1) k_noalloc_search(GridProblem prob, 
     ga_search<GridProblem>(prob, team, m, kHeapsPerCta, smem, ~0ull);
 }
 
-// Result + path, walking prev pointers from the goal (one thread), then
-// reversing the path in place to run start -> goal.
-__global__ void k_noalloc_finish(const unsigned char *scratch, int32_t *path, int64_t cap,
-                                 uastar_noalloc_grid_result *out) {
+// Result + path: walked from the goal (ga_walk.cuh), then reversed in place to
+// run start -> goal.
+constexpr uint32_t kFinishBlock = 1024;
+__global__ void __launch_bounds__(kFinishBlock) k_noalloc_finish(GridProblem prob, const unsigned char *scratch,
+                                                                 int32_t *path, int64_t cap,
+                                                                 uastar_noalloc_grid_result *out) {
     const TeamState *st = reinterpret_cast<const TeamState *>(scratch + kOffState);
     const Slot *tab = reinterpret_cast<const Slot *>(scratch + kOffTable);
-    __shared__ long long s_len;
+    __shared__ GridWalkSmem walk;
+    const uint32_t status = ldcg_u32(&st->status);
+    long long n = 0;
+    if (status == ST_OK)
+        n = (long long)walk_grid(tab, kTableSlots - 1, prob, ldcg_u32(&st->goal_slot), (uint64_t)cap, walk,
+                                 [&](unsigned long long i, uint32_t cell) { path[i] = (int32_t)cell; });
+    const bool fits = n <= cap;  // else the caller's path buffer is too small
+    if (!fits) n = 0;
     if (threadIdx.x == 0) {
         uastar_noalloc_grid_result r;
         memset(&r, 0, sizeof r);
-        r.status = (int32_t)__ldcg(&st->status);
+        r.status = fits ? (int32_t)status : UASTAR_ARENA_FULL;
         r.expanded = (int64_t)__ldcg(&st->expanded);
         r.generated = (int64_t)__ldcg(&st->generated);
         r.rounds = (int64_t)__ldcg(&st->steps);
-        long long n = 0;
-        if (r.status == ST_OK) {
+        if (status == ST_OK) {
             const unsigned long long gbest = __ldcg(&st->goal_best);
             r.straight = (int64_t)(gbest >> 32);
             r.diagonal = (int64_t)(gbest & 0xffffffffu);
-            uint32_t s = __ldcg(&st->goal_slot);
-            while (s != kNone && n < cap) {
-                uint64_t key;
-                uint32_t prev;
-                slot_key_prev(tab + s, GridProblem::kLink, key, prev);
-                path[n++] = (int32_t)key;
-                s = prev;
-            }
-            if (s != kNone) {
-                r.status = UASTAR_ARENA_FULL;  // the caller's path buffer is too small
-                n = 0;
-            }
         }
         r.path_len = n;
         *out = r;
-        s_len = n;
     }
-    __syncthreads();
-    const long long n = s_len;
+    // (one thread wrote the path, and walk_grid's last barrier lies behind it)
     for (long long i = threadIdx.x; i < n / 2; i += blockDim.x) {
         const int32_t a = path[i], b = path[n - 1 - i];
         path[i] = b;
@@ -203,6 +198,6 @@ extern "C" int32_t uastar_grid_solve_noalloc(const uint64_t *d_words, int32_t H,
     if (cudaLaunchCooperativeKernel((const void *)k_noalloc_search, dim3(kCtas), dim3(kBlock), args, smem, s) !=
         cudaSuccess)
         return UASTAR_CUDA_ERROR;
-    k_noalloc_finish<<<1, 256, 0, s>>>(scratch, d_path, path_cap, d_result);
+    k_noalloc_finish<<<1, kFinishBlock, 0, s>>>(prob, scratch, d_path, path_cap, d_result);
     return cudaGetLastError() == cudaSuccess ? UASTAR_OK : UASTAR_CUDA_ERROR;
 }
