@@ -62,7 +62,9 @@ typedef struct {
     int32_t block_threads;   /* CTA size of the plain engine's persistent kernel (0 -> 256) */
     int32_t heap_capacity;   /* entries per heap (0 -> auto, grown on overflow) */
     int32_t hash_log2_slots; /* dedup table = 2^n slots of 32 B, n <= 31 (0 -> sized from the instance and
-                              grown 4x in place whenever it is half full) */
+                              grown 4x in place whenever it is half full).  A grid that fits these bytes
+                              with 8 a cell has one word per cell there; max_load * 2^n limits its
+                              states all the same */
     double max_load;         /* dedup table load limit in (0,1) (0 -> 0.8) */
     int64_t max_rounds;      /* limit on expansion steps per solve (0 -> 2^31): a GA* round is one, and
                               each further pass of expansions that it makes at once is one more */

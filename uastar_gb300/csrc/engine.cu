@@ -32,7 +32,8 @@ __global__ void k_fill_ff(uint4 *p, size_t n16) {
 }
 
 // A plain solve's memory before its first round: empty table and heaps, fresh
-// team state.  Bound by the table's bytes (8.6 GB: 1.29 ms, 6.7 TB/s); one launch
+// team state.  Bound by the table's bytes (8.6 GB: 1.29 ms, 6.7 TB/s; with a
+// word per cell the 20000^2 grid clears 3.2 GB); one launch
 // instead of a fill, a memset and a copy, and the walk queued behind the search
 // (run_plain), take four trips to the driver and one wait off a solve: 61 x 67
 // 340 -> 306 us, an 8-puzzle 134 -> 115 us.
@@ -165,15 +166,16 @@ __global__ void k_walk_solved(const S *tab, const TeamState *st, unsigned long l
     walk_boards_dev(tab, ldcg_u32(&st->goal_slot), keys, cap, len);
 }
 // The grid's (ga_walk.cuh); nothing either if the path has more than cap cells.
-__global__ void __launch_bounds__(1024) k_walk_grid_solved(GridProblem prob, const Slot *tab, uint64_t mask,
-                                                           const TeamState *st, int32_t *cells, uint64_t cap,
-                                                           unsigned long long *len) {
+template <class P>
+__global__ void __launch_bounds__(1024) k_walk_grid_solved(P prob, const Slot *tab, uint64_t mask, const TeamState *st,
+                                                           int32_t *cells, uint64_t cap, unsigned long long *len) {
     __shared__ GridWalkSmem s;
     if (ldcg_u32(&st->status) != ST_OK) return;
-    const uint64_t g = ldcg_u64(&st->goal_best);
+    uint64_t g = ldcg_u64(&st->goal_best);
+    if constexpr (P::kDirect) g = P::pair(g);
     if ((g >> 32) + (g & 0xffffffffull) + 1 > cap) return;
-    const unsigned long long n = walk_grid(tab, mask, prob, ldcg_u32(&st->goal_slot), cap, s,
-                                           [&](unsigned long long i, uint32_t cell) { cells[i] = (int32_t)cell; });
+    const unsigned long long n =
+        walk_grid(tab, mask, prob, cap, s, [&](unsigned long long i, uint32_t cell) { cells[i] = (int32_t)cell; });
     if (threadIdx.x == 0) *len = n;
 }
 
@@ -282,6 +284,15 @@ void plain_shape(const uastar_engine *eng, uint32_t block, uint32_t tph, uint32_
     if (eng->cfg.heaps <= 0) *n = (*n + sms - 1) / sms * sms;
 }
 
+// Whether an unbounded search of this map is expected to outgrow the growth
+// point (2^19 states) of the auto-sized table's first 2^20 slots without
+// outgrowing the table: a map of at most 2^20 cells, of which a search that
+// crosses it at 30 % blocked reaches five eighths.
+bool may_outgrow(int32_t H, int32_t W) {
+    const uint64_t cells = (uint64_t)H * (uint64_t)W;
+    return cells * 5 > (8ull << 19) && cells <= (1ull << 20);
+}
+
 // Moves a paused search's table to one 4x larger (k_grow_*), swapping it in
 // as eng->tab.  Returns false (and changes nothing) if the memory is not there.
 template <class P>
@@ -351,6 +362,8 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
     }
     bool sorted = false;
     uint32_t sort_bits = 0;
+    uint64_t direct_b = 0;  // bytes of a table with a word per cell
+    if constexpr (P::kDirect) direct_b = ((uint64_t)prob.H * (uint64_t)prob.W * 8 + 15) / 16 * 16;
     if constexpr (std::is_same<P, GridProblem>::value) {
         sorted = c.dedup == 1;
         sort_bits = (uint32_t)std::max(1, ceil_log2_u64((uint64_t)prob.H * (uint64_t)prob.W));
@@ -397,7 +410,7 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
 
     for (int attempt = 0; attempt < 6; ++attempt) {
         const uint64_t slots = 1ull << log2;
-        const size_t tab_b = slots * sizeof(Slot);
+        const size_t tab_b = P::kDirect ? direct_b : slots * sizeof(Slot);
         const size_t heap_b = (size_t)k * hg.stride * sizeof(E);
         const size_t cand_b = cand_records<P>(nblocks, H) * sizeof(Cand);
         // the batched engine's cached buffers give way to a table that does not fit
@@ -428,7 +441,9 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
         SearchMem<E> m;
         m.tab = eng->tab.as<Slot>();
         m.mask = slots - 1;
-        m.max_inserted = (uint64_t)((double)slots * c.max_load);
+        // (a word per cell never runs full: only the caller's limit applies)
+        const bool bounded_tab = !P::kDirect || c.hash_log2_slots > 0;
+        m.max_inserted = bounded_tab ? (uint64_t)((double)slots * c.max_load) : ~0ull;
         m.max_probe = 4096;
         m.heaps = eng->heaps.as<E>();
         m.stride = hg.stride;
@@ -439,14 +454,11 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
         m.max_rounds = (uint64_t)c.max_rounds;
         if (!sorted) m.set(prob.expansion(k));
         if constexpr (std::is_same<P, GridProblem>::value) {
-            // An auto-sized table starts at 2^20 slots.  Maps of 2^19 to 2^20
-            // cells keep the open frontier unbounded: their search is expected
-            // to outgrow that table's growth point (2^19 states; the in-place
-            // growth of a grid is pinned by a test on the 1000^2 map), and so
-            // few states stay in L2.  1000^2: 12.6 ms -> 9.7 ms so (2 passes),
-            // 6.4 ms with the bound.
-            const uint64_t cells = (uint64_t)prob.H * (uint64_t)prob.W;
-            if (!sorted && c.hash_log2_slots <= 0 && cells > (1ull << 19) && cells <= (1ull << 20)) {
+            // Hashed only because it may outgrow the auto-sized table
+            // (grid_is_direct): the open frontier is left unbounded, so that
+            // it does and the few states stay in L2.  1000^2: 12.6 ms -> 9.7
+            // ms so (2 passes).
+            if (!sorted && c.hash_log2_slots <= 0 && may_outgrow(prob.H, prob.W)) {
                 m.slack = 0.f;
                 m.cont = 2;
             }
@@ -465,7 +477,7 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
             if (max_log2 <= 0 || n < (1ull << max_log2)) return n / 2;
             return m.max_inserted > round_max ? m.max_inserted - round_max : 0ull;
         };
-        m.grow_at = auto_table ? pause_point(slots) : ~0ull;
+        m.grow_at = auto_table && !P::kDirect ? pause_point(slots) : ~0ull;
         uint64_t timeout_ns = (uint64_t)(c.wait_timeout_s * 1e9);
         P pr = prob;
         uint32_t h_arg = H;
@@ -490,7 +502,9 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
             if (out->st.status != ST_RUNNING) break;
             // paused: at the cap the caller takes over; otherwise grow
             if (max_log2 > 0 && m.mask + 1 >= (1ull << max_log2)) break;
-            if (grow_table<P>(eng, m, k, st)) {
+            bool grown = false;
+            if constexpr (!P::kDirect) grown = grow_table<P>(eng, m, k, st);
+            if (grown) {
                 out->grows += 1;
                 m.grow_at = pause_point(m.mask + 1);
             } else {
@@ -525,17 +539,18 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
 }
 
 // Tails (run_plain): the path's length, then its cells or boards, goal first.
-struct GridTail {
-    GridProblem prob;
+template <class P> struct GridTail {
+    P prob;
     uint64_t cap;
     size_t bytes;
-    GridTail(const GridProblem &p, uint64_t c) : prob(p), cap(c), bytes(16 + (size_t)c * 4) {}
+    uastar_engine *eng;
+    GridTail(uastar_engine *e, const P &p, uint64_t c) : prob(p), cap(c), bytes(16 + (size_t)c * 4), eng(e) {}
     void operator()(const SearchMem<GridEntry> &m, const TeamState *st, unsigned char *at) const {
-        k_walk_grid_solved<<<1, 1024, 0, eng->stream>>>(prob, m.tab, m.mask, st, reinterpret_cast<int32_t *>(at + 16),
-                                                       cap, reinterpret_cast<unsigned long long *>(at));
+        k_walk_grid_solved<<<1, 1024, 0, eng->stream>>>(prob, (const Slot *)m.tab, m.mask, st,
+                                                       reinterpret_cast<int32_t *>(at + 16), cap,
+                                                       reinterpret_cast<unsigned long long *>(at));
         eng->launches++;
     }
-    uastar_engine *eng = nullptr;
 };
 template <int N> struct PuzzleTail {
     static constexpr uint64_t cap = 256;  // boards
@@ -553,7 +568,8 @@ template <int N> struct PuzzleTail {
 };
 
 // The path of a solved grid search whose tail had no room for it, goal first.
-int32_t walk_grid_long(uastar_engine *eng, const GridProblem &prob, uint64_t mask, uint64_t n, uint64_t cap,
+template <class P>
+int32_t walk_grid_long(uastar_engine *eng, const P &prob, uint64_t mask, uint64_t n, uint64_t cap,
                        std::vector<int32_t> *cells) {
     cudaError_t e;
     if (n > cap) {
@@ -562,7 +578,7 @@ int32_t walk_grid_long(uastar_engine *eng, const GridProblem &prob, uint64_t mas
     }
     if ((e = eng->walk.ensure(16 + (size_t)n * 4)) != cudaSuccess) return fail_cuda(eng, e, "alloc walk");
     unsigned char *at = eng->walk.as<unsigned char>();
-    k_walk_grid_solved<<<1, 1024, 0, eng->stream>>>(prob, eng->tab.as<Slot>(), mask, eng->team.as<TeamState>(),
+    k_walk_grid_solved<<<1, 1024, 0, eng->stream>>>(prob, (const Slot *)eng->tab.p, mask, eng->team.as<TeamState>(),
                                                    reinterpret_cast<int32_t *>(at + 16), n,
                                                    reinterpret_cast<unsigned long long *>(at));
     eng->launches++;
@@ -633,6 +649,42 @@ int32_t grid_load_impl(uastar_engine *eng, const uint64_t *words, int32_t H, int
     return UASTAR_OK;
 }
 
+// Whether a grid is searched with a word per cell (GridDirect) instead of the
+// hashed table: its costs have to fit the word (kLimit), and 8 bytes a cell to
+// fit the 32-byte slots that the caller asked for (an auto-sized table is one
+// slot for two cells or more).  Where both forms apply the word is faster at
+// every size measured, 61 x 67 to 20000^2 (GridDirect).
+bool grid_is_direct(const uastar_config &c, int32_t H, int32_t W) {
+    const uint64_t cells = (uint64_t)H * (uint64_t)W;
+    if (c.dedup != 0 || (uint64_t)H + (uint64_t)W > (GridDirect::kLimit >> GridDirect::kFrac)) return false;
+    if (c.hash_log2_slots > 0) return c.hash_log2_slots <= 31 && cells <= 4ull << c.hash_log2_slots;
+    // (the in-place growth of a grid's auto-sized table is pinned by a test on
+    // the 1000^2 map: maps whose first table it applies to stay hashed)
+    return !may_outgrow(H, W) && cells <= 1ull << 30;
+}
+
+// One search of a grid; `far` gets a path that the tail had no room for.
+template <class P>
+int32_t run_grid(uastar_engine *eng, const P &prob, uint64_t tail_cap, PlainOut *po, std::vector<int32_t> *far) {
+    const uint64_t cells = (uint64_t)prob.H * (uint64_t)prob.W;
+    const int log2_auto = std::min(28, std::max(20, ceil_log2_u64(cells) - 1));
+    const uint32_t per_heap =
+        (uint32_t)std::min<uint64_t>(8192, std::max<uint64_t>(64, 4 * cells / plain_heaps<GridProblem>(eng->cfg)));
+    const GridTail<P> tail(eng, prob, tail_cap);
+    if (int32_t rc = run_plain(eng, prob, log2_auto, next_pow2_u32(per_heap), po, 0, tail)) return rc;
+    if (po->st.status != ST_OK) return UASTAR_OK;
+    uint64_t g = po->st.goal_best;
+    if constexpr (P::kDirect) g = P::pair(g);
+    const uint64_t n = (g >> 32) + (g & 0xffffffffull) + 1;
+    if (n > tail_cap)
+        return walk_grid_long(eng, prob, po->slots - 1, n, std::min<uint64_t>(cells + 1, 1ull << 26), far);
+    unsigned long long got = 0;
+    std::memcpy(&got, po->tail, 8);
+    if (got == n) return UASTAR_OK;
+    eng->set_err("solution path of another length than its cost");
+    return UASTAR_CUDA_ERROR;
+}
+
 int32_t grid_solve_impl(uastar_engine *eng, const uint64_t *host_words, int32_t sx, int32_t sy,
                         int32_t ex, int32_t ey, uastar_grid_result *out) {
     const double t0 = now_ms();
@@ -659,15 +711,26 @@ int32_t grid_solve_impl(uastar_engine *eng, const uint64_t *host_words, int32_t 
     prob.ey = ey;
     prob.w_inv = GridProblem::row_inverse(prob.W);
     const uint64_t cells = (uint64_t)H * W;
-    const int log2_auto = std::min(28, std::max(20, ceil_log2_u64(cells) - 1));
-    const uint32_t per_heap =
-        (uint32_t)std::min<uint64_t>(8192, std::max<uint64_t>(64, 4 * cells / plain_heaps<GridProblem>(eng->cfg)));
     // room for the path beside the result: a few times the straight way
     // across, at most 128 KB (a longer path is walked after it)
-    GridTail tail(prob, std::min<uint64_t>(32768, std::min<uint64_t>(cells, 2ull * ((uint64_t)H + W) + 256)));
-    tail.eng = eng;
+    const uint64_t tail_cap = std::min<uint64_t>(32768, std::min<uint64_t>(cells, 2ull * ((uint64_t)H + W) + 256));
     PlainOut po;
-    int32_t rc = run_plain(eng, prob, log2_auto, next_pow2_u32(per_heap), &po, 0, tail);
+    std::vector<int32_t> far;
+    bool direct = grid_is_direct(eng->cfg, H, W);
+    int32_t rc = UASTAR_OK;
+    double kernel_ms = 0;
+    if (direct) {
+        GridDirect dp;
+        static_cast<GridProblem &>(dp) = prob;
+        rc = run_grid(eng, dp, tail_cap, &po, &far);
+        direct = rc == UASTAR_OK && po.st.status != ST_COST_RANGE;
+        kernel_ms = po.kernel_ms;
+        po.st.goal_best = GridDirect::pair(po.st.goal_best);
+    }
+    if (!direct && rc == UASTAR_OK) {
+        rc = run_grid(eng, prob, tail_cap, &po, &far);
+        po.kernel_ms += kernel_ms;
+    }
     if (rc) return out->status = rc;
     const TeamState &st = po.st;
     out->status = (int32_t)st.status;
@@ -691,19 +754,7 @@ int32_t grid_solve_impl(uastar_engine *eng, const uint64_t *host_words, int32_t 
         eng->ley = ey;
         // Path: walked on the device (goal first), re-validated on the host.
         const uint64_t n = (uint64_t)out->straight + (uint64_t)out->diagonal + 1;
-        const uint64_t cap = std::min<uint64_t>(cells + 1, 1ull << 26);
-        std::vector<int32_t> far;
-        const int32_t *walked = reinterpret_cast<const int32_t *>(po.tail + 16);
-        unsigned long long got = 0;
-        std::memcpy(&got, po.tail, 8);
-        if (n > tail.cap) {
-            rc = walk_grid_long(eng, prob, po.slots - 1, n, cap, &far);
-            if (rc) return out->status = rc;
-            walked = far.data();
-        } else if (got != n) {
-            eng->set_err("solution path of another length than its cost");
-            return out->status = UASTAR_CUDA_ERROR;
-        }
+        const int32_t *walked = far.empty() ? reinterpret_cast<const int32_t *>(po.tail + 16) : far.data();
         eng->path.resize(n);
         for (uint64_t i = 0; i < n; ++i) eng->path[i] = walked[n - 1 - i];
         eng->path_cached = true;

@@ -27,6 +27,7 @@ enum : uint32_t {
     ST_BAD_INPUT = 7,
     ST_TIMEOUT = 8,
     ST_RUNNING = 9,
+    ST_COST_RANGE = 10,  // a cost beyond GridDirect's exact range (never leaves the library)
 };
 
 // One dedup-table slot: exactly one 32-byte sector, so a probe, the g update
@@ -64,6 +65,7 @@ enum SlotLink : int { LINK_FIELD = 0, LINK_IN_KEY = 1, LINK_IN_G = 2 };
 struct NarrowSlots {
     using Key = uint64_t;
     static constexpr bool kWide = false;
+    static constexpr bool kDirect = false;     // see GridDirect
     static constexpr bool kPrevInKey = false;  // see GridProblem
     static constexpr int kLink = LINK_FIELD;
     // the g word that the relax CAS installs, and its cost
@@ -79,6 +81,7 @@ struct NarrowSlots {
 struct WideSlots {
     using Key = Key128;
     static constexpr bool kWide = true;
+    static constexpr bool kDirect = false;
     static constexpr bool kPrevInKey = false;
     static constexpr int kLink = LINK_FIELD;
     __device__ static const WideSlot *w(const Slot *s) { return reinterpret_cast<const WideSlot *>(s); }

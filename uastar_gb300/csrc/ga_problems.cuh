@@ -205,11 +205,12 @@ struct GridProblem : NarrowSlots {
         return rows_moves(key, k);
     }
     // Three passes a round, within 1/64 of the straight distance between the
-    // query's ends, 1 to 16.  Measured on 20000^2 (distance 28283): slack 4 /
-    // 8 / 16 / 32: 272 / 224 / 215 / 277 ms (narrow: more rounds; wide: every
-    // state expanded again), passes 2 / 3 / 4 / 5 at 8: 238 / 224 / 220 / 234;
-    // six queries on 1537 x 2049: 33-35 ms throughout; 61 x 67 (distance 84):
-    // slack 1 0.21 ms, 8 0.27, 32 0.32.
+    // query's ends, 1 to 16.  Measured on 20000^2 (distance 28283), hashed:
+    // slack 4 / 8 / 16 / 32: 272 / 224 / 215 / 277 ms (narrow: more rounds;
+    // wide: every state expanded again); on words: slack 12 / 16 / 24: 107 /
+    // 107 / 112, passes 2 / 3 / 4 / 5 / 7 at 16: 108 / 107 / 112 / 115 / 138;
+    // six queries on 1537 x 2049 with these passes 14.6 / 13.8 / 14.0 / 15.0 /
+    // 16.8 ms; 61 x 67 (distance 84): slack 1 0.21 ms, 8 0.27, 32 0.32.
     __host__ __device__ Expansion expansion(uint32_t) const {
         const int dx = sx < ex ? ex - sx : sx - ex, dy = sy < ey ? ey - sy : sy - ey;
         const int mn = dx < dy ? dx : dy, mx = dx < dy ? dy : dx;
@@ -290,6 +291,66 @@ struct GridProblem : NarrowSlots {
         key = v.x & 0xffffffffull;
         g = v.y;
         aux = (uint32_t)key;
+    }
+};
+
+// x with x * odd = 1 modulo 2^64 (Newton's iteration: the correct low bits double).
+__host__ __device__ constexpr uint64_t odd_inverse(uint64_t odd) {
+    uint64_t x = odd;
+    for (int i = 0; i < 6; ++i) x *= 2 - odd * x;
+    return x;
+}
+
+// A grid search whose table is one 8-byte word per cell instead of hashed
+// 32-byte slots: slot = cell, word = g << 3 | the move that reached the cell
+// (all ones: unreached).  A relax is then one 64-bit atomicMin, one memory trip
+// whatever it finds, where the hashed table's 16-byte CAS takes one to claim
+// and two or more to improve or on a collision.  For that a cost has to be one
+// number: g = A * 2^40 + B * kDiag for A straight and B diagonal steps, kDiag an
+// odd number next to sqrt2 * 2^40.  Sums of costs are exact, (A, B) come back
+// from the number (pair) and numbers compare as the costs do while B < 600000:
+// two costs with B apart by n differ by at least 1 / (2 sqrt2 n + 1) and the
+// number's error in the difference is at most n * 2^-40, less while n (2.83 n
+// + 1) < 2^40.  Costs that could reach kLimit (800000, so B < 566000) end the
+// search with ST_COST_RANGE, and the hashed search takes the problem over.
+// Comparing two costs is one integer compare, and a map's words are a quarter of
+// the bytes of its hashed slots at the sizes taken before.  Kernels, hashed ->
+// word: 20000^2 165 -> 103 ms (5.35 -> 3.34 us a step), six queries on 1537 x
+// 2049 20.2 -> 13.3 ms, 61 x 67 0.24 -> 0.20 ms, the allocation-free 700 x 1021
+// 7.1 -> 4.8 ms.  Still bound by the latency of a step's chain, not by bytes.
+struct GridDirect : GridProblem {
+    static constexpr bool kDirect = true;
+    static constexpr int kFrac = 40;
+    static constexpr uint64_t kStraight = 1ull << kFrac, kDiag = 1554944255987ull;
+    static constexpr uint64_t kLimit = 800000ull << kFrac;
+    // A cost as the pair A << 32 | B.
+    __host__ __device__ static uint64_t pair(uint64_t c) {
+        if (c == kInfCost) return c;
+        constexpr uint64_t inv = odd_inverse(kDiag);
+        const uint64_t b = (c * inv) & (kStraight - 1);
+        return ((c - b * kDiag) >> kFrac << 32) | b;
+    }
+    __device__ __forceinline__ static int cost_cmp(uint64_t a, uint64_t b) { return a < b ? -1 : a > b ? 1 : 0; }
+    __device__ __forceinline__ static float cost_val(uint64_t c) { return __ull2float_rn(c) * (1.f / (float)kStraight); }
+    __device__ __forceinline__ uint64_t h_of(uint64_t key) const {
+        const uint64_t h = GridProblem::h_of(key);
+        return (h >> 32 << kFrac) + (uint64_t)(uint32_t)h * kDiag;
+    }
+    __device__ __forceinline__ uint64_t f_of(uint64_t key, uint64_t g, uint32_t) const { return g + h_of(key); }
+    __device__ __forceinline__ bool peek(const Succ &s, float bound) const { return cost_val(s.f) <= bound; }
+    __device__ __forceinline__ void succ_begin(uint64_t key, uint64_t g, uint32_t, int mv, Succ &s) const {
+        const uint32_t c = (uint32_t)key;
+        const int x = (int)row_of(c), y = (int)(c - (uint32_t)x * (uint32_t)W);
+        const int nx = x + c_dx(mv), ny = y + c_dy(mv);
+        s.key = (uint64_t)nx * W + (uint64_t)ny;
+        s.g = g + (mv < 4 ? kStraight : kDiag);
+        const int dx = abs(nx - ex), dy = abs(ny - ey);
+        const int mn = min(dx, dy), mx = max(dx, dy);
+        s.f = s.g + ((uint64_t)(uint32_t)(mx - mn) << kFrac) + (uint64_t)(uint32_t)mn * kDiag;
+    }
+    __device__ __forceinline__ static bool less(const Entry &a, const Entry &b) { return entry_cost(a) < entry_cost(b); }
+    __device__ __forceinline__ static const unsigned long long *words(const Slot *tab) {
+        return reinterpret_cast<const unsigned long long *>(tab);
     }
 };
 

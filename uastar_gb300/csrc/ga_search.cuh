@@ -567,6 +567,7 @@ template <class P> __device__ __forceinline__ uint64_t warp_min_cost(uint64_t v)
 // iff this call strictly lowered the word.
 template <class P>
 __device__ __forceinline__ bool atomic_min_cost(unsigned long long *addr, uint64_t v) {
+    if constexpr (P::kDirect) return v < atomicMin(addr, (unsigned long long)v);
     unsigned long long cur = kInfCost;
     while (P::cost_cmp(v, cur) < 0) {
         const unsigned long long old = atomicCAS(addr, cur, (unsigned long long)v);
@@ -700,11 +701,23 @@ __device__ __forceinline__ int relax_wide(Slot *tab, uint64_t mask, uint32_t max
     return RELAX_FULL;
 }
 
+// One word per cell (GridDirect).  Of two moves that reach a cell at the same g
+// the lower-numbered one stays: both are shortest so far.
+template <class P>
+__device__ __forceinline__ int relax_direct(Slot *tab, uint64_t key, uint64_t g, uint32_t *slot_out, int mv) {
+    const unsigned long long old = atomicMin(reinterpret_cast<unsigned long long *>(tab) + key,
+                                             (unsigned long long)(g << 3 | (uint32_t)max(mv, 0)));
+    *slot_out = (uint32_t)key;
+    return old == kInfCost ? RELAX_INSERTED : (old >> 3) > g ? RELAX_IMPROVED : RELAX_NONE;
+}
+
 template <class P, bool kBeside = true>
 __device__ __forceinline__ int relax_key(Slot *tab, uint64_t mask, uint32_t max_probe, const typename P::Key &key,
                                          uint64_t g, uint32_t prev, uint32_t *slot_out, int mv = -1) {
     if constexpr (P::kWide)
         return relax_wide<P>(tab, mask, max_probe, key, g, slot_out);
+    else if constexpr (P::kDirect)
+        return relax_direct<P>(tab, key, g, slot_out, mv);
     else
         return relax<P, kBeside>(tab, mask, max_probe, key, g, prev, slot_out, mv);
 }
@@ -933,7 +946,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             if (relax_key<P>(m.tab, m.mask, m.max_probe, key0, 0, kNone, &s0) == RELAX_FULL) {
                 set_error(&st->error, ST_HASH_FULL);
             } else {
-                P::set_link(m.tab + s0, kNone, aux0);
+                if constexpr (!P::kDirect) P::set_link(m.tab + s0, kNone, aux0);
                 uint32_t sz = 0;
                 heap_push<P>(heap_of(), sz, prob.make_entry(prob.f_of(key0, 0, aux0), 0, s0, aux0));
                 m.heap_size[myh] = sz;
@@ -1052,7 +1065,13 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                 Key key;
                 uint64_t g;
                 uint32_t aux;
-                P::load_node(m.tab + e.slot, key, g, aux);
+                if constexpr (P::kDirect) {
+                    key = e.slot;
+                    g = __ldcg(P::words(m.tab) + e.slot) >> 3;
+                    aux = e.slot;
+                } else {
+                    P::load_node(m.tab + e.slot, key, g, aux);
+                }
                 // where the entry names its node (grids), the neighbourhood
                 // reads go out beside the node record's, in one round trip
                 uint32_t mv_pre = 0;
@@ -1257,6 +1276,8 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                             const int r =
                                 relax_key<P, Team::kBeside>(m.tab, m.mask, m.max_probe, sc.key, sc.g, oslot, &nslot, move);
                             prob.succ_end(sc, paux, move, naux, nf);
+                            if constexpr (P::kDirect)
+                                if (nf >= P::kLimit) set_error(&st->err[r3], ST_COST_RANGE);
                             if (r == RELAX_FULL) {
                                 set_error(&st->err[r3], ST_HASH_FULL);
                             } else {

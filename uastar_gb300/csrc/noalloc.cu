@@ -12,7 +12,7 @@
 //   - every GPU that loads the library holds kScratchBytes (about 53 MB)
 //     of device memory until the process exits;
 //   - grids are limited to kMaxCells cells; the search itself is limited to
-//     kTableSlots * 0.8 dedup slots and kHeaps heaps of kHeapCap entries
+//     kTableSlots * 0.8 states and kHeaps heaps of kHeapCap entries
 //     (an instance that needs more reports UASTAR_HASH_FULL or
 //     UASTAR_HEAP_OVERFLOW in its result);
 //   - all calls share the one array: two calls whose work overlaps on the
@@ -59,11 +59,13 @@ constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // (heap_geometry<GridProblem>(6, 4095) = {4672, 4095}, checked at set-up)
 constexpr uint32_t kHeapStride = 4672;
 constexpr size_t kOffState = 0;
-constexpr size_t kOffSizes = align256(kOffState + sizeof(TeamState));
+constexpr size_t kOffMode = align256(kOffState + sizeof(TeamState));  // uint32_t: 1 = hashed table, 0 = a word per cell
+constexpr size_t kOffSizes = align256(kOffMode + sizeof(uint32_t));
 constexpr size_t kOffCand = align256(kOffSizes + kHeaps * sizeof(uint32_t));
 constexpr size_t kOffHeaps = align256(kOffCand + cand_records<GridProblem>(kCtas, kHeapsPerCta) * sizeof(Cand));
 constexpr size_t kOffTable = align256(kOffHeaps + (size_t)kHeaps * kHeapStride * sizeof(GridEntry));
 constexpr size_t kScratchBytes = align256(kOffTable + kTableSlots * sizeof(Slot));
+static_assert(kMaxCells * 8 <= kTableSlots * sizeof(Slot), "a word per cell fits the table's bytes");
 
 // The only device memory this entry point uses besides the caller's buffers.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
@@ -73,40 +75,58 @@ constexpr int kMaxDevices = 64;
 unsigned char *g_scratch_ptr[kMaxDevices] = {nullptr};
 std::mutex g_setup_mu;
 
-__global__ void k_noalloc_reset(unsigned char *scratch) {
+// The search runs on a word per cell (GridDirect); a problem whose costs leave
+// that form's range is searched again on the hashed table, in the same bytes.
+// The second reset and search are always queued and return at once otherwise.
+__device__ __forceinline__ uint32_t *mode_of(unsigned char *scratch) {
+    return reinterpret_cast<uint32_t *>(scratch + kOffMode);
+}
+
+// `again`: only if the search before asked for it.
+__global__ void k_noalloc_reset(unsigned char *scratch, uint64_t table_bytes, uint32_t mode, bool again) {
+    if (again && ldcg_u32(mode_of(scratch)) != mode) return;
     // team state: everything zero except the "unset" costs and statuses
     TeamState *st = reinterpret_cast<TeamState *>(scratch + kOffState);
     uint32_t *sizes = reinterpret_cast<uint32_t *>(scratch + kOffSizes);
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t == 0) team_state_init(st);
+    if (t == 0) {
+        team_state_init(st);
+        if (!again) *mode_of(scratch) = mode;
+    }
     for (uint32_t i = t; i < kHeaps; i += gridDim.x * blockDim.x) sizes[i] = 0;
-    // dedup table: every slot empty (key and g all ones, prev = none)
+    // dedup table: every word all ones (an empty slot, an unreached cell)
     uint4 *tab = reinterpret_cast<uint4 *>(scratch + kOffTable);
     const uint4 ff = make_uint4(~0u, ~0u, ~0u, ~0u);
-    for (uint64_t i = t; i < kTableSlots * 2; i += (uint64_t)gridDim.x * blockDim.x) tab[i] = ff;
+    for (uint64_t i = t; i < (table_bytes + 15) / 16; i += (uint64_t)gridDim.x * blockDim.x) tab[i] = ff;
 }
 
-__global__ void __launch_bounds__(kBlock, 1) k_noalloc_search(GridProblem prob, SearchMem<GridEntry> m,
-                                                              TeamState *st, uint64_t timeout_ns) {
+template <class P>
+__global__ void __launch_bounds__(kBlock, 1) k_noalloc_search(P prob, SearchMem<GridEntry> m, TeamState *st,
+                                                              uint32_t *mode, uint64_t timeout_ns) {
     extern __shared__ __align__(128) unsigned char smem[];
+    if (!P::kDirect && ldcg_u32(mode) == 0) return;
     GridTeam team{st, 0u, timeout_ns};
-    ga_search<GridProblem>(prob, team, m, kHeapsPerCta, smem, ~0ull);
+    const uint32_t status = ga_search<P>(prob, team, m, kHeapsPerCta, smem, ~0ull);
+    if (P::kDirect && blockIdx.x == 0 && threadIdx.x == 0 && status == ST_COST_RANGE) *mode = 1;
 }
 
 // Result + path: walked from the goal (ga_walk.cuh), then reversed in place to
 // run start -> goal.
 constexpr uint32_t kFinishBlock = 1024;
-__global__ void __launch_bounds__(kFinishBlock) k_noalloc_finish(GridProblem prob, const unsigned char *scratch,
+__global__ void __launch_bounds__(kFinishBlock) k_noalloc_finish(GridDirect prob, const unsigned char *scratch,
                                                                  int32_t *path, int64_t cap,
                                                                  uastar_noalloc_grid_result *out) {
     const TeamState *st = reinterpret_cast<const TeamState *>(scratch + kOffState);
     const Slot *tab = reinterpret_cast<const Slot *>(scratch + kOffTable);
     __shared__ GridWalkSmem walk;
+    const bool hashed = ldcg_u32(reinterpret_cast<const uint32_t *>(scratch + kOffMode)) != 0;
     const uint32_t status = ldcg_u32(&st->status);
     long long n = 0;
+    const auto put = [&](unsigned long long i, uint32_t cell) { path[i] = (int32_t)cell; };
     if (status == ST_OK)
-        n = (long long)walk_grid(tab, kTableSlots - 1, prob, ldcg_u32(&st->goal_slot), (uint64_t)cap, walk,
-                                 [&](unsigned long long i, uint32_t cell) { path[i] = (int32_t)cell; });
+        n = (long long)(hashed ? walk_grid(tab, kTableSlots - 1, static_cast<const GridProblem &>(prob), (uint64_t)cap,
+                                           walk, put)
+                               : walk_grid(tab, 0, prob, (uint64_t)cap, walk, put));
     const bool fits = n <= cap;  // else the caller's path buffer is too small
     if (!fits) n = 0;
     if (threadIdx.x == 0) {
@@ -117,14 +137,14 @@ __global__ void __launch_bounds__(kFinishBlock) k_noalloc_finish(GridProblem pro
         r.generated = (int64_t)__ldcg(&st->generated);
         r.rounds = (int64_t)__ldcg(&st->steps);
         if (status == ST_OK) {
-            const unsigned long long gbest = __ldcg(&st->goal_best);
+            const unsigned long long gbest = hashed ? __ldcg(&st->goal_best) : GridDirect::pair(__ldcg(&st->goal_best));
             r.straight = (int64_t)(gbest >> 32);
             r.diagonal = (int64_t)(gbest & 0xffffffffu);
         }
         r.path_len = n;
         *out = r;
     }
-    // (one thread wrote the path, and walk_grid's last barrier lies behind it)
+    // (the path is written before walk_grid's last barrier)
     for (long long i = threadIdx.x; i < n / 2; i += blockDim.x) {
         const int32_t a = path[i], b = path[n - 1 - i];
         path[i] = b;
@@ -155,9 +175,9 @@ extern "C" int32_t uastar_grid_solve_noalloc(const uint64_t *d_words, int32_t H,
             void *p = nullptr;
             if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || !p) return UASTAR_CUDA_ERROR;
             const size_t smem = SearchSmem<GridProblem>::bytes(kHeapsPerCta, kTopLevels);
-            if (cudaFuncSetAttribute(k_noalloc_search, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-                cudaSuccess)
-                return UASTAR_CUDA_ERROR;
+            for (const void *k : {(const void *)k_noalloc_search<GridDirect>, (const void *)k_noalloc_search<GridProblem>})
+                if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+                    return UASTAR_CUDA_ERROR;
             const HeapGeometry<GridProblem> hg = heap_geometry<GridProblem>(kTopLevels, kHeapCap);
             if (hg.stride != kHeapStride) return UASTAR_CUDA_ERROR;  // layout constants out of date
             g_scratch_ptr[dev] = static_cast<unsigned char *>(p);
@@ -166,10 +186,13 @@ extern "C" int32_t uastar_grid_solve_noalloc(const uint64_t *d_words, int32_t H,
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
 
-    k_noalloc_reset<<<256, 256, 0, s>>>(scratch);
+    // (a straight way across must be within the words' range of costs)
+    const uint64_t cells = (uint64_t)H * (uint64_t)W, table_bytes = kTableSlots * sizeof(Slot);
+    const bool direct = (uint64_t)H + (uint64_t)W <= (GridDirect::kLimit >> GridDirect::kFrac);
+    k_noalloc_reset<<<256, 256, 0, s>>>(scratch, direct ? cells * 8 : table_bytes, direct ? 0u : 1u, false);
     if (cudaGetLastError() != cudaSuccess) return UASTAR_CUDA_ERROR;
 
-    GridProblem prob;
+    GridDirect prob;
     prob.bm = reinterpret_cast<const uint32_t *>(d_words);
     prob.H = H;
     prob.W = W;
@@ -193,10 +216,19 @@ extern "C" int32_t uastar_grid_solve_noalloc(const uint64_t *d_words, int32_t H,
     m.set(prob.expansion(kHeaps));
     TeamState *st = reinterpret_cast<TeamState *>(scratch + kOffState);
     uint64_t timeout_ns = 10ull * 1000000000ull;  // bound on every team-barrier wait (UASTAR_TIMEOUT)
-    void *args[] = {&prob, &m, &st, &timeout_ns};
+    uint32_t *mode = reinterpret_cast<uint32_t *>(scratch + kOffMode);
+    GridProblem hashed = prob;
+    void *args[] = {&prob, &m, &st, &mode, &timeout_ns}, *args_hashed[] = {&hashed, &m, &st, &mode, &timeout_ns};
     const size_t smem = SearchSmem<GridProblem>::bytes(kHeapsPerCta, kTopLevels);
-    if (cudaLaunchCooperativeKernel((const void *)k_noalloc_search, dim3(kCtas), dim3(kBlock), args, smem, s) !=
-        cudaSuccess)
+    if (direct) {
+        if (cudaLaunchCooperativeKernel((const void *)k_noalloc_search<GridDirect>, dim3(kCtas), dim3(kBlock), args,
+                                        smem, s) != cudaSuccess)
+            return UASTAR_CUDA_ERROR;
+        k_noalloc_reset<<<256, 256, 0, s>>>(scratch, table_bytes, 1u, true);
+        if (cudaGetLastError() != cudaSuccess) return UASTAR_CUDA_ERROR;
+    }
+    if (cudaLaunchCooperativeKernel((const void *)k_noalloc_search<GridProblem>, dim3(kCtas), dim3(kBlock), args_hashed,
+                                    smem, s) != cudaSuccess)
         return UASTAR_CUDA_ERROR;
     k_noalloc_finish<<<1, kFinishBlock, 0, s>>>(prob, scratch, d_path, path_cap, d_result);
     return cudaGetLastError() == cudaSuccess ? UASTAR_OK : UASTAR_CUDA_ERROR;
