@@ -292,8 +292,9 @@ typedef struct {
  * first wave each CTA takes instances from a device work queue and runs GA*
  * on one with its own heap slice and dedup partition, under a budget of
  * expansion steps (tier1_rounds); grids above 2048^2 and the instances that ran
- * out of steps or space go to a second wave of 8-CTA cluster teams with 16x the
- * partition (puzzles under tier2_puzzle_rounds), and what fails there is
+ * out of steps or space go to a second wave of 8-CTA cluster teams with a larger
+ * partition (32x after an overflow, else what their budget of steps can fill, 8x
+ * by default; puzzles under tier2_puzzle_rounds), and what fails there is
  * solved by the plain engine, one instance at a time.  The last instances of a
  * wave (few enough to leave most of the GPU idle) move on without using up
  * their budget.  No counterpart in the
