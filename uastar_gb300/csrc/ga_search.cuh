@@ -589,18 +589,13 @@ __device__ __forceinline__ KeyG cas128(Slot *s, KeyG cmp, KeyG val) {
 // probe limit was reached.
 enum : int { RELAX_NONE = 0, RELAX_IMPROVED = 1, RELAX_CLAIMED = 2, RELAX_INSERTED = 3, RELAX_FULL = 4 };
 
-// Find-or-insert `key` and lower its g to `g` in one pass (the probe order is
-// probe_slot's).  The first turn tries the home slot with one 16-byte CAS,
-// which claims it empty with (key, g) or returns what it holds, and reads the
-// other three slots of its 128-byte line beside it; so a claim takes one memory
-// trip, an improvement or a collision two.  The lanes of a warp take their
-// turns together, whatever each one's next access is (the trips would add up
-// in diverged branches).  A turn under the load of a round is ~2.5 k cycles
-// and a warp waits for its slowest lane, so the number of turns is the relax
-// phase: with a look at the line as a turn of its own a warp took 3-4 turns, up
-// to 16 near half load.  Returns RELAX_INSERTED (new slot, g set),
-// RELAX_IMPROVED (existing slot, g strictly lowered), RELAX_NONE (existing
-// slot, g not better) or RELAX_FULL (probe limit).
+// Find-or-insert `key` and lower its g to `g` (the probe order is
+// probe_slot's): one 16-byte CAS per turn, which claims the slot empty with
+// (key, g), lowers the key's g, or returns what the slot holds.  The lanes of a
+// warp take their turns together, and a warp waits for its slowest lane, so the
+// number of turns is the relax phase.  Returns RELAX_INSERTED (new slot, g set),
+// RELAX_IMPROVED (existing slot, g strictly lowered), RELAX_NONE (existing slot,
+// g not better) or RELAX_FULL (probe limit).
 //
 // Where the problem keeps the parent link in the key word (P::kPrevInKey:
 // grid cells are 32 bits), the word is cell | prev << 32 and the CAS sets g
@@ -615,15 +610,54 @@ template <class P> __device__ __forceinline__ bool key_match(uint64_t word, uint
         return word == key;
 }
 
-template <class P, bool kBeside = true>
+template <class P>
 __device__ __forceinline__ int relax(Slot *tab, uint64_t mask, uint32_t max_probe, uint64_t key, uint64_t g,
                                      uint32_t prev, uint32_t *slot_out, int mv = -1) {
+    const KeyG mine{P::kPrevInKey ? (key | (uint64_t)prev << 32) : key, P::g_word(g, prev, mv)};
+    const uint64_t home = mix64(key) & mask;
+    uint64_t h = home;
+    uint32_t i = 0;
+    KeyG cur{kEmptyKey, kInfCost};  // what the CAS expects
+    for (;;) {
+        const KeyG old = cas128(tab + h, cur, mine);
+        if (old.key == cur.key && old.g == cur.g) {
+            *slot_out = (uint32_t)h;
+            return old.key == kEmptyKey ? RELAX_INSERTED : RELAX_IMPROVED;
+        }
+        if (key_match<P>(old.key, key)) {
+            if (P::cost_cmp(g, P::word_g(old.g)) >= 0) {
+                *slot_out = (uint32_t)h;
+                return RELAX_NONE;
+            }
+            cur = old;
+        } else {
+            if (++i >= max_probe) return RELAX_FULL;
+            h = probe_slot(home, i, mask);
+        }
+    }
+}
+
+// The same for a fuller table: the first turn also reads the other three slots
+// of the home slot's 128-byte line, and a collision goes on at the first of them
+// that holds the key or is free, so that it takes two turns where slot by slot a
+// warp of 28 lanes takes 3 at a quarter load and 8 at half.  But reads of a
+// line's other sectors beside a CAS that misses L2 hold it up (random slots of
+// 2 GB, 29 k threads: CAS 2.7 k cycles, with one neighbour read 24 k, with a
+// sector of another line 3.8 k), and the longer loop costs every turn.  So a
+// whole-GPU search changes over at a sixth of its table: 15-puzzles below it
+// 5.9 -> 5.2 us a step slot by slot (8-puzzles 3.3 -> 2.9), above it 9.9 -> 8.8
+// line by line; changing over at a third, a fifth, an eighth: 2.56 / 2.27 / 2.28
+// ms for a 58-move board.  CTA and cluster teams stay with slots: 64 grids up to
+// 1500^2 21.8 -> 18.9 ms, 160 15-puzzles 56.6 -> 53.2.
+template <class P>
+__device__ __forceinline__ int relax_beside(Slot *tab, uint64_t mask, uint32_t max_probe, uint64_t key, uint64_t g,
+                                            uint32_t prev, uint32_t *slot_out, int mv = -1) {
     const KeyG mine{P::kPrevInKey ? (key | (uint64_t)prev << 32) : key, P::g_word(g, prev, mv)};
     const uint64_t home = mix64(key) & mask;
     uint64_t h = home;              // the slot at probe index i
     uint32_t i = 0;
     KeyG cur{kEmptyKey, kInfCost};  // what the CAS expects there
-    bool cas = true, look = kBeside;  // this turn's accesses: CAS slot h; read the slots i (+ 1 with a CAS) .. end of line
+    bool cas = true, look = true;  // this turn's accesses: CAS slot h; read the slots i (+ 1 with a CAS) .. end of line
     for (;;) {
         const uint32_t from = i + (cas ? 1u : 0u), n = look ? 4u - (i & 3u) - (cas ? 1u : 0u) : 0u;
         ulonglong2 v[4];
@@ -711,15 +745,17 @@ __device__ __forceinline__ int relax_direct(Slot *tab, uint64_t key, uint64_t g,
     return old == kInfCost ? RELAX_INSERTED : (old >> 3) > g ? RELAX_IMPROVED : RELAX_NONE;
 }
 
-template <class P, bool kBeside = true>
+template <class P, bool kBeside = false>
 __device__ __forceinline__ int relax_key(Slot *tab, uint64_t mask, uint32_t max_probe, const typename P::Key &key,
-                                         uint64_t g, uint32_t prev, uint32_t *slot_out, int mv = -1) {
+                                         uint64_t g, uint32_t prev, uint32_t *slot_out, int mv = -1, bool beside = false) {
     if constexpr (P::kWide)
         return relax_wide<P>(tab, mask, max_probe, key, g, slot_out);
     else if constexpr (P::kDirect)
         return relax_direct<P>(tab, key, g, slot_out, mv);
+    else if (kBeside && beside)
+        return relax_beside<P>(tab, mask, max_probe, key, g, prev, slot_out, mv);
     else
-        return relax<P, kBeside>(tab, mask, max_probe, key, g, prev, slot_out, mv);
+        return relax<P>(tab, mask, max_probe, key, g, prev, slot_out, mv);
 }
 
 __device__ __forceinline__ Cand load_cand(const Cand *p) {
@@ -760,7 +796,7 @@ struct RoundState {
     uint32_t cont;                 // its continuation passes at most
     uint32_t status, pause;        // the last decision
     uint32_t nshare;               // candidates in this CTA's share
-    uint32_t pad;
+    uint32_t beside;               // 1: relaxes read the rest of a line beside the first CAS (relax_beside)
 };
 static_assert(sizeof(RoundState) == 88, "22 words of the scratch");
 
@@ -979,6 +1015,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
     if (lead) {
         rs->gbest = team.rd64(&st->goal_best);
         rs->inserted = team.rd64(&st->inserted);
+        rs->beside = rs->inserted * 6 > m.mask;
         rs->rounds = round0;
         rs->steps = team.rd64(&st->steps);
         rs->stop_at = budget < ~rs->steps ? rs->steps + budget : ~0ull;
@@ -1274,7 +1311,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                             const bool peek = pass < rs->cont && prob.peek(sc, rs->bound);
                             if (peek) prob.look_begin(sc.key, look);
                             const int r =
-                                relax_key<P, Team::kBeside>(m.tab, m.mask, m.max_probe, sc.key, sc.g, oslot, &nslot, move);
+                                relax_key<P, Team::kBeside>(m.tab, m.mask, m.max_probe, sc.key, sc.g, oslot, &nslot, move, rs->beside);
                             prob.succ_end(sc, paux, move, naux, nf);
                             if constexpr (P::kDirect)
                                 if (nf >= P::kLimit) set_error(&st->err[r3], ST_COST_RANGE);
@@ -1405,6 +1442,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             uint64_t gbest = rs->gbest;
             if (P::cost_cmp(gmin, gbest) < 0) rs->gbest = gbest = gmin;
             const uint64_t inserted = rs->inserted += ins;
+            rs->beside = inserted * 6 > m.mask;
             const uint64_t steps = rs->steps += 1 + pass;
             rs->rounds += 1;
             uint32_t err = e1 ? e1 : e2;
