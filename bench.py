@@ -616,7 +616,7 @@ def section_mb(eng, args):
                        "exact_nodes": r["exact_nodes"], "exact_ms": round(r["exact_ms"], 1)}
     for log2 in (20, 22, 24):
         r = eng.puzzle_solve_bounded(4, tiles, log2)
-        out.append({"max_table_slots": 1 << log2, "table_mb": (1 << log2) * 32 >> 20, "status": r["status"],
+        out.append({"max_table_slots": 1 << log2, "table_mb": (1 << log2) * 16 >> 20, "status": r["status"],
                     "steps": r["steps"], "lower_bound": r["lower_bound"], "segments": r["segments"],
                     "expanded": r["expanded"], "solve_ms": round(r["solve_ms"], 1), **exact(r)})
     opt = eng.puzzle_solve(4, tiles)

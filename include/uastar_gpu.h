@@ -61,7 +61,7 @@ typedef struct {
                               rounded up to a whole number of CTAs per SM) */
     int32_t block_threads;   /* CTA size of the plain engine's persistent kernel (0 -> 256) */
     int32_t heap_capacity;   /* entries per heap (0 -> auto, grown on overflow) */
-    int32_t hash_log2_slots; /* dedup table = 2^n slots of 32 B, n <= 31 (0 -> sized from the instance and
+    int32_t hash_log2_slots; /* dedup table = 2^n slots of 16 B (5x5: 32 B), n <= 31 (0 -> sized from the instance and
                               grown 4x in place whenever it is half full).  A grid that fits these bytes
                               with 8 a cell has one word per cell there; max_load * 2^n limits its
                               states all the same */
@@ -203,7 +203,7 @@ int64_t uastar_puzzle_moves(uastar_engine *eng, int32_t *moves, int64_t cap);
 /* Memory-bounded solve for puzzles too large for the dedup table (the
  * reference's README.md:30-34 describes such a mode; it has no code for it).
  * Phase 1 runs segments of exact GA* with the table capped at
- * 2^max_log2_slots slots (32 B each).  A segment that fills the table pauses;
+ * 2^max_log2_slots slots (16 B each, 32 on 5x5).  A segment that fills the table pauses;
  * the open list's minimum f is then a lower bound on the remaining optimum,
  * the search commits to the open node holding it and the next segment starts
  * there; one segment means the solution is optimal.  Phase 2, when phase 1

@@ -120,7 +120,7 @@ __device__ unsigned long long walk_chain(const Slot *part, uint32_t goal_slot, u
 __device__ void clear_partition(Slot *tab, uint64_t slots) {
     uint4 *p = reinterpret_cast<uint4 *>(tab);
     const uint4 v = make_uint4(~0u, ~0u, ~0u, ~0u);
-    for (uint64_t j = threadIdx.x; j < slots * 2; j += blockDim.x) p[j] = v;
+    for (uint64_t j = threadIdx.x; j < slots; j += blockDim.x) p[j] = v;
 }
 
 __device__ void init_state(TeamState *st) { team_state_init(st); }
@@ -309,7 +309,7 @@ __global__ void k_serve_walk(const Slot *part, uint32_t goal_slot, unsigned long
 __device__ void clear_partition_team(Slot *tab, uint64_t slots, uint32_t rank, uint32_t nranks) {
     uint4 *p = reinterpret_cast<uint4 *>(tab);
     const uint4 v = make_uint4(~0u, ~0u, ~0u, ~0u);
-    for (uint64_t j = (uint64_t)rank * blockDim.x + threadIdx.x; j < slots * 2; j += (uint64_t)nranks * blockDim.x)
+    for (uint64_t j = (uint64_t)rank * blockDim.x + threadIdx.x; j < slots; j += (uint64_t)nranks * blockDim.x)
         p[j] = v;
 }
 

@@ -94,7 +94,7 @@ __global__ void k_best_open(PuzzleProblem<N> prob, SearchMem<PuzzleEntry> m, uin
         typename PuzzleProblem<N>::Key key;
         uint64_t g;
         uint32_t aux;
-        PuzzleProblem<N>::load_node(m.tab + e.slot, key, g, aux);
+        PuzzleProblem<N>::load_node(PuzzleProblem<N>::at(m.tab, e.slot), e, key, g, aux);
         if (prob.f_of(key, g, aux) != PuzzleProblem<N>::entry_cost(e)) continue;  // stale
         atomicMin(best, ((unsigned long long)e.key << 32) | e.slot);
     }
@@ -300,7 +300,7 @@ bool grow_table(uastar_engine *eng, SearchMem<typename P::Entry> &m, uint32_t k,
     const uint64_t old_n = m.mask + 1, new_n = old_n * 4;
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
-    const size_t need = (new_n * sizeof(Slot) > eng->tab_next.bytes ? new_n * sizeof(Slot) : 0) +
+    const size_t need = (new_n * P::kSlotBytes > eng->tab_next.bytes ? new_n * P::kSlotBytes : 0) +
                         (old_n * 4 > eng->grow_map.bytes ? old_n * 4 : 0);
     // at most 2^31 slots: every slot index stays below the no-parent mark kNone
     if (new_n > (1ull << 31)) return false;
@@ -309,9 +309,9 @@ bool grow_table(uastar_engine *eng, SearchMem<typename P::Entry> &m, uint32_t k,
         cudaMemGetInfo(&free_b, &total_b);
         if (need + (256ull << 20) > free_b) return false;
     }
-    if (eng->tab_next.ensure(new_n * sizeof(Slot)) != cudaSuccess) return false;
+    if (eng->tab_next.ensure(new_n * P::kSlotBytes) != cudaSuccess) return false;
     if (eng->grow_map.ensure(old_n * 4) != cudaSuccess) return false;
-    if (fill_ff(eng, eng->tab_next.p, new_n * sizeof(Slot)) != UASTAR_OK) return false;
+    if (fill_ff(eng, eng->tab_next.p, new_n * P::kSlotBytes) != UASTAR_OK) return false;
     const int blocks = std::max(1, eng->sms * 8);
     Slot *src = m.tab, *dst = eng->tab_next.as<Slot>();
     uint32_t *map = eng->grow_map.as<uint32_t>();
@@ -410,7 +410,7 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
 
     for (int attempt = 0; attempt < 6; ++attempt) {
         const uint64_t slots = 1ull << log2;
-        const size_t tab_b = P::kDirect ? direct_b : slots * sizeof(Slot);
+        const size_t tab_b = P::kDirect ? direct_b : slots * P::kSlotBytes;
         const size_t heap_b = (size_t)k * hg.stride * sizeof(E);
         const size_t cand_b = cand_records<P>(nblocks, H) * sizeof(Cand);
         // the batched engine's cached buffers give way to a table that does not fit
@@ -524,7 +524,7 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
         size_t free_b = 0, total_b = 0;
         cudaMemGetInfo(&free_b, &total_b);
         if (s == ST_HASH_FULL && auto_table && log2 + 2 <= 31 && (max_log2 <= 0 || log2 + 2 <= max_log2) &&
-            (out->slots * 4 * sizeof(Slot)) < free_b + eng->tab.bytes) {
+            (out->slots * 4 * P::kSlotBytes) < free_b + eng->tab.bytes) {
             log2 += 2;
             continue;
         }
@@ -651,13 +651,13 @@ int32_t grid_load_impl(uastar_engine *eng, const uint64_t *words, int32_t H, int
 
 // Whether a grid is searched with a word per cell (GridDirect) instead of the
 // hashed table: its costs have to fit the word (kLimit), and 8 bytes a cell to
-// fit the 32-byte slots that the caller asked for (an auto-sized table is one
+// fit the 16-byte slots that the caller asked for (an auto-sized table is one
 // slot for two cells or more).  Where both forms apply the word is faster at
 // every size measured, 61 x 67 to 20000^2 (GridDirect).
 bool grid_is_direct(const uastar_config &c, int32_t H, int32_t W) {
     const uint64_t cells = (uint64_t)H * (uint64_t)W;
     if (c.dedup != 0 || (uint64_t)H + (uint64_t)W > (GridDirect::kLimit >> GridDirect::kFrac)) return false;
-    if (c.hash_log2_slots > 0) return c.hash_log2_slots <= 31 && cells <= 4ull << c.hash_log2_slots;
+    if (c.hash_log2_slots > 0) return c.hash_log2_slots <= 31 && cells <= 2ull << c.hash_log2_slots;
     // (the in-place growth of a grid's auto-sized table is pinned by a test on
     // the 1000^2 map: maps whose first table it applies to stay hashed)
     return !may_outgrow(H, W) && cells <= 1ull << 30;
@@ -1044,11 +1044,14 @@ int32_t puzzle_bounded_n(uastar_engine *eng, const uint8_t *tiles, int max_log2,
         if ((e = cudaStreamSynchronize(eng->stream)) != cudaSuccess) return fail_cuda(eng, e, "best open node");
         // a goal at or below every open node (the pause came before the decision
         // that takes it): this segment's optimum
-        if (po.st.goal_best <= best >> 48) return solved(po.st.goal_best, po.st.goal_slot);
+        const uint64_t least = PuzzleProblem<N>::entry_cost(PuzzleEntry{(uint32_t)(best >> 32), 0u});
+        if (best == ~0ull || po.st.goal_best <= least) {
+            if (po.st.goal_best != kInfCost) return solved(po.st.goal_best, po.st.goal_slot);
+        }
         if (best == ~0ull) {
             return fallback(UASTAR_HASH_FULL, "bounded search: no current open node at the memory bound");
         }
-        const uint32_t f = (uint32_t)(best >> 48);  // entry key = f << 16 | (0xffff - g)
+        const uint32_t f = (uint32_t)least;
         if (seg == 0) out->lower_bound = (int32_t)f;
         if ((rc = walk_boards<N>(eng, (uint32_t)best, &boards))) return rc;
         if (boards.size() < 2) {

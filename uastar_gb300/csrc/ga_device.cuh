@@ -30,22 +30,23 @@ enum : uint32_t {
     ST_COST_RANGE = 10,  // a cost beyond GridDirect's exact range (never leaves the library)
 };
 
-// One dedup-table slot: exactly one 32-byte sector, so a probe, the g update
-// and the pop-time read of a node each touch a single sector.
-struct __align__(32) Slot {
+// One dedup-table slot: the 16 bytes that one CAS sets.  Random accesses are
+// what the searches wait for, and their latency under load grows with the table
+// (30 k threads' CAS on 32 / 128 / 512 / 2048 MB: 2.0 / 3.4 / 6.5 / 7.9 k
+// cycles), so a slot holds nothing else: with a puzzle's pattern parts and
+// padding it took 32 bytes.  58-move 15-puzzle 9.2 -> 8.6 us a step, 96 mixed
+// instances 45 -> 41.7 ms, 160 15-puzzles in a batch 53.7 -> 49.2.
+struct __align__(16) Slot {
     unsigned long long key;  // state key (grid cell id / the cells of a board's tiles); kEmptyKey = free
     unsigned long long g;    // cost from the start (problem-specific packing)
-    uint32_t aux;            // problem data (puzzle: PDB parts and last move)
-    uint32_t prev;           // parent slot, kNone for the root
-    uint32_t pad0, pad1;
 };
-static_assert(sizeof(Slot) == 32, "slot must be one sector");
+static_assert(sizeof(Slot) == 16, "a slot is one CAS");
 
 // Slot access by key width.  Narrow keys (grid cells, boards of up to 16
 // cells in 4-bit fields) use the layout above; wide keys (a 5x5 board: 24
-// cells in 5-bit fields, the 25th implied) read the same 32 bytes as
-// {key lo, key hi, g, aux, prev}: the 16-byte key is claimed with one
-// 16-byte CAS and g is lowered with its own 8-byte CAS.
+// cells in 5-bit fields, the 25th implied) slots of 32 bytes: the 16-byte key is
+// claimed with one 16-byte CAS and g is lowered with its own 8-byte CAS.  A
+// table is a Slot pointer in either case; at() finds its i-th slot.
 struct Key128 {
     unsigned long long lo, hi;
 };
@@ -67,16 +68,11 @@ struct NarrowSlots {
     static constexpr bool kWide = false;
     static constexpr bool kDirect = false;     // see GridDirect
     static constexpr bool kPrevInKey = false;  // see GridProblem
-    static constexpr int kLink = LINK_FIELD;
+    static constexpr size_t kSlotBytes = sizeof(Slot);
+    __device__ static Slot *at(Slot *tab, uint64_t i) { return tab + i; }
     // the g word that the relax CAS installs, and its cost
     __device__ static uint64_t g_word(uint64_t g, uint32_t, int) { return g; }
     __device__ static uint64_t word_g(uint64_t w) { return w; }
-    __device__ static uint64_t slot_g(const Slot *s) { return __ldcg(&s->g); }
-    __device__ static uint32_t slot_prev(const Slot *s) { return __ldcg(&s->prev); }
-    __device__ static void set_link(Slot *s, uint32_t prev, uint32_t aux) {
-        s->prev = prev;
-        s->aux = aux;
-    }
 };
 struct WideSlots {
     using Key = Key128;
@@ -84,6 +80,8 @@ struct WideSlots {
     static constexpr bool kDirect = false;
     static constexpr bool kPrevInKey = false;
     static constexpr int kLink = LINK_FIELD;
+    static constexpr size_t kSlotBytes = sizeof(WideSlot);
+    __device__ static Slot *at(Slot *tab, uint64_t i) { return reinterpret_cast<Slot *>(w(tab) + i); }
     __device__ static const WideSlot *w(const Slot *s) { return reinterpret_cast<const WideSlot *>(s); }
     __device__ static WideSlot *w(Slot *s) { return reinterpret_cast<WideSlot *>(s); }
     __device__ static uint64_t slot_g(const Slot *s) { return __ldcg(&w(s)->g); }
@@ -103,7 +101,7 @@ __device__ __forceinline__ void slot_key_prev(const Slot *s, int link, uint64_t 
         prev = (uint32_t)(w >> 32);
     } else {
         key = w;
-        prev = link == LINK_IN_G ? (uint32_t)__ldcg(&s->g) : __ldcg(&s->prev);
+        prev = (uint32_t)__ldcg(&s->g);  // (LINK_IN_G)
     }
 }
 
@@ -203,9 +201,9 @@ __host__ __device__ __forceinline__ uint64_t mix64(uint64_t k) {
 __host__ __device__ __forceinline__ uint64_t key_hash(uint64_t k) { return mix64(k); }
 __host__ __device__ __forceinline__ uint64_t key_hash(const Key128 &k) { return mix64(k.lo ^ mix64(k.hi)); }
 
-// Probe order of the dedup table: the four slots of the home slot's 128-byte
-// line, from the home slot round, then the following lines from their first
-// slot.  A new key takes the first free slot in this order (slots are never
+// Probe order of the dedup table: the home slot's group of four slots (two
+// memory sectors; wide slots: a line), from the home slot round, then the
+// following groups from their first slot.  A new key takes the first free slot in this order (slots are never
 // freed), so a search for it may stop at the first free one.
 __device__ __forceinline__ uint64_t probe_slot(uint64_t home, uint32_t i, uint64_t mask) {
     return i < 4 ? (home & ~3ull) | ((home + i) & 3ull) : ((home & ~3ull) + i) & mask;

@@ -22,17 +22,18 @@ namespace {
 template <bool Wide, bool PrevInKey>
 __global__ void k_grow_move(const Slot *src, uint64_t n, Slot *dst, uint64_t mask, uint32_t *map) {
     for (uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; s < n; s += (uint64_t)gridDim.x * blockDim.x) {
-        const uint4 a = __ldcg(reinterpret_cast<const uint4 *>(src + s));
+        constexpr uint64_t words = Wide ? 2 : 1;  // of 16 bytes a slot
+        const uint4 *from = reinterpret_cast<const uint4 *>(src) + s * words;
+        const uint4 a = __ldcg(from);
         const unsigned long long key = ((unsigned long long)a.y << 32) | a.x;
         if (key == kEmptyKey) continue;
-        const uint4 b = __ldcg(reinterpret_cast<const uint4 *>(src + s) + 1);
         uint64_t h;
         if constexpr (Wide) {
             const Key128 k{key, ((unsigned long long)a.w << 32) | a.z};
             const uint64_t home = key_hash(k) & mask;
             h = home;
             for (uint32_t probe = 1; probe <= mask; ++probe) {
-                const KeyG old = cas128(dst + h, KeyG{kEmptyKey, kEmptyKey}, KeyG{k.lo, k.hi});
+                const KeyG old = cas128(WideSlots::at(dst, h), KeyG{kEmptyKey, kEmptyKey}, KeyG{k.lo, k.hi});
                 if (old.key == kEmptyKey && old.g == kEmptyKey) break;
                 h = probe_slot(home, probe, mask);
             }
@@ -44,9 +45,9 @@ __global__ void k_grow_move(const Slot *src, uint64_t n, Slot *dst, uint64_t mas
                 h = probe_slot(home, probe, mask);
             }
         }
-        uint4 *d = reinterpret_cast<uint4 *>(dst + h);
-        d[0] = make_uint4(a.x, a.y, a.z, a.w);  // key and g (narrow), key (wide)
-        d[1] = b;                               // aux, prev (old index) and pad (narrow); g, aux, prev (wide)
+        uint4 *d = reinterpret_cast<uint4 *>(dst) + h * words;
+        d[0] = a;                                  // key and g (narrow), key (wide)
+        if constexpr (Wide) d[1] = __ldcg(from + 1);  // g, aux, prev (old index)
         map[s] = (uint32_t)h;
     }
 }
@@ -55,21 +56,19 @@ __global__ void k_grow_move(const Slot *src, uint64_t n, Slot *dst, uint64_t mas
 template <bool Wide, int Link>
 __global__ void k_grow_links(const Slot *src, uint64_t n, Slot *dst, const uint32_t *map) {
     for (uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; s < n; s += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t w = __ldcg(&src[s].key);
+        const Slot *from = src + (Wide ? 2 * s : s);
+        const uint64_t w = __ldcg(&from->key);
         if (w == kEmptyKey) continue;
         if constexpr (Link == LINK_IN_KEY) {
             const uint32_t p = (uint32_t)(w >> 32);
             dst[map[s]].key = (w & 0xffffffffull) | (uint64_t)(p == kNone ? kNone : map[p]) << 32;
         } else if constexpr (Link == LINK_IN_G) {
-            const uint64_t gw = __ldcg(&src[s].g);
+            const uint64_t gw = __ldcg(&from->g);
             const uint32_t p = (uint32_t)gw;
             dst[map[s]].g = (gw & ~0xffffffffull) | (p == kNone ? kNone : map[p]);
-        } else if constexpr (Wide) {
-            const uint32_t p = __ldcg(&WideSlots::w(src + s)->prev);
-            WideSlots::w(dst + map[s])->prev = p == kNone ? kNone : map[p];
         } else {
-            const uint32_t p = __ldcg(&src[s].prev);
-            dst[map[s]].prev = p == kNone ? kNone : map[p];
+            const uint32_t p = __ldcg(&WideSlots::w(from)->prev);
+            WideSlots::w(WideSlots::at(dst, map[s]))->prev = p == kNone ? kNone : map[p];
         }
     }
 }

@@ -67,8 +67,6 @@ struct GridProblem : NarrowSlots {
     // sets g and the parent link together, so no push-phase winner check.
     static constexpr bool kPrevInKey = true;
     static constexpr int kLink = LINK_IN_KEY;
-    __device__ static uint32_t slot_prev(const Slot *s) { return (uint32_t)(__ldcg(&s->key) >> 32); }
-    __device__ static void set_link(Slot *, uint32_t, uint32_t) {}  // the link lives in the key word
 
     struct Succ {  // see succ_begin
         uint64_t key, g, f;
@@ -285,7 +283,7 @@ struct GridProblem : NarrowSlots {
         *reinterpret_cast<uint4 *>(p) = make_uint4(e.fa, e.fb, e.slot, e.cell);
     }
     // Node record fields needed at pop time: key and g share the first 16 B.
-    __device__ __forceinline__ static void load_node(const Slot *s, uint64_t &key, uint64_t &g,
+    __device__ __forceinline__ static void load_node(const Slot *s, const Entry &, uint64_t &key, uint64_t &g,
                                                      uint32_t &aux) {
         const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2 *>(s));
         key = v.x & 0xffffffffull;
@@ -356,7 +354,7 @@ struct GridDirect : GridProblem {
 
 // --------------------------------------------------------------- puzzle ---
 struct __align__(8) PuzzleEntry {
-    uint32_t key;   // f << 16 | (0xFFFF - g): min f, then max g
+    uint32_t key;   // min f, then max g: 5x5 f << 16 | (0xFFFF - g), else see PuzzleProblem::make_entry
     uint32_t slot;
 };
 
@@ -422,16 +420,13 @@ template <int N> struct PuzzleProblem : NarrowSlots {
     // The slot's g word is g << 40 | (last move + 1) << 32 | prev: the relax
     // CAS sets the cost and the path link together, so the push phase checks
     // no winner (a candidate that lost is a stale entry, dropped at its pop).
-    // The aux field keeps the pattern parts, which depend on the board alone:
-    // the relaxer that claims the slot writes them.
+    // The pattern parts depend on the board alone and travel in its entries
+    // (make_entry).
     static constexpr int kLink = LINK_IN_G;
     __device__ static uint64_t g_word(uint64_t g, uint32_t prev, int mv) {
         return g << 40 | (uint64_t)(uint32_t)(mv + 1) << 32 | prev;
     }
     __device__ static uint64_t word_g(uint64_t w) { return w >> 40; }
-    __device__ static uint64_t slot_g(const Slot *s) { return __ldcg(&s->g) >> 40; }
-    __device__ static uint32_t slot_prev(const Slot *s) { return (uint32_t)__ldcg(&s->g); }
-    __device__ static void set_link(Slot *s, uint32_t, uint32_t aux) { s->aux = aux & 0xffffu; }
 
     // The key is the board's inverse: nibble t = cell of tile t (tile 0 = the
     // blank), nibbles past the last tile all ones (no cell has that number).
@@ -566,13 +561,17 @@ template <int N> struct PuzzleProblem : NarrowSlots {
         return moves(key, naux);
     }
     static constexpr bool kEntryKey = false;
-    __device__ __forceinline__ Entry make_entry(uint64_t f, uint64_t g, uint32_t slot, uint32_t) const {
+    // f in 10 bits, 255 - g in 8 from bit 14 on (every board searched is
+    // solvable, so g and the parts stay below 128), the first pattern's part in
+    // the low 8: with h = f - g it gives the second's, so a slot needs no more
+    // than its CAS word.
+    __device__ __forceinline__ Entry make_entry(uint64_t f, uint64_t g, uint32_t slot, uint32_t aux) const {
         Entry e;
-        e.key = ((uint32_t)f << 16) | (0xffffu - (uint32_t)g);
+        e.key = (uint32_t)f << 22 | (255u - (uint32_t)g) << 14 | (aux & 0xffu);
         e.slot = slot;
         return e;
     }
-    __device__ __forceinline__ static uint64_t entry_cost(const Entry &e) { return e.key >> 16; }
+    __host__ __device__ __forceinline__ static uint64_t entry_cost(const Entry &e) { return e.key >> 22; }
     __device__ __forceinline__ static bool less(const Entry &a, const Entry &b) { return a.key < b.key; }
     __device__ __forceinline__ static Entry load(const Entry *p) {
         const uint2 u = __ldcg(reinterpret_cast<const uint2 *>(p));
@@ -584,12 +583,13 @@ template <int N> struct PuzzleProblem : NarrowSlots {
     __device__ __forceinline__ static void store(Entry *p, const Entry &e) {
         *reinterpret_cast<uint2 *>(p) = make_uint2(e.key, e.slot);
     }
-    __device__ __forceinline__ static void load_node(const Slot *s, uint64_t &key, uint64_t &g,
+    __device__ __forceinline__ static void load_node(const Slot *s, const Entry &e, uint64_t &key, uint64_t &g,
                                                      uint32_t &aux) {
         const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2 *>(s));
         key = v.x;
         g = v.y >> 40;
-        aux = (__ldcg(&s->aux) & 0xffffu) | ((uint32_t)(v.y >> 32) & 0xffu) << kLastMoveShift;
+        const uint32_t part0 = e.key & 0xffu, h = (e.key >> 22) - (255u - ((e.key >> 14) & 0xffu));
+        aux = part0 | (h - part0) << 8 | ((uint32_t)(v.y >> 32) & 0xffu) << kLastMoveShift;
     }
 };
 
@@ -740,7 +740,7 @@ template <> struct PuzzleProblem<5> : WideSlots {
         e.slot = slot;
         return e;
     }
-    __device__ __forceinline__ static uint64_t entry_cost(const Entry &e) { return e.key >> 16; }
+    __host__ __device__ __forceinline__ static uint64_t entry_cost(const Entry &e) { return e.key >> 16; }
     __device__ __forceinline__ static bool less(const Entry &a, const Entry &b) { return a.key < b.key; }
     __device__ __forceinline__ static Entry load(const Entry *p) {
         const uint2 u = __ldcg(reinterpret_cast<const uint2 *>(p));
@@ -752,7 +752,8 @@ template <> struct PuzzleProblem<5> : WideSlots {
     __device__ __forceinline__ static void store(Entry *p, const Entry &e) {
         *reinterpret_cast<uint2 *>(p) = make_uint2(e.key, e.slot);
     }
-    __device__ __forceinline__ static void load_node(const Slot *s, Key128 &key, uint64_t &g, uint32_t &aux) {
+    __device__ __forceinline__ static void load_node(const Slot *s, const Entry &, Key128 &key, uint64_t &g,
+                                                     uint32_t &aux) {
         const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2 *>(s));
         const ulonglong2 w = __ldcg(reinterpret_cast<const ulonglong2 *>(s) + 1);
         key.lo = v.x;

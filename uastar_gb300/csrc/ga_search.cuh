@@ -638,15 +638,15 @@ __device__ __forceinline__ int relax(Slot *tab, uint64_t mask, uint32_t max_prob
 }
 
 // The same for a fuller table: the first turn also reads the other three slots
-// of the home slot's 128-byte line, and a collision goes on at the first of them
+// of the home slot's group, and a collision goes on at the first of them
 // that holds the key or is free, so that it takes two turns where slot by slot a
 // warp of 28 lanes takes 3 at a quarter load and 8 at half.  But reads of a
-// line's other sectors beside a CAS that misses L2 hold it up (random slots of
+// line's other slots beside a CAS that misses L2 hold it up (random slots of
 // 2 GB, 29 k threads: CAS 2.7 k cycles, with one neighbour read 24 k, with a
 // sector of another line 3.8 k), and the longer loop costs every turn.  So a
 // whole-GPU search changes over at a sixth of its table: 15-puzzles below it
 // 5.9 -> 5.2 us a step slot by slot (8-puzzles 3.3 -> 2.9), above it 9.9 -> 8.8
-// line by line; changing over at a third, a fifth, an eighth: 2.56 / 2.27 / 2.28
+// group by group; changing over at a third, a fifth, an eighth: 2.56 / 2.27 / 2.28
 // ms for a 58-move board.  CTA and cluster teams stay with slots: 64 grids up to
 // 1500^2 21.8 -> 18.9 ms, 160 15-puzzles 56.6 -> 53.2.
 template <class P>
@@ -718,11 +718,11 @@ __device__ __forceinline__ int relax_wide(Slot *tab, uint64_t mask, uint32_t max
     const KeyG empty{kEmptyKey, kEmptyKey};
     for (uint32_t probe = 0; probe < max_probe; ++probe) {
         const uint64_t h = probe_slot(home, probe, mask);
-        const KeyG cur = cas128(tab + h, empty, KeyG{key.lo, key.hi});
+        const KeyG cur = cas128(WideSlots::at(tab, h), empty, KeyG{key.lo, key.hi});
         const bool claimed = cur.key == kEmptyKey && cur.g == kEmptyKey;
         if (claimed || (cur.key == key.lo && cur.g == key.hi)) {
             *slot_out = (uint32_t)h;
-            unsigned long long *gp = &WideSlots::w(tab + h)->g;
+            unsigned long long *gp = &WideSlots::w(WideSlots::at(tab, h))->g;
             unsigned long long old = claimed ? kInfCost : __ldcg(gp);
             while (P::cost_cmp(g, old) < 0) {
                 const unsigned long long seen = atomicCAS(gp, old, (unsigned long long)g);
@@ -796,7 +796,7 @@ struct RoundState {
     uint32_t cont;                 // its continuation passes at most
     uint32_t status, pause;        // the last decision
     uint32_t nshare;               // candidates in this CTA's share
-    uint32_t beside;               // 1: relaxes read the rest of a line beside the first CAS (relax_beside)
+    uint32_t beside;               // 1: relaxes read the home group beside the first CAS (relax_beside)
 };
 static_assert(sizeof(RoundState) == 88, "22 words of the scratch");
 
@@ -982,7 +982,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             if (relax_key<P>(m.tab, m.mask, m.max_probe, key0, 0, kNone, &s0) == RELAX_FULL) {
                 set_error(&st->error, ST_HASH_FULL);
             } else {
-                if constexpr (!P::kDirect) P::set_link(m.tab + s0, kNone, aux0);
+                if constexpr (P::kLink == LINK_FIELD) P::set_link(P::at(m.tab, s0), kNone, aux0);
                 uint32_t sz = 0;
                 heap_push<P>(heap_of(), sz, prob.make_entry(prob.f_of(key0, 0, aux0), 0, s0, aux0));
                 m.heap_size[myh] = sz;
@@ -1107,7 +1107,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                     g = __ldcg(P::words(m.tab) + e.slot) >> 3;
                     aux = e.slot;
                 } else {
-                    P::load_node(m.tab + e.slot, key, g, aux);
+                    P::load_node(P::at(m.tab, e.slot), e, key, g, aux);
                 }
                 // where the entry names its node (grids), the neighbourhood
                 // reads go out beside the node record's, in one round trip
@@ -1320,10 +1320,6 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                             } else {
                                 inserted = (r & RELAX_CLAIMED) != 0;
                                 improved = (r & RELAX_IMPROVED) != 0;
-                                // (link in the g word: the claimer stores the node's
-                                // pattern parts, the same for every writer of the key)
-                                if constexpr (P::kLink == LINK_IN_G)
-                                    if (inserted) P::set_link(m.tab + nslot, oslot, naux);
                             }
                             if (improved) {
                                 goal = prob.is_goal(sc.key);
@@ -1586,8 +1582,8 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             const Cand c = load_cand(sreg + q);
             E e = prob.make_entry(c.f, c.g, c.slot, c.aux);
             if constexpr (P::kLink == LINK_FIELD) {
-                if (P::slot_g(m.tab + c.slot) == c.g)
-                    P::set_link(m.tab + c.slot, c.parent, c.aux);
+                if (P::slot_g(P::at(m.tab, c.slot)) == c.g)
+                    P::set_link(P::at(m.tab, c.slot), c.parent, c.aux);
                 else
                     e.slot = kNone;  // lost to a better writer
                 if (c.pad) e.slot = kNone;  // continued: already expanded, only its link was due

@@ -34,8 +34,8 @@ struct GridWalkSmem {
 };
 
 // Slot and parent slot of a cell; kNone if the table does not hold it.  Most
-// cells are in their home slot or have it free: the other three of a line are
-// read only for the rest (each is a memory sector of its own).
+// cells are in their home slot or have it free: the other three of its group are
+// read only for the rest.
 __device__ __forceinline__ void find_cell(const Slot *tab, uint64_t mask, uint32_t cell, uint32_t &slot,
                                           uint32_t &prev) {
     const uint64_t home = mix64(cell) & mask;

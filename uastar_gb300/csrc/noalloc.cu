@@ -53,6 +53,8 @@ constexpr uint32_t kHeapCap = 4095;              // entries per heap
 constexpr uint32_t kTableLog2 = 20;              // dedup slots
 constexpr uint64_t kTableSlots = 1ull << kTableLog2;
 constexpr uint64_t kMaxCells = 1ull << 22;       // largest grid accepted (e.g. 2048 x 2048)
+constexpr size_t kTableBytes = kMaxCells * 8;    // a word per cell, or the hashed slots
+static_assert(kTableSlots * sizeof(Slot) <= kTableBytes, "the hashed slots fit");
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // heap block per heap: saved top (64 entries) + 576 bricks of 8 entries
@@ -64,8 +66,7 @@ constexpr size_t kOffSizes = align256(kOffMode + sizeof(uint32_t));
 constexpr size_t kOffCand = align256(kOffSizes + kHeaps * sizeof(uint32_t));
 constexpr size_t kOffHeaps = align256(kOffCand + cand_records<GridProblem>(kCtas, kHeapsPerCta) * sizeof(Cand));
 constexpr size_t kOffTable = align256(kOffHeaps + (size_t)kHeaps * kHeapStride * sizeof(GridEntry));
-constexpr size_t kScratchBytes = align256(kOffTable + kTableSlots * sizeof(Slot));
-static_assert(kMaxCells * 8 <= kTableSlots * sizeof(Slot), "a word per cell fits the table's bytes");
+constexpr size_t kScratchBytes = align256(kOffTable + kTableBytes);
 
 // The only device memory this entry point uses besides the caller's buffers.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
