@@ -101,7 +101,8 @@ __global__ void __launch_bounds__(256) k_ida_cut(P prob, const IdaRoot *in, IdaR
 #pragma unroll
         for (int mv = 0; mv < 4; ++mv) {
             if (!(mask >> mv & 1u)) continue;
-            prob.succ_begin(key, d, r.aux, mv, sc[mv]);
+            prob.succ_key(key, d, mv, sc[mv]);
+            prob.succ_rest(sc[mv]);
             uint64_t nf;
             prob.succ_end(sc[mv], r.aux, mv, naux[mv], nf);
             if (nf > t) {
@@ -169,7 +170,8 @@ __global__ void __launch_bounds__(128) k_ida_pass(P prob, const IdaRoot *roots, 
             const int mv = __ffs(rem[d]) - 1;
             rem[d] &= (uint8_t)(rem[d] - 1);
             typename P::Succ sc;
-            prob.succ_begin(ks[d], g0 + d, as[d], mv, sc);
+            prob.succ_key(ks[d], g0 + d, mv, sc);
+            prob.succ_rest(sc);
             uint32_t naux;
             uint64_t nf;
             prob.succ_end(sc, as[d], mv, naux, nf);

@@ -68,8 +68,9 @@ struct GridProblem : NarrowSlots {
     static constexpr bool kPrevInKey = true;
     static constexpr int kLink = LINK_IN_KEY;
 
-    struct Succ {  // see succ_begin
+    struct Succ {  // see succ_key
         uint64_t key, g, f;
+        int x, y;
     };
     const uint32_t *bm;  // bitmap as 32-bit words (same bytes as the uint64 words)
     int32_t H, W;
@@ -135,6 +136,9 @@ struct GridProblem : NarrowSlots {
     __device__ __forceinline__ uint64_t h_of(uint64_t key) const {
         const uint32_t c = (uint32_t)key;  // H*W < 2^32 is checked on the host
         const int x = (int)row_of(c), y = (int)(c - (uint32_t)x * (uint32_t)W);
+        return h_at(x, y);
+    }
+    __device__ __forceinline__ uint64_t h_at(int x, int y) const {
         const int dx = abs(x - ex), dy = abs(y - ey);
         const int mn = min(dx, dy), mx = max(dx, dy);
         return ((uint64_t)(mx - mn) << 32) | (uint64_t)mn;
@@ -168,9 +172,7 @@ struct GridProblem : NarrowSlots {
         if (y == W - 1) bits &= ~4u;          // (r, W) is no cell (the next row's first)
         return bits;
     }
-    __device__ __forceinline__ void look_begin(uint64_t key, Look &k) const {
-        const uint32_t c = (uint32_t)key;
-        const int x = (int)row_of(c), y = (int)(c - (uint32_t)x * (uint32_t)W);
+    __device__ __forceinline__ void look_begin(int x, int y, Look &k) const {
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             const int r = x - 1 + i;
@@ -183,9 +185,7 @@ struct GridProblem : NarrowSlots {
     // (CPU-solver.cpp:98-100).  A move into a blocked cell is legal in the
     // reference but such a cell has no out-moves, so it is generated only
     // when it is the goal: no path cost changes.
-    __device__ __forceinline__ uint32_t rows_moves(uint64_t key, const Look &k) const {
-        const uint32_t c = (uint32_t)key;
-        const int x = (int)row_of(c), y = (int)(c - (uint32_t)x * (uint32_t)W);
+    __device__ __forceinline__ uint32_t rows_moves(int x, int y, const Look &k) const {
         const uint32_t rows[3] = {row_bits(k.v[0], x - 1, y), row_bits(k.v[1], x, y), row_bits(k.v[2], x + 1, y)};
         if (!(rows[1] & 2u)) return 0;
         uint32_t m = 0;
@@ -198,9 +198,11 @@ struct GridProblem : NarrowSlots {
         return m;
     }
     __device__ __forceinline__ uint32_t moves(uint64_t key, uint32_t) const {
+        const uint32_t c = (uint32_t)key;
+        const int x = (int)row_of(c), y = (int)(c - (uint32_t)x * (uint32_t)W);
         Look k;
-        look_begin(key, k);
-        return rows_moves(key, k);
+        look_begin(x, y, k);
+        return rows_moves(x, y, k);
     }
     // Three passes a round, within 1/64 of the straight distance between the
     // query's ends, 1 to 16.  Measured on 20000^2 (distance 28283), hashed:
@@ -216,12 +218,13 @@ struct GridProblem : NarrowSlots {
         return Expansion{3u, ~0u, slack < 1.f ? 1.f : slack > 16.f ? 16.f : slack};
     }
     // Continuation (ga_search): whether this successor is within the bound, and
-    // the moves of one that is, looked at in look_begin; naux names its
-    // incoming move (entry_moves).
+    // the moves of one that is, reached by move mv (see entry_moves).
     __device__ __forceinline__ bool peek(const Succ &s, float bound) const { return cost_val(s.f) <= bound; }
-    __device__ __forceinline__ uint32_t look_moves(uint64_t key, uint32_t naux, const Look &k) const {
-        uint32_t m = rows_moves(key, k);
-        if (dirs()) m &= ~pruned(naux >> kCellBits);
+    __device__ __forceinline__ uint32_t next_moves(const Succ &s, int mv) const {
+        Look k;
+        look_begin(s.x, s.y, k);
+        uint32_t m = rows_moves(s.x, s.y, k);
+        if (dirs()) m &= ~pruned((uint32_t)mv);
         return m;
     }
     __device__ __forceinline__ static int c_dx(int i) {
@@ -230,22 +233,21 @@ struct GridProblem : NarrowSlots {
     __device__ __forceinline__ static int c_dy(int i) {
         return i < 2 ? 0 : i == 2 ? 1 : i == 3 ? -1 : ((i & 1) ? -1 : 1);
     }
-    __device__ void apply(uint64_t key, uint64_t g, uint32_t, int mv, uint64_t &nkey,
-                          uint64_t &ng, uint32_t &naux, uint64_t &nf) const {
+    // Successor in three steps: its key and g, which its relax needs; the rest
+    // (a grid's f, a puzzle's database load) beside the relax's memory trip; and
+    // what waits for that load, after it.
+    __device__ __forceinline__ void succ_place(uint64_t key, int mv, Succ &s) const {
         const uint32_t c = (uint32_t)key;
         const int x = (int)row_of(c), y = (int)(c - (uint32_t)x * (uint32_t)W);
-        nkey = (uint64_t)(x + c_dx(mv)) * W + (uint64_t)(y + c_dy(mv));
-        ng = g + (mv < 4 ? (1ull << 32) : 1ull);
-        naux = in_aux(nkey, mv);
-        nf = ng + h_of(nkey);
+        s.x = x + c_dx(mv);
+        s.y = y + c_dy(mv);
+        s.key = (uint64_t)s.x * W + (uint64_t)s.y;
     }
-    // Successor in two steps (the puzzle's second step waits on a database
-    // load that is issued in the first, so that it overlaps the table CAS);
-    // for grids everything is register arithmetic in the first.
-    __device__ __forceinline__ void succ_begin(uint64_t key, uint64_t g, uint32_t aux, int mv, Succ &s) const {
-        uint32_t naux;
-        apply(key, g, aux, mv, s.key, s.g, naux, s.f);
+    __device__ __forceinline__ void succ_key(uint64_t key, uint64_t g, int mv, Succ &s) const {
+        succ_place(key, mv, s);
+        s.g = g + (mv < 4 ? (1ull << 32) : 1ull);
     }
+    __device__ __forceinline__ void succ_rest(Succ &s) const { s.f = s.g + h_at(s.x, s.y); }
     __device__ __forceinline__ void succ_end(const Succ &s, uint32_t, int mv, uint32_t &naux, uint64_t &nf) const {
         naux = in_aux(s.key, mv);
         nf = s.f;
@@ -330,22 +332,16 @@ struct GridDirect : GridProblem {
     }
     __device__ __forceinline__ static int cost_cmp(uint64_t a, uint64_t b) { return a < b ? -1 : a > b ? 1 : 0; }
     __device__ __forceinline__ static float cost_val(uint64_t c) { return __ull2float_rn(c) * (1.f / (float)kStraight); }
-    __device__ __forceinline__ uint64_t h_of(uint64_t key) const {
-        const uint64_t h = GridProblem::h_of(key);
-        return (h >> 32 << kFrac) + (uint64_t)(uint32_t)h * kDiag;
+    __device__ __forceinline__ static uint64_t number(uint64_t p) {  // of a cost as a pair
+        return (p >> 32 << kFrac) + (uint64_t)(uint32_t)p * kDiag;
     }
-    __device__ __forceinline__ uint64_t f_of(uint64_t key, uint64_t g, uint32_t) const { return g + h_of(key); }
+    __device__ __forceinline__ uint64_t f_of(uint64_t key, uint64_t g, uint32_t) const { return g + number(h_of(key)); }
     __device__ __forceinline__ bool peek(const Succ &s, float bound) const { return cost_val(s.f) <= bound; }
-    __device__ __forceinline__ void succ_begin(uint64_t key, uint64_t g, uint32_t, int mv, Succ &s) const {
-        const uint32_t c = (uint32_t)key;
-        const int x = (int)row_of(c), y = (int)(c - (uint32_t)x * (uint32_t)W);
-        const int nx = x + c_dx(mv), ny = y + c_dy(mv);
-        s.key = (uint64_t)nx * W + (uint64_t)ny;
+    __device__ __forceinline__ void succ_key(uint64_t key, uint64_t g, int mv, Succ &s) const {
+        succ_place(key, mv, s);
         s.g = g + (mv < 4 ? kStraight : kDiag);
-        const int dx = abs(nx - ex), dy = abs(ny - ey);
-        const int mn = min(dx, dy), mx = max(dx, dy);
-        s.f = s.g + ((uint64_t)(uint32_t)(mx - mn) << kFrac) + (uint64_t)(uint32_t)mn * kDiag;
     }
+    __device__ __forceinline__ void succ_rest(Succ &s) const { s.f = s.g + number(h_at(s.x, s.y)); }
     __device__ __forceinline__ static bool less(const Entry &a, const Entry &b) { return entry_cost(a) < entry_cost(b); }
     __device__ __forceinline__ static const unsigned long long *words(const Slot *tab) {
         return reinterpret_cast<const unsigned long long *>(tab);
@@ -512,16 +508,15 @@ template <int N> struct PuzzleProblem : NarrowSlots {
         if (last) m &= ~(1u << ((last - 1) ^ 1));
         return m;
     }
-    // Two-step successor (see GridProblem::Succ): the first step computes the
-    // board and issues the load of the moved tile's pattern entry, the second
-    // (after the table CAS) folds it into aux and f.
+    // Successor in three steps (see GridProblem): the board; the load of the
+    // moved tile's pattern entry; and what follows from it, aux and f.
     struct Succ {
         uint64_t key, g;
         uint32_t part;  // the loaded pattern entry
         uint32_t which; // its pattern
     };
     static constexpr uint64_t kPatternOf = pattern_bits<N>();
-    __device__ __forceinline__ void succ_begin(uint64_t key, uint64_t g, uint32_t, int mv, Succ &s) const {
+    __device__ __forceinline__ void succ_key(uint64_t key, uint64_t g, int mv, Succ &s) const {
         const int b = blank(key);
         const int q = b + (mv == 0 ? N : mv == 1 ? -N : mv == 2 ? 1 : -1);
         const int t = tile_on(key, q);
@@ -529,8 +524,8 @@ template <int N> struct PuzzleProblem : NarrowSlots {
         s.key = key ^ swap ^ (swap << (4 * t));
         s.g = g + 1;
         s.which = (uint32_t)(kPatternOf >> (2 * t)) & 3u;
-        s.part = part((int)s.which, s.key);
     }
+    __device__ __forceinline__ void succ_rest(Succ &s) const { s.part = part((int)s.which, s.key); }
     __device__ __forceinline__ void succ_end(const Succ &s, uint32_t aux, int mv, uint32_t &naux,
                                              uint64_t &nf) const {
         uint32_t a = aux & 0xffffu;
@@ -554,11 +549,9 @@ template <int N> struct PuzzleProblem : NarrowSlots {
     // Continuation (see GridProblem): f is known only once the pattern entry
     // has arrived (ga_search tests it then), and the moves follow from the
     // board alone.
-    struct Look {};
     __device__ __forceinline__ bool peek(const Succ &, float) const { return true; }
-    __device__ __forceinline__ void look_begin(const uint64_t &, Look &) const {}
-    __device__ __forceinline__ uint32_t look_moves(const uint64_t & key, uint32_t naux, const Look &) const {
-        return moves(key, naux);
+    __device__ __forceinline__ uint32_t next_moves(const Succ &s, int mv) const {
+        return moves(s.key, (uint32_t)(mv + 1) << kLastMoveShift);
     }
     static constexpr bool kEntryKey = false;
     // f in 10 bits, 255 - g in 8 from bit 14 on (every board searched is
@@ -704,7 +697,7 @@ template <> struct PuzzleProblem<5> : WideSlots {
         uint32_t which;  // its pattern
     };
     static constexpr uint64_t kPatternOf = pattern_bits<5>();
-    __device__ __forceinline__ void succ_begin(const Key128 &key, uint64_t g, uint32_t, int mv, Succ &s) const {
+    __device__ __forceinline__ void succ_key(const Key128 &key, uint64_t g, int mv, Succ &s) const {
         const int b = blank(key);
         const int q = b + (mv == 0 ? N : mv == 1 ? -N : mv == 2 ? 1 : -1);
         const int t = tile_on(key, q);
@@ -713,8 +706,8 @@ template <> struct PuzzleProblem<5> : WideSlots {
         s.key.hi = key.hi ^ (t >= 12 && t < 24 ? swap << (5 * (t - 12)) : 0ull);
         s.g = g + 1;
         s.which = (uint32_t)(kPatternOf >> (2 * t)) & 3u;
-        s.part = part((int)s.which, s.key);
     }
+    __device__ __forceinline__ void succ_rest(Succ &s) const { s.part = part((int)s.which, s.key); }
     __device__ __forceinline__ void succ_end(const Succ &s, uint32_t aux, int mv, uint32_t &naux,
                                              uint64_t &nf) const {
         const uint32_t sh = 7u * s.which;
@@ -727,11 +720,9 @@ template <> struct PuzzleProblem<5> : WideSlots {
     // Continuation (see GridProblem): f is known only once the pattern entry
     // has arrived (ga_search tests it then), and the moves follow from the
     // board alone.
-    struct Look {};
     __device__ __forceinline__ bool peek(const Succ &, float) const { return true; }
-    __device__ __forceinline__ void look_begin(const Key128 &, Look &) const {}
-    __device__ __forceinline__ uint32_t look_moves(const Key128 & key, uint32_t naux, const Look &) const {
-        return moves(key, naux);
+    __device__ __forceinline__ uint32_t next_moves(const Succ &s, int mv) const {
+        return moves(s.key, (uint32_t)(mv + 1) << 28);
     }
     static constexpr bool kEntryKey = false;
     __device__ __forceinline__ Entry make_entry(uint64_t f, uint64_t g, uint32_t slot, uint32_t) const {

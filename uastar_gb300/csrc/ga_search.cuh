@@ -151,7 +151,7 @@ __device__ __forceinline__ void named_arrive(uint32_t id, uint32_t n) {
 // their chores.  The grid team has no split form.
 struct GridTeam {
     static constexpr bool kSplit = false;
-    static constexpr bool kBeside = true;
+    static constexpr bool kGroups = true;
     __device__ void early_arrive() {}  // (no split form: never called)
     __device__ void relaxers_sync(uint32_t) {}
     __device__ void late_wait() {}
@@ -176,7 +176,7 @@ struct GridTeam {
 // ones included, so no separate fence is needed.
 struct ClusterTeam {
     static constexpr bool kSplit = true;
-    static constexpr bool kBeside = false;
+    static constexpr bool kGroups = false;
     TeamState *st;  // global memory
     __device__ uint32_t cta() const {
         uint32_t r;
@@ -209,7 +209,7 @@ struct ClusterTeam {
 
 struct BlockTeam {
     static constexpr bool kSplit = true;
-    static constexpr bool kBeside = false;
+    static constexpr bool kGroups = false;
     TeamState *st;  // shared memory
     __device__ uint32_t cta() const { return 0; }
     __device__ uint32_t ctas() const { return 1; }
@@ -610,16 +610,20 @@ template <class P> __device__ __forceinline__ bool key_match(uint64_t word, uint
         return word == key;
 }
 
-template <class P>
+struct NoBeside {
+    __device__ void operator()() const {}
+};
+template <class P, class Beside = NoBeside>
 __device__ __forceinline__ int relax(Slot *tab, uint64_t mask, uint32_t max_probe, uint64_t key, uint64_t g,
-                                     uint32_t prev, uint32_t *slot_out, int mv = -1) {
+                                     uint32_t prev, uint32_t *slot_out, int mv = -1, Beside &&beside = NoBeside()) {
     const KeyG mine{P::kPrevInKey ? (key | (uint64_t)prev << 32) : key, P::g_word(g, prev, mv)};
     const uint64_t home = mix64(key) & mask;
     uint64_t h = home;
     uint32_t i = 0;
     KeyG cur{kEmptyKey, kInfCost};  // what the CAS expects
+    KeyG old = cas128(tab + h, cur, mine);
+    beside();
     for (;;) {
-        const KeyG old = cas128(tab + h, cur, mine);
         if (old.key == cur.key && old.g == cur.g) {
             *slot_out = (uint32_t)h;
             return old.key == kEmptyKey ? RELAX_INSERTED : RELAX_IMPROVED;
@@ -634,6 +638,7 @@ __device__ __forceinline__ int relax(Slot *tab, uint64_t mask, uint32_t max_prob
             if (++i >= max_probe) return RELAX_FULL;
             h = probe_slot(home, i, mask);
         }
+        old = cas128(tab + h, cur, mine);
     }
 }
 
@@ -649,15 +654,16 @@ __device__ __forceinline__ int relax(Slot *tab, uint64_t mask, uint32_t max_prob
 // group by group; changing over at a third, a fifth, an eighth: 2.56 / 2.27 / 2.28
 // ms for a 58-move board.  CTA and cluster teams stay with slots: 64 grids up to
 // 1500^2 21.8 -> 18.9 ms, 160 15-puzzles 56.6 -> 53.2.
-template <class P>
-__device__ __forceinline__ int relax_beside(Slot *tab, uint64_t mask, uint32_t max_probe, uint64_t key, uint64_t g,
-                                            uint32_t prev, uint32_t *slot_out, int mv = -1) {
+template <class P, class Beside>
+__device__ __forceinline__ int relax_group(Slot *tab, uint64_t mask, uint32_t max_probe, uint64_t key, uint64_t g,
+                                           uint32_t prev, uint32_t *slot_out, int mv, Beside &&beside) {
     const KeyG mine{P::kPrevInKey ? (key | (uint64_t)prev << 32) : key, P::g_word(g, prev, mv)};
     const uint64_t home = mix64(key) & mask;
     uint64_t h = home;              // the slot at probe index i
     uint32_t i = 0;
     KeyG cur{kEmptyKey, kInfCost};  // what the CAS expects there
-    bool cas = true, look = true;  // this turn's accesses: CAS slot h; read the slots i (+ 1 with a CAS) .. end of line
+    // this turn's accesses: CAS slot h; read the slots i (+ 1 with a CAS) .. end of the group
+    bool cas = true, look = true, first = true;
     for (;;) {
         const uint32_t from = i + (cas ? 1u : 0u), n = look ? 4u - (i & 3u) - (cas ? 1u : 0u) : 0u;
         ulonglong2 v[4];
@@ -667,6 +673,8 @@ __device__ __forceinline__ int relax_beside(Slot *tab, uint64_t mask, uint32_t m
         KeyG old = cur;
         if (cas) {
             old = cas128(tab + h, cur, mine);
+            if (first) beside();
+            first = false;
             if (old.key == cur.key && old.g == cur.g) {
                 *slot_out = (uint32_t)h;
                 return old.key == kEmptyKey ? RELAX_INSERTED : RELAX_IMPROVED;
@@ -685,7 +693,7 @@ __device__ __forceinline__ int relax_beside(Slot *tab, uint64_t mask, uint32_t m
                     cur = KeyG{v[q].x, v[q].y};
                 }
             i = from + at;
-            if (at == n) {  // none: the next line
+            if (at == n) {  // none: the next group
                 if (i >= max_probe) return RELAX_FULL;
                 cas = false;
                 continue;
@@ -711,11 +719,12 @@ __device__ __forceinline__ int relax_beside(Slot *tab, uint64_t mask, uint32_t m
 // Wide keys: find-or-claim the 16-byte key with one 16-byte CAS per probed
 // slot, then lower the slot's g with an 8-byte CAS loop.  A claimer whose g
 // another writer of the same key has already undercut reports RELAX_CLAIMED.
-template <class P>
+template <class P, class Beside>
 __device__ __forceinline__ int relax_wide(Slot *tab, uint64_t mask, uint32_t max_probe, const Key128 &key,
-                                          uint64_t g, uint32_t *slot_out) {
+                                          uint64_t g, uint32_t *slot_out, Beside &&beside) {
     const uint64_t home = key_hash(key) & mask;
     const KeyG empty{kEmptyKey, kEmptyKey};
+    beside();  // (between the CAS and its use, or with the next moves, it cost up to 8 %)
     for (uint32_t probe = 0; probe < max_probe; ++probe) {
         const uint64_t h = probe_slot(home, probe, mask);
         const KeyG cur = cas128(WideSlots::at(tab, h), empty, KeyG{key.lo, key.hi});
@@ -737,25 +746,33 @@ __device__ __forceinline__ int relax_wide(Slot *tab, uint64_t mask, uint32_t max
 
 // One word per cell (GridDirect).  Of two moves that reach a cell at the same g
 // the lower-numbered one stays: both are shortest so far.
-template <class P>
-__device__ __forceinline__ int relax_direct(Slot *tab, uint64_t key, uint64_t g, uint32_t *slot_out, int mv) {
+template <class P, class Beside>
+__device__ __forceinline__ int relax_direct(Slot *tab, uint64_t key, uint64_t g, uint32_t *slot_out, int mv,
+                                            Beside &&beside) {
     const unsigned long long old = atomicMin(reinterpret_cast<unsigned long long *>(tab) + key,
                                              (unsigned long long)(g << 3 | (uint32_t)max(mv, 0)));
+    beside();
     *slot_out = (uint32_t)key;
     return old == kInfCost ? RELAX_INSERTED : (old >> 3) > g ? RELAX_IMPROVED : RELAX_NONE;
 }
 
-template <class P, bool kBeside = false>
+// A relax of any problem.  `beside` is work that needs none of its result: it
+// runs once, while the first access is in flight (a successor's f and next
+// moves, a puzzle's rank and database load: ~600 cycles of a grid's 4200-cycle
+// pass.  20000^2 104 -> 98 ms, a query on 1537 x 2049 3.05 -> 2.85 us a step, a
+// 58-move 15-puzzle 8.9 -> 8.4).  `grouped`: relax_group.
+template <class P, bool kGroups = false, class Beside = NoBeside>
 __device__ __forceinline__ int relax_key(Slot *tab, uint64_t mask, uint32_t max_probe, const typename P::Key &key,
-                                         uint64_t g, uint32_t prev, uint32_t *slot_out, int mv = -1, bool beside = false) {
+                                         uint64_t g, uint32_t prev, uint32_t *slot_out, int mv = -1,
+                                         bool grouped = false, Beside &&beside = NoBeside()) {
     if constexpr (P::kWide)
-        return relax_wide<P>(tab, mask, max_probe, key, g, slot_out);
+        return relax_wide<P>(tab, mask, max_probe, key, g, slot_out, beside);
     else if constexpr (P::kDirect)
-        return relax_direct<P>(tab, key, g, slot_out, mv);
-    else if (kBeside && beside)
-        return relax_beside<P>(tab, mask, max_probe, key, g, prev, slot_out, mv);
+        return relax_direct<P>(tab, key, g, slot_out, mv, beside);
+    else if (kGroups && grouped)
+        return relax_group<P>(tab, mask, max_probe, key, g, prev, slot_out, mv, beside);
     else
-        return relax<P>(tab, mask, max_probe, key, g, prev, slot_out, mv);
+        return relax<P>(tab, mask, max_probe, key, g, prev, slot_out, mv, beside);
 }
 
 __device__ __forceinline__ Cand load_cand(const Cand *p) {
@@ -796,7 +813,7 @@ struct RoundState {
     uint32_t cont;                 // its continuation passes at most
     uint32_t status, pause;        // the last decision
     uint32_t nshare;               // candidates in this CTA's share
-    uint32_t beside;               // 1: relaxes read the home group beside the first CAS (relax_beside)
+    uint32_t grouped;              // 1: relaxes read the home group beside the first CAS (relax_group)
 };
 static_assert(sizeof(RoundState) == 88, "22 words of the scratch");
 
@@ -1015,7 +1032,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
     if (lead) {
         rs->gbest = team.rd64(&st->goal_best);
         rs->inserted = team.rd64(&st->inserted);
-        rs->beside = rs->inserted * 6 > m.mask;
+        rs->grouped = rs->inserted * 6 > m.mask;
         rs->rounds = round0;
         rs->steps = team.rd64(&st->steps);
         rs->stop_at = budget < ~rs->steps ? rs->steps + budget : ~0ull;
@@ -1260,7 +1277,8 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                     const PopInfo<Key> &pi = source(q);
                     const int move = nth_bit(pi.mask, q);
                     typename P::Succ sc;
-                    prob.succ_begin(pi.key, pi.g, pi.aux, move, sc);
+                    prob.succ_key(pi.key, pi.g, move, sc);
+                    prob.succ_rest(sc);
                     uint32_t naux;
                     uint64_t nf;
                     prob.succ_end(sc, pi.aux, move, naux, nf);
@@ -1305,13 +1323,17 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                         const uint32_t acts = __ballot_sync(kFull, act);
                         if (lane == 0) atomicAdd(&s_stat[1], (uint32_t)__popc(acts));
                         if (act) {
-                            prob.succ_begin(pkey, pg, paux, move, sc);
-                            // the successor's neighbourhood is read beside the CAS
-                            typename P::Look look;
-                            const bool peek = pass < rs->cont && prob.peek(sc, rs->bound);
-                            if (peek) prob.look_begin(sc.key, look);
-                            const int r =
-                                relax_key<P, Team::kBeside>(m.tab, m.mask, m.max_probe, sc.key, sc.g, oslot, &nslot, move, rs->beside);
+                            prob.succ_key(pkey, pg, move, sc);
+                            // the rest of the successor, and the moves that
+                            // follow it, beside the relax
+                            bool peek = false;
+                            const int r = relax_key<P, Team::kGroups>(
+                                m.tab, m.mask, m.max_probe, sc.key, sc.g, oslot, &nslot, move, rs->grouped, [&] {
+                                    prob.succ_rest(sc);
+                                    peek = pass < rs->cont && prob.peek(sc, rs->bound);
+                                    if constexpr (!P::kWide)
+                                        if (peek) mask = prob.next_moves(sc, move);
+                                });
                             prob.succ_end(sc, paux, move, naux, nf);
                             if constexpr (P::kDirect)
                                 if (nf >= P::kLimit) set_error(&st->err[r3], ST_COST_RANGE);
@@ -1324,7 +1346,8 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                             if (improved) {
                                 goal = prob.is_goal(sc.key);
                                 cand = peek && !goal && P::cost_val(nf) <= rs->bound && P::cost_cmp(nf, rs->gbest) < 0;
-                                if (cand) mask = prob.look_moves(sc.key, naux, look);
+                                if constexpr (P::kWide)
+                                    if (cand) mask = prob.next_moves(sc, move);
                                 if constexpr (P::kLink != LINK_FIELD) {
                                     // the goal's link is in place: the decision
                                     // may take it this round, no pop needed
@@ -1337,6 +1360,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
                                 }
                             }
                         }
+                        if (!cand) mask = 0;
                         const uint32_t ib = __ballot_sync(kFull, inserted);
                         if (ib && lane == (uint32_t)(__ffs(ib) - 1)) atomicAdd(s_ins, (uint32_t)__popc(ib));
                         // nodes to continue: as many (in lane order) as have at
@@ -1438,7 +1462,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             uint64_t gbest = rs->gbest;
             if (P::cost_cmp(gmin, gbest) < 0) rs->gbest = gbest = gmin;
             const uint64_t inserted = rs->inserted += ins;
-            rs->beside = inserted * 6 > m.mask;
+            rs->grouped = inserted * 6 > m.mask;
             const uint64_t steps = rs->steps += 1 + pass;
             rs->rounds += 1;
             uint32_t err = e1 ? e1 : e2;
