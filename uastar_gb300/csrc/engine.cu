@@ -144,8 +144,8 @@ __device__ void walk_boards_dev(const WideSlot *tab, uint32_t goal_slot, unsigne
     uint64_t n = 0;
     while (s != kNone && n < cap) {
         const WideSlot *w = tab + s;
-        keys[2 * n] = __ldcg(&w->lo);
-        keys[2 * n + 1] = __ldcg(&w->hi);
+        keys[2 * n] = __ldcg(&w->lo) & WideSlots::kKeyMask;
+        keys[2 * n + 1] = __ldcg(&w->hi) & WideSlots::kKeyMask;
         ++n;
         s = __ldcg(&w->prev);
     }

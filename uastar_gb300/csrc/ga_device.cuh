@@ -44,14 +44,17 @@ static_assert(sizeof(Slot) == 16, "a slot is one CAS");
 
 // Slot access by key width.  Narrow keys (grid cells, boards of up to 16
 // cells in 4-bit fields) use the layout above; wide keys (a 5x5 board: 24
-// cells in 5-bit fields, the 25th implied) slots of 32 bytes: the 16-byte key is
-// claimed with one 16-byte CAS and g is lowered with its own 8-byte CAS.  A
-// table is a Slot pointer in either case; at() finds its i-th slot.
+// cells in 5-bit fields, the 25th implied) slots of 32 bytes, the first 16 of
+// them for the CAS: 60 bits of the key in each word and 4 of g above them (g =
+// the moves from the start: at most 208 lie between two boards, and a search
+// looks a few further).  A table is a Slot pointer in either case; at() finds
+// its i-th slot.
 struct Key128 {
     unsigned long long lo, hi;
 };
 struct __align__(32) WideSlot {
-    unsigned long long lo, hi, g;
+    unsigned long long lo, hi;  // key | g in the top bits (WideSlots)
+    unsigned long long pad;
     uint32_t aux, prev;
 };
 static_assert(sizeof(WideSlot) == 32, "wide slot must be one sector");
@@ -63,6 +66,11 @@ static_assert(sizeof(WideSlot) == 32, "wide slot must be one sector");
 // same 16-byte CAS that sets g, so the push phase checks no winner.
 enum SlotLink : int { LINK_FIELD = 0, LINK_IN_KEY = 1, LINK_IN_G = 2 };
 
+// The first 16 bytes of a slot, set by one CAS.
+struct __align__(16) KeyG {
+    unsigned long long key, g;
+};
+
 struct NarrowSlots {
     using Key = uint64_t;
     static constexpr bool kWide = false;
@@ -70,9 +78,6 @@ struct NarrowSlots {
     static constexpr bool kPrevInKey = false;  // see GridProblem
     static constexpr size_t kSlotBytes = sizeof(Slot);
     __device__ static Slot *at(Slot *tab, uint64_t i) { return tab + i; }
-    // the g word that the relax CAS installs, and its cost
-    __device__ static uint64_t g_word(uint64_t g, uint32_t, int) { return g; }
-    __device__ static uint64_t word_g(uint64_t w) { return w; }
 };
 struct WideSlots {
     using Key = Key128;
@@ -84,8 +89,21 @@ struct WideSlots {
     __device__ static Slot *at(Slot *tab, uint64_t i) { return reinterpret_cast<Slot *>(w(tab) + i); }
     __device__ static const WideSlot *w(const Slot *s) { return reinterpret_cast<const WideSlot *>(s); }
     __device__ static WideSlot *w(Slot *s) { return reinterpret_cast<WideSlot *>(s); }
-    __device__ static uint64_t slot_g(const Slot *s) { return __ldcg(&w(s)->g); }
-    __device__ static uint32_t slot_prev(const Slot *s) { return __ldcg(&w(s)->prev); }
+    static constexpr int kKeyBits = 60;
+    static constexpr unsigned long long kKeyMask = (1ull << kKeyBits) - 1;
+    __device__ static KeyG cas_word(const Key128 &k, uint64_t g, uint32_t, int) {
+        return KeyG{k.lo | g << kKeyBits, k.hi | g >> 4 << kKeyBits};
+    }
+    __device__ static Key128 word_key(KeyG w) { return Key128{w.key & kKeyMask, w.g & kKeyMask}; }
+    __device__ static bool word_is(KeyG w, const Key128 &k) {
+        return (w.key & kKeyMask) == k.lo && (w.g & kKeyMask) == k.hi;
+    }
+    __device__ static uint64_t word_g(KeyG w) { return w.key >> kKeyBits | w.g >> kKeyBits << 4; }
+    __device__ static KeyG cas_half(const Slot *s) {
+        const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2 *>(s));
+        return KeyG{v.x, v.y};
+    }
+    __device__ static uint64_t slot_g(const Slot *s) { return word_g(cas_half(s)); }
     __device__ static void set_link(Slot *s, uint32_t prev, uint32_t aux) {
         w(s)->prev = prev;
         w(s)->aux = aux;

@@ -29,11 +29,11 @@ __global__ void k_grow_move(const Slot *src, uint64_t n, Slot *dst, uint64_t mas
         if (key == kEmptyKey) continue;
         uint64_t h;
         if constexpr (Wide) {
-            const Key128 k{key, ((unsigned long long)a.w << 32) | a.z};
-            const uint64_t home = key_hash(k) & mask;
+            const KeyG k{key, ((unsigned long long)a.w << 32) | a.z};
+            const uint64_t home = key_hash(WideSlots::word_key(k)) & mask;
             h = home;
             for (uint32_t probe = 1; probe <= mask; ++probe) {
-                const KeyG old = cas128(WideSlots::at(dst, h), KeyG{kEmptyKey, kEmptyKey}, KeyG{k.lo, k.hi});
+                const KeyG old = cas128(WideSlots::at(dst, h), KeyG{kEmptyKey, kEmptyKey}, k);
                 if (old.key == kEmptyKey && old.g == kEmptyKey) break;
                 h = probe_slot(home, probe, mask);
             }
@@ -46,8 +46,8 @@ __global__ void k_grow_move(const Slot *src, uint64_t n, Slot *dst, uint64_t mas
             }
         }
         uint4 *d = reinterpret_cast<uint4 *>(dst) + h * words;
-        d[0] = a;                                  // key and g (narrow), key (wide)
-        if constexpr (Wide) d[1] = __ldcg(from + 1);  // g, aux, prev (old index)
+        d[0] = a;                                     // key and g
+        if constexpr (Wide) d[1] = __ldcg(from + 1);  // aux, prev (old index)
         map[s] = (uint32_t)h;
     }
 }

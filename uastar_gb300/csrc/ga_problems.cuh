@@ -67,6 +67,13 @@ struct GridProblem : NarrowSlots {
     // sets g and the parent link together, so no push-phase winner check.
     static constexpr bool kPrevInKey = true;
     static constexpr int kLink = LINK_IN_KEY;
+    __device__ static KeyG cas_word(uint64_t key, uint64_t g, uint32_t prev, int) {
+        return KeyG{key | (uint64_t)prev << 32, g};
+    }
+    __device__ static bool word_is(KeyG w, uint64_t key) {
+        return (w.key & 0xffffffffull) == key && w.key != kEmptyKey;
+    }
+    __device__ static uint64_t word_g(KeyG w) { return w.g; }
 
     struct Succ {  // see succ_key
         uint64_t key, g, f;
@@ -419,10 +426,11 @@ template <int N> struct PuzzleProblem : NarrowSlots {
     // The pattern parts depend on the board alone and travel in its entries
     // (make_entry).
     static constexpr int kLink = LINK_IN_G;
-    __device__ static uint64_t g_word(uint64_t g, uint32_t prev, int mv) {
-        return g << 40 | (uint64_t)(uint32_t)(mv + 1) << 32 | prev;
+    __device__ static KeyG cas_word(uint64_t key, uint64_t g, uint32_t prev, int mv) {
+        return KeyG{key, g << 40 | (uint64_t)(uint32_t)(mv + 1) << 32 | prev};
     }
-    __device__ static uint64_t word_g(uint64_t w) { return w >> 40; }
+    __device__ static bool word_is(KeyG w, uint64_t key) { return w.key == key; }
+    __device__ static uint64_t word_g(KeyG w) { return w.g >> 40; }
 
     // The key is the board's inverse: nibble t = cell of tile t (tile 0 = the
     // blank), nibbles past the last tile all ones (no cell has that number).
@@ -589,8 +597,11 @@ template <int N> struct PuzzleProblem : NarrowSlots {
 // ------------------------------------------------------- 24-puzzle ---
 // 5x5 board, 128-bit key: the cells of tiles 0 (the blank) .. 11 in `lo` and
 // 12 .. 23 in `hi`, 5 bits each; tile 24's cell is implied (the cells sum to
-// 300), so every state has one key and bits 60..63 of both words stay zero
-// (the all-ones empty key is never a board).  aux = the four pattern parts, 7
+// 300), so every state has one key and bits 60..63 of both words are left for g
+// (WideSlots; the all-ones empty key is never a board).  With g in the CAS that
+// claims the key, a relax of a new board takes one memory trip instead of two
+// and of an old one two instead of three: a step of three boards of 60 random
+// moves 7.2 / 7.9 / 5.3 -> 5.9 / 6.9 / 4.5 us.  aux = the four pattern parts, 7
 // bits each, | (last move + 1) << 28.
 template <> struct PuzzleProblem<5> : WideSlots {
     using Entry = PuzzleEntry;
@@ -745,12 +756,10 @@ template <> struct PuzzleProblem<5> : WideSlots {
     }
     __device__ __forceinline__ static void load_node(const Slot *s, const Entry &, Key128 &key, uint64_t &g,
                                                      uint32_t &aux) {
-        const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2 *>(s));
-        const ulonglong2 w = __ldcg(reinterpret_cast<const ulonglong2 *>(s) + 1);
-        key.lo = v.x;
-        key.hi = v.y;
-        g = w.x;
-        aux = (uint32_t)w.y;
+        const KeyG v = cas_half(s);
+        key = word_key(v);
+        g = word_g(v);
+        aux = __ldcg(&w(s)->aux);
     }
 };
 

@@ -577,10 +577,6 @@ __device__ __forceinline__ bool atomic_min_cost(unsigned long long *addr, uint64
     return false;
 }
 
-// (key, g) half of a slot, updated as one 16-byte word.
-struct __align__(16) KeyG {
-    unsigned long long key, g;
-};
 __device__ __forceinline__ KeyG cas128(Slot *s, KeyG cmp, KeyG val) {
     return atomicCAS(reinterpret_cast<KeyG *>(s), cmp, val);
 }
@@ -590,46 +586,36 @@ __device__ __forceinline__ KeyG cas128(Slot *s, KeyG cmp, KeyG val) {
 enum : int { RELAX_NONE = 0, RELAX_IMPROVED = 1, RELAX_CLAIMED = 2, RELAX_INSERTED = 3, RELAX_FULL = 4 };
 
 // Find-or-insert `key` and lower its g to `g` (the probe order is
-// probe_slot's): one 16-byte CAS per turn, which claims the slot empty with
-// (key, g), lowers the key's g, or returns what the slot holds.  The lanes of a
-// warp take their turns together, and a warp waits for its slowest lane, so the
-// number of turns is the relax phase.  Returns RELAX_INSERTED (new slot, g set),
-// RELAX_IMPROVED (existing slot, g strictly lowered), RELAX_NONE (existing slot,
-// g not better) or RELAX_FULL (probe limit).
-//
-// Where the problem keeps the parent link in the key word (P::kPrevInKey:
-// grid cells are 32 bits), the word is cell | prev << 32 and the CAS sets g
-// and prev together, so the slot's link always belongs to its g: the push
-// phase then needs no winner check.  Keys compare on the cell half.  Where it
-// keeps the link in the g word (P::kLink == LINK_IN_G), the CAS installs
-// P::g_word(g, prev, move) and costs compare on P::word_g of it.
-template <class P> __device__ __forceinline__ bool key_match(uint64_t word, uint64_t key) {
-    if constexpr (P::kPrevInKey)
-        return (word & 0xffffffffull) == key && word != kEmptyKey;
-    else
-        return word == key;
-}
-
+// probe_slot's): one 16-byte CAS per turn on the slot's first 16 bytes, which
+// hold the key, g and, but for wide keys, the parent link (P::cas_word): it
+// claims the slot empty, lowers the key's g, or returns what the slot holds.
+// So a slot's link always belongs to its g, and the push phase needs no winner
+// check.  The lanes of a warp take their turns together, and a warp waits for
+// its slowest lane, so the number of turns is the relax phase.  Returns
+// RELAX_INSERTED (new slot, g set), RELAX_IMPROVED (existing slot, g strictly
+// lowered), RELAX_NONE (existing slot, g not better) or RELAX_FULL (probe
+// limit).
 struct NoBeside {
     __device__ void operator()() const {}
 };
 template <class P, class Beside = NoBeside>
-__device__ __forceinline__ int relax(Slot *tab, uint64_t mask, uint32_t max_probe, uint64_t key, uint64_t g,
-                                     uint32_t prev, uint32_t *slot_out, int mv = -1, Beside &&beside = NoBeside()) {
-    const KeyG mine{P::kPrevInKey ? (key | (uint64_t)prev << 32) : key, P::g_word(g, prev, mv)};
-    const uint64_t home = mix64(key) & mask;
+__device__ __forceinline__ int relax(Slot *tab, uint64_t mask, uint32_t max_probe, const typename P::Key &key,
+                                     uint64_t g, uint32_t prev, uint32_t *slot_out, int mv = -1,
+                                     Beside &&beside = NoBeside()) {
+    const KeyG mine = P::cas_word(key, g, prev, mv);
+    const uint64_t home = key_hash(key) & mask;
     uint64_t h = home;
     uint32_t i = 0;
-    KeyG cur{kEmptyKey, kInfCost};  // what the CAS expects
-    KeyG old = cas128(tab + h, cur, mine);
+    KeyG cur{kEmptyKey, kEmptyKey};  // what the CAS expects
+    KeyG old = cas128(P::at(tab, h), cur, mine);
     beside();
     for (;;) {
         if (old.key == cur.key && old.g == cur.g) {
             *slot_out = (uint32_t)h;
-            return old.key == kEmptyKey ? RELAX_INSERTED : RELAX_IMPROVED;
+            return old.key == kEmptyKey && old.g == kEmptyKey ? RELAX_INSERTED : RELAX_IMPROVED;
         }
-        if (key_match<P>(old.key, key)) {
-            if (P::cost_cmp(g, P::word_g(old.g)) >= 0) {
+        if (P::word_is(old, key)) {
+            if (P::cost_cmp(g, P::word_g(old)) >= 0) {
                 *slot_out = (uint32_t)h;
                 return RELAX_NONE;
             }
@@ -638,7 +624,7 @@ __device__ __forceinline__ int relax(Slot *tab, uint64_t mask, uint32_t max_prob
             if (++i >= max_probe) return RELAX_FULL;
             h = probe_slot(home, i, mask);
         }
-        old = cas128(tab + h, cur, mine);
+        old = cas128(P::at(tab, h), cur, mine);
     }
 }
 
@@ -657,8 +643,8 @@ __device__ __forceinline__ int relax(Slot *tab, uint64_t mask, uint32_t max_prob
 template <class P, class Beside>
 __device__ __forceinline__ int relax_group(Slot *tab, uint64_t mask, uint32_t max_probe, uint64_t key, uint64_t g,
                                            uint32_t prev, uint32_t *slot_out, int mv, Beside &&beside) {
-    const KeyG mine{P::kPrevInKey ? (key | (uint64_t)prev << 32) : key, P::g_word(g, prev, mv)};
-    const uint64_t home = mix64(key) & mask;
+    const KeyG mine = P::cas_word(key, g, prev, mv);
+    const uint64_t home = key_hash(key) & mask;
     uint64_t h = home;              // the slot at probe index i
     uint32_t i = 0;
     KeyG cur{kEmptyKey, kInfCost};  // what the CAS expects there
@@ -680,7 +666,7 @@ __device__ __forceinline__ int relax_group(Slot *tab, uint64_t mask, uint32_t ma
                 return old.key == kEmptyKey ? RELAX_INSERTED : RELAX_IMPROVED;
             }
         }
-        if (cas && key_match<P>(old.key, key)) {
+        if (cas && P::word_is(old, key)) {
             cur = old;
             look = false;
         } else if (look) {
@@ -688,7 +674,7 @@ __device__ __forceinline__ int relax_group(Slot *tab, uint64_t mask, uint32_t ma
             uint32_t at = n;
 #pragma unroll
             for (uint32_t q = 4; q-- > 0;)
-                if (q < n && (v[q].x == kEmptyKey || key_match<P>(v[q].x, key))) {
+                if (q < n && (v[q].x == kEmptyKey || P::word_is(KeyG{v[q].x, v[q].y}, key))) {
                     at = q;
                     cur = KeyG{v[q].x, v[q].y};
                 }
@@ -709,39 +695,11 @@ __device__ __forceinline__ int relax_group(Slot *tab, uint64_t mask, uint32_t ma
             look = true;
             continue;
         }
-        if (cur.key != kEmptyKey && P::cost_cmp(g, P::word_g(cur.g)) >= 0) {
+        if (cur.key != kEmptyKey && P::cost_cmp(g, P::word_g(cur)) >= 0) {
             *slot_out = (uint32_t)h;
             return RELAX_NONE;
         }
     }
-}
-
-// Wide keys: find-or-claim the 16-byte key with one 16-byte CAS per probed
-// slot, then lower the slot's g with an 8-byte CAS loop.  A claimer whose g
-// another writer of the same key has already undercut reports RELAX_CLAIMED.
-template <class P, class Beside>
-__device__ __forceinline__ int relax_wide(Slot *tab, uint64_t mask, uint32_t max_probe, const Key128 &key,
-                                          uint64_t g, uint32_t *slot_out, Beside &&beside) {
-    const uint64_t home = key_hash(key) & mask;
-    const KeyG empty{kEmptyKey, kEmptyKey};
-    beside();  // (between the CAS and its use, or with the next moves, it cost up to 8 %)
-    for (uint32_t probe = 0; probe < max_probe; ++probe) {
-        const uint64_t h = probe_slot(home, probe, mask);
-        const KeyG cur = cas128(WideSlots::at(tab, h), empty, KeyG{key.lo, key.hi});
-        const bool claimed = cur.key == kEmptyKey && cur.g == kEmptyKey;
-        if (claimed || (cur.key == key.lo && cur.g == key.hi)) {
-            *slot_out = (uint32_t)h;
-            unsigned long long *gp = &WideSlots::w(WideSlots::at(tab, h))->g;
-            unsigned long long old = claimed ? kInfCost : __ldcg(gp);
-            while (P::cost_cmp(g, old) < 0) {
-                const unsigned long long seen = atomicCAS(gp, old, (unsigned long long)g);
-                if (seen == old) return claimed ? RELAX_INSERTED : RELAX_IMPROVED;
-                old = seen;
-            }
-            return claimed ? RELAX_CLAIMED : RELAX_NONE;
-        }
-    }
-    return RELAX_FULL;
 }
 
 // One word per cell (GridDirect).  Of two moves that reach a cell at the same g
@@ -765,14 +723,13 @@ template <class P, bool kGroups = false, class Beside = NoBeside>
 __device__ __forceinline__ int relax_key(Slot *tab, uint64_t mask, uint32_t max_probe, const typename P::Key &key,
                                          uint64_t g, uint32_t prev, uint32_t *slot_out, int mv = -1,
                                          bool grouped = false, Beside &&beside = NoBeside()) {
-    if constexpr (P::kWide)
-        return relax_wide<P>(tab, mask, max_probe, key, g, slot_out, beside);
-    else if constexpr (P::kDirect)
+    if constexpr (P::kDirect) {
         return relax_direct<P>(tab, key, g, slot_out, mv, beside);
-    else if (kGroups && grouped)
-        return relax_group<P>(tab, mask, max_probe, key, g, prev, slot_out, mv, beside);
-    else
+    } else {
+        if constexpr (kGroups && !P::kWide)
+            if (grouped) return relax_group<P>(tab, mask, max_probe, key, g, prev, slot_out, mv, beside);
         return relax<P>(tab, mask, max_probe, key, g, prev, slot_out, mv, beside);
+    }
 }
 
 __device__ __forceinline__ Cand load_cand(const Cand *p) {
