@@ -62,7 +62,8 @@ typedef struct {
     int32_t block_threads;   /* CTA size of the plain engine's persistent kernel (0 -> 256) */
     int32_t heap_capacity;   /* entries per heap (0 -> auto, grown on overflow) */
     int32_t hash_log2_slots; /* dedup table = 2^n slots of 16 B (5x5: 32 B), n <= 31 (0 -> sized from the instance and
-                              grown 4x in place whenever it is half full).  A grid that fits these bytes
+                              grown 4x in place when a quarter full, 5x5 and from 2^27 slots on
+                              half full).  A grid that fits these bytes
                               with 8 a cell has one word per cell there; max_load * 2^n limits its
                               states all the same */
     double max_load;         /* dedup table load limit in (0,1) (0 -> 0.8) */
@@ -293,8 +294,8 @@ typedef struct {
  * on one with its own heap slice and dedup partition, under a budget of
  * expansion steps (tier1_rounds); grids above 2048^2 and the instances that ran
  * out of steps or space go to a second wave of 8-CTA cluster teams with a larger
- * partition (32x after an overflow, else what their budget of steps can fill, 8x
- * by default; puzzles under tier2_puzzle_rounds), and what fails there is
+ * partition (32x after an overflow, else sized by what their budget of steps can
+ * fill, 16x by default; puzzles under tier2_puzzle_rounds), and what fails there is
  * solved by the plain engine, one instance at a time.  The last instances of a
  * wave (few enough to leave most of the GPU idle) move on without using up
  * their budget.  No counterpart in the

@@ -968,15 +968,16 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
         rc = run_wave(eng, insts, tier1, g, m, use_graph, b1, 0, 2 * clusters, 256, results, stats, &retry);
         if (rc) return rc;
         // Space for the next tier: 16x after an overflow.  One that ran out of
-        // steps or gave up its team gets what it can fill there, a puzzle by its
-        // budget of steps (384 new states each at 256 heaps), a grid by its
-        // cells: a partition is cleared by its team before the search, 1 GB per
-        // puzzle at 16x.  96 mixed instances 50.6 -> 46.3 ms, 160 15-puzzles
-        // 64.3 -> 56.3, 64 grids up to 1500^2 24.3 -> 21.7 (8x: 45.9 / 57.1 / 22.4,
-        // 2x: 52.2 / 59.9 / 21.4).
+        // steps or gave up its team gets what it can fill there to a third, a
+        // puzzle by its budget of steps (384 new states each at 256 heaps), a
+        // grid by its cells: a partition is cleared by its team before the
+        // search, 0.5 GB per puzzle at 16x, but a relax slows down as it fills.
+        // 96 mixed instances 16x / 8x / 4x: 50.6 / 45.9 / 46.3 ms, 160 15-puzzles
+        // 64.3 / 57.1 / 56.3 (32-byte slots); with 16-byte ones 8x / 4x 38.0 /
+        // 41.4 and 46.4 / 47.9.  64 grids up to 1500^2 16x / 4x 24.3 / 21.7.
         for (int i : retry) {
             const bool over = results[i].status == UASTAR_HASH_FULL || results[i].status == UASTAR_HEAP_OVERFLOW;
-            const uint64_t fill = insts[i].kind == UASTAR_KIND_PUZZLE ? std::clamp<uint64_t>(b2 / 4096, 4, 16) : 4;
+            const uint64_t fill = insts[i].kind == UASTAR_KIND_PUZZLE ? std::clamp<uint64_t>(b2 / 2048, 8, 16) : 4;
             mult[i] = over ? 16 : (int)fill;
             tier2.push_back(i);
         }
@@ -1026,11 +1027,11 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
                 stats->generated += gr.generated;
             }
         } else {
-            // the plain engine starts this puzzle's table at 2^26 slots: it
+            // the plain engine starts this puzzle's table at 2^27 slots: it
             // filled a cluster's partition or ran out of its round budget
             // there, and every 4x growth on the way up pauses the search
             uastar_puzzle_result pr;
-            eng->puzzle_log2_start = 26;
+            eng->puzzle_log2_start = 27;
             rc = uastar_puzzle_solve(eng, in.n, in.tiles, &pr);
             eng->puzzle_log2_start = 0;
             r.status = pr.status;
@@ -1313,7 +1314,7 @@ static void serve_complete(ServeState *S, ServeReq &r, int32_t status) {
 
 // A request's first dedup partition: its estimate, but at most 2^20 slots
 // times its growth multiplier; the search grows it 4x in place whenever it
-// is half full (serve_grow), so admission reserves what a request has shown
+// is a quarter full (serve_grow), so admission reserves what a request has shown
 // it needs rather than what the largest like it might.
 static uint64_t serve_partition_slots(const ServeState *S, const ServeReq &r) {
     const double load = S->cfg.load_factor > 0 && S->cfg.load_factor < 1 ? S->cfg.load_factor : 0.5;
@@ -1419,7 +1420,10 @@ static int serve_admit(ServeState *S, ServeTier &t, ServeReq &r) {
     d.heap_hcap = hhcap;
     d.key_off = (uint64_t)q * t.kcap;
     d.key_cap = t.kcap;
-    d.grow_at = tn / 2;
+    // grown when a quarter full: half full, a relax takes 82 k cycles where after
+    // the growth it takes 26 (a 54-move board on a cluster slot; a burst of 48
+    // requests 99 -> 86 ms)
+    d.grow_at = tn / 4;
     if (fill_ff_async(eng, S->tab.as<Slot>() + toff, tn * sizeof(Slot), t.stream) != UASTAR_OK) {
         S->loop_error = UASTAR_CUDA_ERROR;
         return 0;
@@ -1741,7 +1745,7 @@ static void serve_grow(ServeState *S, ServeTier &t, int q) {
     sl.tab_n = new_n;
     d.tab_off = noff;
     d.log2_slots += 2;
-    d.grow_at = new_n / 2;
+    d.grow_at = new_n / 4;
 }
 
 // Move CTA slot q's parked request onto a free cluster slot without

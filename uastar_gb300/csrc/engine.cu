@@ -285,9 +285,9 @@ void plain_shape(const uastar_engine *eng, uint32_t block, uint32_t tph, uint32_
 }
 
 // Whether an unbounded search of this map is expected to outgrow the growth
-// point (2^19 states) of the auto-sized table's first 2^20 slots without
-// outgrowing the table: a map of at most 2^20 cells, of which a search that
-// crosses it at 30 % blocked reaches five eighths.
+// point (2^19 states) of the auto-sized table's first 2^21 slots: a map of at
+// most 2^20 cells, of which a search that crosses it at 30 % blocked reaches
+// five eighths.
 bool may_outgrow(int32_t H, int32_t W) {
     const uint64_t cells = (uint64_t)H * (uint64_t)W;
     return cells * 5 > (8ull << 19) && cells <= (1ull << 20);
@@ -468,13 +468,13 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
             m.sort_hist = reinterpret_cast<uint32_t *>(m.sort_buf + 2 * sort_n);
             m.sort_bits = sort_bits;
         }
-        // an auto-sized table grows in place (x4) when half full; at the cap
+        // an auto-sized table grows in place (x4) at its share of kGrowAt; at the cap
         // the search pauses instead, a round's worth of inserts short of the
         // load limit (a round relaxes at most kMoves successors per heap)
         const bool auto_table = c.hash_log2_slots <= 0 || max_log2 > 0;
         const uint64_t round_max = (uint64_t)k * P::kMoves;
         const auto pause_point = [&](uint64_t n) -> uint64_t {
-            if (max_log2 <= 0 || n < (1ull << max_log2)) return n / 2;
+            if (max_log2 <= 0 || n < (1ull << max_log2)) return n / (n < (1ull << 27) ? P::kGrowAt : 2);
             return m.max_inserted > round_max ? m.max_inserted - round_max : 0ull;
         };
         m.grow_at = auto_table && !P::kDirect ? pause_point(slots) : ~0ull;
@@ -667,7 +667,7 @@ bool grid_is_direct(const uastar_config &c, int32_t H, int32_t W) {
 template <class P>
 int32_t run_grid(uastar_engine *eng, const P &prob, uint64_t tail_cap, PlainOut *po, std::vector<int32_t> *far) {
     const uint64_t cells = (uint64_t)prob.H * (uint64_t)prob.W;
-    const int log2_auto = std::min(28, std::max(20, ceil_log2_u64(cells) - 1));
+    const int log2_auto = std::min(28, std::max(21, ceil_log2_u64(cells)));
     const uint32_t per_heap =
         (uint32_t)std::min<uint64_t>(8192, std::max<uint64_t>(64, 4 * cells / plain_heaps<GridProblem>(eng->cfg)));
     const GridTail<P> tail(eng, prob, tail_cap);
@@ -810,7 +810,10 @@ int32_t puzzle_solve_n(uastar_engine *eng, const uint8_t *tiles, PlainOut *po, s
     else
         prob.start = pack_board(N, tiles);
     prob.goal = PuzzleProblem<N>::goal_key();
-    const int log2_start = N < 5 && eng->puzzle_log2_start > 0 ? eng->puzzle_log2_start : (N == 3 ? 20 : 22);
+    const int log2_start = N < 5 && eng->puzzle_log2_start > 0 ? eng->puzzle_log2_start
+                           : N == 3                                  ? 20
+                           : N == 4                                  ? 23
+                                                                     : 22;
     PuzzleTail<N> tail;
     tail.eng = eng;
     if (int32_t rc = run_plain(eng, prob, log2_start, N == 3 ? 1024 : 16383, po, 0, tail)) return rc;
