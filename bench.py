@@ -344,7 +344,7 @@ def run_ours(args, rank, world, local_rank):
                 "d2h_bytes_per_step": d2h, "steps": e2e_steps},
         "roofline": {"bound": "hbm", "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 5), "traffic": traffic, "peak_kind": peak_kind,
-                     "kernel": "k_plain_search<GridProblem>", "kernel_ms_mean": round(mean_kernel_ms, 3),
+                     "kernel": "k_plain_search<GridDirect>", "kernel_ms_mean": round(mean_kernel_ms, 3),
                      "bytes_per_launch": int(sum(per_launch_bytes) / len(per_launch_bytes)),
                      "bytes_model": "160*expanded + 32*generated + 64*pushed"},
         "gpu_launches": int(launches),
@@ -759,7 +759,7 @@ def run_case(args) -> None:
                 print(f"pdb4: built in {eng.pdb_build(4):.1f} ms", flush=True)
     elif c == "grow":
         # an auto-sized dedup table that starts at 2^22 slots and grows in
-        # place (k_grow_move / k_grow_links / k_grow_heaps) when half full:
+        # place (k_grow_move / k_grow_links / k_grow_heaps) at its growth point:
         # a 15-puzzle whose search stores ~4 M states (200-move walk, seed 1039)
         with Engine(0) as eng:
             eng.pdb_build(4)

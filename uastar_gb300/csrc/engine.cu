@@ -35,7 +35,7 @@ __global__ void k_fill_ff(uint4 *p, size_t n16) {
 // team state.  Bound by the table's bytes (8.6 GB: 1.29 ms, 6.7 TB/s; with a
 // word per cell the 20000^2 grid clears 3.2 GB); one launch
 // instead of a fill, a memset and a copy, and the walk queued behind the search
-// (run_plain), take four trips to the driver and one wait off a solve: 61 x 67
+// (run_plain), take four launch calls and one wait off a solve: 61 x 67
 // 340 -> 306 us, an 8-puzzle 134 -> 115 us.
 __global__ void k_plain_reset(uint4 *tab, size_t n16, uint32_t *heap_size, uint32_t k, TeamState *st) {
     const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;

@@ -27,7 +27,7 @@ enum : uint32_t {
     ST_BAD_INPUT = 7,
     ST_TIMEOUT = 8,
     ST_RUNNING = 9,
-    ST_COST_RANGE = 10,  // a cost beyond GridDirect's exact range (never leaves the library)
+    ST_COST_RANGE = 100,  // a cost beyond GridDirect's exact range (never leaves the library)
 };
 
 // One dedup-table slot: the 16 bytes that one CAS sets.  Random accesses are
