@@ -330,7 +330,7 @@ def run_ours(args, rank, world, local_rank):
         "config": {"workload": WORKLOAD, "grid": "20000x20000", "block_rate": 0.30, "seed": sp.seed,
                    "heaps": 8192, "block_threads": 256, "threads_per_heap": 4, "hash_slots": 2 ** 28,
                    "parallelism": f"replicas x{world}" if world > 1 else "single GPU",
-                   "l2": "inputs larger than L2: each solve rewrites its 8.6 GB dedup table first",
+                   "l2": "inputs larger than L2: each solve rewrites its 3.2 GB table of cells first",
                    "step": "one full solve (search + path walk + host validation), bitmap resident"},
         "result": {"straight": r0.straight, "diagonal": r0.diagonal, "cost": r0.cost,
                    "expanded": r0.expanded, "generated": r0.generated, "pushed": r0.pushed,
@@ -718,7 +718,7 @@ def run_case(args) -> None:
     """One named workload, for profilers: each repeat solves it once and
     prints a line; captures take the second launch of the kernel of interest
     (`-s 1 -c 1`).  Every case holds a few GB on the device at most, except
-    grid_20000 (the headline query, 8.6 GB table: launch lists only)."""
+    grid_20000 (the headline query, 3.2 GB table: launch lists only)."""
     import numpy as np
     from uastar_gb300 import Engine, workloads as WL
     c = args.case
