@@ -92,7 +92,9 @@ struct WideSlots {
     static constexpr bool kPrevInKey = false;
     static constexpr int kLink = LINK_FIELD;
     static constexpr size_t kSlotBytes = sizeof(WideSlot);
-    static constexpr uint64_t kGrowAt = 2;  // (the same states in the same bytes)
+    // (32 bytes a slot: with twice the slots and growth at a quarter, boards of 2 M
+    // states take 6.5 ms instead of 7.0, small ones 1.01 instead of 0.92)
+    static constexpr uint64_t kGrowAt = 2;
     __device__ static Slot *at(Slot *tab, uint64_t i) { return reinterpret_cast<Slot *>(w(tab) + i); }
     __device__ static const WideSlot *w(const Slot *s) { return reinterpret_cast<const WideSlot *>(s); }
     __device__ static WideSlot *w(Slot *s) { return reinterpret_cast<WideSlot *>(s); }
