@@ -884,11 +884,51 @@ int32_t run_wave(uastar_engine *eng, const uastar_instance *insts, const std::ve
     return UASTAR_OK;
 }
 
+// The batched engine solves an instance on the plain engine through that
+// engine's public calls, which replace the loaded grid and the last solution.
+// Those belong to the caller (uastar_grid_load, then uastar_grid_solve_loaded
+// and uastar_grid_path around a batch): they are set aside for as long as this
+// object lives, and the solves get a bitmap of their own, kept for the next batch.
+class BatchPlain {
+  public:
+    explicit BatchPlain(uastar_engine *e) : eng(e) { swap(); }
+    ~BatchPlain() { swap(); }
+    BatchPlain(const BatchPlain &) = delete;
+    BatchPlain &operator=(const BatchPlain &) = delete;
+
+  private:
+    void swap() {
+        // (the caller's map waits here, not in b_plain_map: that is a buffer to release)
+        if (!inside) {
+            map = eng->bitmap;
+            eng->bitmap = eng->b_plain_map;
+            eng->b_plain_map = DevBuf{};
+        } else {
+            eng->b_plain_map = eng->bitmap;
+            eng->bitmap = map;
+        }
+        inside = !inside;
+        std::swap(H, eng->gH);
+        std::swap(W, eng->gW);
+        std::swap(loaded, eng->grid_loaded);
+        std::swap(kind, eng->last_kind);
+        std::swap(ok, eng->last_ok);
+        std::swap(cached, eng->path_cached);
+        std::swap(path, eng->path);
+    }
+    uastar_engine *eng;
+    bool inside = false, loaded = false, ok = false, cached = false;
+    DevBuf map;
+    int32_t H = 0, W = 0;
+    int kind = 0;
+    std::vector<int32_t> path;
+};
+
 }  // namespace
 
 namespace uastar {
 void release_batch_buffers(uastar_engine *eng) {
-    for (DevBuf *b : {&eng->b_tab, &eng->b_heaps, &eng->b_bitmaps, &eng->b_cand, &eng->b_hsize, &eng->b_walk})
+    for (DevBuf *b : {&eng->b_tab, &eng->b_heaps, &eng->b_bitmaps, &eng->b_cand, &eng->b_hsize, &eng->b_walk, &eng->b_plain_map})
         b->release();
 }
 }  // namespace uastar
@@ -1007,6 +1047,7 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
             eng->b_bitmaps.release();
         }
     }
+    const BatchPlain own(eng);
     for (int i : todo) {
         const uastar_instance &in = insts[i];
         uastar_instance_result &r = results[i];

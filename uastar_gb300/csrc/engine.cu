@@ -1108,7 +1108,7 @@ void uastar_destroy(uastar_engine *eng) {
                       &eng->tab_next, &eng->grow_map, &eng->sortb,
                       &eng->bitmap, &eng->b_desc, &eng->b_out, &eng->b_queue, &eng->b_bitmaps,
                       &eng->b_tab, &eng->b_heaps, &eng->b_hsize, &eng->b_cand, &eng->b_walk,
-                      &eng->b_walklen, &eng->b_cstate, &eng->b_cnext, &eng->ida})
+                      &eng->b_walklen, &eng->b_cstate, &eng->b_cnext, &eng->ida, &eng->b_plain_map})
         b->release();
     if (eng->h_pin) cudaFreeHost(eng->h_pin);
     for (auto &b : eng->pdb) b.release();

@@ -127,6 +127,7 @@ struct uastar_engine {
     uint8_t last_tiles[25] = {0};
     bool path_cached = false;
     std::vector<int32_t> path;  // grid: cell ids; puzzle: moves
+    uastar::DevBuf b_plain_map; // bitmap of the batched engine's own plain solves (BatchPlain)
 
     // batched / serving engines
     uastar::DevBuf b_desc, b_out, b_queue, b_bitmaps, b_tab, b_heaps, b_hsize, b_cand, b_walk,
