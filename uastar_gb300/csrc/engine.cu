@@ -16,6 +16,7 @@
 #include "ga_problems.cuh"
 #include "ga_search.cuh"
 #include "ga_grow.cuh"
+#include "ga_open.cuh"
 #include "ga_ida.cuh"
 #include "ga_walk.cuh"
 
@@ -74,30 +75,6 @@ __global__ void __launch_bounds__(256, 1) k_team_sort(const uint32_t *keys, uint
         reinterpret_cast<uint32_t *>(smem), &st->error);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         perm[i] = (uint32_t)__ldcg(out + i);
-}
-
-// The best open node of a paused puzzle search: the minimum entry (least f,
-// then deepest) among the entries of the heaps' saved shared tops that are
-// current (their f still matches the node's g), as key << 32 | slot into
-// *best by atomicMin.  The heap roots are the per-heap minima, so this is the
-// open list's minimum unless every root near it is stale.
-template <int N>
-__global__ void k_best_open(PuzzleProblem<N> prob, SearchMem<PuzzleEntry> m, uint32_t k,
-                            unsigned long long *best) {
-    const uint32_t topn = (1u << m.L) - 1u;
-    const uint64_t total = (uint64_t)k * topn;
-    for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total;
-         t += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t h = (uint32_t)(t / topn), i = (uint32_t)(t % topn) + 1;
-        if (i > __ldcg(&m.heap_size[h])) continue;
-        const PuzzleEntry e = PuzzleProblem<N>::load(m.heaps + (size_t)h * m.stride + i);
-        typename PuzzleProblem<N>::Key key;
-        uint64_t g;
-        uint32_t aux;
-        PuzzleProblem<N>::load_node(PuzzleProblem<N>::at(m.tab, e.slot), e, key, g, aux);
-        if (prob.f_of(key, g, aux) != PuzzleProblem<N>::entry_cost(e)) continue;  // stale
-        atomicMin(best, ((unsigned long long)e.key << 32) | e.slot);
-    }
 }
 
 // Round-latency floor of the plain engine's launch geometry: `rounds` rounds
@@ -1046,7 +1023,8 @@ int32_t puzzle_bounded_n(uastar_engine *eng, const uint8_t *tiles, int max_log2,
         cudaMemcpyAsync(&best, d_best, 8, cudaMemcpyDeviceToHost, eng->stream);
         if ((e = cudaStreamSynchronize(eng->stream)) != cudaSuccess) return fail_cuda(eng, e, "best open node");
         // a goal at or below every open node (the pause came before the decision
-        // that takes it): this segment's optimum
+        // that takes it): this segment's optimum.  `least` is the minimum over all
+        // current entries, so it is a lower bound whatever lies stale above it.
         const uint64_t least = PuzzleProblem<N>::entry_cost(PuzzleEntry{(uint32_t)(best >> 32), 0u});
         if (best == ~0ull || po.st.goal_best <= least) {
             if (po.st.goal_best != kInfCost) return solved(po.st.goal_best, po.st.goal_slot);
