@@ -270,11 +270,12 @@ bool may_outgrow(int32_t H, int32_t W) {
     return cells * 5 > (8ull << 19) && cells <= (1ull << 20);
 }
 
-// Moves a paused search's table to one 4x larger (k_grow_*), swapping it in
-// as eng->tab.  Returns false (and changes nothing) if the memory is not there.
+// Moves a paused search's table to one 4x larger, or as large as `limit` slots
+// allow (k_grow_*), swapping it in as eng->tab.  Returns false (and changes
+// nothing) if the memory is not there.
 template <class P>
-bool grow_table(uastar_engine *eng, SearchMem<typename P::Entry> &m, uint32_t k, TeamState *st) {
-    const uint64_t old_n = m.mask + 1, new_n = old_n * 4;
+bool grow_table(uastar_engine *eng, SearchMem<typename P::Entry> &m, uint32_t k, TeamState *st, uint64_t limit) {
+    const uint64_t old_n = m.mask + 1, new_n = std::min(old_n * 4, limit);
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
     const size_t need = (new_n * P::kSlotBytes > eng->tab_next.bytes ? new_n * P::kSlotBytes : 0) +
@@ -480,7 +481,7 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
             // paused: at the cap the caller takes over; otherwise grow
             if (max_log2 > 0 && m.mask + 1 >= (1ull << max_log2)) break;
             bool grown = false;
-            if constexpr (!P::kDirect) grown = grow_table<P>(eng, m, k, st);
+            if constexpr (!P::kDirect) grown = grow_table<P>(eng, m, k, st, max_log2 > 0 ? 1ull << max_log2 : ~0ull);
             if (grown) {
                 out->grows += 1;
                 m.grow_at = pause_point(m.mask + 1);
@@ -500,9 +501,10 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
         if (s != ST_HASH_FULL && s != ST_HEAP_OVERFLOW) break;
         size_t free_b = 0, total_b = 0;
         cudaMemGetInfo(&free_b, &total_b);
-        if (s == ST_HASH_FULL && auto_table && log2 + 2 <= 31 && (max_log2 <= 0 || log2 + 2 <= max_log2) &&
-            (out->slots * 4 * P::kSlotBytes) < free_b + eng->tab.bytes) {
-            log2 += 2;
+        const int larger = max_log2 > 0 ? std::min(log2 + 2, max_log2) : log2 + 2;
+        if (s == ST_HASH_FULL && auto_table && larger > log2 && larger <= 31 &&
+            (P::kSlotBytes << larger) < free_b + eng->tab.bytes) {
+            log2 = larger;
             continue;
         }
         if (s == ST_HEAP_OVERFLOW && c.heap_capacity <= 0 && hg.hcap < (1u << 22) &&
