@@ -1,0 +1,41 @@
+"""The last instances of a batch's waves, which move on to larger teams.
+
+Tolerance: the exact (straight, diagonal) optimum must be identical to the
+oracle's."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from uastar_gb300 import Engine, GridInstance, PuzzleInstance
+from uastar_gb300 import _lib as L
+from uastar_gb300 import engine as E
+
+pytestmark = pytest.mark.gpu
+
+
+def open_grid(H, W):
+    """All cells open, corner to corner: min(H, W) - 1 diagonal steps, the rest straight."""
+    words = np.full(E.grid_words(H, W), np.uint64(0xFFFFFFFFFFFFFFFF), dtype=np.uint64)
+    return GridInstance(words, H, W, (0, 0), (H - 1, W - 1))
+
+
+# what a program may give its engine for plain solves, and too little of it for these instances
+LIMITS = [{"hash_log2_slots": 12}, {"heap_capacity": 3, "heaps": 32, "block_threads": 32, "threads_per_heap": 1,
+                                    "heap_top_levels": -1},
+          {"heaps": 1 << 20}]
+
+
+@pytest.mark.parametrize("limit", range(len(LIMITS)))
+def test_limits_of_plain_solves_refuse_no_instance(limit):
+    grids = [open_grid(2100, 2300), open_grid(1200, 1300)]
+    with Engine(0, **LIMITS[limit]) as eng:
+        eng.pdb_build(4)
+        for insts in (grids[:1], grids[1:], grids + [PuzzleInstance(4, E.gen_puzzle(1001, 4, 200))]):
+            res, _ = eng.batch_solve(insts)
+            for i, r in zip(insts, res):
+                assert r["status"] == L.OK, r
+                if isinstance(i, GridInstance):
+                    assert (r["straight"], r["diagonal"]) == (abs(i.H - i.W), min(i.H, i.W) - 1)
+                else:
+                    assert r["steps"] == 50

@@ -1023,9 +1023,9 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
         }
     }
     todo.clear();
+    bool heap_over = false;
     if (!tier2.empty()) {
         if (cluster_rc) return cluster_rc;
-        bool heap_over = false;
         for (int i : tier2) heap_over |= results[i].status == UASTAR_HEAP_OVERFLOW;
         if (heap_over) gc.set_capacity(g.want * 16 + 15);
         std::vector<int> m(tier2.size());
@@ -1036,6 +1036,8 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
         if (rc) return rc;
         todo = retry;
     }
+    bool over2 = false;  // heaps overflowed in the cluster tier
+    for (int i : todo) over2 |= results[i].status == UASTAR_HEAP_OVERFLOW;
     // The team regions are kept for the next batch (teams x region, tens of
     // GB at most); only a plain-engine escalation that finds too little free
     // memory for its table gets them back.
@@ -1047,6 +1049,7 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
             eng->b_bitmaps.release();
         }
     }
+    std::vector<int> failed;  // not solved by the plain engine
     const BatchPlain own(eng);
     for (int i : todo) {
         const uastar_instance &in = insts[i];
@@ -1085,10 +1088,29 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
                 stats->generated += pr.generated;
             }
         }
+        if (r.status != UASTAR_OK && r.status != UASTAR_NO_SOLUTION) failed.push_back(i);
         if (stats) stats->escalated += 1;
         if (debug_log())
             std::fprintf(stderr, "[uastar] escalated instance %d (%s) to the plain engine: status %d, %.1f ms\n", i,
                          in.kind == UASTAR_KIND_GRID ? "grid" : "puzzle", r.status, now_ms() - te);
+    }
+    // What the plain engine could not solve, because the engine's own limits for
+    // plain solves are too small (hash_log2_slots, heap_capacity, heaps) or the
+    // memory is not there, may have been well on its way on a cluster when it
+    // gave up its team: it gets one again, with that tier's largest space and no
+    // early end.  If that fails too, the plain engine's status stands.
+    if (!failed.empty() && !cluster_rc) {
+        if (over2 && !heap_over) gc.set_capacity(g.want * 16 + 15);
+        std::vector<int> m;
+        for (int i : failed) m.push_back(mult[i] > 1 ? 32 : 2);
+        std::vector<uastar_instance_result> before;
+        for (int i : failed) before.push_back(results[i]);
+        retry.clear();
+        rc = run_wave(eng, insts, failed, gc, m, use_graph, ~0ull, b2, 0, 0, results, stats, &retry);
+        if (rc) return rc;
+        for (size_t j = 0; j < failed.size(); ++j)
+            if (std::find(retry.begin(), retry.end(), failed[j]) != retry.end())
+                results[failed[j]].status = before[j].status;
     }
     if (stats) {
         stats->wall_ms = now_ms() - t0;
