@@ -388,7 +388,8 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
 
     for (int attempt = 0; attempt < 6; ++attempt) {
         const uint64_t slots = 1ull << log2;
-        const size_t tab_b = P::kDirect ? direct_b : slots * P::kSlotBytes;
+        // (a key's first probes are its group of four slots: smaller tables have one all the same)
+        const size_t tab_b = P::kDirect ? direct_b : std::max<uint64_t>(slots, 4) * P::kSlotBytes;
         const size_t heap_b = (size_t)k * hg.stride * sizeof(E);
         const size_t cand_b = cand_records<P>(nblocks, H) * sizeof(Cand);
         // the batched engine's cached buffers give way to a table that does not fit
