@@ -156,6 +156,18 @@ __global__ void __launch_bounds__(1024) k_walk_grid_solved(P prob, const Slot *t
     if (threadIdx.x == 0) *len = n;
 }
 
+cudaError_t open_smem(int device, const void *kernel) {
+    int optin = 0;
+    cudaFuncAttributes a;
+    cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+    if (e != cudaSuccess) return e;
+    const int most = optin - (int)a.sharedSizeBytes;  // (the limit counts the kernel's static part too)
+    return a.maxDynamicSharedSizeBytes >= most
+               ? cudaSuccess
+               : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 int32_t fill_ff_async(uastar_engine *eng, void *p, size_t bytes, cudaStream_t stream) {
     const size_t n16 = bytes / 16;
     const int blocks = (int)std::min<size_t>((n16 + 255) / 256, (size_t)std::max(1, eng->sms * 8));
@@ -359,10 +371,9 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
     const uint32_t L = fit_levels<P>(H, c.heap_top_levels, smem_budget - sort_extra);
     const size_t smem = sorted ? SearchSmem<P>::bytes_sorted(H, L, block) : SearchSmem<P>::bytes(H, L);
     cudaError_t e = cudaSuccess;
-    if (eng->smem_limit[kfn] < smem) {
-        e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return fail_cuda(eng, e, "smem attribute");
-        eng->smem_limit[kfn] = smem;
+    if (!eng->smem_open.count(kfn)) {
+        if ((e = open_smem(eng->device, kfn)) != cudaSuccess) return fail_cuda(eng, e, "smem attribute");
+        eng->smem_open.insert(kfn);
     }
     int max_active = 0;
     const auto occ_key = std::make_tuple(kfn, block, smem);
