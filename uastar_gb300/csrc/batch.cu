@@ -928,7 +928,8 @@ class BatchPlain {
 
 namespace uastar {
 void release_batch_buffers(uastar_engine *eng) {
-    for (DevBuf *b : {&eng->b_tab, &eng->b_heaps, &eng->b_bitmaps, &eng->b_cand, &eng->b_hsize, &eng->b_walk, &eng->b_plain_map})
+    for (DevBuf *b : {&eng->b_tab, &eng->b_heaps, &eng->b_bitmaps, &eng->b_cand, &eng->b_hsize, &eng->b_walk,
+                      &eng->b_plain_map, &eng->ida})
         b->release();
 }
 }  // namespace uastar

@@ -874,22 +874,24 @@ int32_t ida_exact(uastar_engine *eng, const uint8_t *tiles, int32_t lb, int32_t 
         out->exact_ms = now_ms() - t0;
         return UASTAR_OK;
     }
-    // pass state, cut state, the start, two levels of the cut
+    // pass state, cut state, the cut's levels
     constexpr size_t kCutAt = (sizeof(IdaPass) + 255) & ~(size_t)255;
-    constexpr size_t kStartAt = (kCutAt + sizeof(IdaCut) + 255) & ~(size_t)255;
-    constexpr size_t kLevelAt = (kStartAt + sizeof(IdaRoot) + 255) & ~(size_t)255;
-    const size_t room = 4 * (size_t)kIdaRoots;  // a level's children
+    constexpr size_t kRingAt = (kCutAt + sizeof(IdaCut) + 255) & ~(size_t)255;
     cudaError_t e;
-    if ((e = eng->ida.ensure(kLevelAt + 2 * room * sizeof(IdaRoot))) != cudaSuccess)
-        return fail_cuda(eng, e, "alloc ida");
+    // Where the memory is not there, fewer roots; and without any (or none for the
+    // passes' stacks, below) the segments' answer stands, unproven.
+    uint32_t roots = kIdaRoots;
+    const auto room = [&] { return kRingAt + 4 * (size_t)roots * sizeof(IdaRoot); };
+    while ((e = eng->ida.ensure(room())) != cudaSuccess && roots > kIdaLeastRoots) roots /= 4;
+    if (e != cudaSuccess) {
+        out->exact_ms = now_ms() - t0;
+        return UASTAR_OK;
+    }
     unsigned char *const base = eng->ida.as<unsigned char>();
     IdaPass *d_pass = reinterpret_cast<IdaPass *>(base);
     IdaCut *d_cut = reinterpret_cast<IdaCut *>(base + kCutAt);
-    IdaRoot *d_start = reinterpret_cast<IdaRoot *>(base + kStartAt);
-    IdaRoot *const d_level[2] = {reinterpret_cast<IdaRoot *>(base + kLevelAt),
-                                 reinterpret_cast<IdaRoot *>(base + kLevelAt) + room};
-    k_ida_start<PuzzleProblem<N>><<<1, 1, 0, eng->stream>>>(prob, d_start);
-    eng->launches++;
+    IdaRoot *const d_ring = reinterpret_cast<IdaRoot *>(base + kRingAt);
+    const uint32_t wrap = 4 * roots - 1;
     uint32_t t = (uint32_t)std::max(lb, 0);
     bool optimal = false;
     while (t < (uint32_t)ub) {
@@ -906,18 +908,22 @@ int32_t ida_exact(uastar_engine *eng, const uint8_t *tiles, int32_t lb, int32_t 
                 cudaSuccess ||
             (e = cudaMemcpyAsync(d_cut, &init.cut, sizeof init.cut, cudaMemcpyHostToDevice, eng->stream)) != cudaSuccess)
             return fail_cuda(eng, e, "ida state");
-        for (uint32_t d = 0; d < kIdaCutDepth; ++d) {
-            k_ida_cut<PuzzleProblem<N>><<<std::max(1, eng->sms * 4), 256, 0, eng->stream>>>(
-                prob, d == 0 ? d_start : d_level[d & 1], d_level[(d + 1) & 1], d, t, d_cut);
-            eng->launches++;
-        }
+        k_ida_start<PuzzleProblem<N>><<<1, 1, 0, eng->stream>>>(prob, d_ring);
+        for (uint32_t d = 0; d < kIdaCutDepth; ++d)
+            k_ida_cut<PuzzleProblem<N>><<<std::max(1, eng->sms * 4), 256, 0, eng->stream>>>(prob, d_ring, roots, d, t,
+                                                                                          d_cut);
+        eng->launches += 1 + kIdaCutDepth;
         IdaCut cut;
-        if ((e = cudaGetLastError()) != cudaSuccess) return fail_cuda(eng, e, "ida cut");
+        if ((e = cudaGetLastError()) == cudaErrorMemoryAllocation) break;
+        if (e != cudaSuccess) return fail_cuda(eng, e, "ida cut");
         if ((e = cudaMemcpyAsync(&cut, d_cut, sizeof cut, cudaMemcpyDeviceToHost, eng->stream)) != cudaSuccess ||
             (e = cudaStreamSynchronize(eng->stream)) != cudaSuccess)
             return fail_cuda(eng, e, "ida cut");
-        uint32_t depth = 0;
-        while (depth < kIdaCutDepth && cut.count[depth + 1]) out->exact_nodes += cut.count[++depth];
+        uint32_t depth = 0, first = 0;  // the last level, its first record in the ring
+        while (depth < kIdaCutDepth && cut.count[depth + 1]) {
+            first += cut.count[depth];
+            out->exact_nodes += cut.count[++depth];
+        }
         if (cut.goal) {
             out->exact_passes += 1;
             moves->clear();
@@ -926,17 +932,17 @@ int32_t ida_exact(uastar_engine *eng, const uint8_t *tiles, int32_t lb, int32_t 
             optimal = true;
             break;
         }
-        const IdaRoot *const d_roots = d_level[depth & 1];
         // (level `depth` is whole only if it is where the cut stopped; otherwise
         // the tree below t ended within the cut)
-        const bool ended = depth < kIdaCutDepth && cut.count[depth] < kIdaRoots;
+        const bool ended = depth < kIdaCutDepth && cut.count[depth] < roots;
         const uint32_t nroots = ended ? 0u : cut.count[depth];
         // threads read the device clock at their start: the pass ends
         // `left_ms` after it began
         k_ida_pass<PuzzleProblem<N>, kMaxDepth><<<std::max(1, eng->sms * 8), 128, 0, eng->stream>>>(
-            prob, d_roots, nroots, t, d_pass, (unsigned long long)(left_ms * 1e6));
+            prob, d_ring, wrap, first, nroots, t, d_pass, (unsigned long long)(left_ms * 1e6));
+        if ((e = cudaGetLastError()) == cudaErrorMemoryAllocation) break;
+        if (e != cudaSuccess) return fail_cuda(eng, e, "ida launch");
         eng->launches++;
-        if ((e = cudaGetLastError()) != cudaSuccess) return fail_cuda(eng, e, "ida launch");
         IdaPass res;
         if ((e = cudaMemcpyAsync(&res, d_pass, sizeof res, cudaMemcpyDeviceToHost, eng->stream)) != cudaSuccess ||
             (e = cudaStreamSynchronize(eng->stream)) != cudaSuccess)
@@ -945,8 +951,8 @@ int32_t ida_exact(uastar_engine *eng, const uint8_t *tiles, int32_t lb, int32_t 
         out->exact_nodes += (int64_t)res.nodes;
         if (res.found) {
             IdaRoot r;
-            if ((e = cudaMemcpyAsync(&r, d_roots + res.found_root, sizeof r, cudaMemcpyDeviceToHost, eng->stream)) !=
-                    cudaSuccess ||
+            if ((e = cudaMemcpyAsync(&r, d_ring + ((first + res.found_root) & wrap), sizeof r, cudaMemcpyDeviceToHost,
+                                     eng->stream)) != cudaSuccess ||
                 (e = cudaStreamSynchronize(eng->stream)) != cudaSuccess)
                 return fail_cuda(eng, e, "ida root");
             moves->clear();

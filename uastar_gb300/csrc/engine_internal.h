@@ -155,7 +155,8 @@ cudaError_t open_smem(int device, const void *kernel);
 // pdb.cu
 int32_t pdb_build_device(uastar_engine *eng, int n, double *ms);
 // batch.cu: the batched engine keeps its team regions, heaps and bitmaps for
-// the next batch; a caller that needs the memory (the serving loop, a plain
-// solve that cannot get its table) gives them back.
+// the next batch, the memory-bounded mode those of its exact phase; a caller
+// that needs the memory (the serving loop, a plain solve that cannot get its
+// table) gives them back.
 void release_batch_buffers(uastar_engine *eng);
 }  // namespace uastar

@@ -36,10 +36,14 @@ struct IdaRoot {
     unsigned long long prefix;
 };
 
-// The cut: the first depth with this many nodes, at most kIdaCutDepth (what a
-// prefix holds).
-constexpr uint32_t kIdaRoots = 1u << 20;
+// The cut: the first depth with kIdaRoots nodes (down to kIdaLeastRoots where the
+// memory for more is not there), at most kIdaCutDepth (what a prefix holds).
+constexpr uint32_t kIdaRoots = 1u << 20, kIdaLeastRoots = 1u << 12;
 constexpr uint32_t kIdaCutDepth = 32;
+// The levels follow each other in a ring of 4 records per root: a level that is
+// expanded has fewer nodes than there are roots and at most three children each
+// (the start four), so it and its children fit, whatever came before.
+// 134 MB for 2^20 roots (two buffers of a level's children each took 268).
 struct IdaCut {
     uint32_t count[kIdaCutDepth + 1];  // nodes per level; 0 past the last
     uint32_t goal;                     // a goal's depth (0: none met)
@@ -85,15 +89,19 @@ template <class P> __global__ void k_ida_start(P prob, IdaRoot *out) {
 }
 
 // One level of the cut: the children of level d's nodes with f <= t, appended
-// to `out` in any order, unless level d is the last.
+// behind it in the ring in any order, unless level d is the last.  `roots`: a
+// power of two.
 template <class P>
-__global__ void __launch_bounds__(256) k_ida_cut(P prob, const IdaRoot *in, IdaRoot *out, uint32_t d, uint32_t t,
+__global__ void __launch_bounds__(256) k_ida_cut(P prob, IdaRoot *ring, uint32_t roots, uint32_t d, uint32_t t,
                                                  IdaCut *cut) {
     const uint32_t n = ldcg_u32(&cut->count[d]);
-    if (n == 0 || n >= kIdaRoots) return;
+    if (n == 0 || n >= roots) return;
+    const uint32_t wrap = 4u * roots - 1u;
+    uint32_t first = 0;  // level d's first record
+    for (uint32_t q = 0; q < d; ++q) first += ldcg_u32(&cut->count[q]);
     uint32_t minx = ~0u;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const IdaRoot r = in[i];
+        const IdaRoot r = ring[(first + i) & wrap];
         const typename P::Key key = ida_key<P>(r);
         const uint32_t mask = prob.moves(key, r.aux);
         typename P::Succ sc[4];
@@ -114,7 +122,7 @@ __global__ void __launch_bounds__(256) k_ida_cut(P prob, const IdaRoot *in, IdaR
                 cut->goal_prefix = r.prefix | (unsigned long long)mv << (2 * d);
         }
         if (!keep) continue;
-        uint32_t at = atomicAdd(&cut->count[d + 1], (uint32_t)__popc(keep));
+        uint32_t at = first + n + atomicAdd(&cut->count[d + 1], (uint32_t)__popc(keep));
 #pragma unroll
         for (int mv = 0; mv < 4; ++mv) {
             if (!(keep >> mv & 1u)) continue;
@@ -129,15 +137,16 @@ __global__ void __launch_bounds__(256) k_ida_cut(P prob, const IdaRoot *in, IdaR
             c.g = d + 1;
             c.aux = naux[mv];
             c.prefix = r.prefix | (unsigned long long)mv << (2 * d);
-            out[at++] = c;
+            ring[at++ & wrap] = c;
         }
     }
     if (minx != ~0u) atomicMin(&cut->min_exceed, minx);
 }
 
 template <class P, int kMaxDepth>
-__global__ void __launch_bounds__(128) k_ida_pass(P prob, const IdaRoot *roots, uint32_t nroots, uint32_t t,
-                                                  IdaPass *out, unsigned long long budget_ns) {
+__global__ void __launch_bounds__(128) k_ida_pass(P prob, const IdaRoot *ring, uint32_t wrap, uint32_t first,
+                                                  uint32_t nroots, uint32_t t, IdaPass *out,
+                                                  unsigned long long budget_ns) {
     using Key = typename P::Key;
     // the pass ends budget_ns after this thread started (the threads of a
     // launch start together: the grid fits the GPU at once)
@@ -156,7 +165,7 @@ __global__ void __launch_bounds__(128) k_ida_pass(P prob, const IdaRoot *roots, 
         }
         const uint32_t i = atomicAdd(&out->next_root, 1u);
         if (i >= nroots) break;
-        const IdaRoot r = roots[i];
+        const IdaRoot r = ring[(first + i) & wrap];
         const uint32_t g0 = r.g;
         ks[0] = ida_key<P>(r);
         as[0] = r.aux;
