@@ -14,10 +14,10 @@ from uastar_gb300 import engine as E
 pytestmark = pytest.mark.gpu
 
 
-def open_grid(H, W):
+def open_grid(H, W, est_nodes=0):
     """All cells open, corner to corner: min(H, W) - 1 diagonal steps, the rest straight."""
     words = np.full(E.grid_words(H, W), np.uint64(0xFFFFFFFFFFFFFFFF), dtype=np.uint64)
-    return GridInstance(words, H, W, (0, 0), (H - 1, W - 1))
+    return GridInstance(words, H, W, (0, 0), (H - 1, W - 1), est_nodes)
 
 
 # what a program may give its engine for plain solves, and too little of it for these instances
@@ -39,3 +39,15 @@ def test_limits_of_plain_solves_refuse_no_instance(limit):
                     assert (r["straight"], r["diagonal"]) == (abs(i.H - i.W), min(i.H, i.W) - 1)
                 else:
                     assert r["steps"] == 50
+
+
+@pytest.mark.parametrize("ctas", [1, 8])
+def test_no_early_end_while_instances_wait(ctas):
+    # grids of ~600 steps on few teams: only those running when the queue has
+    # run empty may be handed on, so all but one team's worth finish where they
+    # began (est_nodes: with room for every cell, none overflows)
+    grids = [open_grid(600, 400 + 7 * i, 600 * (400 + 7 * i)) for i in range(4 * ctas)]
+    with Engine(0) as eng:
+        res, _ = eng.batch_solve(grids, ctas=ctas)
+    assert all(r["status"] == L.OK for r in res)
+    assert sum(r["attempts"] == 1 for r in res) >= len(grids) - ctas

@@ -717,7 +717,9 @@ int32_t run_wave(uastar_engine *eng, const uastar_instance *insts, const std::ve
     a.keys = eng->b_walk.as<unsigned long long>();
     // the last `keep` running instances give up their teams
     a.idle = a.queue + 1;
-    a.idle_min = (uint32_t)std::max(0, teams - keep);
+    // (an idle team says that the queue is empty: with more instances than teams
+    // one at least has to be, however few the teams are)
+    a.idle_min = (uint32_t)std::max(cnt > teams ? 1 : 0, teams - keep);
     a.yield_steps = yield_steps;
     int ctas = std::min(g.ctas, cnt);
     cudaLaunchConfig_t lc = {};
