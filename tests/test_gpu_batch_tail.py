@@ -51,3 +51,20 @@ def test_no_early_end_while_instances_wait(ctas):
         res, _ = eng.batch_solve(grids, ctas=ctas)
     assert all(r["status"] == L.OK for r in res)
     assert sum(r["attempts"] == 1 for r in res) >= len(grids) - ctas
+
+
+def test_short_grids_finish_where_they_began():
+    grids = [open_grid(200 + 3 * i, 320, 320 * 320) for i in range(36)]
+    with Engine(0) as eng:
+        res, stats = eng.batch_solve(grids)
+    assert stats["waves"] == 1 and stats["escalated"] == 0
+    assert all(r["status"] == L.OK and r["attempts"] == 1 for r in res)
+
+
+@pytest.mark.parametrize("W,escalated", [(513, 0), (514, 0), (2049, 0), (2050, 1)])
+def test_a_grid_alone_is_started_once(W, escalated):
+    # 2 x 256 and 2 x 1024 steps are where one team or a cluster is sure not to keep it
+    with Engine(0) as eng:
+        (r,), stats = eng.batch_solve([open_grid(300, W, 300 * W)])
+    assert r["status"] == L.OK and (r["straight"], r["diagonal"]) == (W - 300, 299)
+    assert r["attempts"] == 1 and stats["escalated"] == escalated

@@ -180,6 +180,8 @@ __device__ uint32_t run_instance(const BatchArgs &a, const InstDesc &d, Team &te
             m.idle = a.idle;
             m.idle_min = a.idle_min;
             m.yield_steps = a.yield_steps;
+            // a grid past half of its way is left to finish (see uastar_batch_solve)
+            m.yield_end = grid ? (uint32_t)max(abs(d.sx - d.ex), abs(d.sy - d.ey)) / 2u : ~0u;
             m.sort_buf = nullptr;
             m.sort_hist = nullptr;
             m.sort_bits = 0;
@@ -995,6 +997,24 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
     // to 400 instances: 1092 ms without, 605 with the second rule (2 / 4 / 8 /
     // 16 of 36 teams: 710 / 605 / 603 / 756), 536 with both (18 / 36 / 72 / 150
     // instances: 583 / 574 / 536 / 539).
+    // A grid takes at least as many steps as its ends are rows or columns apart, so
+    // what is left of one can be told.  One that has made half of that many is
+    // left to finish: without that, 36 grids of 200 to 320 cells a side start
+    // over (4.7 ms, with it 3.9) and so do the last of eight of 3000 (53-65, 41).
+    // And where a wave is so small that it would give up its instances from the
+    // outset, a grid that is sure to get there is not started in it: two grids of
+    // 900 to 1500 cells a side 24.8 -> 8.0 ms, one of 3000 18.2 -> 11.4.
+    constexpr uint32_t kYield1 = 256, kYield2 = 1024;
+    const auto given_up = [&](std::vector<int> &tier, int teams, int keep, uint32_t yield, std::vector<int> *next) {
+        if ((int)tier.size() > std::min(teams, keep)) return;
+        std::vector<int> stay;
+        for (int i : tier) {
+            const uastar_instance &in = insts[i];
+            const int apart = std::max(std::abs(in.sx - in.ex), std::abs(in.sy - in.ey));
+            (in.kind == UASTAR_KIND_GRID && apart > 2 * (int)yield ? *next : stay).push_back(i);
+        }
+        tier.swap(stay);
+    };
     BatchGeometry gc = g;
     rc = resolve_cluster_geometry(eng, cfg && cfg->cluster_size >= 2 && cfg->cluster_size <= 16 ? cfg->cluster_size : 8,
                                   &gc);
@@ -1005,10 +1025,14 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
     // tail.  Grids do not: their steps are bounded by the path length, which
     // costs a cluster no more of them than the whole GPU.
     const uint64_t b2 = cfg && cfg->tier2_puzzle_rounds > 0 ? (uint64_t)cfg->tier2_puzzle_rounds : 16384;
+    const int keep1 = 2 * clusters, keep2 = std::max(1, clusters / 8);
+    const size_t large = tier2.size();
+    given_up(tier1, g.ctas, keep1, kYield1, &tier2);
+    for (size_t j = large; j < tier2.size(); ++j) mult[tier2[j]] = insts[tier2[j]].est_nodes > 0 ? 16 : 4;
     if (!tier1.empty()) {
         std::vector<int> m(tier1.size(), 1);
         const uint64_t b1 = cfg && cfg->tier1_rounds > 0 ? (uint64_t)cfg->tier1_rounds : 2048;
-        rc = run_wave(eng, insts, tier1, g, m, use_graph, b1, 0, 2 * clusters, 256, results, stats, &retry);
+        rc = run_wave(eng, insts, tier1, g, m, use_graph, b1, 0, keep1, kYield1, results, stats, &retry);
         if (rc) return rc;
         // Space for the next tier: 16x after an overflow.  One that ran out of
         // steps or gave up its team gets what it can fill there to a third, a
@@ -1027,6 +1051,7 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
     }
     todo.clear();
     bool heap_over = false;
+    given_up(tier2, clusters, keep2, kYield2, &todo);
     if (!tier2.empty()) {
         if (cluster_rc) return cluster_rc;
         for (int i : tier2) heap_over |= results[i].status == UASTAR_HEAP_OVERFLOW;
@@ -1034,10 +1059,9 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
         std::vector<int> m(tier2.size());
         for (size_t j = 0; j < tier2.size(); ++j) m[j] = mult[tier2[j]] * 2;
         retry.clear();
-        rc = run_wave(eng, insts, tier2, gc, m, use_graph, ~0ull, b2, std::max(1, clusters / 8), 1024, results, stats,
-                      &retry);
+        rc = run_wave(eng, insts, tier2, gc, m, use_graph, ~0ull, b2, keep2, kYield2, results, stats, &retry);
         if (rc) return rc;
-        todo = retry;
+        todo.insert(todo.end(), retry.begin(), retry.end());
     }
     bool over2 = false;  // heaps overflowed in the cluster tier
     for (int i : todo) over2 |= results[i].status == UASTAR_HEAP_OVERFLOW;
