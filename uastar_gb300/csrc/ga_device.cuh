@@ -75,6 +75,7 @@ struct NarrowSlots {
     using Key = uint64_t;
     static constexpr bool kWide = false;
     static constexpr bool kDirect = false;     // see GridDirect
+    static constexpr bool kNeedsBound = false; // see PuzzleProblem
     static constexpr bool kPrevInKey = false;  // see GridProblem
     static constexpr size_t kSlotBytes = sizeof(Slot);
     // An auto-sized table grows when a quarter full: a relax goes slot by slot,

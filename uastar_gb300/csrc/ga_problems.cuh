@@ -426,6 +426,7 @@ template <int N> struct PuzzleProblem : NarrowSlots {
     // The pattern parts depend on the board alone and travel in its entries
     // (make_entry).
     static constexpr int kLink = LINK_IN_G;
+    static constexpr bool kNeedsBound = true;  // see make_entry
     __device__ static KeyG cas_word(uint64_t key, uint64_t g, uint32_t prev, int mv) {
         return KeyG{key, g << 40 | (uint64_t)(uint32_t)(mv + 1) << 32 | prev};
     }
@@ -562,10 +563,12 @@ template <int N> struct PuzzleProblem : NarrowSlots {
         return moves(s.key, (uint32_t)(mv + 1) << kLastMoveShift);
     }
     static constexpr bool kEntryKey = false;
-    // f in 10 bits, 255 - g in 8 from bit 14 on (every board searched is
-    // solvable, so g and the parts stay below 128), the first pattern's part in
-    // the low 8: with h = f - g it gives the second's, so a slot needs no more
-    // than its CAS word.
+    // f in 10 bits, 255 - g in 8 from bit 14 on, the first pattern's part in the
+    // low 8: with h = f - g it gives the second's, so a slot needs no more than
+    // its CAS word.  g fits because every board searched is solvable and the
+    // search bounded: it expands nothing whose f is above the optimum (80 moves at
+    // most on 4x4, 208 on 5x5, where the slot has 8 bits for g) plus the slack.
+    // ga_search refuses a puzzle without a bound.
     __device__ __forceinline__ Entry make_entry(uint64_t f, uint64_t g, uint32_t slot, uint32_t aux) const {
         Entry e;
         e.key = (uint32_t)f << 22 | (255u - (uint32_t)g) << 14 | (aux & 0xffu);
@@ -608,6 +611,7 @@ template <> struct PuzzleProblem<5> : WideSlots {
     static constexpr int kMoves = 4;
     static constexpr int N = 5;
     static constexpr int NN = 25;
+    static constexpr bool kNeedsBound = true;  // 8 bits of g (PuzzleProblem::make_entry)
     static constexpr uint64_t kFieldLow = 0x0084210842108421ull;  // bit 0 of each of 12 fields
 
     const uint8_t *pdb;  // four concatenated tables

@@ -891,6 +891,13 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
     TeamState *const st = team.st;
     const uint32_t T = blockDim.x, tid = threadIdx.x, lane = tid & 31u;
     const uint32_t C = team.ctas(), cta = team.cta();
+    // a problem whose fields hold only what a bound on f lets in is not searched
+    // without one (SearchMem's default)
+    if constexpr (P::kNeedsBound)
+        if (!(m.slack > 0.f)) {
+            if (cta == 0 && tid == 0) st->status = ST_BAD_INPUT;
+            return ST_BAD_INPUT;
+        }
     const bool owner = tid < H;
     const uint32_t L = m.L, topn = (1u << L) - 1;
     const uint32_t owner_warps = (H + 31u) / 32u;
