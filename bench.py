@@ -58,9 +58,18 @@ WORKLOAD = "grid_20000"
 # generator, the engine arm with the engine's: the same bits.
 C2_H = C2_W = 20000
 C2_RATE, C2_SEED = 0.30, 7
-# algorithmic bytes per unit of work (sector-granular, 32 B per random access):
-# grid 160 B per expansion + 32 B per generated successor + 64 B per heap push
-GRID_BYTES = (160, 32, 64)
+
+
+def grid_bytes(expanded: int, generated: int, pushed: int) -> int:
+    """Algorithmic bytes of a grid search on one word per cell, 32 (a sector) per
+    random access: three bitmap rows per expansion, the word that a successor's
+    relax changes, the entry of a push, and for a node that came off a heap its
+    entry and its word.  A node expanded at once by the pass that reached it has
+    neither, and no more come off the heaps than were pushed."""
+    return 32 * (3 * expanded + generated + pushed + 2 * min(expanded, pushed))
+
+
+GRID_BYTES_MODEL = "96*expanded + 32*generated + 32*pushed + 64*min(expanded, pushed)"
 
 
 def log(*a):
@@ -284,8 +293,7 @@ def run_ours(args, rank, world, local_rank):
 
     # roofline of the search kernel (one launch per solve)
     peak, peak_kind = measured_peaks()
-    per_launch_bytes = [GRID_BYTES[0] * r.expanded + GRID_BYTES[1] * r.generated + GRID_BYTES[2] * r.pushed
-                        for r in results]
+    per_launch_bytes = [grid_bytes(r.expanded, r.generated, r.pushed) for r in results]
     mean_kernel_ms = sum(kernel_ms) / len(kernel_ms)
     achieved = (sum(per_launch_bytes) / len(per_launch_bytes)) / (mean_kernel_ms / 1e3) / 1e9
     traffic = None
@@ -328,7 +336,7 @@ def run_ours(args, rank, world, local_rank):
         "scaling": "weak", "vs_baseline": None, "dtype": "int64", "data": "synthetic (seeded generator)",
         "s_per_solve": round(elapsed_ms / args.steps / 1e3, 4),
         "config": {"workload": WORKLOAD, "grid": "20000x20000", "block_rate": 0.30, "seed": sp.seed,
-                   "heaps": 8192, "block_threads": 256, "threads_per_heap": 4, "hash_slots": 2 ** 28,
+                   "heaps": 8192, "block_threads": 256, "threads_per_heap": 4, "table": "a word of 8 B per cell (the 2^28 16-byte slots asked for hold it)",
                    "parallelism": f"replicas x{world}" if world > 1 else "single GPU",
                    "l2": "inputs larger than L2: each solve rewrites its 3.2 GB table of cells first",
                    "step": "one full solve (search + path walk + host validation), bitmap resident"},
@@ -346,7 +354,7 @@ def run_ours(args, rank, world, local_rank):
                      "frac": round(achieved / peak, 5), "traffic": traffic, "peak_kind": peak_kind,
                      "kernel": "k_plain_search<GridDirect>", "kernel_ms_mean": round(mean_kernel_ms, 3),
                      "bytes_per_launch": int(sum(per_launch_bytes) / len(per_launch_bytes)),
-                     "bytes_model": "160*expanded + 32*generated + 64*pushed"},
+                     "bytes_model": GRID_BYTES_MODEL},
         "gpu_launches": int(launches),
         "clocks": clocks.summary(),
     }
