@@ -89,6 +89,8 @@ struct BatchArgs {
     uint64_t quantum_ns;   // serving: time slice of the launch, from each team's start (0: rounds only)
     uint32_t *idle;        // batch: teams that found the queue empty (SearchMem::idle)
     uint32_t idle_min, yield_steps;
+    uint32_t yield_short;  // grids with their ends at most this far apart keep their team
+    uint32_t yield_half;   // 1: so do grids past half of their least number of steps
     uint64_t walk_inline;  // serving: paths of more cells are walked after the quantum (0: all inline)
     unsigned long long *keys;  // batch: path keys of solved instances
 };
@@ -180,8 +182,9 @@ __device__ uint32_t run_instance(const BatchArgs &a, const InstDesc &d, Team &te
             m.idle = a.idle;
             m.idle_min = a.idle_min;
             m.yield_steps = a.yield_steps;
-            // a grid past half of its way is left to finish (see uastar_batch_solve)
-            m.yield_end = grid ? (uint32_t)max(abs(d.sx - d.ex), abs(d.sy - d.ey)) / 2u : ~0u;
+            // (see uastar_batch_solve)
+            const uint32_t apart = (uint32_t)max(abs(d.sx - d.ex), abs(d.sy - d.ey));
+            m.yield_end = !grid ? ~0u : a.yield_half ? apart / 2u : apart <= a.yield_short ? 0u : ~0u;
             m.sort_buf = nullptr;
             m.sort_hist = nullptr;
             m.sort_bits = 0;
@@ -723,6 +726,9 @@ int32_t run_wave(uastar_engine *eng, const uastar_instance *insts, const std::ve
     // one at least has to be, however few the teams are)
     a.idle_min = (uint32_t)std::max(cnt > teams ? 1 : 0, teams - keep);
     a.yield_steps = yield_steps;
+    a.yield_half = g.csize > 0 ? 1u : 0u;
+    const auto is_grid = [&](int i) { return insts[i].kind == UASTAR_KIND_GRID; };
+    if (g.csize == 0 && std::all_of(idx.begin(), idx.end(), is_grid)) a.yield_short = 2 * yield_steps;
     int ctas = std::min(g.ctas, cnt);
     cudaLaunchConfig_t lc = {};
     cudaLaunchAttribute lat[1];
@@ -998,9 +1004,12 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
     // 16 of 36 teams: 710 / 605 / 603 / 756), 536 with both (18 / 36 / 72 / 150
     // instances: 583 / 574 / 536 / 539).
     // A grid takes at least as many steps as its ends are rows or columns apart, so
-    // what is left of one can be told.  One that has made half of that many is
-    // left to finish: without that, 36 grids of 200 to 320 cells a side start
-    // over (4.7 ms, with it 3.9) and so do the last of eight of 3000 (53-65, 41).
+    // what is left of one can be told.  On a cluster one that has made half of
+    // that many is left to finish (the last of eight grids of 3000 cells a side
+    // started over: 53-65 ms, so 41; 24 of up to 1500: 33, 20).  On a single CTA
+    // one whose ends are at most twice the 256 steps apart, if the wave has no
+    // puzzles: those would wait for it (36 grids of 200 to 320 cells a side 4.7
+    // -> 3.9 ms; 96 mixed instances with puzzles 40 -> 45, so not there).
     // And where a wave is so small that it would give up its instances from the
     // outset, a grid that is sure to get there is not started in it: two grids of
     // 900 to 1500 cells a side 24.8 -> 8.0 ms, one of 3000 18.2 -> 11.4.
