@@ -919,11 +919,9 @@ int32_t ida_exact(uastar_engine *eng, const uint8_t *tiles, int32_t lb, int32_t 
         if ((e = cudaMemcpyAsync(&cut, d_cut, sizeof cut, cudaMemcpyDeviceToHost, eng->stream)) != cudaSuccess ||
             (e = cudaStreamSynchronize(eng->stream)) != cudaSuccess)
             return fail_cuda(eng, e, "ida cut");
-        uint32_t depth = 0, first = 0;  // the last level, its first record in the ring
-        while (depth < kIdaCutDepth && cut.count[depth + 1]) {
-            first += cut.count[depth];
-            out->exact_nodes += cut.count[++depth];
-        }
+        uint32_t depth = 0;
+        while (depth < kIdaCutDepth && cut.count[depth + 1]) out->exact_nodes += cut.count[++depth];
+        const uint32_t first = cut.first[depth];
         if (cut.goal) {
             out->exact_passes += 1;
             moves->clear();

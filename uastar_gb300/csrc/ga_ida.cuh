@@ -46,6 +46,7 @@ constexpr uint32_t kIdaCutDepth = 32;
 // 134 MB for 2^20 roots (two buffers of a level's children each took 268).
 struct IdaCut {
     uint32_t count[kIdaCutDepth + 1];  // nodes per level; 0 past the last
+    uint32_t first[kIdaCutDepth + 1];  // a level's first record (modulo the ring)
     uint32_t goal;                     // a goal's depth (0: none met)
     uint32_t min_exceed;               // least f above the threshold
     unsigned long long goal_prefix;    // the moves to the goal
@@ -97,8 +98,8 @@ __global__ void __launch_bounds__(256) k_ida_cut(P prob, IdaRoot *ring, uint32_t
     const uint32_t n = ldcg_u32(&cut->count[d]);
     if (n == 0 || n >= roots) return;
     const uint32_t wrap = 4u * roots - 1u;
-    uint32_t first = 0;  // level d's first record
-    for (uint32_t q = 0; q < d; ++q) first += ldcg_u32(&cut->count[q]);
+    const uint32_t first = ldcg_u32(&cut->first[d]);
+    if (blockIdx.x == 0 && threadIdx.x == 0) cut->first[d + 1] = first + n;
     uint32_t minx = ~0u;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const IdaRoot r = ring[(first + i) & wrap];
