@@ -803,7 +803,7 @@ def run_case(args) -> None:
                 r = eng.puzzle_solve_bounded(4, tiles, 20)
                 print(f"bounded: {r['steps']} moves, bound {r['lower_bound']}, {r['segments']} segments", flush=True)
     elif c == "walk":
-        # path walks after solves: k_walk on a 4096^2 grid, the in-kernel
+        # path walks after solves: k_walk_grid_solved on a 4096^2 grid, the in-kernel
         # walk of a batch
         sp = WL.screened_grid(4096, 4096, 0.30, 7)
         words = sp.words()

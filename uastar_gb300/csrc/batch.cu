@@ -469,9 +469,9 @@ inline int log2_u64(uint64_t v) {
 uint64_t est_nodes(const uastar_instance &in) {
     if (in.est_nodes > 0) return (uint64_t)in.est_nodes;
     // Grids: an eighth of the cells (random grids searched corner to corner
-    // touch a few percent to ~20 %).  15-puzzles: 2^19 states, what a single
-    // CTA team inserts in a 4096-round budget (64 heaps, ~2 new states per
-    // expansion), so that a puzzle leaves that tier by running out of rounds
+    // touch a few percent to ~20 %).  15-puzzles: 2^19 states, twice what a single
+    // CTA team inserts in its budget of 2048 steps (64 heaps, ~2 new states per
+    // expansion), so that a puzzle leaves that tier by running out of steps
     // rather than out of space.  An instance that fills its partition is
     // re-run in the next wave with 32x the space.
     if (in.kind == UASTAR_KIND_GRID) return std::max<uint64_t>(4096, (uint64_t)in.H * in.W / 8);

@@ -309,7 +309,7 @@ __host__ __device__ constexpr uint64_t odd_inverse(uint64_t odd) {
 }
 
 // A grid search whose table is one 8-byte word per cell instead of hashed
-// 32-byte slots: slot = cell, word = g << 3 | the move that reached the cell
+// 16-byte slots: slot = cell, word = g << 3 | the move that reached the cell
 // (all ones: unreached).  A relax is then one 64-bit atomicMin, one memory trip
 // whatever it finds, where the hashed table's 16-byte CAS takes one to claim
 // and two or more to improve or on a collision.  For that a cost has to be one
@@ -320,8 +320,8 @@ __host__ __device__ constexpr uint64_t odd_inverse(uint64_t odd) {
 // number's error in the difference is at most n * 2^-40, less while n (2.83 n
 // + 1) < 2^40.  Costs that could reach kLimit (800000, so B < 566000) end the
 // search with ST_COST_RANGE, and the hashed search takes the problem over.
-// Comparing two costs is one integer compare, and a map's words are a quarter of
-// the bytes of its hashed slots at the sizes taken before.  Kernels, hashed ->
+// Comparing two costs is one integer compare, and a map's words are no more bytes
+// than hashed slots for half of its cells.  Kernels, hashed (32-byte slots) ->
 // word: 20000^2 165 -> 103 ms (5.35 -> 3.34 us a step), six queries on 1537 x
 // 2049 20.2 -> 13.3 ms, 61 x 67 0.24 -> 0.20 ms, the allocation-free 700 x 1021
 // 7.1 -> 4.8 ms.  Still bound by the latency of a step's chain, not by bytes.
