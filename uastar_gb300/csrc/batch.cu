@@ -553,7 +553,7 @@ int32_t resolve_block_geometry(uastar_engine *eng, int threads, int tph, BatchGe
     g->split_grid = SearchSmem<GridProblem>::bytes_split(g->H, g->L_grid) <= g->smem ? 1u : 0u;
     g->split_puzzle = SearchSmem<PuzzleProblem<4>>::bytes_split(g->H, g->L_puzzle) <= g->smem ? 1u : 0u;
     g->set_capacity(4095);
-    cudaError_t e = open_smem(eng->device, (const void *)k_batch);
+    cudaError_t e = raise_smem((const void *)k_batch, g->smem);
     if (e != cudaSuccess) return fail_cuda(eng, e, "smem attribute");
     int occ = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch, g->T, g->smem);
@@ -565,7 +565,7 @@ int32_t resolve_block_geometry(uastar_engine *eng, int threads, int tph, BatchGe
 // Cluster teams: the same CTA geometry, `csize` CTAs per team, as many
 // teams as can be co-resident.
 int32_t resolve_cluster_geometry(uastar_engine *eng, int csize, BatchGeometry *g) {
-    cudaError_t e = open_smem(eng->device, (const void *)k_batch_cluster);
+    cudaError_t e = raise_smem((const void *)k_batch_cluster, g->smem);
     if (e == cudaSuccess && csize > 8)
         e = cudaFuncSetAttribute(k_batch_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return fail_cuda(eng, e, "cluster attributes");

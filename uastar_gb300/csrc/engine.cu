@@ -156,16 +156,13 @@ __global__ void __launch_bounds__(1024) k_walk_grid_solved(P prob, const Slot *t
     if (threadIdx.x == 0) *len = n;
 }
 
-cudaError_t open_smem(int device, const void *kernel) {
-    int optin = 0;
+cudaError_t raise_smem(const void *kernel, size_t bytes) {
+    static std::mutex mu;  // (reading and raising are one step for all engines' threads)
+    std::lock_guard<std::mutex> lk(mu);
     cudaFuncAttributes a;
-    cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
-    if (e != cudaSuccess) return e;
-    const int most = optin - (int)a.sharedSizeBytes;  // (the limit counts the kernel's static part too)
-    return a.maxDynamicSharedSizeBytes >= most
-               ? cudaSuccess
-               : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    const cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+    if (e != cudaSuccess || (size_t)a.maxDynamicSharedSizeBytes >= bytes) return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 int32_t fill_ff_async(uastar_engine *eng, void *p, size_t bytes, cudaStream_t stream) {
@@ -371,9 +368,9 @@ int32_t run_plain(uastar_engine *eng, const P &prob, int log2_auto, uint32_t str
     const uint32_t L = fit_levels<P>(H, c.heap_top_levels, smem_budget - sort_extra);
     const size_t smem = sorted ? SearchSmem<P>::bytes_sorted(H, L, block) : SearchSmem<P>::bytes(H, L);
     cudaError_t e = cudaSuccess;
-    if (!eng->smem_open.count(kfn)) {
-        if ((e = open_smem(eng->device, kfn)) != cudaSuccess) return fail_cuda(eng, e, "smem attribute");
-        eng->smem_open.insert(kfn);
+    if (eng->smem_raised[kfn] < smem) {
+        if ((e = raise_smem(kfn, smem)) != cudaSuccess) return fail_cuda(eng, e, "smem attribute");
+        eng->smem_raised[kfn] = smem;
     }
     int max_active = 0;
     const auto occ_key = std::make_tuple(kfn, block, smem);

@@ -11,7 +11,6 @@
 #include <map>
 #include <memory>
 #include <mutex>
-#include <set>
 #include <string>
 #include <thread>
 #include <tuple>
@@ -108,10 +107,10 @@ struct uastar_engine {
         return e;
     }
     uastar::DevBuf ida;                 // memory-bounded mode: IDA* roots and pass state
-    // launch-configuration queries of the plain engine: the kernels whose
-    // shared memory limit it has opened (open_smem), and co-resident CTAs per SM
-    // per (kernel, block, shared memory)
-    std::set<const void *> smem_open;
+    // launch-configuration queries of the plain engine, made once per shape: the
+    // dynamic shared memory asked for per kernel (raise_smem), and co-resident
+    // CTAs per SM per (kernel, block, shared memory)
+    std::map<const void *, size_t> smem_raised;
     std::map<std::tuple<const void *, uint32_t, size_t>, int> occupancy;
     int32_t gH = 0, gW = 0;
     bool grid_loaded = false;
@@ -147,11 +146,11 @@ namespace uastar {
 int32_t fail_cuda(uastar_engine *eng, cudaError_t e, const char *what);
 // Fill `bytes` (a multiple of 16) at `p` with 0xFF on `stream` using the whole GPU.
 int32_t fill_ff_async(uastar_engine *eng, void *p, size_t bytes, cudaStream_t stream);
-// Lets a kernel be launched with all the dynamic shared memory that a CTA of
-// this device can have.  The limit belongs to the kernel and the device, not to
-// an engine: set to what one launch shape needs, a smaller engine (or batch)
-// would lower it under another's next launch.
-cudaError_t open_smem(int device, const void *kernel);
+// Lets a kernel be launched on the current device with `bytes` of dynamic shared
+// memory.  The limit belongs to the kernel and the device, not to an engine, so
+// it is only ever raised: an engine or batch that needs less would lower it under
+// another's next launch.
+cudaError_t raise_smem(const void *kernel, size_t bytes);
 // pdb.cu
 int32_t pdb_build_device(uastar_engine *eng, int n, double *ms);
 // batch.cu: the batched engine keeps its team regions, heaps and bitmaps for
