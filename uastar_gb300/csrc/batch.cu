@@ -583,6 +583,7 @@ int32_t resolve_cluster_geometry(uastar_engine *eng, int csize, BatchGeometry *g
     int nclusters = 0;
     e = cudaOccupancyMaxActiveClusters(&nclusters, k_batch_cluster, &lc);
     if (e != cudaSuccess || nclusters < 1) {
+        (void)cudaGetLastError();  // (as fail_cuda)
         eng->set_err("no cluster of the requested size fits this GPU");
         return UASTAR_BAD_INPUT;
     }

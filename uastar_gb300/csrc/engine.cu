@@ -175,6 +175,7 @@ int32_t fill_ff_async(uastar_engine *eng, void *p, size_t bytes, cudaStream_t st
 }
 
 int32_t fail_cuda(uastar_engine *eng, cudaError_t e, const char *what) {
+    (void)cudaGetLastError();  // reported here, not by the next launch check of this or another engine
     eng->set_err(std::string(what) + ": " + cudaGetErrorString(e));
     return UASTAR_CUDA_ERROR;
 }
