@@ -26,3 +26,15 @@ def test_corridors_fill_the_table(log2):
                 assert r.status == L.HASH_FULL and r.table_used > 0.8 * 2**log2, s
                 r = eng.grid_solve(words, 1, n, (0, s), (0, s))
                 assert r.ok and r.path_len == 1
+
+
+def test_near_goals_fit_a_tiny_table():
+    # 8 slots hold 6 states; a goal two cells away takes at most five, if nothing
+    # away from it is expanded
+    n = 64
+    words = E.pack_words(np.ones((1, n), dtype=np.uint8))
+    with Engine(0, hash_log2_slots=3) as eng:
+        for s in range(2, n - 2):
+            for g in (s - 2, s - 1, s + 1, s + 2):
+                r = eng.grid_solve(words, 1, n, (0, s), (0, g))
+                assert r.ok and r.path_len == abs(g - s) + 1, (s, g)

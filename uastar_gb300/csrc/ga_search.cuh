@@ -967,9 +967,12 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             } else {
                 if constexpr (P::kLink == LINK_FIELD) P::set_link(P::at(m.tab, s0), kNone, aux0);
                 uint32_t sz = 0;
-                heap_push<P>(heap_of(), sz, prob.make_entry(prob.f_of(key0, 0, aux0), 0, s0, aux0));
+                const uint64_t f0 = prob.f_of(key0, 0, aux0);
+                heap_push<P>(heap_of(), sz, prob.make_entry(f0, 0, s0, aux0));
                 m.heap_size[myh] = sz;
                 st->inserted = 1;
+                // (the first round's bound is the start's, or its passes would claim all around it)
+                if (m.slack > 0.f) st->bound = __float_as_uint(P::cost_val(f0) + m.slack);
             }
             st->started = 1;
         }
