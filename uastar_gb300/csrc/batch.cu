@@ -89,6 +89,7 @@ struct BatchArgs {
     uint64_t quantum_ns;   // serving: time slice of the launch, from each team's start (0: rounds only)
     uint32_t *idle;        // batch: teams that found the queue empty (SearchMem::idle)
     uint32_t idle_min, yield_steps;
+    uint32_t idle_late, yield_late;  // the same of puzzles that have made more steps
     uint32_t yield_short;  // grids with their ends at most this far apart keep their team
     uint32_t yield_half;   // 1: so do grids past half of their least number of steps
     uint64_t walk_inline;  // serving: paths of more cells are walked after the quantum (0: all inline)
@@ -181,6 +182,8 @@ __device__ uint32_t run_instance(const BatchArgs &a, const InstDesc &d, Team &te
             m.split = grid ? a.split_grid : a.split_puzzle;
             m.idle = a.idle;
             m.idle_min = a.idle_min;
+            m.idle_late = a.idle_late;
+            m.yield_late = grid ? ~0u : a.yield_late;
             m.yield_steps = a.yield_steps;
             // (see uastar_batch_solve)
             const uint32_t apart = (uint32_t)max(abs(d.sx - d.ex), abs(d.sy - d.ey));
@@ -607,7 +610,8 @@ int32_t resolve_geometry(uastar_engine *eng, const uastar_batch_config *cfg, Bat
 // wave's table memory is teams x region, not the sum over instances.
 // `budget` and `puzzle_budget` (0: none; puzzle instances only) count expansion
 // steps.  Once no more than `keep` instances are left running, those that have
-// made yield_steps steps return unfinished as if out of budget.
+// made yield_steps steps return unfinished as if out of budget (see
+// uastar_batch_solve).
 int32_t run_wave(uastar_engine *eng, const uastar_instance *insts, const std::vector<int> &idx,
                  const BatchGeometry &g, const std::vector<int> &space_mult, bool use_graph, uint64_t budget,
                  uint64_t puzzle_budget, int keep, uint32_t yield_steps, uastar_instance_result *results,
@@ -726,6 +730,8 @@ int32_t run_wave(uastar_engine *eng, const uastar_instance *insts, const std::ve
     // (an idle team says that the queue is empty: with more instances than teams
     // one at least has to be, however few the teams are)
     a.idle_min = (uint32_t)std::max(cnt > teams ? 1 : 0, teams - keep);
+    a.idle_late = (uint32_t)std::max(cnt > teams ? 1 : 0, teams - 2 * keep);
+    a.yield_late = g.csize > 0 ? 4 * yield_steps : ~0u;
     a.yield_steps = yield_steps;
     a.yield_half = g.csize > 0 ? 1u : 0u;
     const auto is_grid = [&](int i) { return insts[i].kind == UASTAR_KIND_GRID; };
@@ -1003,7 +1009,11 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
     // once an eighth of its teams is busy (after 1024).  Eight batches of 16
     // to 400 instances: 1092 ms without, 605 with the second rule (2 / 4 / 8 /
     // 16 of 36 teams: 710 / 605 / 603 / 756), 536 with both (18 / 36 / 72 / 150
-    // instances: 583 / 574 / 536 / 539).
+    // instances: 583 / 574 / 536 / 539).  A puzzle that has made 4096 is a hard one and
+    // gives up its cluster once a quarter of the teams is busy: five of them among
+    // 72 held theirs to the end of the budget (302 ms; 286 without any rule), and now
+    // 144; after 2048 / 4096 / 8192 steps 72 other boards 82 / 82 / 96 (97 without),
+    // 36 boards 59 / 65 / 89 (89), 36 mixed instances 26.4 / 24.1 / 24.7 (24.5).
     // A grid takes at least as many steps as its ends are rows or columns apart, so
     // what is left of one can be told.  On a cluster one that has made half of
     // that many is left to finish (the last of eight grids of 3000 cells a side

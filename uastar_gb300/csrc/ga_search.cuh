@@ -99,10 +99,10 @@ template <class E> struct SearchMem {
     uint64_t deadline_ns = 0;
     // Yielding: the search also pauses once *idle (teams of the launch that have
     // run out of instances) reaches idle_min and it has made yield_steps
-    // expansion steps, but not yield_end; looked at every 32nd round.
-    // nullptr = never.
+    // expansion steps, but not yield_end; or idle_late and yield_late steps.
+    // Looked at every 32nd round.  nullptr = never.
     const uint32_t *idle = nullptr;
-    uint32_t idle_min = 0, yield_steps = 0, yield_end = ~0u;
+    uint32_t idle_min = 0, yield_steps = 0, yield_end = ~0u, idle_late = ~0u, yield_late = ~0u;
     // Split rounds (CTA and cluster teams, table-minimum dedup, separate
     // owner warps): the heap owners arrive at the team barrier as soon as
     // their pops are published and refill their heaps while the relaxers
@@ -1412,7 +1412,7 @@ __device__ uint32_t ga_search(const P &prob, Team &team, const SearchMem<typenam
             // threads take the same decision
             if (cta == 0 && m.deadline_ns) st->quit[r3] = globaltimer_ns() >= m.deadline_ns ? 1u : 0u;
             if (cta == 0 && m.idle && (rs->rounds & 31u) == 31u && rs->steps >= m.yield_steps && rs->steps < m.yield_end)
-                st->quit[r3] = ldcg_u32(m.idle) >= m.idle_min ? 1u : 0u;
+                st->quit[r3] = ldcg_u32(m.idle) >= (rs->steps < m.yield_late ? m.idle_min : m.idle_late) ? 1u : 0u;
         };
         // The decision, taken by one thread of each CTA once the barrier is
         // complete and handed to the others in shared memory: the same words
