@@ -70,11 +70,12 @@ def test_a_grid_alone_is_started_once(W, escalated):
     assert r["attempts"] == 1 and stats["escalated"] == escalated
 
 
-def test_a_budget_of_the_first_tier_is_not_lost():
+@pytest.mark.parametrize("tier1", [1, 1 << 20])
+def test_small_budgets_lose_no_instance(tier1):
     # (200 moves from the goal: more than the 256 steps after which a lone puzzle
-    # moves on, and than the 64 of the second tier; the first alone would do)
+    # moves on, and than the 64 of the second tier)
     tiles = E.gen_puzzle(1008, 4, 200)
     with Engine(0, hash_log2_slots=8) as eng:
         eng.pdb_build(4)
-        (r,), _ = eng.batch_solve([PuzzleInstance(4, tiles)], tier1_rounds=1 << 20, tier2_puzzle_rounds=64)
+        (r,), _ = eng.batch_solve([PuzzleInstance(4, tiles)], tier1_rounds=tier1, tier2_puzzle_rounds=64)
     assert r["status"] == L.OK and r["steps"] == 46

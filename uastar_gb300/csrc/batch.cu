@@ -1045,13 +1045,13 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
     // tail.  Grids do not: their steps are bounded by the path length, which
     // costs a cluster no more of them than the whole GPU.
     const uint64_t b2 = cfg && cfg->tier2_puzzle_rounds > 0 ? (uint64_t)cfg->tier2_puzzle_rounds : 16384;
-    const uint64_t b1 = cfg && cfg->tier1_rounds > 0 ? (uint64_t)cfg->tier1_rounds : 2048;
     const int keep1 = 2 * clusters, keep2 = std::max(1, clusters / 8);
     const size_t large = tier2.size();
     given_up(tier1, g.ctas, keep1, kYield1, &tier2);
     for (size_t j = large; j < tier2.size(); ++j) mult[tier2[j]] = insts[tier2[j]].est_nodes > 0 ? 16 : 4;
     if (!tier1.empty()) {
         std::vector<int> m(tier1.size(), 1);
+        const uint64_t b1 = cfg && cfg->tier1_rounds > 0 ? (uint64_t)cfg->tier1_rounds : 2048;
         rc = run_wave(eng, insts, tier1, g, m, use_graph, b1, 0, keep1, kYield1, results, stats, &retry);
         if (rc) return rc;
         // Space for the next tier: 16x after an overflow.  One that ran out of
@@ -1144,9 +1144,9 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
     // What the plain engine could not solve, because the engine's own limits for
     // plain solves are too small (hash_log2_slots, heap_capacity, heaps) or the
     // memory is not there, may have been well on its way on a cluster when it
-    // gave up its team: it gets one again, with that tier's largest space, the
-    // larger of the two budgets and no early end.  If that fails too, the plain
-    // engine's status stands.
+    // gave up its team: it gets one again, with that tier's largest space, which
+    // is then all that bounds it.  If that fails too, the plain engine's status
+    // stands.
     if (!failed.empty() && !cluster_rc) {
         if (over2 && !heap_over) gc.set_capacity(g.want * 16 + 15);
         std::vector<int> m;
@@ -1154,7 +1154,7 @@ int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int
         std::vector<uastar_instance_result> before;
         for (int i : failed) before.push_back(results[i]);
         retry.clear();
-        rc = run_wave(eng, insts, failed, gc, m, use_graph, ~0ull, std::max(b1, b2), 0, 0, results, stats, &retry);
+        rc = run_wave(eng, insts, failed, gc, m, use_graph, ~0ull, 0, 0, 0, results, stats, &retry);
         if (rc) return rc;
         for (size_t j = 0; j < failed.size(); ++j)
             if (std::find(retry.begin(), retry.end(), failed[j]) != retry.end())
