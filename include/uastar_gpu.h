@@ -301,7 +301,9 @@ typedef struct {
  * fill, 16x by default; puzzles under tier2_puzzle_rounds), and what fails there is
  * solved by the plain engine, one instance at a time.  The last instances of a
  * wave (few enough to leave most of the GPU idle) move on without using up
- * their budget.  No counterpart in the
+ * their budget.  An instance that the plain engine refuses (its limits are the
+ * engine's, its memory may not be there) is run on a cluster once more.  The
+ * engine's loaded grid and last solution stay as they were.  No counterpart in the
  * reference, which solves one instance per process through
  * GPUPathwaySolver / GPUPuzzleSolver. */
 int32_t uastar_batch_solve(uastar_engine *eng, const uastar_instance *insts, int32_t count,
